@@ -1,0 +1,865 @@
+// KxK convolution (INT8 u8 x s8 -> s32, and fp32 as 3xTF32) as an implicit GEMM whose activation operand
+// is fetched ONCE per channel group and reused by every filter tap.
+//
+// Replaces, for filters larger than one pixel or strides above one, the reference's
+// elx_int8_conv_direct_t (src/elx_int8_conv_direct.cpp:502-571, kernels
+// src/kernel/elk_u8s8_conv.hxx:254-677) and elx_conv_direct_t (src/elx_conv_direct.cpp,
+// src/kernel/elk_conv.hxx).
+//
+// Tile: 16 output rows x 8 output columns = the 128 rows of one tcgen05.mma, times BN output channels.
+// The input pixels the tile's taps touch (for a 3x3 stride-1 filter 18 x 10 pixels) are fetched row by row
+// with tiled TMA copies into shared memory as [row][16-byte channel chunk][pixel][16 B].  Eight
+// horizontally adjacent pixels of one chunk are 128 contiguous bytes, i.e. one core matrix of the
+// no-swizzle K-major operand layout, the next eight rows of the operand are the next image row (stride
+// `pitch`), and shifting the tile by a tap moves only the operand's START ADDRESS (16-byte granular in
+// this layout).  So all taps multiply the same bytes: 1.4 x the tile's own pixels cross from L2 instead of
+// the 9 x an implicit GEMM with one copy per tap moves, which is what bounded that form (94 B/clk per
+// SM wanted at BN = 256 for int8, where an SM takes in about 60).  Stride 2 does the same on the four
+// (row, column) parity planes of the input, one tensor map each.
+//
+// Small images: the output rows of all images of the batch are stacked into one tall row space with
+// `period` = OH + the padding rows two neighbours can share, so 16-row tiles run across image borders and
+// a 7x7 layer fills 7/8 of its tile rows; the copies are per row, so each finds its own image, and rows
+// outside an image arrive as zeros.
+//
+// Warp roles: 0 activation rows (TMA) | 1, 3 MMA issuers (even / odd tiles of the CTA, 1 owns tensor memory)
+// | 2 weights (bulk copies) | 4.. epilogue | (fp32) four warps that split the landed rows into tf32 hi / lo
+// planes in shared memory.
+// Two accumulators in tensor memory, each with its own issuer: one warp issues an MMA about every 40 cycles
+// (wait, addresses, descriptors), and on narrow tiles an MMA lasts no longer than that.
+#include "conv_halo.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <type_traits>
+
+#include "host_prep.hpp"
+#include "umma.cuh"
+
+namespace elb {
+
+namespace {
+
+constexpr int BM = 128, TILE_H = 16, TILE_W = 8;
+constexpr int MAX_A = 4, MAX_B = 16, RAW_STAGES = 2, MAX_BUFS = 4;
+// int8: an epilogue group of four warps per (accumulator, half of the column blocks); fp32: per half
+constexpr int EPI_WARP0 = 4, SPLIT_WARPS = 4;
+constexpr int EPI_WARPS_I8 = 16, EPI_WARPS_F32 = 8;
+constexpr int SPLIT_WARP0 = EPI_WARP0 + EPI_WARPS_F32;
+constexpr int THREADS_I8 = (EPI_WARP0 + EPI_WARPS_I8) * 32, THREADS_F32 = (SPLIT_WARP0 + SPLIT_WARPS) * 32;
+constexpr int SMEM_LIMIT = 232448 - 1024;      // dynamic shared memory the plan may fill
+
+struct Bars {
+  uint64_t afull[MAX_A], aempty[MAX_A], rfull[RAW_STAGES], rempty[RAW_STAGES], bfull[MAX_B], bempty[MAX_B], tfull[MAX_BUFS], tempty[MAX_BUFS], turn[2];
+  uint32_t tmem_slot;
+  int abort_flag;
+};
+
+// All lanes wait (one instruction for the converged warp); the verdict is warp-uniform.
+__device__ __forceinline__ bool wait_all(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+  const bool ok = mbar_wait(bar, parity, abort_flag);
+  return __all_sync(0xFFFFFFFFu, ok ? 1 : 0) != 0;
+}
+
+// Lane 0's value: the compiler then knows that the value is the same in the whole warp.  The MMA operands live in
+// uniform registers; from values it cannot prove uniform (anything behind a branch on threadIdx) it builds them
+// with a loop around every MMA.
+__device__ __forceinline__ int uni(int v) { return __shfl_sync(0xFFFFFFFFu, v, 0); }
+
+// requant_store16 for the common case: u8 result, ReLU at zero without an upper bound, no residual.  The
+// saturating conversion is the ReLU; scale and shift on channel pairs (each lane rounds as the scalar fma).
+__device__ __forceinline__ void requant_relu_u8(const int (&acc)[16], const float *sc, const float *sh, uint8_t *out) {
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const ulonglong2 c = reinterpret_cast<const ulonglong2 *>(sc)[i], h = reinterpret_cast<const ulonglong2 *>(sh)[i];
+    int r[4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      unsigned long long f;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(f) : "f"(__int2float_rn(acc[4 * i + 2 * j])), "f"(__int2float_rn(acc[4 * i + 2 * j + 1])));
+      asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(f) : "l"(f), "l"(j ? c.y : c.x), "l"(j ? h.y : h.x));
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(f));
+      r[2 * j] = __float2int_rn(lo);
+      r[2 * j + 1] = __float2int_rn(hi);
+    }
+    uint32_t t;
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, 0;" : "=r"(t) : "r"(r[3]), "r"(r[2]));
+    asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(w[i]) : "r"(r[1]), "r"(r[0]), "r"(t));
+  }
+  *reinterpret_cast<uint4 *>(out) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// 32 bytes in one store: a lane's two 16-byte stores into one 32-byte sector would be two partial writes
+__device__ __forceinline__ void store_v8(float *p, const float (&f)[16], int at) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + at), "f"(f[at]), "f"(f[at + 1]),
+               "f"(f[at + 2]), "f"(f[at + 3]), "f"(f[at + 4]), "f"(f[at + 5]), "f"(f[at + 6]), "f"(f[at + 7])
+               : "memory");
+}
+
+// PAIRS: K steps of one tap, each two 16-byte channel chunks (fp32: 2).  0: a group is ONE chunk wide (at most
+// 16 int8 channels) and a K step takes the chunk of two neighbouring taps of a filter row.
+// FORM: how the issuer walks the taps.  FORM_3X3_* are 3x3 stride 1 (a weight stage per filter row, per tap, or
+// all weights resident) with a channel group's MMAs as straight-line code; FORM_ANY loops over rows and taps.
+// STACK: fp32 with at most 128 output channels per tile, see HaloParams::stack.
+// All are compile-time because the issuer is one warp: a loop iteration costs it 55 to 65 cycles whatever it
+// does, an address from a table in the parameter space 70, and a wait on a completed barrier 100 to 160.  With
+// loops, tables and a wait per filter row issuing took 2900 cycles per tile of 18 MMAs that last 864 (64 -> 64
+// channels at 224 x 224).
+enum : int { FORM_ANY = 0, FORM_3X3_ROWS = 1, FORM_3X3_TAPS = 2, FORM_3X3_RESIDENT = 3 };
+// pixels of a shared-memory row of a 3x3 stride-1 filter (what halo_plan() computes)
+__host__ __device__ constexpr int pxw_3x3(int kind, int pairs) { return kind == HALO_F32 || pairs == 2 || pairs == 4 ? 10 : pairs == 0 ? 16 : 12; }
+
+template <int KIND, int PAIRS, int FORM, bool STACK>
+__global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
+conv_halo_kernel(const __grid_constant__ HaloParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = smem_aligned(smem_raw);
+  constexpr int PLANES = KIND == HALO_I8 ? 1 : 2, EPI_WARPS = KIND == HALO_I8 ? EPI_WARPS_I8 : EPI_WARPS_F32;
+  const int a_stage = p.a_bytes * PLANES;
+  uint8_t *raw = smem + p.a_stages * a_stage;
+  uint8_t *b_ring = raw + (KIND == HALO_F32 ? RAW_STAGES * p.raw_bytes : 0);
+  float *s_scale = reinterpret_cast<float *>(b_ring + p.b_stages * p.b_stage_bytes);
+  const int n_const = p.n_tiles * p.BN;
+  float *s_shift = KIND == HALO_I8 ? s_scale + n_const : s_scale;
+  Bars &bar = *reinterpret_cast<Bars *>(s_shift + n_const);
+  volatile int *abort_flag = &bar.abort_flag;
+
+  const int warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (warp == 1) {
+    if (lane == 0) {
+      for (int i = 0; i < MAX_A; ++i) {
+        mbar_init(&bar.afull[i], KIND == HALO_I8 ? 1 : SPLIT_WARPS);
+        mbar_init(&bar.aempty[i], 1);
+      }
+      for (int i = 0; i < RAW_STAGES; ++i) { mbar_init(&bar.rfull[i], 1); mbar_init(&bar.rempty[i], SPLIT_WARPS); }
+      for (int i = 0; i < MAX_B; ++i) { mbar_init(&bar.bfull[i], 1); mbar_init(&bar.bempty[i], 1); }
+      for (int i = 0; i < 2; ++i) mbar_init(&bar.turn[i], 1);
+      for (int i = 0; i < MAX_BUFS; ++i) { mbar_init(&bar.tfull[i], 1); mbar_init(&bar.tempty[i], p.bufs == 4 ? 4 : 8); }
+      *abort_flag = 0;
+      fence_barrier_init();
+      fence_proxy_async_smem();
+    }
+    __syncwarp();
+    tmem_alloc(&bar.tmem_slot, 512);
+  } else if (warp == 0) {
+    if (lane < p.planes) { tma_prefetch_desc(&p.tmap[lane][HALO_HEIGHTS - 1]); tma_prefetch_desc(&p.tmap[lane][3]); }
+  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
+    const int OCP = p.OCB * 16;
+    for (int i = threadIdx.x - EPI_WARP0 * 32; i < n_const; i += EPI_WARPS * 32) {
+      if (KIND == HALO_I8) s_scale[i] = i < OCP ? p.scale[i] : 0.0f;
+      s_shift[i] = (i < OCP && p.shift) ? p.shift[i] : 0.0f;
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = bar.tmem_slot;
+  // (the kernel behind this one may set itself up now; see griddep_wait)
+  if (threadIdx.x == 0) griddep_launch_dependents();
+  int fail_code = 0;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- activation rows
+    griddep_wait();
+    uint64_t *full = KIND == HALO_I8 ? bar.afull : bar.rfull, *empty = KIND == HALO_I8 ? bar.aempty : bar.rempty;
+    const int stages = KIND == HALO_I8 ? p.a_stages : RAW_STAGES;
+    uint8_t *ring = KIND == HALO_I8 ? smem : raw;
+    const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
+    const int groups = uni(p.groups), planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
+    const bool strided = uni(p.strided) != 0;
+    // stride 1: 8-byte elements, so that the copy engine moves whole rows
+    const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+      const int mt = p.div_n.div(tile);
+      const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
+      for (int g = 0; g < groups && ok; ++g)
+      for (int q = 0; q < planes; ++q) {
+        const int rows = p.rows[q], x = (ct * TILE_W + p.col0[q]) * x_unit, v0 = rt * TILE_H + p.row0[q];
+        int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
+        if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
+        uint8_t *dst = ring + s * stage_bytes;
+        if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
+        if (h + rows <= period) {
+          // all rows belong to one image: one copy
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(rows * pitch));
+            if (!strided) tma_tile_4d(dst, &p.tmap[0][HALO_HEIGHTS - 1], x, g * cb_step, h, n, &full[s]);
+            else tma_tile_5d(dst, &p.tmap[q][HALO_HEIGHTS - 1], 0, x, g * cb_step, h, n, &full[s]);
+          }
+        } else {
+          // Lane r stands for row r.  Issuing a copy costs the warp about 100 cycles, so each image's share goes in
+          // pieces of 8, 4, 2 and 1 rows; the lane of a piece's first row issues it.
+          if (lane == 0) mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(rows * pitch));
+          const int v = v0 + lane;
+          n = v > 0 ? p.div_period.div(v) : 0;
+          h = v - n * period;
+          const int n_prev = __shfl_up_sync(0xFFFFFFFFu, n, 1);
+          const uint32_t starts = __ballot_sync(0xFFFFFFFFu, lane == 0 || n != n_prev || lane == rows);
+          if (lane < rows) {
+            const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
+            const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
+            const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
+            int idx = -1;
+            if (at < (len & ~7)) {
+              if ((at & 7) == 0) idx = 3;
+            } else {
+              const int sub = at & 7, rest = len - at;
+              if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx = 31 - __clz(rest);
+            }
+            if (idx >= 0) {
+              if (!strided) tma_tile_4d(dst + lane * pitch, &p.tmap[0][idx], x, g * cb_step, h, n, &full[s]);
+              else tma_tile_5d(dst + lane * pitch, &p.tmap[q][idx], 0, x, g * cb_step, h, n, &full[s]);
+            }
+          }
+        }
+        __syncwarp();
+        if (++s == stages) { s = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- weights
+    // (written before this launch's stream could reach it and never again: no griddep_wait)
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    const size_t group_bytes = static_cast<size_t>(p.ksteps) * p.kstep_bytes;
+    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+      const int nt = tile - p.div_n.div(tile) * p.n_tiles;
+      const uint8_t *src = p.b_img + static_cast<size_t>(nt) * p.groups * group_bytes;
+      for (int g = 0; g < p.groups && ok; ++g)
+      for (int q = 0; q < p.planes && ok; ++q) {
+        const int cols = p.tap_cols[q], row_steps = PAIRS == 0 ? (cols + 1) >> 1 : cols * PAIRS;
+        const int units = p.row_units ? p.tap_rows[q] : p.tap_rows[q] * cols;
+        const uint32_t bytes = static_cast<uint32_t>(p.row_units ? row_steps : PAIRS) * p.kstep_bytes;
+        for (int u = 0; u < units; ++u) {
+          if (!wait_all(&bar.bempty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&bar.bfull[s], bytes);
+            tma_bulk_g2s(b_ring + s * p.b_stage_bytes, src, bytes, &bar.bfull[s]);
+          }
+          __syncwarp();
+          src += bytes;
+          if (++s == p.b_stages) { s = 0; ph ^= 1u; }
+        }
+      }
+      if (p.resident) break;
+    }
+  } else if (warp == 1 || warp == 3) {
+    // ---------------------------------------------------------------- MMA issuers
+    constexpr bool STRAIGHT = FORM != FORM_ANY;
+    constexpr int PXW = pxw_3x3(KIND, PAIRS), CHUNKS = PAIRS ? 2 * PAIRS : 1;
+    const int BN = uni(p.BN), total = uni(p.total_tiles), groups = uni(p.groups), planes = STRAIGHT ? 1 : uni(p.planes),
+              b_stages = uni(p.b_stages), a_stages = uni(p.a_stages), bufs = uni(p.bufs);
+    const bool row_units = uni(p.row_units) != 0, resident = FORM == FORM_ANY ? uni(p.resident) != 0 : FORM == FORM_3X3_RESIDENT;
+    const uint32_t idesc = KIND == HALO_I8 ? umma_idesc(2, 0, 1, BM, BN) : umma_idesc(1, 2, 2, BM, BN);
+    const uint32_t idesc2 = umma_idesc(1, 2, 2, BM, 2 * BN);
+    const uint32_t a_base = smem_u32(smem) >> 4, b_base = smem_u32(b_ring) >> 4;
+    // descriptors: low word = address | chunk distance << 16, high word = 8-row group distance | version
+    const uint32_t pitch16 = STRAIGHT ? CHUNKS * PXW : uni(p.pitch) >> 4, pair16 = STRAIGHT ? 2 * PXW : 2u * uni(p.pxw);
+    const uint32_t a_hi = pitch16 | (1u << 14), b_hi = (128u >> 4) | (1u << 14);
+    const uint32_t b_lbo = static_cast<uint32_t>(STACK ? 2 * BN : BN) << 16;
+    const uint32_t ks16 = uni(p.kstep_bytes) >> 4, lo16 = uni(p.a_bytes) >> 4, a16 = lo16 * PLANES, b16 = uni(p.b_stage_bytes) >> 4;
+    const uint32_t a_lbo = static_cast<uint32_t>(PAIRS == 0 ? 1 : pair16 >> 1) << 16;      // (one pixel / one chunk further)
+    auto desc = [](uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32); };
+    const uint32_t el = elect_one() ? 1u : 0u;
+    const int me = warp >> 1;      // this issuer takes tiles me, me + 2, ... of the CTA's
+    // ring positions; the stages of the other issuer's tiles are skipped
+    const int skip_a = groups * planes, skip_b = resident ? 0 : uni(p.b_per_tile);
+    int as = 0, bs = 0;
+    uint32_t aph = 0, bph = 0;
+    auto skip = [&]() {
+      as += skip_a;
+      while (as >= a_stages) { as -= a_stages; aph ^= 1u; }
+      bs += skip_b;
+      while (bs >= b_stages) { bs -= b_stages; bph ^= 1u; }
+    };
+    auto next_b = [&]() {
+      if (++bs == b_stages) { bs = 0; bph ^= 1u; }
+    };
+    if (me) skip();
+    bool ok = true, b_ready = false;
+    int t = me;
+    for (int tile = blockIdx.x + me * gridDim.x; tile < total && ok; tile += 2 * gridDim.x, t += 2, skip()) {
+      const uint32_t buf = t & (bufs - 1), tph = (bufs == 4 ? t >> 2 : t >> 1) & 1u, my_ph = (t >> 1) & 1u;
+      const uint32_t d_tmem = tmem_base + buf * (bufs == 4 ? 128u : 256u);
+      // An issuer looks at the rings only once the other has seen every stage of the tile before: a barrier tells
+      // the last completed phase from the one before it, not from older ones.
+      if ((t > 0 && !wait_all(&bar.turn[me], my_ph ^ (me ^ 1u), abort_flag)) ||
+          !wait_all(&bar.tempty[buf], tph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
+      uint32_t acc = 0;
+      for (int g = 0; g < groups && ok; ++g)
+      for (int q = 0; q < planes && ok; ++q) {
+        if (!wait_all(&bar.afull[as], aph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
+        if (resident && g == groups - 1 && q == planes - 1 && el) mbar_arrive(&bar.turn[me ^ 1u]);
+        tc_fence_after_sync();
+        uint32_t a_row = (a_base + as * a16) | a_lbo, b_lo = 0;
+        auto mma = [&](uint32_t al, uint32_t bl, uint32_t accumulate) {
+          if (KIND == HALO_I8) {
+            umma_i8_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
+          } else if (STACK) {
+            // hi * [hi; lo] in one MMA of 2 * BN columns, lo * hi in one of BN (the first BN rows are hi)
+            umma_tf32_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc2, accumulate, el);
+            umma_tf32_el(d_tmem, desc(al + lo16, a_hi), desc(bl, b_hi), idesc, 1u, el);
+          } else {
+            // planes: the two hi chunks, then the two lo chunks
+            const uint64_t bh = desc(bl, b_hi), blo = desc(bl + (ks16 >> 1), b_hi);
+            umma_tf32_el(d_tmem, desc(al + lo16, a_hi), bh, idesc, accumulate, el);
+            umma_tf32_el(d_tmem, desc(al, a_hi), blo, idesc, 1u, el);
+            umma_tf32_el(d_tmem, desc(al, a_hi), bh, idesc, 1u, el);
+          }
+        };
+        // `n` taps from column c of the row at a_row (PAIRS = 0: n pairs of taps), unrolled
+        auto taps = [&](auto n, int c) {
+          constexpr int N = decltype(n)::value, P = PAIRS ? PAIRS : 1;
+#pragma unroll
+          for (int i = 0; i < N; ++i)
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+              mma(a_row + c + i * (PAIRS ? 1 : 2) + j * pair16, b_lo + (i * P + j) * ks16, (i | j) == 0 ? acc : 1u);
+          acc = 1u;
+          b_lo += N * P * ks16;
+        };
+        constexpr int ROW_STEPS = PAIRS ? 3 : 2;      // of a 3x3 filter row, for taps()
+        if constexpr (FORM == FORM_3X3_RESIDENT) {
+          if (!b_ready)      // the first tile waits for the weights, stage by stage; after that they stay
+            for (int i = 0; i < b_stages && ok; ++i) ok = wait_all(&bar.bfull[i], 0u, abort_flag);
+          b_ready = true;
+          b_lo = (b_base + (groups == 1 ? 0u : g * 3 * b16)) | b_lbo;
+#pragma unroll
+          for (int r = 0; r < 3; ++r, a_row += pitch16) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
+        } else if constexpr (STRAIGHT) {
+          constexpr int UNITS = FORM == FORM_3X3_ROWS ? 3 : 9;
+          bool seen = mbar_test_wait(&bar.bfull[bs], bph);
+#pragma unroll
+          for (int u = 0; u < UNITS; ++u) {
+            if (!__all_sync(0xFFFFFFFFu, seen)) {
+              ok = wait_all(&bar.bfull[bs], bph, abort_flag);
+              if (!ok) break;
+            }
+            tc_fence_after_sync();
+            b_lo = (b_base + bs * b16) | b_lbo;
+            uint64_t *done = &bar.bempty[bs];
+            next_b();
+            // the next stage is tested in front of this one's MMAs, so the answer is there when they are issued
+            if (u + 1 < UNITS) seen = mbar_test_wait(&bar.bfull[bs], bph);
+            if (FORM == FORM_3X3_ROWS) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
+            else taps(std::integral_constant<int, 1>{}, u % 3);
+            umma_commit_el(done, el);
+            if (FORM == FORM_3X3_ROWS || u % 3 == 2) a_row += pitch16;
+          }
+        } else {
+          const int rows = uni(p.tap_rows[q]), cols = uni(p.tap_cols[q]);
+          auto begin_unit = [&]() {
+            ok = wait_all(&bar.bfull[bs], resident ? 0u : bph, abort_flag);
+            tc_fence_after_sync();
+            b_lo = (b_base + bs * b16) | b_lbo;
+          };
+          auto end_unit = [&]() {
+            if (!resident) umma_commit_el(&bar.bempty[bs], el);
+            next_b();
+          };
+          if (row_units) {
+            const int steps = PAIRS ? cols : (cols + 1) >> 1;
+#pragma unroll 1
+            for (int r = 0; r < rows; ++r, a_row += pitch16) {
+              begin_unit();
+              if (!ok) break;
+#pragma unroll 1
+              for (int c = 0; c < steps; c += 4) {
+                const int at = PAIRS ? c : 2 * c;
+                switch (min(steps - c, 4)) {
+                  case 1: taps(std::integral_constant<int, 1>{}, at); break;
+                  case 2: taps(std::integral_constant<int, 2>{}, at); break;
+                  case 3: taps(std::integral_constant<int, 3>{}, at); break;
+                  default: taps(std::integral_constant<int, 4>{}, at);
+                }
+              }
+              end_unit();
+            }
+          } else {
+#pragma unroll 1
+            for (int r = 0; r < rows && ok; ++r, a_row += pitch16)
+#pragma unroll 1
+              for (int c = 0; c < cols; ++c) {
+                begin_unit();
+                if (!ok) break;
+                taps(std::integral_constant<int, 1>{}, c);
+                end_unit();
+              }
+          }
+        }
+        if (!ok) { fail_code = ST_WAIT_TIMEOUT_MMA; break; }
+        umma_commit_el(&bar.aempty[as], el);
+        if (++as == a_stages) { as = 0; aph ^= 1u; }
+      }
+      if (resident) bs = 0;
+      if (ok) umma_commit_el(&bar.tfull[buf], el);
+      if (!resident && el) mbar_arrive(&bar.turn[me ^ 1u]);
+      __syncwarp();
+    }
+  } else if (KIND == HALO_F32 && warp >= SPLIT_WARP0) {
+    // ---------------------------------------------------------------- fp32 rows -> tf32 hi / lo planes
+    // hi = round-to-nearest tf32(x), lo = x - hi (exact); done once per pixel, used by every tap
+    const int tid = threadIdx.x - SPLIT_WARP0 * 32;
+    int rs = 0, as = 0;
+    uint32_t rph = 0, aph = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+      for (int g = 0; g < p.groups && ok; ++g)
+      for (int q = 0; q < p.planes; ++q) {
+        const int items = p.rows[q] * p.pxw * 4;       // 16-byte pieces: [row][pixel][4 chunks]
+        if (!mbar_wait_warp(&bar.rfull[rs], rph, abort_flag) || !mbar_wait_warp(&bar.aempty[as], aph ^ 1u, abort_flag)) {
+          ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break;
+        }
+        const float4 *src = reinterpret_cast<const float4 *>(raw + rs * p.raw_bytes);
+        uint8_t *hi = smem + as * a_stage;
+        for (int i = tid; i < items; i += SPLIT_WARPS * 32) {
+          const float4 v = src[i];
+          const int px_all = i >> 2, c = i & 3;
+          const int row = p.div_px.div(px_all), px = px_all - row * p.pxw;
+          const float x[4] = {v.x, v.y, v.z, v.w};
+          float h[4], l[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t hb;
+            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hb) : "f"(x[j]));
+            h[j] = __uint_as_float(hb);
+            l[j] = __fsub_rn(x[j], h[j]);
+          }
+          uint8_t *d = hi + row * p.pitch + (c * p.pxw + px) * 16;
+          *reinterpret_cast<float4 *>(d) = make_float4(h[0], h[1], h[2], h[3]);
+          *reinterpret_cast<float4 *>(d + p.a_bytes) = make_float4(l[0], l[1], l[2], l[3]);
+        }
+        fence_proxy_async_smem();      // these stores -> visible to the tensor core's reads
+        __syncwarp();
+        if (lane == 0) { mbar_arrive(&bar.afull[as]); mbar_arrive(&bar.rempty[rs]); }
+        if (++rs == RAW_STAGES) { rs = 0; rph ^= 1u; }
+        if (++as == p.a_stages) { as = 0; aph ^= 1u; }
+      }
+    }
+  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
+    // ---------------------------------------------------------------- epilogue: one output pixel per thread
+    // int8: group g of four warps serves accumulator g of four, or column half g & 1 of accumulator g >> 1 of two
+    const int quarter = warp & 3, group = (warp - EPI_WARP0) >> 2;
+    const bool whole = p.bufs == 4;
+    const int half = whole ? 0 : group & 1, blk_step = whole ? 1 : 2;
+    const int row = quarter * 32 + lane;
+    const int elt = KIND == HALO_F32 || p.rq.out_type == OUT_F32 ? 4 : 1;
+    const size_t blk_stride = static_cast<size_t>(p.OH) * p.OW;
+    const int nb16 = p.BN >> 4, cnt = whole ? nb16 : (nb16 - half + 1) >> 1;
+    const int t_step = KIND == HALO_F32 ? 1 : p.bufs, t_shift = whole ? 2 : 1;
+    int t = KIND == HALO_F32 ? 0 : whole ? group : group >> 1;
+    bool ok = true;
+    for (int tile = blockIdx.x + t * gridDim.x; tile < p.total_tiles && ok; tile += t_step * gridDim.x, t += t_step) {
+      const int mt = p.div_n.div(tile), nt = tile - mt * p.n_tiles;
+      const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
+      const int v = rt * TILE_H + (row >> 3);
+      const int n = p.div_period.div(v), oh = v - n * p.period, ow = ct * TILE_W + (row & 7);
+      const bool valid = n < p.N && oh < p.OH && ow < p.OW;
+      const size_t pix = (static_cast<size_t>(n) * p.OCB * p.OH + oh) * p.OW + ow;
+      const float *shift_row = s_shift;
+      if (KIND == HALO_I8 && p.shift_tbl && valid) {
+        const int cls = __ldg(p.hclass + oh) * p.zp_nw + __ldg(p.wclass + ow);
+        if (cls != p.zp_full) shift_row = p.shift_tbl + static_cast<size_t>(cls) * (p.OCB * 16);
+      }
+      const uint32_t buf = t & (p.bufs - 1), tph = (t >> t_shift) & 1u;
+      if (!wait_all(&bar.tfull[buf], tph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
+      tc_fence_after_sync();
+      const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (whole ? 128u : 256u) + half * 16;
+      auto emit = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16]) {
+        const int ocb = nt * nb16 + blk;
+        if (!valid || ocb >= p.OCB) return;
+        const size_t off = (pix + ocb * blk_stride) * 16;
+        if (KIND == HALO_I8) {
+          int a[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) a[i] = static_cast<int>(r[i]);
+          if (p.acc_dump) {
+            int4 *d = reinterpret_cast<int4 *>(p.acc_dump + off);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) d[i] = make_int4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+          }
+          if (p.fast == 2) requant_relu_u8(a, s_scale + ocb * 16, s_shift + ocb * 16, static_cast<uint8_t *>(p.out) + off);
+          else if (p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
+          else requant_store16(a, s_scale + ocb * 16, shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * elt, p.rq);
+        } else {
+          float f[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            f[i] = __uint_as_float(r[i]);
+            if (STACK) f[i] = __fadd_rn(f[i], __uint_as_float(r2[i]));
+          }
+          float *o = static_cast<float *>(p.out) + off;
+          if (p.shift) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 b = reinterpret_cast<const float4 *>(s_shift + ocb * 16)[i];
+              f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
+              f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
+            }
+          }
+          if (p.rq.with_sum) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const float4 b = reinterpret_cast<const float4 *>(o)[i];
+              f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
+              f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
+            }
+          }
+          if (p.rq.relu) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) f[i] = fminf(fmaxf(f[i], p.rq.relu_lo), p.rq.relu_hi);
+          }
+          store_v8(o, f, 0);
+          store_v8(o, f, 8);
+        }
+      };
+      auto release = [&]() {
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.tempty[buf]);
+      };
+      {
+      // blocks half, half + blk_step, ... of this warp, two in flight: while one is converted and stored the next is
+        // on its way out of tensor memory
+        uint32_t r0[16], r1[16], q0[16], q1[16];
+        constexpr bool pair = STACK;
+        auto load = [&](int k, uint32_t (&r)[16], uint32_t (&q)[16]) {
+          tmem_ld16(t_addr + k * (16 * blk_step), r);
+          if (pair) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
+        };
+        if (cnt > 0) load(0, r0, q0);
+#pragma unroll 1
+        for (int k = 0; k < cnt; k += 2) {
+          tmem_ld_wait16(r0);
+          if (pair) tmem_ld_wait16(q0);
+          if (k + 1 < cnt) load(k + 1, r1, q1);
+          emit(half + blk_step * k, r0, q0);
+          if (k + 1 < cnt) {
+            tmem_ld_wait16(r1);
+            if (pair) tmem_ld_wait16(q1);
+            if (k + 2 < cnt) load(k + 2, r0, q0);
+            emit(half + blk_step * (k + 1), r1, q1);
+          }
+        }
+        release();
+      }
+    }
+  }
+
+  if (fail_code != 0) atomicCAS(p.status, 0, fail_code);
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  if (warp == 1) tmem_dealloc(tmem_base, 512);
+}
+
+int alignup(int v, int a) { return (v + a - 1) / a * a; }
+
+// Cycles one K step keeps the tensor pipe busy: N / 2 for an MMA of 128 x N x 32 bytes, unless reading
+// its operands from shared memory (128 B/clk) takes longer, which it does below N = 128.
+double mma_cycles(int n) { return std::max(n / 2.0, 32.0 + n / 4.0); }
+double kstep_cycles(int kind, int BN) {
+  if (kind == HALO_I8) return mma_cycles(BN);
+  return BN <= 128 ? mma_cycles(2 * BN) + mma_cycles(BN) : 3 * mma_cycles(BN);
+}
+
+}  // namespace
+
+bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, int oh, int ow, int kh, int kw, int stride,
+               int pad_t, int pad_l, int num_sms, std::string &err) {
+  HaloParams &p = hp.p;
+  hp.kind = kind; hp.stride = stride; hp.IH = ih; hp.IW = iw;
+  hp.CB = (ic + 15) / 16;
+  p.OCB = (oc + 15) / 16;
+  if (stride < 1 || stride > 2 || ih < stride || iw < stride) { err = "stride"; return false; }
+  p.N = n; p.OH = oh; p.OW = ow; p.strided = stride > 1;
+  auto fdiv = [](int e, int s) { return e >= 0 ? e / s : -((-e + s - 1) / s); };
+  // which parity plane each tap reads, and by how many rows / columns it shifts there
+  const int taps = kh * kw;
+  std::vector<int> plane(taps), dr(taps), dc(taps);
+  int rmin[4], rmax[4], cmin[4], cmax[4];
+  for (int i = 0; i < 4; ++i) { rmin[i] = cmin[i] = 1 << 20; rmax[i] = cmax[i] = -(1 << 20); }
+  for (int t = 0; t < taps; ++t) {
+    const int eh = t / kw - pad_t, ew = t % kw - pad_l;
+    dr[t] = fdiv(eh, stride); dc[t] = fdiv(ew, stride);
+    plane[t] = (eh - dr[t] * stride) * stride + (ew - dc[t] * stride);
+    const int q = plane[t];
+    rmin[q] = std::min(rmin[q], dr[t]); rmax[q] = std::max(rmax[q], dr[t]);
+    cmin[q] = std::min(cmin[q], dc[t]); cmax[q] = std::max(cmax[q], dc[t]);
+  }
+  int span_c = 0, rows = 0, period = oh;
+  p.planes = 0;
+  for (int q = 0; q < stride * stride; ++q) {
+    if (rmin[q] > rmax[q]) continue;
+    if (rmin[q] < -24 || rmax[q] > 24) { err = "padding"; return false; }
+    const int i = p.planes++;
+    hp.parity[i] = q;
+    p.row0[i] = rmin[q]; p.rows[i] = TILE_H + rmax[q] - rmin[q]; p.col0[i] = cmin[q];
+    span_c = std::max(span_c, cmax[q] - cmin[q]);
+    if (p.rows[i] > 32) { err = "filter height"; return false; }
+    rows = std::max(rows, p.rows[i]);
+    // Stacked images: the rows above image i are read as rows period + d of image i - 1 and must lie outside
+    // it (zeros); the rows below its last output row must not reach image i + 1.
+    const int hp_rows = (ih - q / stride + stride - 1) / stride;
+    if (rmax[q] > 0) period = std::max(period, oh + rmax[q]);
+    if (rmin[q] < 0) period = std::max(period, hp_rows - rmin[q]);
+  }
+  p.period = period;
+  p.div_period.set(period);
+  // Channel groups.  fp32: one 16-channel block (four chunks).  int8: an even number of blocks, at most eight,
+  // that wastes the fewest chunks past the last block (narrow groups cost more hand-overs per MMA), or one.
+  int kch = 4;
+  if (kind == HALO_I8) {
+    double best_k = 0;
+    kch = 0;
+    for (int k = 8; k >= 2; k -= 2) {
+      if (k > 2 && k - 2 >= hp.CB) continue;
+      if (rows * alignup((TILE_W + span_c) * k, 8) * 16 > 48 * 1024) continue;
+      const double c = static_cast<double>((hp.CB + k - 1) / k) * (k + 0.5);
+      if (kch == 0 || c < best_k) { best_k = c; kch = k; }
+    }
+    if (hp.CB == 1 || kch == 0) kch = 1;
+  }
+  int pxw = TILE_W + span_c + (kch == 1 && !(span_c & 1));      // (the last tap of an odd row pairs up with a zero weight)
+  while ((kind == HALO_F32 ? pxw * 64 : kch * pxw * 16) % 128) ++pxw;      // (a TMA destination is 128-byte aligned)
+  if (pxw > 32) { err = "filter width"; return false; }
+  p.kch = kch; p.pxw = pxw;
+  p.div_px.set(pxw);
+  p.pitch = kch * pxw * 16;
+  p.a_bytes = rows * p.pitch;
+  if (p.a_bytes > 48 * 1024) { err = "filter size"; return false; }
+  p.cb_step = kind == HALO_F32 ? 1 : kch;
+  p.groups = kind == HALO_F32 ? hp.CB : (hp.CB + kch - 1) / kch;
+  p.raw_bytes = kind == HALO_F32 ? p.a_bytes : 0;
+  // K steps in the order the issuer takes them: two chunks each
+  hp.order.clear();
+  p.ksteps = 0;
+  for (int i = 0; i < p.planes; ++i) {
+    const int q = hp.parity[i], ph = q / stride, pw = q % stride;
+    p.tap_rows[i] = rmax[q] - rmin[q] + 1; p.tap_cols[i] = cmax[q] - cmin[q] + 1;
+    for (int r = 0; r < p.tap_rows[i]; ++r)
+      for (int c = 0; c < p.tap_cols[i]; c += kch == 1 ? 2 : 1) {
+        const int t = ((rmin[q] + r) * stride + ph + pad_t) * kw + (cmin[q] + c) * stride + pw + pad_l;
+        if (kch == 1) {
+          hp.order.push_back({t, 0});
+          if (c + 1 < p.tap_cols[i]) hp.order.push_back({t + stride, 0});
+          else hp.order.push_back({-1, 0});
+        } else {
+          for (int b = 0; b < kch; ++b) hp.order.push_back({t, b});
+        }
+      }
+  }
+  p.ksteps = static_cast<int>(hp.order.size()) / 2;
+  // tile width: the smallest modelled time over the whole chip
+  const int OCP = p.OCB * 16;
+  p.row_tiles = (static_cast<int>((static_cast<long long>(n - 1) * period) + oh) + TILE_H - 1) / TILE_H;
+  p.col_tiles = (ow + TILE_W - 1) / TILE_W;
+  const double m_tiles = static_cast<double>(p.row_tiles) * p.col_tiles;
+  if (m_tiles * p.OCB > 1e9 || OCP > HALO_MAX_OC) { err = "size"; return false; }
+  const int planes_bytes = p.a_bytes * (kind == HALO_F32 ? 2 : 1);
+  double best = 0;
+  p.BN = 0;
+  for (int nt = (OCP + 255) / 256; nt <= p.OCB; ++nt) {
+    const int BN = alignup((OCP + nt - 1) / nt, 16);
+    if ((OCP + BN - 1) / BN != nt) continue;
+    const double kb = BN * (kind == HALO_F32 ? 64.0 : 32.0), ab = static_cast<double>(p.a_bytes) * p.planes / p.ksteps;
+    const double writes = (kb + ab * (kind == HALO_F32 ? 4 : 1)) / 128, ingest = (kb + ab) / 50;
+    const double tile = std::max(kstep_cycles(kind, BN) + writes, ingest) * p.ksteps * p.groups + 1500;
+    const double t = std::ceil(m_tiles * nt / num_sms) * tile;
+    if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; }
+  }
+  p.stack = kind == HALO_F32 && p.BN <= 128;
+  p.bufs = kind == HALO_I8 && p.BN <= 128 ? 4 : 2;      // accumulators in the 512 columns of tensor memory
+  p.div_n.set(p.n_tiles);
+  p.div_col.set(p.col_tiles);
+  // shared memory: operand rows first, the rest is the weight ring
+  p.kstep_bytes = p.BN * (kind == HALO_F32 ? 64 : 32);
+  const int fixed = p.n_tiles * p.BN * (kind == HALO_F32 ? 4 : 8) + static_cast<int>(sizeof(Bars)) + 256;
+  const int room = SMEM_LIMIT - fixed - RAW_STAGES * p.raw_bytes;
+  int b_per_group = 0, most_c = 0;      // weight stages of a channel group; longest filter row
+  for (int i = 0; i < p.planes; ++i) most_c = std::max(most_c, p.tap_cols[i]);
+  const int pairs = kch / 2, row_steps = kch == 1 ? (most_c + 1) / 2 : most_c * pairs;
+  // a stage costs its hand-over whatever it holds: whole filter rows while they are small
+  auto set_units = [&](bool rows_of_taps) {
+  p.row_units = rows_of_taps;
+  b_per_group = 0;
+  for (int i = 0; i < p.planes; ++i) b_per_group += p.row_units ? p.tap_rows[i] : p.tap_rows[i] * p.tap_cols[i];
+  p.b_per_tile = b_per_group * p.groups;
+  p.b_stage_bytes = (p.row_units ? row_steps : pairs) * p.kstep_bytes;
+  };
+  auto fit_b = [&](int a_stages) -> bool {
+    p.a_stages = a_stages;
+    p.b_stages = std::min(MAX_B, (room - a_stages * planes_bytes) / p.b_stage_bytes);
+    return p.b_stages >= 1;
+  };
+  const long long b_all = static_cast<long long>(p.groups) * p.ksteps * p.kstep_bytes;
+  p.resident = 0;
+  if (p.n_tiles == 1 && b_all <= room - 2ll * planes_bytes) {
+    // the whole filter fits: it is fetched once per CTA
+    set_units(true);
+    for (int a = MAX_A; a >= 2 && !p.resident; --a)
+      if (a * static_cast<long long>(planes_bytes) + b_all <= room) {
+        fit_b(a);
+        if (p.groups * b_per_group <= MAX_B && p.groups * b_per_group <= p.b_stages) {
+          p.resident = 1;
+          p.b_stages = p.groups * b_per_group;
+        }
+      }
+  }
+  if (!p.resident) {
+    set_units(kch == 1 || row_steps * p.kstep_bytes <= 24 * 1024);
+    bool ok = false;
+    for (int a = planes_bytes <= 24 * 1024 ? 3 : 2; a >= 1 && !ok; --a) ok = fit_b(a) && p.b_stages >= 3;
+    if (!ok) { err = "shared memory"; return false; }
+  }
+  hp.smem_bytes = static_cast<size_t>(p.a_stages) * planes_bytes + RAW_STAGES * static_cast<size_t>(p.raw_bytes) +
+                  static_cast<size_t>(p.b_stages) * p.b_stage_bytes + fixed;
+  hp.b_bytes = static_cast<size_t>(p.n_tiles) * b_all;
+  return true;
+}
+
+std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP) {
+  const HaloParams &p = hp.p;
+  std::vector<uint8_t> img(hp.b_bytes, 0);
+  uint8_t *dst = img.data();
+  for (int nt = 0; nt < p.n_tiles; ++nt)
+    for (int g = 0; g < p.groups; ++g)
+      for (int k = 0; k < p.ksteps * 2; ++k, dst += p.BN * 16) {
+        const HaloPlan::Chunk c = hp.order[k];
+        const int cb = g * p.kch + c.cb;
+        if (c.tap < 0 || cb >= hp.CB) continue;
+        for (int r = 0; r < p.BN && nt * p.BN + r < OCP; ++r)
+          std::memcpy(dst + r * 16, q + (static_cast<size_t>(nt * p.BN + r) * taps + c.tap) * ICP + cb * 16, 16);
+      }
+  return img;
+}
+
+std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, int taps, int ICP) {
+  const HaloParams &p = hp.p;
+  std::vector<uint8_t> img(hp.b_bytes, 0);
+  float *dst = reinterpret_cast<float *>(img.data());
+  const int BN = p.BN;
+  for (int nt = 0; nt < p.n_tiles; ++nt)
+    for (int g = 0; g < p.groups; ++g)
+      for (int k = 0; k < p.ksteps; ++k, dst += BN * 16)
+        for (int j = 0; j < 2; ++j) {
+          const HaloPlan::Chunk c = hp.order[2 * k + j];      // cb: which four channels of the block
+          float *hi = dst + static_cast<size_t>(j) * (p.stack ? 2 * BN : BN) * 4;
+          float *lo = p.stack ? hi + BN * 4 : hi + static_cast<size_t>(2) * BN * 4;
+          for (int r = 0; r < BN && nt * BN + r < OCP; ++r) {
+            const float *src = u + (static_cast<size_t>(nt * BN + r) * taps + c.tap) * ICP + g * 16 + c.cb * 4;
+            for (int e = 0; e < 4; ++e) {
+              const float h = host::tf32_rna(src[e]);
+              volatile float l = src[e] - h;
+              hi[r * 4 + e] = h;
+              lo[r * 4 + e] = l;
+            }
+          }
+        }
+  return img;
+}
+
+namespace {
+
+// Tensor maps of `cnt` images at `in`.
+bool encode_maps(const HaloPlan &hp, const void *in, int cnt, CUtensorMap (*out)[HALO_HEIGHTS], std::string &err) {
+  PFN_encodeTiled enc = get_encode_tiled();
+  if (!enc) { err = "cuTensorMapEncodeTiled is not available from the driver"; return false; }
+  const HaloParams &p = hp.p;
+  const cuuint64_t px = hp.kind == HALO_F32 ? 64 : 16, IW = hp.IW, IH = hp.IH, CB = hp.CB;
+  const cuuint32_t blocks = p.cb_step, estr[5] = {1, 1, 1, 1, 1};
+  CUresult r = CUDA_SUCCESS;
+  // (dimensions in the order the operand rows lie in shared memory: pixels, channel blocks, rows)
+  for (int q = 0; q < p.planes; ++q)
+    for (int i = 0; i < HALO_HEIGHTS && r == CUDA_SUCCESS; ++i) {
+      const cuuint32_t height = i == HALO_HEIGHTS - 1 ? p.rows[q] : 1u << i;
+      if (!p.strided) {
+        cuuint64_t dims[4] = {IW * px / 8, CB, IH, static_cast<cuuint64_t>(cnt)};
+        cuuint64_t strides[3] = {IH * IW * px, IW * px, CB * IH * IW * px};
+        cuuint32_t box[4] = {static_cast<cuuint32_t>(p.pxw * px / 8), blocks, height, 1};
+        r = enc(&out[q][i], CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<void *>(in), dims, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      } else {
+        const int s = hp.stride, ph = hp.parity[q] / s, pw = hp.parity[q] % s;
+        cuuint64_t dims[5] = {16, static_cast<cuuint64_t>((hp.IW - pw + s - 1) / s), CB,
+                              static_cast<cuuint64_t>((hp.IH - ph + s - 1) / s), static_cast<cuuint64_t>(cnt)};
+        cuuint64_t strides[4] = {s * px, IH * IW * px, s * IW * px, CB * IH * IW * px};
+        cuuint32_t box[5] = {16, static_cast<cuuint32_t>(p.pxw), blocks, height, 1};
+        uint8_t *base = const_cast<uint8_t *>(static_cast<const uint8_t *>(in)) + (static_cast<size_t>(ph) * IW + pw) * px;
+        r = enc(&out[q][i], hp.kind == HALO_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dims,
+                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      }
+    }
+  if (r != CUDA_SUCCESS) { err = "cuTensorMapEncodeTiled failed (" + std::to_string(static_cast<int>(r)) + ")"; return false; }
+  return true;
+}
+
+}  // namespace
+
+namespace {
+
+typedef void (*HaloKernel)(HaloParams);
+template <int FORM>
+HaloKernel pick_kernel(const HaloPlan &hp) {
+  if (hp.kind == HALO_F32) return hp.p.stack ? conv_halo_kernel<HALO_F32, 2, FORM, true> : conv_halo_kernel<HALO_F32, 2, FORM, false>;
+  switch (hp.p.kch) {
+    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false>;
+    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false>;
+    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false>;
+    case 2: return conv_halo_kernel<HALO_I8, 1, FORM, false>;
+    default: return conv_halo_kernel<HALO_I8, 0, FORM, false>;
+  }
+}
+HaloKernel pick_kernel(const HaloPlan &hp) {
+  const HaloParams &p = hp.p;
+  if (p.strided || p.tap_cols[0] != 3 || p.tap_rows[0] != 3 || p.pxw != pxw_3x3(hp.kind, p.kch / 2)) return pick_kernel<FORM_ANY>(hp);
+  if (p.resident && p.b_stages == 3 * p.groups) return pick_kernel<FORM_3X3_RESIDENT>(hp);
+  if (p.resident) return pick_kernel<FORM_ANY>(hp);
+  return p.row_units ? pick_kernel<FORM_3X3_ROWS>(hp) : pick_kernel<FORM_3X3_TAPS>(hp);
+}
+
+}  // namespace
+
+cudaError_t halo_init(const HaloPlan &hp) {
+  return cudaFuncSetAttribute(pick_kernel(hp), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
+}
+
+bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err) {
+  const HaloPlan::Maps *hit = nullptr;
+  for (const auto &m : hp.maps)
+    if (m.base == in && m.cnt == images) { hit = &m; break; }
+  if (!hit) {
+    HaloPlan::Maps m{};
+    m.base = in; m.cnt = images;
+    if (!encode_maps(hp, in, images, m.m, err)) return false;
+    if (hp.maps.size() >= 64) hp.maps.erase(hp.maps.begin());
+    hp.maps.push_back(m);
+    hit = &hp.maps.back();
+  }
+  std::memcpy(p.tmap, hit->m, sizeof(p.tmap[0]) * p.planes);
+  p.b_img = static_cast<const uint8_t *>(hp.d_b);
+  const bool fast = p.rq.out_type == OUT_U8 && p.rq.relu && p.rq.relu_lo == 0.0f && p.rq.relu_hi >= 3.0e38f && !p.rq.with_sum &&
+                    !p.shift_tbl;
+  p.fast = !fast ? 0 : p.OCB * 16 <= HALO_PARAM_OC ? 1 : 2;
+  if (p.fast == 1)
+    for (int i = 0; i < p.OCB * 16; ++i) { p.cst[0][i] = hp.scale[i]; p.cst[1][i] = hp.shift[i]; }
+  p.N = images;
+  p.row_tiles = ((images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
+  p.total_tiles = p.row_tiles * p.col_tiles * p.n_tiles;
+  const dim3 grid(std::min(p.total_tiles, num_sms));
+  const cudaError_t e = launch_overlapped(pick_kernel(hp), grid, dim3(hp.kind == HALO_F32 ? THREADS_F32 : THREADS_I8),
+                                          hp.smem_bytes, s, p);
+  if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
+  return true;
+}
+
+}  // namespace elb

@@ -13,6 +13,7 @@
 
 #include "../../include/euler_b200.h"
 #include "elb_common.cuh"
+#include "conv_halo.cuh"
 #include "host_prep.hpp"
 #include "wino.cuh"
 #include "depthwise.cuh"
@@ -162,6 +163,7 @@ struct elb_conv {
   // int8 direct
   I8ConvParams i8{};
   I8UmmaConfig i8cfg{};
+  HaloPlan *halo = nullptr;             // KxK and strided int8: the halo-tiled kernel
   struct TmapEntry { const void *base; int cnt; CUtensorMap m[4]; };
   std::vector<TmapEntry> tmaps;         // tensor maps encoded so far, keyed by (first image address, image count)
   // host-pointer callers: copy streams and events of the chunked, overlapped execute
@@ -184,6 +186,8 @@ struct elb_conv {
     for (void *p : {d_wpack, d_wplain, d_scale, d_shift, d_shift_tbl, d_tap_cls, d_tap_tbl, (void *)d_status, d_in_stage, d_out_stage,
                     d_cvt_in, d_cvt_out})
       if (p) cudaFree(p);
+    if (halo && halo->d_b) cudaFree(halo->d_b);
+    delete halo;
     wino_release(wino);
     dw_release(dw);
     if (stream) cudaStreamSynchronize(stream);
@@ -359,6 +363,20 @@ int setup_i8_direct(elb_conv &pl) {
   // applies the 1x1 semantics there as well (f += prev * sum_scale); with the flag off the two agree bit for bit.
   p.rq.with_sum = d.with_ip_sum && d.dt_output != ELB_F32;
   p.rq.sum_scale = d.sum_scale;
+  if (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA) {
+    // (ELB_I8_CTA2=1 asks for the pair kernel, which takes the one-copy-per-tap form below)
+    const char *on2 = getenv("ELB_I8_CTA2");
+    std::string why;
+    pl.halo = new HaloPlan();
+    if (!(on2 && atoi(on2) > 0) &&
+        halo_plan(*pl.halo, HALO_I8, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, pl.num_sms, why)) {
+      CUDA_TRY(halo_init(*pl.halo));
+      pl.info.launches_per_call = 1;
+      return ELB_OK;
+    }
+    delete pl.halo;
+    pl.halo = nullptr;
+  }
   if (pl.info.kernel == ELB_KERNEL_I8_GEMM_UMMA || pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA) {
     // A 1x1 stride-1 convolution has no halo, so its image plane is viewed as ONE row of oh*ow
     // pixels: the tile becomes 128 consecutive pixels of one image and a whole K stage of A is a
@@ -502,6 +520,13 @@ int prepare_i8_direct(elb_conv &pl, const void *weights, const void *bias) {
     CUDA_TRY(cudaMalloc(&pl.d_wplain, wq.q.size()));
     CUDA_TRY(cudaMemcpy(pl.d_wplain, wq.q.data(), wq.q.size(), cudaMemcpyHostToDevice));
     pl.info.workspace_bytes += wq.q.size();
+  } else if (pl.halo) {
+    pl.halo->scale = scale;
+    pl.halo->shift = shift;
+    const std::vector<uint8_t> pk = halo_pack_i8(*pl.halo, wq.q.data(), wq.OCP, wq.taps, wq.ICP);
+    CUDA_TRY(cudaMalloc(&pl.halo->d_b, pk.size()));
+    CUDA_TRY(cudaMemcpy(pl.halo->d_b, pk.data(), pk.size(), cudaMemcpyHostToDevice));
+    pl.info.workspace_bytes += pk.size();
   } else {
     int n_tiles, CBG, k_stages;
     std::vector<int8_t> pk = host::pack_b_i8(wq, pl.i8cfg.BN, pl.i8cfg.KC, n_tiles, CBG, k_stages,
@@ -533,6 +558,16 @@ int run_i8_direct(elb_conv &pl, void *out, const void *in, int n0, int cnt, cuda
   p.N = cnt;
   p.M = cnt * p.HW;
   cudaError_t e;
+  if (pl.halo) {
+    HaloParams hp = pl.halo->p;
+    hp.scale = p.scale; hp.shift = p.shift;
+    hp.shift_tbl = p.shift_tbl; hp.hclass = p.hclass; hp.wclass = p.wclass; hp.zp_nw = p.zp_nw; hp.zp_full = p.zp_full;
+    hp.out = p.out; hp.acc_dump = p.acc_dump; hp.status = p.status; hp.rq = p.rq;
+    std::string err;
+    if (!halo_launch(*pl.halo, hp, p.in, cnt, pl.num_sms, s, err)) return fail(ELB_GENERAL_ERROR, "%s", err.c_str());
+    pl.launches += 1;
+    return ELB_OK;
+  }
   if (pl.info.kernel == ELB_KERNEL_I8_SIMT) {
     e = launch_i8_simt(p, s);
   } else {

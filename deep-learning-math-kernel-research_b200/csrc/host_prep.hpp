@@ -20,6 +20,15 @@ inline size_t w_index(int I2, int KH, int KW, int o, int i, int kh, int kw) {
   return (((((size_t)(o / 16) * I2 + i / 16) * KH + kh) * KW + kw) * 16 + i % 16) * 16 + o % 16;
 }
 
+inline float tf32_rna(float x) {            // what cvt.rna.tf32.f32 returns for finite x
+  uint32_t u;
+  std::memcpy(&u, &x, 4);
+  u = (u + 0x1000u) & 0xFFFFE000u;
+  float r;
+  std::memcpy(&r, &u, 4);
+  return r;
+}
+
 struct I8Weights {
   int OCP = 0, ICP = 0, taps = 0;
   std::vector<int8_t> q;        // [OCP][taps][ICP]

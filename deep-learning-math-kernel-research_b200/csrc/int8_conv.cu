@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) i8_umma_kernel(const __grid_co
   const bool merged_rows = SPEC == 1 ? true : SPEC == 2 ? false : p.merged_rows != 0;
   const bool use_tbl = SPEC != 0 ? true : p.tap_tbl != nullptr;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  uint8_t *smem = smem_aligned(smem_raw);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::BAR_OFF);
   uint64_t *empty = full + STAGES;
   uint64_t *tfull = empty + STAGES;

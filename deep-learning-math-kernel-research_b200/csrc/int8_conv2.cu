@@ -49,7 +49,7 @@ template <int BN, int KC, int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) i8_umma2_kernel(const __grid_constant__ I8ConvParams p) {
   using L = Smem2<BN, KC, STAGES>;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  uint8_t *smem = smem_aligned(smem_raw);
   uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::BAR_OFF);
   uint64_t *empty = full + STAGES;
   uint64_t *pfull = empty + STAGES;       // leader only: the peer's stage s has landed

@@ -16,6 +16,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The next 128-byte boundary of the dynamic shared memory.  As an offset from the array: through an integer the
+// compiler loses track of the address space and every access becomes a generic load or store.
+__device__ __forceinline__ uint8_t *smem_aligned(uint8_t *base) { return base + ((128u - (smem_u32(base) & 127u)) & 127u); }
+
 __device__ __forceinline__ unsigned long long global_timer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -245,6 +249,32 @@ __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t adesc, uint6
       "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same MMAs for a whole CONVERGED warp: `el` (0 / 1) is nonzero in the one lane that issues.  The lane is
+// selected by a predicate on the instruction instead of a branch around it, so the operands stay
+// warp-uniform values: measured with back-to-back MMAs whose addresses are computed on the way, 8 cycles per
+// issue against 44 from inside an `if (lane == 0)` -- and an MMA of 128 x 64 x 32 bytes lasts only 48.
+__device__ __forceinline__ void umma_i8_el(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                           uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P, Q;\n\t"
+      "setp.ne.b32 P, %4, 0;\n\t"
+      "setp.ne.b32 Q, %5, 0;\n\t"
+      "@Q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, P;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void umma_tf32_el(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                             uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P, Q;\n\t"
+      "setp.ne.b32 P, %4, 0;\n\t"
+      "setp.ne.b32 Q, %5, 0;\n\t"
+      "@Q tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, P;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
+      : "memory");
+}
 // Same with the A operand in TENSOR memory: a_tmem addresses 128 lanes (the M rows) x 8 columns,
 // one tf32 value per 32-bit column (written with tmem_st16).  A read from tensor memory does not
 // use the shared-memory port, which the B operand and the incoming copies need.
@@ -262,6 +292,16 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
                ::"r"(smem_u32(bar)) : "memory");
+}
+
+__device__ __forceinline__ void umma_commit_el(uint64_t *bar, uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred Q;\n\t"
+      "setp.ne.b32 Q, %1, 0;\n\t"
+      "@Q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(smem_u32(bar)), "r"(el)
+      : "memory");
 }
 
 // ------------------------------------------------------------------------------------ CTA pairs

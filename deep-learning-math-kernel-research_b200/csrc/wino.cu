@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "elb_common.cuh"
+#include "conv_halo.cuh"
 #include "host_prep.hpp"
 #include "umma.cuh"
 #include <type_traits>
@@ -630,7 +631,7 @@ struct WinoGemmParams {
 template <bool CTA2, int KMUL = 1, int SPEC = 0, int TBN = 0>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid_constant__ WinoGemmParams p) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+  uint8_t *smem = smem_aligned(smem_raw);
   constexpr int GEMM_STAGES = CTA2 ? GEMM_STAGES_2 : GEMM_STAGES_1;
   constexpr int STAGE_BYTES = A_STAGE_BYTES + (CTA2 ? B_STAGE_MAX / 2 : B_STAGE_MAX);
   // ring of operand stages (fp32: the copy of V lands in the first half of the A region and is split
@@ -1547,15 +1548,6 @@ __global__ void __launch_bounds__(128) f32_epilogue_kernel(const __grid_constant
 }
 
 // ------------------------------------------------------------------------------ host side
-inline float tf32_rna(float x) {            // what cvt.rna.tf32.f32 returns for finite x
-  uint32_t u;
-  std::memcpy(&u, &x, 4);
-  u = (u + 0x1000u) & 0xFFFFE000u;
-  float r;
-  std::memcpy(&r, &u, 4);
-  return r;
-}
-
 // G with the reference's constants and order (src/kernel/elk_conv_wino_4x4_3x3_weights.hxx:25-58)
 inline void g3(float f0, float f1, float f2, float o[6]) {
   const float z0 = 0.26890756302521f, z1 = -0.688403361344538f, z2 = 0.119514472455649f,
@@ -1677,6 +1669,7 @@ struct WinoImpl {
   float relu_lo = 0.f, relu_hi = 3.402823466e38f;
   bool direct = false;     // fp32 direct convolution on the GEMM kernel (g.A == 1)
   bool flat = false;       // ... 1x1 stride 1 without padding: the GEMM kernel alone, reading the user's tensor
+  HaloPlan *halo = nullptr;   // fp32 KxK / strided: the halo-tiled kernel (conv_halo.cu) does the whole convolution
   bool small_ic = false;   // fp32 Winograd asked for a layer with <= 4 input channels: the CUDA-core direct kernel
   void *d_w_small = nullptr;
   int ic_real = 0;
@@ -1686,6 +1679,10 @@ struct WinoImpl {
   bool stack = false;      // fp32, BN <= 128: hi and lo weight rows stacked per K chunk (two MMAs per K step instead of three)
   int max_clusters = 0;    // pairs the device holds at once
   void *d_a = nullptr, *d_b = nullptr, *d_m = nullptr, *d_bias = nullptr, *d_scale = nullptr, *d_shift = nullptr;
+  ~WinoImpl() {
+    if (halo && halo->d_b) cudaFree(halo->d_b);
+    delete halo;
+  }
 };
 
 int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, std::string &err) {
@@ -1727,6 +1724,22 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   g.k_stages = w->kind == KIND_F32 ? g.CB * g.taps : (g.CB + 7) / 8;
   w->n_tiles = (w->OCP + MAX_BN - 1) / MAX_BN;
   w->BN = host::alignup((w->OCP + w->n_tiles - 1) / w->n_tiles, 16);
+  // Direct convolutions other than the plain 1x1: one kernel that reads the caller's tensor, instead of an
+  // im2col tensor written and read once per tap (3x3 stride 2, 64 x 128 -> 256 channels 56x56: 231 MB of it).
+  if (direct && !(d.kh == 1 && d.kw == 1 && d.stride_h == 1)) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    w->halo = new HaloPlan();
+    std::string why;
+    if (!halo_plan(*w->halo, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why)) {
+      delete w->halo;
+      w->halo = nullptr;
+    } else if (halo_init(*w->halo) != cudaSuccess) {
+      err = "cudaFuncSetAttribute failed";
+      return ELB_GENERAL_ERROR;
+    }
+  }
   // chunk of whole images whose transform-domain buffers fit the budget
   const size_t tiles_img = static_cast<size_t>(g.ht) * g.wt;
   const size_t a_gbytes = w->kind == KIND_F32 ? A_RAW_BYTES : A_STAGE_BYTES;    // one stage of A in global memory
@@ -1735,7 +1748,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   budget = static_cast<size_t>(tune_env("ELB_WINO_CHUNK_MB", static_cast<int>(budget >> 20))) << 20;
   size_t imgs = budget / (per_tile * tiles_img);
   if (imgs < 1) imgs = 1;
-  if (imgs > static_cast<size_t>(d.n) || w->flat || w->small_ic) imgs = d.n;       // (no transform-domain buffers in these modes)
+  if (imgs > static_cast<size_t>(d.n) || w->flat || w->small_ic || w->halo) imgs = d.n;       // (no transform-domain buffers in these modes)
   w->imgs_per_chunk = static_cast<int>(imgs);
   g.N = w->imgs_per_chunk;
   g.T = static_cast<int>(imgs * tiles_img);
@@ -1744,7 +1757,8 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   w->a_bytes = static_cast<size_t>(AA) * g.m_tiles * g.k_stages * a_gbytes;
   w->b_bytes = static_cast<size_t>(AA) * w->n_tiles * g.k_stages * 128 * w->BN;
   w->m_bytes = static_cast<size_t>(AA) * g.OCB * g.Tpad * 16 * 4;
-  if (w->flat || w->small_ic) { w->a_bytes = 256; w->m_bytes = 256; }
+  if (w->flat || w->small_ic || w->halo) { w->a_bytes = 256; w->m_bytes = 256; }
+  if (w->halo) w->b_bytes = w->halo->b_bytes;
   w->in_img_bytes = static_cast<size_t>(w->ICP) * d.ih * d.iw * (d.dt_input == ELB_F32 ? 4 : 1);
   w->out_type = d.dt_output == ELB_F32 ? OUT_F32 : d.dt_output == ELB_U8 ? OUT_U8 : OUT_S8;
   w->out_img_bytes = static_cast<size_t>(w->OCP) * d.oh * d.ow * (w->out_type == OUT_F32 ? 4 : 1);
@@ -1790,7 +1804,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     }
   }
   w->stack = w->kind == KIND_F32 && !w->cta2 && w->BN <= 128 && tune_env("ELB_F32_STACK", 1) > 0;
-  info.launches_per_call = (w->flat || w->small_ic) ? 1 : 3 * ((d.n + w->imgs_per_chunk - 1) / w->imgs_per_chunk);
+  info.launches_per_call = (w->flat || w->small_ic || w->halo) ? 1 : 3 * ((d.n + w->imgs_per_chunk - 1) / w->imgs_per_chunk);
   if (w->small_ic) {
     e = init_f32_small_ic(g.OCB);
     if (e != cudaSuccess) { err = std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e); return ELB_GENERAL_ERROR; }
@@ -1841,6 +1855,15 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
   } else {
     u = transform_weights(hw.data(), d.oc, d.ic, w->OCP, w->ICP, g.A);
   }
+  if (w->halo) {
+    const std::vector<uint8_t> img = halo_pack_f32(*w->halo, u.data(), w->OCP, g.taps, w->ICP);
+    W_TRY(cudaMalloc(&w->halo->d_b, img.size()));
+    W_TRY(cudaMemcpy(w->halo->d_b, img.data(), img.size(), cudaMemcpyHostToDevice));
+    W_TRY(cudaMalloc(&w->d_bias, static_cast<size_t>(w->OCP) * 4));
+    W_TRY(cudaMemcpy(w->d_bias, hb.data(), static_cast<size_t>(w->OCP) * 4, cudaMemcpyHostToDevice));
+    info.workspace_bytes += img.size() + static_cast<size_t>(w->OCP) * 4;
+    return ELB_OK;
+  }
   const int BN = w->BN, KS = g.k_stages, AA = g.A * g.A;
   const size_t KTOT = static_cast<size_t>(g.taps) * w->ICP;      // K extent of one position
   std::vector<uint8_t> img(w->b_bytes, 0);
@@ -1858,7 +1881,7 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
             const int BNH = w->cta2 ? BN / 2 : BN, hf = r / BNH, rr = r % BNH;
             float *stage = dst + ((static_cast<size_t>(a) * w->n_tiles + nt) * KS + ks) * (32 * BN) + static_cast<size_t>(hf) * 32 * BNH;
             for (int c = 0; c < 16; ++c) {
-              const float hi = tf32_rna(src[c]);
+              const float hi = host::tf32_rna(src[c]);
               volatile float lo = src[c] - hi;
               const int j = c >> 2, e = c & 3;
               if (w->stack) {      // [chunk j][hi rows | lo rows][4 floats]
@@ -1946,6 +1969,22 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[0], s)); W_TRY(cudaEventRecord(pl.stage_ev[1], s)); }
     if (f32_rgb_umma_supported(sp) && tune_env("ELB_RGB_UMMA", 1) != 0) W_TRY(launch_f32_rgb_umma(sp, num_sms, status, s));
     else W_TRY(launch_f32_small_ic(sp, s));
+    if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[2], s)); W_TRY(cudaEventRecord(pl.stage_ev[3], s)); }
+    launches = 1;
+    return ELB_OK;
+  }
+  if (w->halo) {
+    HaloParams hp = w->halo->p;
+    hp.shift = w->with_bias ? static_cast<const float *>(w->d_bias) : nullptr;
+    hp.out = static_cast<float *>(out) + static_cast<size_t>(first) * (w->out_img_bytes / 4);
+    hp.status = status;
+    hp.rq.out_type = OUT_F32; hp.rq.relu = w->with_relu; hp.rq.with_sum = w->with_sum;
+    hp.rq.relu_lo = w->relu_lo; hp.rq.relu_hi = w->relu_hi;
+    const bool timed = pl.stage_ev[0] != nullptr;
+    if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[0], s)); W_TRY(cudaEventRecord(pl.stage_ev[1], s)); }
+    if (!halo_launch(*w->halo, hp, static_cast<const float *>(in) + static_cast<size_t>(first) * (w->in_img_bytes / 4), count,
+                     num_sms, s, err))
+      return ELB_GENERAL_ERROR;
     if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[2], s)); W_TRY(cudaEventRecord(pl.stage_ev[3], s)); }
     launches = 1;
     return ELB_OK;

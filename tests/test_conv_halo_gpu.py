@@ -1,0 +1,51 @@
+"""The halo-tiled kernel (conv_halo.cu) at the edges of its tiles, channel groups and weight-stage forms, against
+the C restatement: INT8 bit-exact (accumulators and outputs), fp32 to the direct path's tolerance."""
+import numpy as np
+import pytest
+
+import refutil as R
+
+pytestmark = pytest.mark.gpu
+
+
+def _c(name, n, ic, oc, ih, iw, types="u8f32u8f32", **kw):
+    kw.setdefault("relu", True)
+    kw.setdefault("bias", True)
+    kw.setdefault("algo", "direct")
+    if types != "fp32":
+        kw.setdefault("oscale", 0.3)
+    return R.ConvCase(name, n, ic, oc, ih, iw, types=types, **kw)
+
+
+SHAPES = [                                            # n, ic, oc, ih, iw, extra
+    (1, 16, 16, 16, 8, {}),                           # exactly one tile, one chunk per group
+    (2, 32, 24, 17, 9, {}),                           # one row and one column over a tile
+    (5, 96, 48, 7, 7, {}),                            # six blocks, tiles across several small images
+    (3, 64, 64, 14, 14, {}),                          # weights resident, four accumulators
+    (2, 144, 80, 15, 15, {}),                         # nine blocks: a padded group
+    (4, 128, 256, 14, 13, {}),                        # 256-wide tiles
+    (3, 256, 272, 9, 9, {}),                          # two groups, two channel tiles
+    (2, 64, 32, 21, 10, dict(stride=2)),              # four parity planes, odd extents
+    (1, 32, 48, 12, 12, dict(kh=5, kw=5, pad=2)),
+    (2, 16, 32, 20, 20, dict(kh=7, kw=7, pad=3, stride=2)),
+    (2, 48, 64, 9, 11, dict(kh=1, kw=1, pad=0, stride=2)),
+]
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s[:5])) + "".join(f"_{k}{v}" for k, v in s[5].items()))
+@pytest.mark.parametrize("types", ["u8f32u8f32", "fp32"])
+def test_halo_matches_oracle(pkg, shape, types):
+    import gpuutil as G
+    n, ic, oc, ih, iw, kw = shape
+    case = _c("halo", n, ic, oc, ih, iw, types=types, **kw)
+    t = R.make_tensors(case)
+    if types == "fp32":
+        got, d = G.run_gpu(case, t)
+        assert d.launch_count() == 1 and d.device_status() == 0
+        assert R.rel_l2(got, R.oracle_direct_f64(case, t)) <= 1e-5
+    else:
+        want, want_acc = R.oracle_int8_conv(case, t, want_acc=True)
+        got, d, acc = G.run_gpu(case, t, want_acc=True)
+        assert d.launch_count() == 1 and d.device_status() == 0
+        assert np.array_equal(acc, want_acc) and np.array_equal(got, want)
+    d.close()
