@@ -42,7 +42,7 @@ namespace elb {
 namespace {
 
 constexpr int BM = 128, TILE_H = 16, TILE_W = 8;
-constexpr int MAX_A = 4, MAX_B = 16, RAW_STAGES = 2, MAX_BUFS = 4;
+constexpr int MAX_A = 4, MAX_B = 16, RAW_STAGES = 4, MAX_BUFS = 4;
 // int8: an epilogue group of four warps per (accumulator, half of the column blocks); fp32: per half
 constexpr int EPI_WARP0 = 4, SPLIT_WARPS = 4;
 constexpr int EPI_WARPS_I8 = 16, EPI_WARPS_F32 = 8;
@@ -112,7 +112,11 @@ enum : int { FORM_ANY = 0, FORM_3X3_ROWS = 1, FORM_3X3_TAPS = 2, FORM_3X3_RESIDE
 // pixels of a shared-memory row of a 3x3 stride-1 filter (what halo_plan() computes)
 __host__ __device__ constexpr int pxw_3x3(int kind, int pairs) { return kind == HALO_F32 || pairs == 2 || pairs == 4 ? 10 : pairs == 0 ? 16 : 12; }
 
-template <int KIND, int PAIRS, int FORM, bool STACK>
+// PAIR: clusters of two CTAs.  One tcgen05.mma.cta_group::2 multiplies two row tiles (128 rows per CTA) by the BN
+// weight rows of which each CTA stages HALF: what an SM takes in per MMA from L2 and what the MMA reads from its
+// shared memory both fall by the weights' half, and these two (about 50 B/clk, 128 B/clk) bound the tiles of
+// 256 output channels on single CTAs.
+template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR>
 __global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
 conv_halo_kernel(const __grid_constant__ HaloParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -128,22 +132,25 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
   volatile int *abort_flag = &bar.abort_flag;
 
   const int warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;      // this CTA's (pair's) tiles
   if (warp == 1) {
     if (lane == 0) {
       for (int i = 0; i < MAX_A; ++i) {
-        mbar_init(&bar.afull[i], KIND == HALO_I8 ? 1 : SPLIT_WARPS);
+        mbar_init(&bar.afull[i], KIND == HALO_I8 ? 1 : SPLIT_WARPS * (PAIR ? 2 : 1));
         mbar_init(&bar.aempty[i], 1);
       }
       for (int i = 0; i < RAW_STAGES; ++i) { mbar_init(&bar.rfull[i], 1); mbar_init(&bar.rempty[i], SPLIT_WARPS); }
       for (int i = 0; i < MAX_B; ++i) { mbar_init(&bar.bfull[i], 1); mbar_init(&bar.bempty[i], 1); }
       for (int i = 0; i < 2; ++i) mbar_init(&bar.turn[i], 1);
-      for (int i = 0; i < MAX_BUFS; ++i) { mbar_init(&bar.tfull[i], 1); mbar_init(&bar.tempty[i], p.bufs == 4 ? 4 : 8); }
+      for (int i = 0; i < MAX_BUFS; ++i) { mbar_init(&bar.tfull[i], 1); mbar_init(&bar.tempty[i], (p.bufs == 4 ? 4 : 8) * (PAIR ? 2 : 1)); }
       *abort_flag = 0;
       fence_barrier_init();
       fence_proxy_async_smem();
     }
     __syncwarp();
-    tmem_alloc(&bar.tmem_slot, 512);
+    if (PAIR) tmem_alloc2(&bar.tmem_slot, 512);
+    else tmem_alloc(&bar.tmem_slot, 512);
   } else if (warp == 0) {
     if (lane < p.planes) { tma_prefetch_desc(&p.tmap[lane][HALO_HEIGHTS - 1]); tma_prefetch_desc(&p.tmap[lane][3]); }
   } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
@@ -155,6 +162,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
   }
   tc_fence_before_sync();
   __syncthreads();
+  if (PAIR) cluster_sync_all();          // the peer's barriers exist before anyone signals them
   tc_fence_after_sync();
   const uint32_t tmem_base = bar.tmem_slot;
   // (the kernel behind this one may set itself up now; see griddep_wait)
@@ -164,38 +172,36 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
   if (warp == 0) {
     // ---------------------------------------------------------------- activation rows
     griddep_wait();
+    constexpr bool PAIR_A = PAIR && KIND == HALO_I8;      // (fp32 rows are split first: they count on their own CTA's barrier)
     uint64_t *full = KIND == HALO_I8 ? bar.afull : bar.rfull, *empty = KIND == HALO_I8 ? bar.aempty : bar.rempty;
     const int stages = KIND == HALO_I8 ? p.a_stages : RAW_STAGES;
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
     const int groups = uni(p.groups), planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    const bool strided = uni(p.strided) != 0;
+    const bool strided = FORM == FORM_ANY && uni(p.strided) != 0;
     // stride 1: 8-byte elements, so that the copy engine moves whole rows
     const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
-      const int mt = p.div_n.div(tile);
+    for (int tile = first; tile < p.total_tiles && ok; tile += step) {
+      const int mt = PAIR ? 2 * p.div_n.div(tile) + rank : p.div_n.div(tile);
       const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
-      for (int g = 0; g < groups && ok; ++g)
-      for (int q = 0; q < planes; ++q) {
-        const int rows = p.rows[q], x = (ct * TILE_W + p.col0[q]) * x_unit, v0 = rt * TILE_H + p.row0[q];
+      // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
+      // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
+      // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
+      constexpr int Q = FORM == FORM_ANY ? 4 : 1;      // planes the code is written out for
+      int idx[Q], img[Q], row[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (Q > 1 && q >= planes) continue;
+        const int rows = p.rows[q], v0 = rt * TILE_H + p.row0[q];
         int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
         if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
-        uint8_t *dst = ring + s * stage_bytes;
-        if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
+        idx[q] = -1;
         if (h + rows <= period) {
-          // all rows belong to one image: one copy
-          if (elect_one()) {
-            mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(rows * pitch));
-            if (!strided) tma_tile_4d(dst, &p.tmap[0][HALO_HEIGHTS - 1], x, g * cb_step, h, n, &full[s]);
-            else tma_tile_5d(dst, &p.tmap[q][HALO_HEIGHTS - 1], 0, x, g * cb_step, h, n, &full[s]);
-          }
+          if (lane == 0) idx[q] = HALO_HEIGHTS - 1;
         } else {
-          // Lane r stands for row r.  Issuing a copy costs the warp about 100 cycles, so each image's share goes in
-          // pieces of 8, 4, 2 and 1 rows; the lane of a piece's first row issues it.
-          if (lane == 0) mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(rows * pitch));
           const int v = v0 + lane;
           n = v > 0 ? p.div_period.div(v) : 0;
           h = v - n * period;
@@ -205,21 +211,38 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
             const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
             const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
             const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
-            int idx = -1;
             if (at < (len & ~7)) {
-              if ((at & 7) == 0) idx = 3;
+              if ((at & 7) == 0) idx[q] = 3;
             } else {
               const int sub = at & 7, rest = len - at;
-              if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx = 31 - __clz(rest);
-            }
-            if (idx >= 0) {
-              if (!strided) tma_tile_4d(dst + lane * pitch, &p.tmap[0][idx], x, g * cb_step, h, n, &full[s]);
-              else tma_tile_5d(dst + lane * pitch, &p.tmap[q][idx], 0, x, g * cb_step, h, n, &full[s]);
+              if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx[q] = 31 - __clz(rest);
             }
           }
         }
-        __syncwarp();
-        if (++s == stages) { s = 0; ph ^= 1u; }
+        img[q] = n; row[q] = h;
+      }
+      for (int g = 0; g < groups && ok; ++g) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          if (Q > 1 && (q >= planes || !ok)) continue;
+          if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; continue; }
+          if (lane == 0 && (rank == 0 || !PAIR_A))
+            mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(p.rows[q] * pitch) * (PAIR_A ? 2u : 1u));
+          if (idx[q] >= 0) {
+            uint8_t *d = ring + s * stage_bytes + lane * pitch;
+            const int x = (ct * TILE_W + p.col0[q]) * x_unit, c = g * cb_step;
+            if (PAIR_A) {
+              const uint32_t pair_bar = mapa_u32(&full[s], 0);
+              if (!strided) tma_tile_4d_pair(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], pair_bar);
+              else tma_tile_5d_pair(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], pair_bar);
+            } else {
+              if (!strided) tma_tile_4d(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], &full[s]);
+              else tma_tile_5d(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], &full[s]);
+            }
+          }
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1u; }
+        }
       }
     }
   } else if (warp == 2) {
@@ -228,8 +251,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     int s = 0;
     uint32_t ph = 0;
     bool ok = true;
-    const size_t group_bytes = static_cast<size_t>(p.ksteps) * p.kstep_bytes;
-    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+    const size_t group_bytes = static_cast<size_t>(p.ksteps) * p.kstep_bytes * (PAIR ? 2 : 1);
+    for (int tile = first; tile < p.total_tiles && ok; tile += step) {
       const int nt = tile - p.div_n.div(tile) * p.n_tiles;
       const uint8_t *src = p.b_img + static_cast<size_t>(nt) * p.groups * group_bytes;
       for (int g = 0; g < p.groups && ok; ++g)
@@ -240,34 +263,45 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         for (int u = 0; u < units; ++u) {
           if (!wait_all(&bar.bempty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
           if (elect_one()) {
-            mbar_arrive_expect_tx(&bar.bfull[s], bytes);
-            tma_bulk_g2s(b_ring + s * p.b_stage_bytes, src, bytes, &bar.bfull[s]);
+            if (PAIR) {      // (a stage in memory: the leader's half, the peer's half)
+              if (rank == 0) mbar_arrive_expect_tx(&bar.bfull[s], 2 * bytes);
+              tma_tile_2d_pair(b_ring + s * p.b_stage_bytes, &p.tmap_b, 0, static_cast<int>((src - p.b_img + rank * bytes) >> 9),
+                               mapa_u32(&bar.bfull[s], 0));
+            } else {
+              mbar_arrive_expect_tx(&bar.bfull[s], bytes);
+              tma_bulk_g2s(b_ring + s * p.b_stage_bytes, src, bytes, &bar.bfull[s]);
+            }
           }
           __syncwarp();
-          src += bytes;
+          src += PAIR ? 2 * bytes : bytes;
           if (++s == p.b_stages) { s = 0; ph ^= 1u; }
         }
       }
       if (p.resident) break;
     }
   } else if (warp == 1 || warp == 3) {
-    // ---------------------------------------------------------------- MMA issuers
+    // ---------------------------------------------------------------- MMA issuers (pairs: the leader's)
+    if (rank == 0) {
     constexpr bool STRAIGHT = FORM != FORM_ANY;
-    constexpr int PXW = pxw_3x3(KIND, PAIRS), CHUNKS = PAIRS ? 2 * PAIRS : 1;
+    constexpr int M = PAIR ? 2 * BM : BM, PXW = pxw_3x3(KIND, PAIRS), CHUNKS = PAIRS ? 2 * PAIRS : 1;
     const int BN = uni(p.BN), total = uni(p.total_tiles), groups = uni(p.groups), planes = STRAIGHT ? 1 : uni(p.planes),
               b_stages = uni(p.b_stages), a_stages = uni(p.a_stages), bufs = uni(p.bufs);
     const bool row_units = uni(p.row_units) != 0, resident = FORM == FORM_ANY ? uni(p.resident) != 0 : FORM == FORM_3X3_RESIDENT;
-    const uint32_t idesc = KIND == HALO_I8 ? umma_idesc(2, 0, 1, BM, BN) : umma_idesc(1, 2, 2, BM, BN);
-    const uint32_t idesc2 = umma_idesc(1, 2, 2, BM, 2 * BN);
+    const uint32_t idesc = KIND == HALO_I8 ? umma_idesc(2, 0, 1, M, BN) : umma_idesc(1, 2, 2, M, BN);
+    const uint32_t idesc2 = umma_idesc(1, 2, 2, M, 2 * BN);
     const uint32_t a_base = smem_u32(smem) >> 4, b_base = smem_u32(b_ring) >> 4;
     // descriptors: low word = address | chunk distance << 16, high word = 8-row group distance | version
     const uint32_t pitch16 = STRAIGHT ? CHUNKS * PXW : uni(p.pitch) >> 4, pair16 = STRAIGHT ? 2 * PXW : 2u * uni(p.pxw);
     const uint32_t a_hi = pitch16 | (1u << 14), b_hi = (128u >> 4) | (1u << 14);
-    const uint32_t b_lbo = static_cast<uint32_t>(STACK ? 2 * BN : BN) << 16;
+    const uint32_t b_lbo = static_cast<uint32_t>(STACK ? 2 * BN : PAIR ? BN / 2 : BN) << 16;
     const uint32_t ks16 = uni(p.kstep_bytes) >> 4, lo16 = uni(p.a_bytes) >> 4, a16 = lo16 * PLANES, b16 = uni(p.b_stage_bytes) >> 4;
     const uint32_t a_lbo = static_cast<uint32_t>(PAIRS == 0 ? 1 : pair16 >> 1) << 16;      // (one pixel / one chunk further)
     auto desc = [](uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32); };
     const uint32_t el = elect_one() ? 1u : 0u;
+    auto commit = [](uint64_t *b, uint32_t e) {
+      if (PAIR) umma_commit_2cta_el(b, e);
+      else umma_commit_el(b, e);
+    };
     const int me = warp >> 1;      // this issuer takes tiles me, me + 2, ... of the CTA's
     // ring positions; the stages of the other issuer's tiles are skipped
     const int skip_a = groups * planes, skip_b = resident ? 0 : uni(p.b_per_tile);
@@ -285,7 +319,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     if (me) skip();
     bool ok = true, b_ready = false;
     int t = me;
-    for (int tile = blockIdx.x + me * gridDim.x; tile < total && ok; tile += 2 * gridDim.x, t += 2, skip()) {
+    for (int tile = first + me * step; tile < total && ok; tile += 2 * step, t += 2, skip()) {
       const uint32_t buf = t & (bufs - 1), tph = (bufs == 4 ? t >> 2 : t >> 1) & 1u, my_ph = (t >> 1) & 1u;
       const uint32_t d_tmem = tmem_base + buf * (bufs == 4 ? 128u : 256u);
       // An issuer looks at the rings only once the other has seen every stage of the tile before: a barrier tells
@@ -301,7 +335,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         uint32_t a_row = (a_base + as * a16) | a_lbo, b_lo = 0;
         auto mma = [&](uint32_t al, uint32_t bl, uint32_t accumulate) {
           if (KIND == HALO_I8) {
-            umma_i8_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
+            if (PAIR) umma_i8_2cta_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
+            else umma_i8_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
           } else if (STACK) {
             // hi * [hi; lo] in one MMA of 2 * BN columns, lo * hi in one of BN (the first BN rows are hi)
             umma_tf32_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc2, accumulate, el);
@@ -309,9 +344,13 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
           } else {
             // planes: the two hi chunks, then the two lo chunks
             const uint64_t bh = desc(bl, b_hi), blo = desc(bl + (ks16 >> 1), b_hi);
-            umma_tf32_el(d_tmem, desc(al + lo16, a_hi), bh, idesc, accumulate, el);
-            umma_tf32_el(d_tmem, desc(al, a_hi), blo, idesc, 1u, el);
-            umma_tf32_el(d_tmem, desc(al, a_hi), bh, idesc, 1u, el);
+            auto one = [&](uint64_t ad, uint64_t bd, uint32_t ac) {
+              if (PAIR) umma_tf32_2cta_el(d_tmem, ad, bd, idesc, ac, el);
+              else umma_tf32_el(d_tmem, ad, bd, idesc, ac, el);
+            };
+            one(desc(al + lo16, a_hi), bh, accumulate);
+            one(desc(al, a_hi), blo, 1u);
+            one(desc(al, a_hi), bh, 1u);
           }
         };
         // `n` taps from column c of the row at a_row (PAIRS = 0: n pairs of taps), unrolled
@@ -350,7 +389,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
             if (u + 1 < UNITS) seen = mbar_test_wait(&bar.bfull[bs], bph);
             if (FORM == FORM_3X3_ROWS) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
             else taps(std::integral_constant<int, 1>{}, u % 3);
-            umma_commit_el(done, el);
+            commit(done, el);
             if (FORM == FORM_3X3_ROWS || u % 3 == 2) a_row += pitch16;
           }
         } else {
@@ -361,7 +400,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
             b_lo = (b_base + bs * b16) | b_lbo;
           };
           auto end_unit = [&]() {
-            if (!resident) umma_commit_el(&bar.bempty[bs], el);
+            if (!resident) commit(&bar.bempty[bs], el);
             next_b();
           };
           if (row_units) {
@@ -395,13 +434,14 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
           }
         }
         if (!ok) { fail_code = ST_WAIT_TIMEOUT_MMA; break; }
-        umma_commit_el(&bar.aempty[as], el);
+        commit(&bar.aempty[as], el);
         if (++as == a_stages) { as = 0; aph ^= 1u; }
       }
       if (resident) bs = 0;
-      if (ok) umma_commit_el(&bar.tfull[buf], el);
+      if (ok) commit(&bar.tfull[buf], el);
       if (!resident && el) mbar_arrive(&bar.turn[me ^ 1u]);
       __syncwarp();
+    }
     }
   } else if (KIND == HALO_F32 && warp >= SPLIT_WARP0) {
     // ---------------------------------------------------------------- fp32 rows -> tf32 hi / lo planes
@@ -410,15 +450,18 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     int rs = 0, as = 0;
     uint32_t rph = 0, aph = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
+    for (int tile = first; tile < p.total_tiles && ok; tile += step) {
       for (int g = 0; g < p.groups && ok; ++g)
       for (int q = 0; q < p.planes; ++q) {
         const int items = p.rows[q] * p.pxw * 4;       // 16-byte pieces: [row][pixel][4 chunks]
-        if (!mbar_wait_warp(&bar.rfull[rs], rph, abort_flag) || !mbar_wait_warp(&bar.aempty[as], aph ^ 1u, abort_flag)) {
+        if (!wait_all(&bar.rfull[rs], rph, abort_flag) || !wait_all(&bar.aempty[as], aph ^ 1u, abort_flag)) {
           ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break;
         }
         const float4 *src = reinterpret_cast<const float4 *>(raw + rs * p.raw_bytes);
         uint8_t *hi = smem + as * a_stage;
+        // (four pieces per thread in flight: one at a time a round trip through shared memory and the
+        // conversions was about 110 cycles)
+#pragma unroll 4
         for (int i = tid; i < items; i += SPLIT_WARPS * 32) {
           const float4 v = src[i];
           const int px_all = i >> 2, c = i & 3;
@@ -438,7 +481,11 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         }
         fence_proxy_async_smem();      // these stores -> visible to the tensor core's reads
         __syncwarp();
-        if (lane == 0) { mbar_arrive(&bar.afull[as]); mbar_arrive(&bar.rempty[rs]); }
+        if (lane == 0) {
+          if (PAIR && rank) mbar_arrive_cluster(mapa_u32(&bar.afull[as], 0));
+          else mbar_arrive(&bar.afull[as]);
+          mbar_arrive(&bar.rempty[rs]);
+        }
         if (++rs == RAW_STAGES) { rs = 0; rph ^= 1u; }
         if (++as == p.a_stages) { as = 0; aph ^= 1u; }
       }
@@ -456,8 +503,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const int t_step = KIND == HALO_F32 ? 1 : p.bufs, t_shift = whole ? 2 : 1;
     int t = KIND == HALO_F32 ? 0 : whole ? group : group >> 1;
     bool ok = true;
-    for (int tile = blockIdx.x + t * gridDim.x; tile < p.total_tiles && ok; tile += t_step * gridDim.x, t += t_step) {
-      const int mt = p.div_n.div(tile), nt = tile - mt * p.n_tiles;
+    for (int tile = first + t * step; tile < p.total_tiles && ok; tile += t_step * step, t += t_step) {
+      const int mu = p.div_n.div(tile), nt = tile - mu * p.n_tiles, mt = PAIR ? 2 * mu + rank : mu;
       const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
       const int v = rt * TILE_H + (row >> 3);
       const int n = p.div_period.div(v), oh = v - n * p.period, ow = ct * TILE_W + (row & 7);
@@ -523,7 +570,10 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       auto release = [&]() {
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bar.tempty[buf]);
+        if (lane == 0) {
+          if (PAIR && rank) mbar_arrive_cluster(mapa_u32(&bar.tempty[buf], 0));
+          else mbar_arrive(&bar.tempty[buf]);
+        }
       };
       {
       // blocks half, half + blk_step, ... of this warp, two in flight: while one is converted and stored the next is
@@ -553,21 +603,30 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     }
   }
 
-  if (fail_code != 0) atomicCAS(p.status, 0, fail_code);
+  if (fail_code != 0) report_status(p.status, fail_code);
   tc_fence_before_sync();
   __syncthreads();
+  if (PAIR) cluster_sync_all();      // nobody leaves (or frees tensor memory) while the other CTA may still use it
   tc_fence_after_sync();
-  if (warp == 1) tmem_dealloc(tmem_base, 512);
+  if (warp == 1) {
+    if (PAIR) tmem_dealloc2(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
+  }
 }
 
 int alignup(int v, int a) { return (v + a - 1) / a * a; }
 
-// Cycles one K step keeps the tensor pipe busy: N / 2 for an MMA of 128 x N x 32 bytes, unless reading
-// its operands from shared memory (128 B/clk) takes longer, which it does below N = 128.
-double mma_cycles(int n) { return std::max(n / 2.0, 32.0 + n / 4.0); }
-double kstep_cycles(int kind, int BN) {
-  if (kind == HALO_I8) return mma_cycles(BN);
-  return BN <= 128 ? mma_cycles(2 * BN) + mma_cycles(BN) : 3 * mma_cycles(BN);
+// Modelled cycles of one K step: the tensor pipe (N / 2 per MMA of 128 or 256 x N x 32 bytes), the shared-memory
+// port at 128 B/clk (operand reads of the MMAs, incoming copies, fp32: the split), the SM's intake from L2 at
+// about 48 B/clk.  b: bytes of weights an SM takes in per K step (0: resident), a: of input.
+double kstep_cycles(int kind, int BN, bool pair, double b, double a) {
+  const double read_n = BN / (pair ? 8.0 : 4.0);
+  double tensor, port;
+  if (kind == HALO_I8) { tensor = BN / 2.0; port = 32 + read_n; }
+  else if (!pair && BN <= 128) { tensor = 1.5 * BN; port = 64 + 3 * read_n; }      // (stacked hi / lo rows)
+  else { tensor = 1.5 * BN; port = 3 * (32 + read_n); }
+  port += (b + a * (kind == HALO_F32 ? 4 : 1)) / 128;
+  return std::max(std::max(tensor, port), (b + a) / 48);
 }
 
 }  // namespace
@@ -664,28 +723,39 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   const double m_tiles = static_cast<double>(p.row_tiles) * p.col_tiles;
   if (m_tiles * p.OCB > 1e9 || OCP > HALO_MAX_OC) { err = "size"; return false; }
   const int planes_bytes = p.a_bytes * (kind == HALO_F32 ? 2 : 1);
+  const int pairs = kch / 2;
   double best = 0;
   p.BN = 0;
   for (int nt = (OCP + 255) / 256; nt <= p.OCB; ++nt) {
     const int BN = alignup((OCP + nt - 1) / nt, 16);
     if ((OCP + BN - 1) / BN != nt) continue;
     const double kb = BN * (kind == HALO_F32 ? 64.0 : 32.0), ab = static_cast<double>(p.a_bytes) * p.planes / p.ksteps;
-    const double writes = (kb + ab * (kind == HALO_F32 ? 4 : 1)) / 128, ingest = (kb + ab) / 50;
-    const double tile = std::max(kstep_cycles(kind, BN) + writes, ingest) * p.ksteps * p.groups + 1500;
-    const double t = std::ceil(m_tiles * nt / num_sms) * tile;
-    if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; }
+    const double all = kb * p.ksteps * p.groups;
+    const bool stays = nt == 1 && all + 2.0 * planes_bytes + 8192 + BN * 8 <= SMEM_LIMIT - RAW_STAGES * p.raw_bytes;
+    // (int8: the epilogue, about 9 outputs per clock)
+    const double epilogue = kind == HALO_I8 ? 400 + 128.0 * BN / 9 : 0;
+    for (int pair = 0; pair < 2; ++pair) {
+      // pairs take the weights tap by tap, in rows of 512 bytes per half
+      // (fp32 with a stride: each CTA waits for the slower of the two splits of a stage, 150 -> 180 us on 128 -> 256, 56x56)
+      if (pair && ((kind == HALO_F32 && stride > 1) || pairs < 2 || BN % 32 || stays || m_tiles < 2 || kb * pairs > 48 * 1024 || kb * pairs * 3 <= 24 * 1024)) continue;
+      const double b = stays ? 0.0 : pair ? kb / 2 : kb;
+      const double tile = std::max(kstep_cycles(kind, BN, pair != 0, b, ab) * p.ksteps * p.groups + 600, epilogue);
+      const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
+      const double t = waves * tile + 4000;
+      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; }
+    }
   }
-  p.stack = kind == HALO_F32 && p.BN <= 128;
+  p.stack = kind == HALO_F32 && p.BN <= 128 && !p.pair;
   p.bufs = kind == HALO_I8 && p.BN <= 128 ? 4 : 2;      // accumulators in the 512 columns of tensor memory
   p.div_n.set(p.n_tiles);
   p.div_col.set(p.col_tiles);
   // shared memory: operand rows first, the rest is the weight ring
-  p.kstep_bytes = p.BN * (kind == HALO_F32 ? 64 : 32);
+  p.kstep_bytes = p.BN * (kind == HALO_F32 ? 64 : 32) / (p.pair ? 2 : 1);      // (of one CTA)
   const int fixed = p.n_tiles * p.BN * (kind == HALO_F32 ? 4 : 8) + static_cast<int>(sizeof(Bars)) + 256;
   const int room = SMEM_LIMIT - fixed - RAW_STAGES * p.raw_bytes;
   int b_per_group = 0, most_c = 0;      // weight stages of a channel group; longest filter row
   for (int i = 0; i < p.planes; ++i) most_c = std::max(most_c, p.tap_cols[i]);
-  const int pairs = kch / 2, row_steps = kch == 1 ? (most_c + 1) / 2 : most_c * pairs;
+  const int row_steps = kch == 1 ? (most_c + 1) / 2 : most_c * pairs;
   // a stage costs its hand-over whatever it holds: whole filter rows while they are small
   auto set_units = [&](bool rows_of_taps) {
   p.row_units = rows_of_taps;
@@ -701,7 +771,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   };
   const long long b_all = static_cast<long long>(p.groups) * p.ksteps * p.kstep_bytes;
   p.resident = 0;
-  if (p.n_tiles == 1 && b_all <= room - 2ll * planes_bytes) {
+  if (p.n_tiles == 1 && !p.pair && b_all <= room - 2ll * planes_bytes) {
     // the whole filter fits: it is fetched once per CTA
     set_units(true);
     for (int a = MAX_A; a >= 2 && !p.resident; --a)
@@ -714,55 +784,58 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       }
   }
   if (!p.resident) {
-    set_units(kch == 1 || row_steps * p.kstep_bytes <= 24 * 1024);
+    set_units(!p.pair && (kch == 1 || row_steps * p.kstep_bytes <= 24 * 1024));
     bool ok = false;
     for (int a = planes_bytes <= 24 * 1024 ? 3 : 2; a >= 1 && !ok; --a) ok = fit_b(a) && p.b_stages >= 3;
     if (!ok) { err = "shared memory"; return false; }
   }
   hp.smem_bytes = static_cast<size_t>(p.a_stages) * planes_bytes + RAW_STAGES * static_cast<size_t>(p.raw_bytes) +
                   static_cast<size_t>(p.b_stages) * p.b_stage_bytes + fixed;
-  hp.b_bytes = static_cast<size_t>(p.n_tiles) * b_all;
+  hp.b_bytes = static_cast<size_t>(p.n_tiles) * b_all * (p.pair ? 2 : 1);
   return true;
 }
 
-std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP) {
+// [n tile][group][K step]: single CTAs: the BN rows of both chunks (fp32: hi and lo rows); pairs: the K steps of
+// one tap for the leader's BN / 2 rows, then for the peer's.
+template <typename PutChunk>
+static void pack_walk(const HaloPlan &hp, uint8_t *dst, PutChunk put) {
   const HaloParams &p = hp.p;
-  std::vector<uint8_t> img(hp.b_bytes, 0);
-  uint8_t *dst = img.data();
+  const int halves = p.pair ? 2 : 1, rows = p.BN / halves, unit = p.pair ? (hp.kind == HALO_F32 ? 2 : p.kch / 2) : 1;
   for (int nt = 0; nt < p.n_tiles; ++nt)
     for (int g = 0; g < p.groups; ++g)
-      for (int k = 0; k < p.ksteps * 2; ++k, dst += p.BN * 16) {
-        const HaloPlan::Chunk c = hp.order[k];
-        const int cb = g * p.kch + c.cb;
-        if (c.tap < 0 || cb >= hp.CB) continue;
-        for (int r = 0; r < p.BN && nt * p.BN + r < OCP; ++r)
-          std::memcpy(dst + r * 16, q + (static_cast<size_t>(nt * p.BN + r) * taps + c.tap) * ICP + cb * 16, 16);
-      }
+      for (int k0 = 0; k0 < p.ksteps; k0 += unit)
+        for (int h = 0; h < halves; ++h)
+          for (int k = k0; k < k0 + unit; ++k, dst += p.kstep_bytes)
+            for (int j = 0; j < 2; ++j) put(dst, j, hp.order[2 * k + j], g, nt * p.BN + h * rows, rows);
+}
+
+std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP) {
+  std::vector<uint8_t> img(hp.b_bytes, 0);
+  pack_walk(hp, img.data(), [&](uint8_t *dst, int j, HaloPlan::Chunk c, int g, int o0, int rows) {
+    const int cb = g * hp.p.kch + c.cb;
+    if (c.tap < 0 || cb >= hp.CB) return;
+    for (int r = 0; r < rows && o0 + r < OCP; ++r)
+      std::memcpy(dst + (j * rows + r) * 16, q + (static_cast<size_t>(o0 + r) * taps + c.tap) * ICP + cb * 16, 16);
+  });
   return img;
 }
 
 std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, int taps, int ICP) {
-  const HaloParams &p = hp.p;
   std::vector<uint8_t> img(hp.b_bytes, 0);
-  float *dst = reinterpret_cast<float *>(img.data());
-  const int BN = p.BN;
-  for (int nt = 0; nt < p.n_tiles; ++nt)
-    for (int g = 0; g < p.groups; ++g)
-      for (int k = 0; k < p.ksteps; ++k, dst += BN * 16)
-        for (int j = 0; j < 2; ++j) {
-          const HaloPlan::Chunk c = hp.order[2 * k + j];      // cb: which four channels of the block
-          float *hi = dst + static_cast<size_t>(j) * (p.stack ? 2 * BN : BN) * 4;
-          float *lo = p.stack ? hi + BN * 4 : hi + static_cast<size_t>(2) * BN * 4;
-          for (int r = 0; r < BN && nt * BN + r < OCP; ++r) {
-            const float *src = u + (static_cast<size_t>(nt * BN + r) * taps + c.tap) * ICP + g * 16 + c.cb * 4;
-            for (int e = 0; e < 4; ++e) {
-              const float h = host::tf32_rna(src[e]);
-              volatile float l = src[e] - h;
-              hi[r * 4 + e] = h;
-              lo[r * 4 + e] = l;
-            }
-          }
-        }
+  pack_walk(hp, img.data(), [&](uint8_t *dst, int j, HaloPlan::Chunk c, int g, int o0, int rows) {
+    // c.cb: which four channels of the block
+    float *hi = reinterpret_cast<float *>(dst) + static_cast<size_t>(j) * (hp.p.stack ? 2 * rows : rows) * 4;
+    float *lo = hi + static_cast<size_t>(hp.p.stack ? rows : 2 * rows) * 4;
+    for (int r = 0; r < rows && o0 + r < OCP; ++r) {
+      const float *src = u + (static_cast<size_t>(o0 + r) * taps + c.tap) * ICP + g * 16 + c.cb * 4;
+      for (int e = 0; e < 4; ++e) {
+        const float h = host::tf32_rna(src[e]);
+        volatile float l = src[e] - h;
+        hi[r * 4 + e] = h;
+        lo[r * 4 + e] = l;
+      }
+    }
+  });
   return img;
 }
 
@@ -808,29 +881,78 @@ bool encode_maps(const HaloPlan &hp, const void *in, int cnt, CUtensorMap (*out)
 namespace {
 
 typedef void (*HaloKernel)(HaloParams);
-template <int FORM>
+template <int FORM, bool PAIR = false>
 HaloKernel pick_kernel(const HaloPlan &hp) {
-  if (hp.kind == HALO_F32) return hp.p.stack ? conv_halo_kernel<HALO_F32, 2, FORM, true> : conv_halo_kernel<HALO_F32, 2, FORM, false>;
-  switch (hp.p.kch) {
-    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false>;
-    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false>;
-    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false>;
-    case 2: return conv_halo_kernel<HALO_I8, 1, FORM, false>;
-    default: return conv_halo_kernel<HALO_I8, 0, FORM, false>;
+  if (hp.kind == HALO_F32) {
+    if constexpr (!PAIR)
+      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false>;
+    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR>;
   }
+  switch (hp.p.kch) {
+    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR>;
+    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR>;
+    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR>;
+  }
+  if constexpr (!PAIR) {
+    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false>;
+    return conv_halo_kernel<HALO_I8, 0, FORM, false, false>;
+  }
+  return nullptr;
 }
 HaloKernel pick_kernel(const HaloPlan &hp) {
   const HaloParams &p = hp.p;
-  if (p.strided || p.tap_cols[0] != 3 || p.tap_rows[0] != 3 || p.pxw != pxw_3x3(hp.kind, p.kch / 2)) return pick_kernel<FORM_ANY>(hp);
+  const bool s3x3 = !p.strided && p.tap_cols[0] == 3 && p.tap_rows[0] == 3 && p.pxw == pxw_3x3(hp.kind, p.kch / 2);
+  if (p.pair) return s3x3 ? pick_kernel<FORM_3X3_TAPS, true>(hp) : pick_kernel<FORM_ANY, true>(hp);
+  if (!s3x3) return pick_kernel<FORM_ANY>(hp);
   if (p.resident && p.b_stages == 3 * p.groups) return pick_kernel<FORM_3X3_RESIDENT>(hp);
   if (p.resident) return pick_kernel<FORM_ANY>(hp);
   return p.row_units ? pick_kernel<FORM_3X3_ROWS>(hp) : pick_kernel<FORM_3X3_TAPS>(hp);
 }
 
+// Launch configuration: may overlap its set-up with the kernel before it (launch_overlapped), pairs as clusters of two.
+struct LaunchConfig {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  LaunchConfig(const HaloPlan &hp, int ctas, cudaStream_t s) {
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(hp.kind == HALO_F32 ? THREADS_F32 : THREADS_I8);
+    cfg.dynamicSmemBytes = hp.smem_bytes;
+    cfg.stream = s;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = hp.p.pair ? 2 : 1;
+  }
+  LaunchConfig(const LaunchConfig &) = delete;
+};
+
 }  // namespace
 
-cudaError_t halo_init(const HaloPlan &hp) {
-  return cudaFuncSetAttribute(pick_kernel(hp), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
+cudaError_t halo_init(HaloPlan &hp) {
+  cudaError_t e = cudaFuncSetAttribute(pick_kernel(hp), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
+  if (e == cudaSuccess && hp.p.pair) {
+    LaunchConfig lc(hp, 2, nullptr);
+    e = cudaOccupancyMaxActiveClusters(&hp.max_clusters, pick_kernel(hp), &lc.cfg);
+    if (e == cudaSuccess && hp.max_clusters < 1) e = cudaErrorInvalidConfiguration;
+  }
+  return e;
+}
+
+// The packed weights as rows of 512 bytes (pairs fetch them with tiled copies, whose bytes may count on the leader's barrier)
+bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err) {
+  hp.d_b = d_b;
+  if (!hp.p.pair) return true;
+  PFN_encodeTiled enc = get_encode_tiled();
+  if (!enc) { err = "cuTensorMapEncodeTiled is not available from the driver"; return false; }
+  cuuint64_t dims[2] = {64, hp.b_bytes / 512}, strides[1] = {512};
+  cuuint32_t box[2] = {64, static_cast<cuuint32_t>(hp.p.b_stage_bytes / 512)}, estr[2] = {1, 1};
+  const CUresult r = enc(&hp.p.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, d_b, dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { err = "cuTensorMapEncodeTiled failed (" + std::to_string(static_cast<int>(r)) + ")"; return false; }
+  return true;
 }
 
 bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err) {
@@ -854,10 +976,10 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
     for (int i = 0; i < p.OCB * 16; ++i) { p.cst[0][i] = hp.scale[i]; p.cst[1][i] = hp.shift[i]; }
   p.N = images;
   p.row_tiles = ((images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
-  p.total_tiles = p.row_tiles * p.col_tiles * p.n_tiles;
-  const dim3 grid(std::min(p.total_tiles, num_sms));
-  const cudaError_t e = launch_overlapped(pick_kernel(hp), grid, dim3(hp.kind == HALO_F32 ? THREADS_F32 : THREADS_I8),
-                                          hp.smem_bytes, s, p);
+  const int m_tiles = p.row_tiles * p.col_tiles;
+  p.total_tiles = (p.pair ? (m_tiles + 1) / 2 : m_tiles) * p.n_tiles;
+  LaunchConfig lc(hp, p.pair ? 2 * std::min(p.total_tiles, hp.max_clusters) : std::min(p.total_tiles, num_sms), s);
+  const cudaError_t e = cudaLaunchKernelEx(&lc.cfg, pick_kernel(hp), p);
   if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
   return true;
 }

@@ -32,6 +32,7 @@ struct FastDiv {
 struct HaloParams {
   // [row / column parity plane of the input (stride 1: one)][rows a copy brings: 1, 2, 4, 8, all of a tile's]
   alignas(64) CUtensorMap tmap[4][HALO_HEIGHTS];
+  CUtensorMap tmap_b;                // pairs of CTAs: the packed weights as rows of 512 bytes
   const uint8_t *b_img;              // packed weights [n tile][group][K step][...]
   const float *scale, *shift;        // int8: [OCP] requantisation constants; f32: shift = bias (null: none)
   const float *shift_tbl;            // int8, zero point with padding: shift vectors by (row class, column class)
@@ -56,6 +57,7 @@ struct HaloParams {
   int fast;                          // int8: u8 result, ReLU at 0, no residual, one shift vector (1: constants in cst)
   int row_units;                     // a weight stage holds a filter row's taps (1) or one tap (0) of a plane
   int kstep_bytes, b_stages, b_stage_bytes;
+  int pair;                          // clusters of two CTAs multiply two row tiles by weights of which each holds half
   int bufs;                          // accumulators in tensor memory: 4 of up to 128 columns or 2 of up to 256
   int resident;                      // every weight stage of the (single) n tile stays in shared memory
   int stack;                         // f32: hi and lo weight rows of a chunk stacked (BN <= 128)
@@ -74,6 +76,7 @@ struct HaloPlan {
   int kind = HALO_I8;
   HaloParams p{};
   size_t smem_bytes = 0, b_bytes = 0;
+  int max_clusters = 0;              // pairs the device holds at once
   int stride = 1, IH = 0, IW = 0, CB = 0;
   int parity[4] = {0, 0, 0, 0};      // of each plane: row parity * stride + column parity
   struct Chunk { int tap, cb; };     // tap -1: zero weights
@@ -89,7 +92,8 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
 // Weights in the order the kernel reads them: i8 from q[OCP][taps][ICP], f32 from u[OCP][taps][ICP].
 std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP);
 std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, int taps, int ICP);
-cudaError_t halo_init(const HaloPlan &hp);      // once per plan and device
+bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err);      // the packed weights on the device
+cudaError_t halo_init(HaloPlan &hp);      // once per plan and device
 // Run `images` images: in / p.out address the first; p: a copy of hp.p with the per-call pointers set.
 bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err);
 

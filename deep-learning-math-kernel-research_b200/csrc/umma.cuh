@@ -362,6 +362,59 @@ __device__ __forceinline__ void umma_commit_2cta(uint64_t *bar) {
                ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)) : "memory");
 }
 
+// The same for a whole converged warp of the leader (see umma_i8_el)
+__device__ __forceinline__ void umma_i8_2cta_el(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+                                                uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P, Q;\n\t"
+      "setp.ne.b32 P, %4, 0;\n\t"
+      "setp.ne.b32 Q, %5, 0;\n\t"
+      "@Q tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, P;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void umma_tf32_2cta_el(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                  uint32_t accumulate, uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P, Q;\n\t"
+      "setp.ne.b32 P, %4, 0;\n\t"
+      "setp.ne.b32 Q, %5, 0;\n\t"
+      "@Q tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, P;\n\t"
+      "}\n" ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(el)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_2cta_el(uint64_t *bar, uint32_t el) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred Q;\n\t"
+      "setp.ne.b32 Q, %2, 0;\n\t"
+      "@Q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+      "}\n" ::"r"(smem_u32(bar)), "h"(static_cast<uint16_t>(3)), "r"(el)
+      : "memory");
+}
+// Tiled copies into THIS CTA's shared memory whose bytes count on a barrier of either CTA of the pair
+// (`bar`: a shared::cluster address, see mapa_u32), so that the leader waits for both CTAs' operands on one barrier.
+__device__ __forceinline__ void tma_tile_2d_pair(void *smem_dst, const void *tmap, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_tile_4d_pair(void *smem_dst, const void *tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
+__device__ __forceinline__ void tma_tile_5d_pair(void *smem_dst, const void *tmap, int c0, int c1, int c2, int c3, int c4, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(smem_u32(smem_dst)), "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+      : "memory");
+}
+
 // Read 16 consecutive 32-bit columns of this thread's TMEM lane (warp-wide, converged).
 // taddr = base + (lane_quarter*32 << 16) + column.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {

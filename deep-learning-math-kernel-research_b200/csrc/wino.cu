@@ -1231,7 +1231,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
     else tile_loop(std::false_type{});
   }
 
-  if (fail_code != 0) atomicCAS(p.status, 0, fail_code);
+  if (fail_code != 0) report_status(p.status, fail_code);
   tc_fence_before_sync();
   __syncthreads();
   if (CTA2) cluster_sync_all();    // nobody leaves (or frees tensor memory) while the other CTA may still signal it
@@ -1857,8 +1857,10 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
   }
   if (w->halo) {
     const std::vector<uint8_t> img = halo_pack_f32(*w->halo, u.data(), w->OCP, g.taps, w->ICP);
-    W_TRY(cudaMalloc(&w->halo->d_b, img.size()));
-    W_TRY(cudaMemcpy(w->halo->d_b, img.data(), img.size(), cudaMemcpyHostToDevice));
+    void *d_b = nullptr;
+    W_TRY(cudaMalloc(&d_b, img.size()));
+    if (!halo_set_weights(*w->halo, d_b, err)) return ELB_GENERAL_ERROR;
+    W_TRY(cudaMemcpy(d_b, img.data(), img.size(), cudaMemcpyHostToDevice));
     W_TRY(cudaMalloc(&w->d_bias, static_cast<size_t>(w->OCP) * 4));
     W_TRY(cudaMemcpy(w->d_bias, hb.data(), static_cast<size_t>(w->OCP) * 4, cudaMemcpyHostToDevice));
     info.workspace_bytes += img.size() + static_cast<size_t>(w->OCP) * 4;

@@ -28,6 +28,8 @@ SHAPES = [                                            # n, ic, oc, ih, iw, extra
     (2, 64, 32, 21, 10, dict(stride=2)),              # four parity planes, odd extents
     (1, 32, 48, 12, 12, dict(kh=5, kw=5, pad=2)),
     (2, 16, 32, 20, 20, dict(kh=7, kw=7, pad=3, stride=2)),
+    (36, 128, 256, 14, 14, {}),                       # pairs of CTAs
+    (37, 64, 256, 28, 28, dict(stride=2)),            # pairs, parity planes; an odd number of row tiles
     (2, 48, 64, 9, 11, dict(kh=1, kw=1, pad=0, stride=2)),
 ]
 
