@@ -137,12 +137,12 @@ def last_error() -> str:
 
 def _ptr(x):
     """Address of a torch tensor / numpy array / int / None."""
-    if x is None:
-        return None
-    if isinstance(x, int):
+    try:
+        return x.data_ptr()                 # (first: what the calls of a running program pass)
+    except AttributeError:
+        pass
+    if x is None or isinstance(x, int):
         return x
-    if hasattr(x, "data_ptr"):
-        return x.data_ptr()
     if hasattr(x, "ctypes"):
         return x.ctypes.data
     raise TypeError(f"cannot take the address of {type(x)}")

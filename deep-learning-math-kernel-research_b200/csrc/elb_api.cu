@@ -150,8 +150,8 @@ struct elb_conv {
   void *d_wpack = nullptr, *d_wplain = nullptr, *d_scale = nullptr, *d_shift = nullptr;
   void *d_shift_tbl = nullptr, *d_tap_cls = nullptr;     // int8 direct, zero point with padding: per-class shifts
   void *d_tap_tbl = nullptr;                             // int8 direct, BOX mode: I8ConvParams::tap_tbl
-  int *d_status = nullptr;
-  int *h_status = nullptr;              // pinned: the status word travels back on the stream, behind the kernels
+  int *h_status = nullptr;              // the status word: pinned host memory ...
+  int *d_status = nullptr;              // ... as the device sees it
   std::string name = "ioi";             // eld_conv_t::name, printed in the euler-perf line
   bool pending = false;                 // an asynchronous execute has not been waited for yet
   bool pending_d2h = false;
@@ -183,7 +183,7 @@ struct elb_conv {
 
   ~elb_conv() {
     cudaSetDevice(device);
-    for (void *p : {d_wpack, d_wplain, d_scale, d_shift, d_shift_tbl, d_tap_cls, d_tap_tbl, (void *)d_status, d_in_stage, d_out_stage,
+    for (void *p : {d_wpack, d_wplain, d_scale, d_shift, d_shift_tbl, d_tap_cls, d_tap_tbl, d_in_stage, d_out_stage,
                     d_cvt_in, d_cvt_out})
       if (p) cudaFree(p);
     if (halo && halo->d_b) cudaFree(halo->d_b);
@@ -524,8 +524,11 @@ int prepare_i8_direct(elb_conv &pl, const void *weights, const void *bias) {
     pl.halo->scale = scale;
     pl.halo->shift = shift;
     const std::vector<uint8_t> pk = halo_pack_i8(*pl.halo, wq.q.data(), wq.OCP, wq.taps, wq.ICP);
-    CUDA_TRY(cudaMalloc(&pl.halo->d_b, pk.size()));
-    CUDA_TRY(cudaMemcpy(pl.halo->d_b, pk.data(), pk.size(), cudaMemcpyHostToDevice));
+    void *d_b = nullptr;
+    std::string err;
+    CUDA_TRY(cudaMalloc(&d_b, pk.size()));
+    if (!halo_set_weights(*pl.halo, d_b, err)) return fail(ELB_GENERAL_ERROR, "%s", err.c_str());
+    CUDA_TRY(cudaMemcpy(d_b, pk.data(), pk.size(), cudaMemcpyHostToDevice));
     pl.info.workspace_bytes += pk.size();
   } else {
     int n_tiles, CBG, k_stages;
@@ -598,17 +601,11 @@ int run_i8_direct(elb_conv &pl, void *out, const void *in, int n0, int cnt, cuda
   return ELB_OK;
 }
 
-// The status word of the kernels follows them on the stream into pinned host memory, so the call's
-// one synchronisation also brings back the verdict (no separate blocking copy).
-int fetch_status_async(elb_conv &pl, cudaStream_t s) {
-  CUDA_TRY(cudaMemcpyAsync(pl.h_status, pl.d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
-  return ELB_OK;
-}
+// What the kernels of the calls waited for left in the status word.
 int check_status(elb_conv &pl) {
-  const int st = *pl.h_status;
+  const int st = *reinterpret_cast<volatile int *>(pl.h_status);
   if (st != 0) {
     *pl.h_status = 0;
-    cudaMemset(pl.d_status, 0, sizeof(int));
     return fail(ELB_GENERAL_ERROR, "device kernel gave up waiting (status %d)", st);
   }
   return ELB_OK;
@@ -813,8 +810,6 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
     CUDA_TRY(cudaEventCreate(&t1));
   }
   auto finish = [&](bool used_d2h) -> int {
-    int r = fetch_status_async(pl, pl.stream);
-    if (r != ELB_OK) return r;
     if (!wait) {
       // the next call must not overwrite the staging buffers before this one has used them
       CUDA_TRY(cudaEventRecord(pl.ev_call_done, pl.stream));
@@ -1005,14 +1000,14 @@ int elb_conv_create(const elb_conv_desc_t *desc, elb_conv_t **plan) {
   if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) { delete pl; return fail(ELB_GENERAL_ERROR, "device query failed"); }
   pl->num_sms = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&pl->d_status, sizeof(int)) != cudaSuccess ||
-      cudaMemset(pl->d_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaHostAlloc(&pl->h_status, sizeof(int), cudaHostAllocDefault) != cudaSuccess ||
+      cudaHostAlloc(&pl->h_status, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess ||
+      cudaHostGetDevicePointer(reinterpret_cast<void **>(&pl->d_status), pl->h_status, 0) != cudaSuccess ||
       cudaEventCreateWithFlags(&pl->ev_call_done, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&pl->ev_d2h_done, cudaEventDisableTiming) != cudaSuccess) {
     delete pl;
     return fail(ELB_GENERAL_ERROR, "device allocation failed");
   }
+  *pl->h_status = 0;
   switch (info.kernel) {
     case ELB_KERNEL_I8_GEMM_UMMA:
     case ELB_KERNEL_I8_CONV_UMMA:
@@ -1144,9 +1139,18 @@ int elb_conv_device_status(elb_conv_t *plan) {
   if (!plan) return -1;
   DeviceGuard guard(plan->device);
   int st = -1;
-  if (cudaMemcpy(&st, plan->d_status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+  if (cudaMemcpy(&st, plan->d_status, sizeof(int), cudaMemcpyDefault) != cudaSuccess) return -1;      // (behind the default stream's work)
   return st;
 }
+
+}  // extern "C"
+
+namespace elb {
+// The status word once every kernel of the plan has been waited for (no copy; elb_multi.cu).
+int plan_status(elb_conv_t *plan) { return *reinterpret_cast<volatile int *>(plan->h_status); }
+}  // namespace elb
+
+extern "C" {
 
 uint64_t elb_conv_launch_count(const elb_conv_t *plan) { return plan ? plan->launches : 0; }
 

@@ -63,6 +63,14 @@ enum : int {
   ST_WAIT_TIMEOUT_TEST = 104        // the deliberate give-up of the wait self-test
 };
 
+// The status word of a plan lies in host memory that the device maps: a kernel that gives up a wait leaves its code
+// there, and a call that has waited for its kernels reads it without a copy of its own (the 4-byte copy behind
+// the kernels cost a single-image call 5 us).
+__device__ __forceinline__ void report_status(int *status, int code) {
+  *reinterpret_cast<volatile int *>(status) = code;
+  __threadfence_system();
+}
+
 enum : int { OUT_F32 = 0, OUT_U8 = 1, OUT_S8 = 2 };
 
 // ---------------------------------------------------------------------------------------------

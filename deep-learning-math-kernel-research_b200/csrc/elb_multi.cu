@@ -28,6 +28,7 @@
 
 namespace elb {
 void set_last_error(const char *msg);   // elb_api.cu
+int plan_status(elb_conv_t *plan);      // elb_api.cu
 }
 
 namespace {
@@ -143,7 +144,7 @@ int stack_enqueue(elb_stack &st, void *output, const void *input, cudaStream_t s
 
 int stack_status(elb_stack &st) {
   for (size_t k = 0; k < st.layers.size(); ++k) {
-    const int v = elb_conv_device_status(st.layers[k].plan);
+    const int v = elb::plan_status(st.layers[k].plan);
     if (v != 0) return mfail(ELB_GENERAL_ERROR, "layer %d: device kernel gave up waiting (status %d)", (int)k, v);
   }
   return ELB_OK;

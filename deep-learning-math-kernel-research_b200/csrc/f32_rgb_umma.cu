@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(RGB_THREADS, 1) f32_rgb_umma_kernel(const __gr
     }
   }
 
-  if (fail_code != 0) atomicCAS(status, 0, fail_code);
+  if (fail_code != 0) report_status(status, fail_code);
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();

@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) i8_umma_kernel(const __grid_co
   }
 
   // ------------------------------------------------------------------ teardown
-  if (fail_code != 0) atomicCAS(p.status, 0, fail_code);
+  if (fail_code != 0) report_status(p.status, fail_code);
   if (threadIdx.x == 0) ELB_TRACE(43);
   tc_fence_before_sync();
   __syncthreads();

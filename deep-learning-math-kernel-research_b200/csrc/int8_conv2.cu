@@ -267,7 +267,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1) i8_u
   }
 
   // ------------------------------------------------------------------ teardown
-  if (fail_code != 0) atomicCAS(p.status, 0, fail_code);
+  if (fail_code != 0) report_status(p.status, fail_code);
   if (threadIdx.x == 0) ELB_TRACE(43);
   tc_fence_before_sync();
   __syncthreads();
