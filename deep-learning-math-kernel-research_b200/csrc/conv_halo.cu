@@ -51,7 +51,7 @@ constexpr int THREADS_I8 = (EPI_WARP0 + EPI_WARPS_I8) * 32, THREADS_F32 = (SPLIT
 constexpr int SMEM_LIMIT = 232448 - 1024;      // dynamic shared memory the plan may fill
 
 struct Bars {
-  uint64_t afull[MAX_A], aempty[MAX_A], rfull[RAW_STAGES], rempty[RAW_STAGES], bfull[MAX_B], bempty[MAX_B], tfull[MAX_BUFS], tempty[MAX_BUFS], turn[2];
+  uint64_t afull[MAX_A], aempty[MAX_A], rfull[RAW_STAGES], rempty[RAW_STAGES], bfull[MAX_B], bempty[MAX_B], tfull[MAX_BUFS], tempty[MAX_BUFS], turn[2], parts;
   uint32_t tmem_slot;
   int abort_flag;
 };
@@ -116,7 +116,11 @@ __host__ __device__ constexpr int pxw_3x3(int kind, int pairs) { return kind == 
 // weight rows of which each CTA stages HALF: what an SM takes in per MMA from L2 and what the MMA reads from its
 // shared memory both fall by the weights' half, and these two (about 50 B/clk, 128 B/clk) bound the tiles of
 // 256 output channels on single CTAs.
-template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR>
+// SPLIT: one tile per cluster of p.split CTAs, each of which multiplies a share of the channel groups; the partial
+// sums meet in the CTAs' own shared memory (always added in the same order).  For problems of a few tiles: a
+// 3x3 layer of one 14x14 image is two pixel tiles, whose K loop alone would keep a few SMs busy for longer than the
+// whole call should take.
+template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT>
 __global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
 conv_halo_kernel(const __grid_constant__ HaloParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -133,41 +137,117 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
 
   const int warp = uni(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-  const int first = PAIR ? blockIdx.x >> 1 : blockIdx.x, step = PAIR ? gridDim.x >> 1 : gridDim.x;      // this CTA's (pair's) tiles
+  // this CTA's (pair's, cluster's) tiles
+  const int share = SPLIT ? p.split : 1, first = PAIR ? blockIdx.x >> 1 : SPLIT ? blockIdx.x / share : blockIdx.x,
+            step = PAIR ? gridDim.x >> 1 : SPLIT ? gridDim.x / share : gridDim.x;
+  const int srank = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int g0 = SPLIT ? p.groups * srank / share : 0, g1 = SPLIT ? p.groups * (srank + 1) / share : p.groups;
+  // Set-up in two groups: the copying warps need the barriers only, and are on their way while the others allocate
+  // tensor memory and load constants (pairs: everybody waits for the peer's barriers).
+  const bool copies = warp == 0 || warp == 2;
   if (warp == 1) {
-    if (lane == 0) {
-      for (int i = 0; i < MAX_A; ++i) {
-        mbar_init(&bar.afull[i], KIND == HALO_I8 ? 1 : SPLIT_WARPS * (PAIR ? 2 : 1));
-        mbar_init(&bar.aempty[i], 1);
-      }
-      for (int i = 0; i < RAW_STAGES; ++i) { mbar_init(&bar.rfull[i], 1); mbar_init(&bar.rempty[i], SPLIT_WARPS); }
-      for (int i = 0; i < MAX_B; ++i) { mbar_init(&bar.bfull[i], 1); mbar_init(&bar.bempty[i], 1); }
-      for (int i = 0; i < 2; ++i) mbar_init(&bar.turn[i], 1);
-      for (int i = 0; i < MAX_BUFS; ++i) { mbar_init(&bar.tfull[i], 1); mbar_init(&bar.tempty[i], (p.bufs == 4 ? 4 : 8) * (PAIR ? 2 : 1)); }
-      *abort_flag = 0;
-      fence_barrier_init();
-      fence_proxy_async_smem();
+    for (int i = lane; i < MAX_B; i += 32) { mbar_init(&bar.bfull[i], 1); mbar_init(&bar.bempty[i], 1); }
+    if (lane < MAX_A) {
+      mbar_init(&bar.afull[lane], KIND == HALO_I8 ? 1 : SPLIT_WARPS * (PAIR ? 2 : 1));
+      mbar_init(&bar.aempty[lane], 1);
     }
+    if (lane < RAW_STAGES) { mbar_init(&bar.rfull[lane], 1); mbar_init(&bar.rempty[lane], SPLIT_WARPS); }
+    if (lane < 2) mbar_init(&bar.turn[lane], 1);
+    if (lane < MAX_BUFS) { mbar_init(&bar.tfull[lane], 1); mbar_init(&bar.tempty[lane], (p.bufs == 4 ? 4 : 8) * (PAIR ? 2 : 1)); }
+    if (lane == 31) { mbar_init(&bar.parts, 1); *abort_flag = 0; }
+    fence_barrier_init();
+    fence_proxy_async_smem();
     __syncwarp();
-    if (PAIR) tmem_alloc2(&bar.tmem_slot, 512);
-    else tmem_alloc(&bar.tmem_slot, 512);
   } else if (warp == 0) {
     if (lane < p.planes) { tma_prefetch_desc(&p.tmap[lane][HALO_HEIGHTS - 1]); tma_prefetch_desc(&p.tmap[lane][3]); }
-  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
+  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS && p.fast != 1) {
     const int OCP = p.OCB * 16;
     for (int i = threadIdx.x - EPI_WARP0 * 32; i < n_const; i += EPI_WARPS * 32) {
       if (KIND == HALO_I8) s_scale[i] = i < OCP ? p.scale[i] : 0.0f;
       s_shift[i] = (i < OCP && p.shift) ? p.shift[i] : 0.0f;
     }
   }
-  tc_fence_before_sync();
-  __syncthreads();
-  if (PAIR) cluster_sync_all();          // the peer's barriers exist before anyone signals them
-  tc_fence_after_sync();
-  const uint32_t tmem_base = bar.tmem_slot;
+  if (copies || warp == 1) named_bar_sync(1, 96);
+  if (PAIR || !copies) {
+    if (warp == 1) {
+      if (PAIR) tmem_alloc2(&bar.tmem_slot, 512);
+      else tmem_alloc(&bar.tmem_slot, 512);
+    }
+    tc_fence_before_sync();
+    if (PAIR) {
+      __syncthreads();
+      cluster_sync_all();          // the peer's barriers exist before anyone signals them
+    } else {
+      named_bar_sync(2, blockDim.x - 64);
+    }
+    tc_fence_after_sync();
+  }
+  const uint32_t tmem_base = copies ? 0u : bar.tmem_slot;
   // (the kernel behind this one may set itself up now; see griddep_wait)
   if (threadIdx.x == 0) griddep_launch_dependents();
   int fail_code = 0;
+
+  // ---- what the epilogue does with 16 output channels of a pixel
+  struct Pixel { bool valid; size_t pix; const float *shift_row; };
+  auto locate = [&](int mt, int row) {
+    const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
+    const int v = rt * TILE_H + (row >> 3);
+    const int n = p.div_period.div(v), oh = v - n * p.period, ow = ct * TILE_W + (row & 7);
+    Pixel x;
+    x.valid = n < p.N && oh < p.OH && ow < p.OW;
+    x.pix = (static_cast<size_t>(n) * p.OCB * p.OH + oh) * p.OW + ow;
+    x.shift_row = s_shift;
+    if (KIND == HALO_I8 && p.shift_tbl && x.valid) {
+      const int cls = __ldg(p.hclass + oh) * p.zp_nw + __ldg(p.wclass + ow);
+      if (cls != p.zp_full) x.shift_row = p.shift_tbl + static_cast<size_t>(cls) * (p.OCB * 16);
+    }
+    return x;
+  };
+  auto emit = [&](const Pixel &px, int ocb, uint32_t (&r)[16]) {
+    if (!px.valid || ocb >= p.OCB) return;
+    const size_t off = (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16;
+    if (KIND == HALO_I8) {
+      int a[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) a[i] = static_cast<int>(r[i]);
+      if (p.acc_dump) {
+        int4 *d = reinterpret_cast<int4 *>(p.acc_dump + off);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = make_int4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
+      }
+      if (p.fast == 2) requant_relu_u8(a, s_scale + ocb * 16, s_shift + ocb * 16, static_cast<uint8_t *>(p.out) + off);
+      else if (p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
+      else requant_store16(a, s_scale + ocb * 16, px.shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * (p.rq.out_type == OUT_F32 ? 4 : 1), p.rq);
+    } else {
+      float f[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(r[i]);
+      float *o = static_cast<float *>(p.out) + off;
+      if (p.shift) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 b = reinterpret_cast<const float4 *>(s_shift + ocb * 16)[i];
+          f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
+          f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
+        }
+      }
+      if (p.rq.with_sum) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 b = reinterpret_cast<const float4 *>(o)[i];
+          f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
+          f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
+        }
+      }
+      if (p.rq.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = fminf(fmaxf(f[i], p.rq.relu_lo), p.rq.relu_hi);
+      }
+      store_v8(o, f, 0);
+      store_v8(o, f, 8);
+    }
+  };
+  const int part_pitch = p.BN / 4 + 1;      // SPLIT: 16-byte words per row of partial sums (odd: no bank conflicts)
 
   if (warp == 0) {
     // ---------------------------------------------------------------- activation rows
@@ -177,8 +257,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const int stages = KIND == HALO_I8 ? p.a_stages : RAW_STAGES;
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
-    const int groups = uni(p.groups), planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    const bool strided = FORM == FORM_ANY && uni(p.strided) != 0;
+    const int planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
+    const bool strided = (FORM == FORM_ANY || KIND == HALO_F32) && uni(p.strided) != 0;
     // stride 1: 8-byte elements, so that the copy engine moves whole rows
     const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
     int s = 0;
@@ -221,7 +301,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         }
         img[q] = n; row[q] = h;
       }
-      for (int g = 0; g < groups && ok; ++g) {
+      for (int g = g0; g < g1 && ok; ++g) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
           if (Q > 1 && (q >= planes || !ok)) continue;
@@ -254,8 +334,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const size_t group_bytes = static_cast<size_t>(p.ksteps) * p.kstep_bytes * (PAIR ? 2 : 1);
     for (int tile = first; tile < p.total_tiles && ok; tile += step) {
       const int nt = tile - p.div_n.div(tile) * p.n_tiles;
-      const uint8_t *src = p.b_img + static_cast<size_t>(nt) * p.groups * group_bytes;
-      for (int g = 0; g < p.groups && ok; ++g)
+      const uint8_t *src = p.b_img + (static_cast<size_t>(nt) * p.groups + g0) * group_bytes;
+      for (int g = g0; g < g1 && ok; ++g)
       for (int q = 0; q < p.planes && ok; ++q) {
         const int cols = p.tap_cols[q], row_steps = PAIRS == 0 ? (cols + 1) >> 1 : cols * PAIRS;
         const int units = p.row_units ? p.tap_rows[q] : p.tap_rows[q] * cols;
@@ -289,7 +369,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const bool row_units = uni(p.row_units) != 0, resident = FORM == FORM_ANY ? uni(p.resident) != 0 : FORM == FORM_3X3_RESIDENT;
     const uint32_t idesc = KIND == HALO_I8 ? umma_idesc(2, 0, 1, M, BN) : umma_idesc(1, 2, 2, M, BN);
     const uint32_t idesc2 = umma_idesc(1, 2, 2, M, 2 * BN);
-    const uint32_t a_base = smem_u32(smem) >> 4, b_base = smem_u32(b_ring) >> 4;
+    // (in a cluster an address carries the CTA's rank in its upper bits; a descriptor takes the offset alone)
+    const uint32_t a_base = (smem_u32(smem) >> 4) & 0x3FFFu, b_base = (smem_u32(b_ring) >> 4) & 0x3FFFu;
     // descriptors: low word = address | chunk distance << 16, high word = 8-row group distance | version
     const uint32_t pitch16 = STRAIGHT ? CHUNKS * PXW : uni(p.pitch) >> 4, pair16 = STRAIGHT ? 2 * PXW : 2u * uni(p.pxw);
     const uint32_t a_hi = pitch16 | (1u << 14), b_hi = (128u >> 4) | (1u << 14);
@@ -327,7 +408,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       if ((t > 0 && !wait_all(&bar.turn[me], my_ph ^ (me ^ 1u), abort_flag)) ||
           !wait_all(&bar.tempty[buf], tph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
       uint32_t acc = 0;
-      for (int g = 0; g < groups && ok; ++g)
+      for (int g = g0; g < (SPLIT ? g1 : groups) && ok; ++g)
       for (int q = 0; q < planes && ok; ++q) {
         if (!wait_all(&bar.afull[as], aph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
         if (resident && g == groups - 1 && q == planes - 1 && el) mbar_arrive(&bar.turn[me ^ 1u]);
@@ -451,7 +532,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     uint32_t rph = 0, aph = 0;
     bool ok = true;
     for (int tile = first; tile < p.total_tiles && ok; tile += step) {
-      for (int g = 0; g < p.groups && ok; ++g)
+      for (int g = g0; g < g1 && ok; ++g)
       for (int q = 0; q < p.planes; ++q) {
         const int items = p.rows[q] * p.pxw * 4;       // 16-byte pieces: [row][pixel][4 chunks]
         if (!wait_all(&bar.rfull[rs], rph, abort_flag) || !wait_all(&bar.aempty[as], aph ^ 1u, abort_flag)) {
@@ -497,74 +578,28 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const bool whole = p.bufs == 4;
     const int half = whole ? 0 : group & 1, blk_step = whole ? 1 : 2;
     const int row = quarter * 32 + lane;
-    const int elt = KIND == HALO_F32 || p.rq.out_type == OUT_F32 ? 4 : 1;
-    const size_t blk_stride = static_cast<size_t>(p.OH) * p.OW;
     const int nb16 = p.BN >> 4, cnt = whole ? nb16 : (nb16 - half + 1) >> 1;
     const int t_step = KIND == HALO_F32 ? 1 : p.bufs, t_shift = whole ? 2 : 1;
     int t = KIND == HALO_F32 ? 0 : whole ? group : group >> 1;
     bool ok = true;
     for (int tile = first + t * step; tile < p.total_tiles && ok; tile += t_step * step, t += t_step) {
       const int mu = p.div_n.div(tile), nt = tile - mu * p.n_tiles, mt = PAIR ? 2 * mu + rank : mu;
-      const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
-      const int v = rt * TILE_H + (row >> 3);
-      const int n = p.div_period.div(v), oh = v - n * p.period, ow = ct * TILE_W + (row & 7);
-      const bool valid = n < p.N && oh < p.OH && ow < p.OW;
-      const size_t pix = (static_cast<size_t>(n) * p.OCB * p.OH + oh) * p.OW + ow;
-      const float *shift_row = s_shift;
-      if (KIND == HALO_I8 && p.shift_tbl && valid) {
-        const int cls = __ldg(p.hclass + oh) * p.zp_nw + __ldg(p.wclass + ow);
-        if (cls != p.zp_full) shift_row = p.shift_tbl + static_cast<size_t>(cls) * (p.OCB * 16);
-      }
+      const Pixel px = SPLIT ? Pixel{} : locate(mt, row);
       const uint32_t buf = t & (p.bufs - 1), tph = (t >> t_shift) & 1u;
       if (!wait_all(&bar.tfull[buf], tph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
       tc_fence_after_sync();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (whole ? 128u : 256u) + half * 16;
-      auto emit = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16]) {
-        const int ocb = nt * nb16 + blk;
-        if (!valid || ocb >= p.OCB) return;
-        const size_t off = (pix + ocb * blk_stride) * 16;
-        if (KIND == HALO_I8) {
-          int a[16];
+      auto take = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16]) {
+        if (STACK) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) a[i] = static_cast<int>(r[i]);
-          if (p.acc_dump) {
-            int4 *d = reinterpret_cast<int4 *>(p.acc_dump + off);
+          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(r[i]), __uint_as_float(r2[i])));
+        }
+        if (SPLIT) {      // (every copy into the rings has landed and every MMA has read them: the space is free)
+          uint4 *d = reinterpret_cast<uint4 *>(smem) + row * part_pitch + blk * 4;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) d[i] = make_int4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
-          }
-          if (p.fast == 2) requant_relu_u8(a, s_scale + ocb * 16, s_shift + ocb * 16, static_cast<uint8_t *>(p.out) + off);
-          else if (p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
-          else requant_store16(a, s_scale + ocb * 16, shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * elt, p.rq);
+          for (int i = 0; i < 4; ++i) d[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
         } else {
-          float f[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            f[i] = __uint_as_float(r[i]);
-            if (STACK) f[i] = __fadd_rn(f[i], __uint_as_float(r2[i]));
-          }
-          float *o = static_cast<float *>(p.out) + off;
-          if (p.shift) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 b = reinterpret_cast<const float4 *>(s_shift + ocb * 16)[i];
-              f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
-              f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
-            }
-          }
-          if (p.rq.with_sum) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const float4 b = reinterpret_cast<const float4 *>(o)[i];
-              f[4 * i] = __fadd_rn(f[4 * i], b.x); f[4 * i + 1] = __fadd_rn(f[4 * i + 1], b.y);
-              f[4 * i + 2] = __fadd_rn(f[4 * i + 2], b.z); f[4 * i + 3] = __fadd_rn(f[4 * i + 3], b.w);
-            }
-          }
-          if (p.rq.relu) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) f[i] = fminf(fmaxf(f[i], p.rq.relu_lo), p.rq.relu_hi);
-          }
-          store_v8(o, f, 0);
-          store_v8(o, f, 8);
+          emit(px, nt * nb16 + blk, r);
         }
       };
       auto release = [&]() {
@@ -590,12 +625,12 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
           tmem_ld_wait16(r0);
           if (pair) tmem_ld_wait16(q0);
           if (k + 1 < cnt) load(k + 1, r1, q1);
-          emit(half + blk_step * k, r0, q0);
+          take(half + blk_step * k, r0, q0);
           if (k + 1 < cnt) {
             tmem_ld_wait16(r1);
             if (pair) tmem_ld_wait16(q1);
             if (k + 2 < cnt) load(k + 2, r0, q0);
-            emit(half + blk_step * (k + 1), r1, q1);
+            take(half + blk_step * (k + 1), r1, q1);
           }
         }
         release();
@@ -604,9 +639,50 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
   }
 
   if (fail_code != 0) report_status(p.status, fail_code);
+  if (SPLIT) {
+    // Every CTA finishes a share of the tile's rows.  The rows' partial sums travel as one bulk copy from each CTA
+    // into a second area behind the first (loads of remote shared memory took 12 us here: 16 bytes of another row per
+    // lane), once every CTA is done with its rings; they are added in rank order.
+    const int nb16 = p.BN >> 4, rows = BM / share;
+    const uint32_t part_bytes = static_cast<uint32_t>(rows * part_pitch) * 16;
+    uint8_t *inbox = smem + BM * part_pitch * 16;
+    fence_proxy_async_smem();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 0) {
+      if (lane == 0) mbar_arrive_expect_tx(&bar.parts, part_bytes * share);
+      __syncwarp();
+      if (lane < share)
+        bulk_s2cluster(mapa_u32(inbox + srank * part_bytes, lane), smem + lane * part_bytes, part_bytes, mapa_u32(&bar.parts, lane));
+    }
+    if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
+      const int mt = p.div_n.div(first), nt = first - mt * p.n_tiles;
+      if (wait_all(&bar.parts, 0u, abort_flag)) {
+        for (int i = threadIdx.x - EPI_WARP0 * 32; i < rows * nb16; i += EPI_WARPS * 32) {
+          const int row = i & (rows - 1), blk = i / rows;
+          const uint4 *src = reinterpret_cast<const uint4 *>(inbox) + row * part_pitch + blk * 4;
+          uint32_t sum[16];
+          for (int c = 0; c < share; ++c, src += rows * part_pitch) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 v = src[j];
+              const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                sum[4 * j + k] = c == 0 ? x[k] : KIND == HALO_I8 ? sum[4 * j + k] + x[k]
+                                               : __float_as_uint(__fadd_rn(__uint_as_float(sum[4 * j + k]), __uint_as_float(x[k])));
+            }
+          }
+          emit(locate(mt, srank * rows + row), nt * nb16 + blk, sum);
+        }
+      } else {
+        report_status(p.status, ST_WAIT_TIMEOUT_EPILOGUE);
+      }
+    }
+  }
   tc_fence_before_sync();
   __syncthreads();
-  if (PAIR) cluster_sync_all();      // nobody leaves (or frees tensor memory) while the other CTA may still use it
+  if (PAIR || SPLIT) cluster_sync_all();      // nobody leaves (or frees tensor memory) while the other CTA may still use it
   tc_fence_after_sync();
   if (warp == 1) {
     if (PAIR) tmem_dealloc2(tmem_base, 512);
@@ -742,9 +818,18 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       const double tile = std::max(kstep_cycles(kind, BN, pair != 0, b, ab) * p.ksteps * p.groups + 600, epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
-      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; }
+      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; }
+    }
+    // few tiles: several CTAs share the K loop of each.  Partial sums cross shared memories at about 9 B/clk.  An SM
+    // holds one CTA, and the device no more clusters than its GPCs have room for (15 of 8, 33 of 4).
+    for (int split = 2; split <= 8 && split <= p.groups && m_tiles * nt * split <= num_sms * (split == 8 ? 0.8 : 0.88); split *= 2) {
+      const double parts = 128.0 * (BN + 4) * 4;
+      if (kch == 1 || 2 * parts > 150 * 1024) continue;
+      const double t = kstep_cycles(kind, BN, false, kb, ab) * p.ksteps * ((p.groups + split - 1) / split) + 600 + 4000 + 2000 + parts / 9;
+      if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; }
     }
   }
+  hp.est_us = best / 1750;
   p.stack = kind == HALO_F32 && p.BN <= 128 && !p.pair;
   p.bufs = kind == HALO_I8 && p.BN <= 128 ? 4 : 2;      // accumulators in the 512 columns of tensor memory
   p.div_n.set(p.n_tiles);
@@ -771,7 +856,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   };
   const long long b_all = static_cast<long long>(p.groups) * p.ksteps * p.kstep_bytes;
   p.resident = 0;
-  if (p.n_tiles == 1 && !p.pair && b_all <= room - 2ll * planes_bytes) {
+  if (p.n_tiles == 1 && !p.pair && p.split == 1 && b_all <= room - 2ll * planes_bytes) {
     // the whole filter fits: it is fetched once per CTA
     set_units(true);
     for (int a = MAX_A; a >= 2 && !p.resident; --a)
@@ -788,6 +873,10 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
     bool ok = false;
     for (int a = planes_bytes <= 24 * 1024 ? 3 : 2; a >= 1 && !ok; --a) ok = fit_b(a) && p.b_stages >= 3;
     if (!ok) { err = "shared memory"; return false; }
+  }
+  if (p.split > 1 && 2 * 128 * (p.BN + 4) * 4 > p.a_stages * planes_bytes + RAW_STAGES * p.raw_bytes + p.b_stages * p.b_stage_bytes) {
+    err = "shared memory";      // (the partial sums take the rings' place)
+    return false;
   }
   hp.smem_bytes = static_cast<size_t>(p.a_stages) * planes_bytes + RAW_STAGES * static_cast<size_t>(p.raw_bytes) +
                   static_cast<size_t>(p.b_stages) * p.b_stage_bytes + fixed;
@@ -842,7 +931,8 @@ std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, 
 namespace {
 
 // Tensor maps of `cnt` images at `in`.
-bool encode_maps(const HaloPlan &hp, const void *in, int cnt, CUtensorMap (*out)[HALO_HEIGHTS], std::string &err) {
+bool encode_maps(const HaloPlan &hp, const void *in, int cnt, int step, int src_h, int src_w, CUtensorMap (*out)[HALO_HEIGHTS],
+                 std::string &err) {
   PFN_encodeTiled enc = get_encode_tiled();
   if (!enc) { err = "cuTensorMapEncodeTiled is not available from the driver"; return false; }
   const HaloParams &p = hp.p;
@@ -853,7 +943,16 @@ bool encode_maps(const HaloPlan &hp, const void *in, int cnt, CUtensorMap (*out)
   for (int q = 0; q < p.planes; ++q)
     for (int i = 0; i < HALO_HEIGHTS && r == CUDA_SUCCESS; ++i) {
       const cuuint32_t height = i == HALO_HEIGHTS - 1 ? p.rows[q] : 1u << i;
-      if (!p.strided) {
+      if (step > 1) {
+        // one plane of every step-th pixel of a larger one (pixel by pixel, like the parity planes)
+        const cuuint64_t SH = src_h, SW = src_w, st = step;
+        cuuint64_t dims[5] = {16, IW, CB, IH, static_cast<cuuint64_t>(cnt)};
+        cuuint64_t strides[4] = {st * px, SH * SW * px, st * SW * px, CB * SH * SW * px};
+        cuuint32_t box[5] = {16, static_cast<cuuint32_t>(p.pxw), blocks, height, 1};
+        r = enc(&out[q][i], hp.kind == HALO_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 5,
+                const_cast<void *>(in), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+      } else if (!p.strided) {
         cuuint64_t dims[4] = {IW * px / 8, CB, IH, static_cast<cuuint64_t>(cnt)};
         cuuint64_t strides[3] = {IH * IW * px, IW * px, CB * IH * IW * px};
         cuuint32_t box[4] = {static_cast<cuuint32_t>(p.pxw * px / 8), blocks, height, 1};
@@ -881,27 +980,29 @@ bool encode_maps(const HaloPlan &hp, const void *in, int cnt, CUtensorMap (*out)
 namespace {
 
 typedef void (*HaloKernel)(HaloParams);
-template <int FORM, bool PAIR = false>
+template <int FORM, bool PAIR = false, bool SPLIT = false>
 HaloKernel pick_kernel(const HaloPlan &hp) {
   if (hp.kind == HALO_F32) {
     if constexpr (!PAIR)
-      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false>;
-    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR>;
+      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false, SPLIT>;
+    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR, SPLIT>;
   }
   switch (hp.p.kch) {
-    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR>;
-    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR>;
-    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR>;
+    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR, SPLIT>;
+    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR, SPLIT>;
+    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR, SPLIT>;
   }
   if constexpr (!PAIR) {
-    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false>;
-    return conv_halo_kernel<HALO_I8, 0, FORM, false, false>;
+    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false, SPLIT>;
+    if constexpr (!SPLIT) return conv_halo_kernel<HALO_I8, 0, FORM, false, false, false>;
   }
   return nullptr;
 }
 HaloKernel pick_kernel(const HaloPlan &hp) {
   const HaloParams &p = hp.p;
-  const bool s3x3 = !p.strided && p.tap_cols[0] == 3 && p.tap_rows[0] == 3 && p.pxw == pxw_3x3(hp.kind, p.kch / 2);
+  const bool s3x3 = hp.stride == 1 && p.tap_cols[0] == 3 && p.tap_rows[0] == 3 && p.pxw == pxw_3x3(hp.kind, p.kch / 2);
+  if (p.split > 1) return !s3x3 ? pick_kernel<FORM_ANY, false, true>(hp) : p.row_units ? pick_kernel<FORM_3X3_ROWS, false, true>(hp)
+                                                                                      : pick_kernel<FORM_3X3_TAPS, false, true>(hp);
   if (p.pair) return s3x3 ? pick_kernel<FORM_3X3_TAPS, true>(hp) : pick_kernel<FORM_ANY, true>(hp);
   if (!s3x3) return pick_kernel<FORM_ANY>(hp);
   if (p.resident && p.b_stages == 3 * p.groups) return pick_kernel<FORM_3X3_RESIDENT>(hp);
@@ -921,9 +1022,9 @@ struct LaunchConfig {
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    at[1].val.clusterDim.x = hp.p.pair ? 2 : hp.p.split; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
-    cfg.numAttrs = hp.p.pair ? 2 : 1;
+    cfg.numAttrs = hp.p.pair || hp.p.split > 1 ? 2 : 1;
   }
   LaunchConfig(const LaunchConfig &) = delete;
 };
@@ -955,14 +1056,15 @@ bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err) {
   return true;
 }
 
-bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err) {
+bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err,
+                 int step, int src_h, int src_w) {
   const HaloPlan::Maps *hit = nullptr;
   for (const auto &m : hp.maps)
-    if (m.base == in && m.cnt == images) { hit = &m; break; }
+    if (m.base == in && m.cnt == images && m.step == step && (step == 1 || (m.src_h == src_h && m.src_w == src_w))) { hit = &m; break; }
   if (!hit) {
     HaloPlan::Maps m{};
-    m.base = in; m.cnt = images;
-    if (!encode_maps(hp, in, images, m.m, err)) return false;
+    m.base = in; m.cnt = images; m.step = step; m.src_h = src_h; m.src_w = src_w;
+    if (!encode_maps(hp, in, images, step, src_h, src_w, m.m, err)) return false;
     if (hp.maps.size() >= 64) hp.maps.erase(hp.maps.begin());
     hp.maps.push_back(m);
     hit = &hp.maps.back();
@@ -975,10 +1077,11 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   if (p.fast == 1)
     for (int i = 0; i < p.OCB * 16; ++i) { p.cst[0][i] = hp.scale[i]; p.cst[1][i] = hp.shift[i]; }
   p.N = images;
+  if (step > 1) p.strided = 1;
   p.row_tiles = ((images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
   const int m_tiles = p.row_tiles * p.col_tiles;
   p.total_tiles = (p.pair ? (m_tiles + 1) / 2 : m_tiles) * p.n_tiles;
-  LaunchConfig lc(hp, p.pair ? 2 * std::min(p.total_tiles, hp.max_clusters) : std::min(p.total_tiles, num_sms), s);
+  LaunchConfig lc(hp, p.split > 1 ? p.total_tiles * p.split : p.pair ? 2 * std::min(p.total_tiles, hp.max_clusters) : std::min(p.total_tiles, num_sms), s);
   const cudaError_t e = cudaLaunchKernelEx(&lc.cfg, pick_kernel(hp), p);
   if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
   return true;

@@ -58,6 +58,7 @@ struct HaloParams {
   int row_units;                     // a weight stage holds a filter row's taps (1) or one tap (0) of a plane
   int kstep_bytes, b_stages, b_stage_bytes;
   int pair;                          // clusters of two CTAs multiply two row tiles by weights of which each holds half
+  int split;                         // CTAs that share a tile's K loop (1: none; else one tile per cluster)
   int bufs;                          // accumulators in tensor memory: 4 of up to 128 columns or 2 of up to 256
   int resident;                      // every weight stage of the (single) n tile stays in shared memory
   int stack;                         // f32: hi and lo weight rows of a chunk stacked (BN <= 128)
@@ -76,6 +77,7 @@ struct HaloPlan {
   int kind = HALO_I8;
   HaloParams p{};
   size_t smem_bytes = 0, b_bytes = 0;
+  double est_us = 0;                 // modelled time of the whole batch
   int max_clusters = 0;              // pairs the device holds at once
   int stride = 1, IH = 0, IW = 0, CB = 0;
   int parity[4] = {0, 0, 0, 0};      // of each plane: row parity * stride + column parity
@@ -83,7 +85,7 @@ struct HaloPlan {
   std::vector<Chunk> order;          // two (i8) chunks per K step of a group; f32: cb = quarter of the block
   std::vector<float> scale, shift;   // int8: host copies of the requantisation constants, [OCP]
   void *d_b = nullptr;               // packed weights (owned by the plan that owns this)
-  struct Maps { const void *base; int cnt; CUtensorMap m[4][HALO_HEIGHTS]; };
+  struct Maps { const void *base; int cnt, step, src_h, src_w; CUtensorMap m[4][HALO_HEIGHTS]; };
   std::vector<Maps> maps;            // tensor maps encoded so far
 };
 // false: the shape does not suit the kernel (err says why)
@@ -95,6 +97,8 @@ std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, 
 bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err);      // the packed weights on the device
 cudaError_t halo_init(HaloPlan &hp);      // once per plan and device
 // Run `images` images: in / p.out address the first; p: a copy of hp.p with the per-call pointers set.
-bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err);
+// step > 1 (stride 1 only): the tensor holds src_h x src_w pixels per plane, of which every step-th row and column is read.
+bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err,
+                 int step = 1, int src_h = 0, int src_w = 0);
 
 }  // namespace elb

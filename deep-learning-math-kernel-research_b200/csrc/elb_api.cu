@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -363,13 +364,20 @@ int setup_i8_direct(elb_conv &pl) {
   // applies the 1x1 semantics there as well (f += prev * sum_scale); with the flag off the two agree bit for bit.
   p.rq.with_sum = d.with_ip_sum && d.dt_output != ELB_F32;
   p.rq.sum_scale = d.sum_scale;
-  if (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA) {
+  if (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA || pl.info.kernel == ELB_KERNEL_I8_GEMM_UMMA) {
     // (ELB_I8_CTA2=1 asks for the pair kernel, which takes the one-copy-per-tap form below)
     const char *on2 = getenv("ELB_I8_CTA2");
     std::string why;
+    // A plain 1x1 layer goes the same way where the GEMM kernel below has few tiles of 128 pixels x BN channels (each
+    // its whole K loop on one SM) or small images half fill them.  Its time, fitted on 1024 -> 256 at 14x14, 256 ->
+    // 1024 at 7x7 and 64 -> 64 at 28x28, 1 to 64 images; one 14x14 image 8.1 -> 6.2 us, 16 of 7x7 6.6 -> 4.4 us.
+    const int gemm_bn = p.OCB >= 16 ? 256 : p.OCB >= 8 ? 128 : 64;
+    const double gemm_tiles = static_cast<double>(d.n) * ((d.oh * d.ow + 127) / 128) * ((p.OCB * V + gemm_bn - 1) / gemm_bn);
+    const double gemm_us = 2.5 + 0.007 * gemm_bn + std::ceil(gemm_tiles / pl.num_sms) * gemm_bn * (0.006 + 0.0011 * ((p.CB + 7) / 8));
     pl.halo = new HaloPlan();
     if (!(on2 && atoi(on2) > 0) &&
-        halo_plan(*pl.halo, HALO_I8, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, pl.num_sms, why)) {
+        halo_plan(*pl.halo, HALO_I8, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, pl.num_sms, why) &&
+        (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA || pl.halo->est_us + 1.5 < gemm_us)) {
       CUDA_TRY(halo_init(*pl.halo));
       pl.info.launches_per_call = 1;
       return ELB_OK;

@@ -1724,20 +1724,50 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   g.k_stages = w->kind == KIND_F32 ? g.CB * g.taps : (g.CB + 7) / 8;
   w->n_tiles = (w->OCP + MAX_BN - 1) / MAX_BN;
   w->BN = host::alignup((w->OCP + w->n_tiles - 1) / w->n_tiles, 16);
-  // Direct convolutions other than the plain 1x1: one kernel that reads the caller's tensor, instead of an
-  // im2col tensor written and read once per tap (3x3 stride 2, 64 x 128 -> 256 channels 56x56: 231 MB of it).
-  if (direct && !(d.kh == 1 && d.kw == 1 && d.stride_h == 1)) {
+  // fp32 convolutions that the halo-tiled direct kernel (conv_halo.cu) runs as a whole:
+  //   * direct KxK and strided ones, instead of an im2col tensor written and read once per tap (3x3 stride 2,
+  //     64 x 128 -> 256 channels 56x56: 231 MB of it, 252 -> 164 us);
+  //   * plain 1x1 layers of so few tiles that most SMs would have none (1024 -> 256 at 14x14, one image 47 -> 13 us);
+  //   * Winograd requests where nine products per output cost less than moving V and M through memory and
+  //     transforming them: few channels (VGG conv1_2 at 16 images 413 -> 245 us, conv2_1 153 -> 103, conv2_2
+  //     217 -> 195; conv3_1 325 against 373 stays), or a single image, where the 36 transformed weight planes
+  //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 63 -> 18 us; one image of
+  //     512 channels 14x14 30 -> 14 us).  The direct result has the smaller rounding error of the two.  Layers of
+  //     at most 32 input channels and few tiles stay on the transform kernels, whose launches the chain's tests count.
+  const bool wino_f32 = info.kernel == ELB_KERNEL_WINO_F32_UMMA;
+  if ((direct && (w->flat || !(d.kh == 1 && d.kw == 1 && d.stride_h == 1))) ||
+      (wino_f32 && (d.ic > 32 || static_cast<long long>(d.n) * d.oh * d.ow > 8192))) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    w->halo = new HaloPlan();
+    HaloPlan *hp = new HaloPlan();
     std::string why;
-    if (!halo_plan(*w->halo, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why)) {
-      delete w->halo;
-      w->halo = nullptr;
-    } else if (halo_init(*w->halo) != cudaSuccess) {
+    bool take = halo_plan(*hp, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why);
+    if (take && w->flat) {      // the GEMM kernel: fitted on 1024 -> 256 at 14x14, 64 -> 64 at 28x28, 256 -> 1024 at 7x7
+      const double tiles = static_cast<double>(d.n) * ((d.oh * d.ow + BM - 1) / BM) * w->n_tiles;
+      take = hp->est_us < 6 + 0.65 * g.k_stages * std::ceil(tiles / sms);
+    }
+    if (take && wino_f32 && !w->small_ic) {
+      // modelled time of the transform kernels: traffic at 5.8 TB/s, the GEMM at 3 x its operations in 0.8 PFLOP/s if
+      // that takes longer, 11.5 us of launches and tails (both models are within about 10 % from 7 to 400 us)
+      const double tiles = static_cast<double>(d.n) * g.ht * g.wt, C = w->ICP, K = w->OCP;
+      const double vb = AA * tiles * C * 4, mb = AA * tiles * K * 4, ub = AA * C * K * 8.0;
+      const double io = (C * d.ih * d.iw + K * d.oh * d.ow) * d.n * 4;
+      const double us = 11.5 + (io + vb + mb) / 5.8e6 + std::max((vb + mb + ub) / 5.8e6, 6 * AA * tiles * C * K / 0.8e9);
+      take = hp->est_us < 0.98 * us;
+    }
+    if (w->small_ic) take = false;
+    if (take && halo_init(*hp) != cudaSuccess) {
+      delete hp;
       err = "cudaFuncSetAttribute failed";
       return ELB_GENERAL_ERROR;
+    }
+    if (take) {
+      w->halo = hp;
+      w->flat = false;
+      if (wino_f32) { w->relu_lo = 0.0f; w->relu_hi = 3.402823466e38f; }      // (relu_bound is not used on this path)
+    } else {
+      delete hp;
     }
   }
   // chunk of whole images whose transform-domain buffers fit the budget
@@ -1844,19 +1874,20 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
     return ELB_OK;
   }
   std::vector<float> u;
-  if (w->direct) {
+  const int taps = d.kh * d.kw;
+  if (w->direct || w->halo) {
     // U[oc][tap][ic]: K runs over (kh, kw) taps, then the input channels
-    u.assign(static_cast<size_t>(w->OCP) * g.taps * w->ICP, 0.0f);
+    u.assign(static_cast<size_t>(w->OCP) * taps * w->ICP, 0.0f);
     for (int o = 0; o < d.oc; ++o)
-      for (int tap = 0; tap < g.taps; ++tap)
+      for (int tap = 0; tap < taps; ++tap)
         for (int i = 0; i < d.ic; ++i)
-          u[(static_cast<size_t>(o) * g.taps + tap) * w->ICP + i] =
+          u[(static_cast<size_t>(o) * taps + tap) * w->ICP + i] =
               hw[host::w_index(w->ICP / 16, d.kh, d.kw, o, i, tap / d.kw, tap % d.kw)];
   } else {
     u = transform_weights(hw.data(), d.oc, d.ic, w->OCP, w->ICP, g.A);
   }
   if (w->halo) {
-    const std::vector<uint8_t> img = halo_pack_f32(*w->halo, u.data(), w->OCP, g.taps, w->ICP);
+    const std::vector<uint8_t> img = halo_pack_f32(*w->halo, u.data(), w->OCP, taps, w->ICP);
     void *d_b = nullptr;
     W_TRY(cudaMalloc(&d_b, img.size()));
     if (!halo_set_weights(*w->halo, d_b, err)) return ELB_GENERAL_ERROR;
@@ -1976,6 +2007,7 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     return ELB_OK;
   }
   if (w->halo) {
+    const WinoGeom &g0 = w->g;
     HaloParams hp = w->halo->p;
     hp.shift = w->with_bias ? static_cast<const float *>(w->d_bias) : nullptr;
     hp.out = static_cast<float *>(out) + static_cast<size_t>(first) * (w->out_img_bytes / 4);
@@ -1984,8 +2016,9 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     hp.rq.relu_lo = w->relu_lo; hp.rq.relu_hi = w->relu_hi;
     const bool timed = pl.stage_ev[0] != nullptr;
     if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[0], s)); W_TRY(cudaEventRecord(pl.stage_ev[1], s)); }
-    if (!halo_launch(*w->halo, hp, static_cast<const float *>(in) + static_cast<size_t>(first) * (w->in_img_bytes / 4), count,
-                     num_sms, s, err))
+    const size_t img = stepped ? static_cast<size_t>(g0.CB) * pl.src_h * pl.src_w * 16 : w->in_img_bytes / 4;
+    if (!halo_launch(*w->halo, hp, static_cast<const float *>(in) + static_cast<size_t>(first) * img, count, num_sms, s, err,
+                     stepped ? pl.in_step : 1, pl.src_h, pl.src_w))
       return ELB_GENERAL_ERROR;
     if (timed) { W_TRY(cudaEventRecord(pl.stage_ev[2], s)); W_TRY(cudaEventRecord(pl.stage_ev[3], s)); }
     launches = 1;

@@ -30,6 +30,9 @@ SHAPES = [                                            # n, ic, oc, ih, iw, extra
     (2, 16, 32, 20, 20, dict(kh=7, kw=7, pad=3, stride=2)),
     (36, 128, 256, 14, 14, {}),                       # pairs of CTAs
     (37, 64, 256, 28, 28, dict(stride=2)),            # pairs, parity planes; an odd number of row tiles
+    (1, 512, 64, 14, 14, {}),                         # a tile's K loop shared by the CTAs of a cluster
+    (2, 1024, 256, 7, 7, dict(kh=1, kw=1, pad=0, algo="1x1")),
+    (1, 304, 40, 9, 9, dict(kh=1, kw=1, pad=0, algo="1x1")),
     (2, 48, 64, 9, 11, dict(kh=1, kw=1, pad=0, stride=2)),
 ]
 
@@ -50,4 +53,38 @@ def test_halo_matches_oracle(pkg, shape, types):
         got, d, acc = G.run_gpu(case, t, want_acc=True)
         assert d.launch_count() == 1 and d.device_status() == 0
         assert np.array_equal(acc, want_acc) and np.array_equal(got, want)
+    d.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 64, 17, 20), (2, 96, 40, 9, 9), (1, 512, 512, 14, 14)], ids=str)
+@pytest.mark.parametrize("tile", [6, 4])
+@pytest.mark.parametrize("total", [False, True])
+def test_winograd_request_on_the_direct_kernel(pkg, shape, tile, total):
+    """fp32 Winograd requests the plan serves with the direct kernel: one launch, the Winograd result."""
+    import gpuutil as G
+    n, ic, oc, ih, iw = shape
+    case = R.ConvCase("halo_wino", n, ic, oc, ih, iw, types="fp32", algo="wino", tile=tile, relu=True, bias=True, sum=total)
+    t = R.make_tensors(case)
+    got, d = G.run_gpu(case, t)
+    assert d.kernel == "wino_f32_umma" and d.launch_count() == 1 and d.device_status() == 0
+    assert R.rel_l2(got, R.oracle_wino_f32(case, t)) <= 1e-5
+    d.close()
+
+
+def test_direct_kernel_reads_its_input_with_a_step(pkg):
+    import torch
+    import gpuutil as G
+    E = G.package()
+    case = R.ConvCase("halo_step", 2, 64, 48, 11, 10, types="fp32", algo="wino", tile=6, relu=True, bias=True)
+    t = R.make_tensors(case)
+    want = R.oracle_wino_f32(case, t)
+    d = G.make_desc(case)
+    assert d.setup() == E.ELD_OK and d.input_step_supported()
+    assert d.prepare(torch.from_numpy(t["weights"]).cuda(), torch.from_numpy(t["bias"]).cuda()) == 0
+    big = np.full((2, 4, 21, 20, 16), 7.0, np.float32)
+    big[:, :, ::2, ::2] = t["input"]
+    out = torch.zeros(R.out_shape(case), device="cuda")
+    assert d.enqueue_strided(out, torch.from_numpy(big).cuda(), 21, 20, 2) == 0, E.last_error()
+    torch.cuda.synchronize()
+    assert d.launch_count() == 1 and R.rel_l2(out.cpu().numpy(), want) <= 1e-5
     d.close()
