@@ -42,7 +42,7 @@ namespace elb {
 namespace {
 
 constexpr int BM = 128, TILE_H = 16, TILE_W = 8;
-constexpr int MAX_A = 4, MAX_B = 16, RAW_STAGES = 4, MAX_BUFS = 4;
+constexpr int MAX_A = 8, MAX_B = 16, RAW_STAGES = 4, MAX_BUFS = 4;
 // int8: an epilogue group of four warps per (accumulator, half of the column blocks); fp32: per half
 constexpr int EPI_WARP0 = 4, SPLIT_WARPS = 4;
 constexpr int EPI_WARPS_I8 = 16, EPI_WARPS_F32 = 8;
@@ -108,9 +108,15 @@ __device__ __forceinline__ void store_v8(float *p, const float (&f)[16], int at)
 // does, an address from a table in the parameter space 70, and a wait on a completed barrier 100 to 160.  With
 // loops, tables and a wait per filter row issuing took 2900 cycles per tile of 18 MMAs that last 864 (64 -> 64
 // channels at 224 x 224).
-enum : int { FORM_ANY = 0, FORM_3X3_ROWS = 1, FORM_3X3_TAPS = 2, FORM_3X3_RESIDENT = 3 };
-// pixels of a shared-memory row of a 3x3 stride-1 filter (what halo_plan() computes)
-__host__ __device__ constexpr int pxw_3x3(int kind, int pairs) { return kind == HALO_F32 || pairs == 2 || pairs == 4 ? 10 : pairs == 0 ? 16 : 12; }
+// FORM_3X3S2: 3x3 stride 2 with one padding column (planes of 1, 2, 2 and 4 taps), FORM_1X1: one tap; a weight stage
+// per tap.  (As loops a unit of four MMAs that last 512 cycles took 500 to 650 to issue.)
+enum : int { FORM_ANY = 0, FORM_3X3_ROWS = 1, FORM_3X3_TAPS = 2, FORM_3X3_RESIDENT = 3, FORM_3X3S2 = 4, FORM_1X1 = 5 };
+// pixels of a shared-memory row (what halo_plan() computes)
+__host__ __device__ constexpr int pxw_of(int form, int kind, int pairs) {
+  return form == FORM_1X1 ? (pairs ? 8 : 16)
+       : form == FORM_3X3S2 ? (kind == HALO_F32 || pairs == 2 ? 10 : pairs == 4 ? 9 : pairs == 0 ? 16 : 12)
+                            : (kind == HALO_F32 || pairs == 2 || pairs == 4 ? 10 : pairs == 0 ? 16 : 12);
+}
 
 // PAIR: clusters of two CTAs.  One tcgen05.mma.cta_group::2 multiplies two row tiles (128 rows per CTA) by the BN
 // weight rows of which each CTA stages HALF: what an SM takes in per MMA from L2 and what the MMA reads from its
@@ -203,7 +209,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     }
     return x;
   };
-  auto emit = [&](const Pixel &px, int ocb, uint32_t (&r)[16]) {
+  auto emit = [&](const Pixel &px, int ocb, uint32_t (&r)[16], const uint4 *prev) {
     if (!px.valid || ocb >= p.OCB) return;
     const size_t off = (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16;
     if (KIND == HALO_I8) {
@@ -217,7 +223,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       }
       if (p.fast == 2) requant_relu_u8(a, s_scale + ocb * 16, s_shift + ocb * 16, static_cast<uint8_t *>(p.out) + off);
       else if (p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
-      else requant_store16(a, s_scale + ocb * 16, px.shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * (p.rq.out_type == OUT_F32 ? 4 : 1), p.rq);
+      else requant_store16(a, s_scale + ocb * 16, px.shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * (p.rq.out_type == OUT_F32 ? 4 : 1), p.rq, prev);
     } else {
       float f[16];
 #pragma unroll
@@ -258,7 +264,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
     const int planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    const bool strided = (FORM == FORM_ANY || KIND == HALO_F32) && uni(p.strided) != 0;
+    const bool strided = FORM == FORM_3X3S2 || ((FORM == FORM_ANY || FORM == FORM_1X1 || KIND == HALO_F32) && uni(p.strided) != 0);
     // stride 1: 8-byte elements, so that the copy engine moves whole rows
     const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
     int s = 0;
@@ -270,7 +276,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
       // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
       // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
-      constexpr int Q = FORM == FORM_ANY ? 4 : 1;      // planes the code is written out for
+      constexpr int Q = FORM == FORM_ANY || FORM == FORM_3X3S2 ? 4 : 1;      // planes the code is written out for
       int idx[Q], img[Q], row[Q];
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
@@ -363,8 +369,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     // ---------------------------------------------------------------- MMA issuers (pairs: the leader's)
     if (rank == 0) {
     constexpr bool STRAIGHT = FORM != FORM_ANY;
-    constexpr int M = PAIR ? 2 * BM : BM, PXW = pxw_3x3(KIND, PAIRS), CHUNKS = PAIRS ? 2 * PAIRS : 1;
-    const int BN = uni(p.BN), total = uni(p.total_tiles), groups = uni(p.groups), planes = STRAIGHT ? 1 : uni(p.planes),
+    constexpr int M = PAIR ? 2 * BM : BM, PXW = pxw_of(FORM, KIND, PAIRS), CHUNKS = PAIRS ? 2 * PAIRS : 1;
+    const int BN = uni(p.BN), total = uni(p.total_tiles), groups = uni(p.groups), planes = FORM == FORM_3X3S2 ? 4 : STRAIGHT ? 1 : uni(p.planes),
               b_stages = uni(p.b_stages), a_stages = uni(p.a_stages), bufs = uni(p.bufs);
     const bool row_units = uni(p.row_units) != 0, resident = FORM == FORM_ANY ? uni(p.resident) != 0 : FORM == FORM_3X3_RESIDENT;
     const uint32_t idesc = KIND == HALO_I8 ? umma_idesc(2, 0, 1, M, BN) : umma_idesc(1, 2, 2, M, BN);
@@ -454,24 +460,40 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
 #pragma unroll
           for (int r = 0; r < 3; ++r, a_row += pitch16) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
         } else if constexpr (STRAIGHT) {
-          constexpr int UNITS = FORM == FORM_3X3_ROWS ? 3 : 9;
-          bool seen = mbar_test_wait(&bar.bfull[bs], bph);
+          // R x C taps of the plane; a weight stage holds one tap or, FORM_3X3_ROWS, a row of them
+          auto units = [&](auto r_const, auto c_const) {
+            constexpr int C = decltype(c_const)::value, UNITS = decltype(r_const)::value * (FORM == FORM_3X3_ROWS ? 1 : C);
+            bool seen = mbar_test_wait(&bar.bfull[bs], bph);
 #pragma unroll
-          for (int u = 0; u < UNITS; ++u) {
-            if (!__all_sync(0xFFFFFFFFu, seen)) {
-              ok = wait_all(&bar.bfull[bs], bph, abort_flag);
-              if (!ok) break;
+            for (int u = 0; u < UNITS; ++u) {
+              if (!__all_sync(0xFFFFFFFFu, seen)) {
+                ok = wait_all(&bar.bfull[bs], bph, abort_flag);
+                if (!ok) break;
+              }
+              tc_fence_after_sync();
+              b_lo = (b_base + bs * b16) | b_lbo;
+              uint64_t *done = &bar.bempty[bs];
+              next_b();
+              // the next stage is tested in front of this one's MMAs, so the answer is there when they are issued
+              if (u + 1 < UNITS) seen = mbar_test_wait(&bar.bfull[bs], bph);
+              if (FORM == FORM_3X3_ROWS) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
+              else taps(std::integral_constant<int, 1>{}, u % C);
+              commit(done, el);
+              if (FORM == FORM_3X3_ROWS || u % C == C - 1) a_row += pitch16;
             }
-            tc_fence_after_sync();
-            b_lo = (b_base + bs * b16) | b_lbo;
-            uint64_t *done = &bar.bempty[bs];
-            next_b();
-            // the next stage is tested in front of this one's MMAs, so the answer is there when they are issued
-            if (u + 1 < UNITS) seen = mbar_test_wait(&bar.bfull[bs], bph);
-            if (FORM == FORM_3X3_ROWS) taps(std::integral_constant<int, ROW_STEPS>{}, 0);
-            else taps(std::integral_constant<int, 1>{}, u % 3);
-            commit(done, el);
-            if (FORM == FORM_3X3_ROWS || u % 3 == 2) a_row += pitch16;
+          };
+          using One = std::integral_constant<int, 1>;
+          using Two = std::integral_constant<int, 2>;
+          using Three = std::integral_constant<int, 3>;
+          if constexpr (FORM == FORM_3X3S2) {
+            if (q == 0) units(One{}, One{});
+            else if (q == 1) units(One{}, Two{});
+            else if (q == 2) units(Two{}, One{});
+            else units(Two{}, Two{});
+          } else if constexpr (FORM == FORM_1X1) {
+            units(One{}, One{});
+          } else {
+            units(Three{}, Three{});
           }
         } else {
           const int rows = uni(p.tap_rows[q]), cols = uni(p.tap_cols[q]);
@@ -586,10 +608,20 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       const int mu = p.div_n.div(tile), nt = tile - mu * p.n_tiles, mt = PAIR ? 2 * mu + rank : mu;
       const Pixel px = SPLIT ? Pixel{} : locate(mt, row);
       const uint32_t buf = t & (p.bufs - 1), tph = (t >> t_shift) & 1u;
+      if (!SPLIT && p.rq.with_sum && px.valid) {
+        // the residual this tile adds: on its way to L2 while the MMAs run
+        const int elt = KIND == HALO_F32 || p.rq.out_type == OUT_F32 ? 4 : 1;
+        for (int k = 0; k < cnt; ++k) {
+          const int ocb = nt * nb16 + half + blk_step * k;
+          if (ocb < p.OCB)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.out) +
+                                                          (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16 * elt));
+        }
+      }
       if (!wait_all(&bar.tfull[buf], tph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
       tc_fence_after_sync();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (whole ? 128u : 256u) + half * 16;
-      auto take = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16]) {
+      auto take = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16], const uint4 &pv) {
         if (STACK) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(r[i]), __uint_as_float(r2[i])));
@@ -599,8 +631,15 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) d[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
         } else {
-          emit(px, nt * nb16 + blk, r);
+          emit(px, nt * nb16 + blk, r, KIND == HALO_I8 ? &pv : nullptr);
         }
+      };
+      // int8: the stored output that block k adds, fetched a block ahead
+      const bool add = KIND == HALO_I8 && !SPLIT && p.rq.with_sum && px.valid;
+      auto residual = [&](int k, uint4 &pv) {
+        const int ocb = nt * nb16 + half + blk_step * k;
+        if (add && ocb < p.OCB)
+          pv = *reinterpret_cast<const uint4 *>(static_cast<const uint8_t *>(p.out) + (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16);
       };
       auto release = [&]() {
         tc_fence_before_sync();
@@ -614,23 +653,24 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       // blocks half, half + blk_step, ... of this warp, two in flight: while one is converted and stored the next is
         // on its way out of tensor memory
         uint32_t r0[16], r1[16], q0[16], q1[16];
+        uint4 pv0 = make_uint4(0, 0, 0, 0), pv1 = pv0;
         constexpr bool pair = STACK;
         auto load = [&](int k, uint32_t (&r)[16], uint32_t (&q)[16]) {
           tmem_ld16(t_addr + k * (16 * blk_step), r);
           if (pair) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
         };
-        if (cnt > 0) load(0, r0, q0);
+        if (cnt > 0) { load(0, r0, q0); residual(0, pv0); }
 #pragma unroll 1
         for (int k = 0; k < cnt; k += 2) {
           tmem_ld_wait16(r0);
           if (pair) tmem_ld_wait16(q0);
-          if (k + 1 < cnt) load(k + 1, r1, q1);
-          take(half + blk_step * k, r0, q0);
+          if (k + 1 < cnt) { load(k + 1, r1, q1); residual(k + 1, pv1); }
+          take(half + blk_step * k, r0, q0, pv0);
           if (k + 1 < cnt) {
             tmem_ld_wait16(r1);
             if (pair) tmem_ld_wait16(q1);
-            if (k + 2 < cnt) load(k + 2, r0, q0);
-            take(half + blk_step * (k + 1), r1, q1);
+            if (k + 2 < cnt) { load(k + 2, r0, q0); residual(k + 2, pv0); }
+            take(half + blk_step * (k + 1), r1, q1, pv1);
           }
         }
         release();
@@ -673,7 +713,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
                                                : __float_as_uint(__fadd_rn(__uint_as_float(sum[4 * j + k]), __uint_as_float(x[k])));
             }
           }
-          emit(locate(mt, srank * rows + row), nt * nb16 + blk, sum);
+          emit(locate(mt, srank * rows + row), nt * nb16 + blk, sum, nullptr);
         }
       } else {
         report_status(p.status, ST_WAIT_TIMEOUT_EPILOGUE);
@@ -704,6 +744,8 @@ double kstep_cycles(int kind, int BN, bool pair, double b, double a) {
   port += (b + a * (kind == HALO_F32 ? 4 : 1)) / 128;
   return std::max(std::max(tensor, port), (b + a) / 48);
 }
+
+int tap_form(const HaloPlan &hp);
 
 }  // namespace
 
@@ -869,9 +911,19 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       }
   }
   if (!p.resident) {
-    set_units(!p.pair && (kch == 1 || row_steps * p.kstep_bytes <= 24 * 1024));
+    const int form = tap_form(hp);
+    set_units(!p.pair && form != FORM_3X3S2 && form != FORM_1X1 && (kch == 1 || row_steps * p.kstep_bytes <= 24 * 1024));
+    // Ring depths.  A stage comes back about 4500 cycles after the MMAs that read it were issued (their end, the
+    // hand-overs, the copy); weights, which wait for nothing else, 3000.  An operand stage may last only a few
+    // hundred cycles (a parity plane, a 1x1 filter).  fp32 rows have the raw ring in front.
+    const double k_cyc = kstep_cycles(kind, p.BN, p.pair != 0, 0, 0);
+    const double a_cyc = k_cyc * p.ksteps / p.planes, b_cyc = k_cyc * p.ksteps / b_per_group;
+    const int a_min = planes_bytes <= 24 * 1024 ? 3 : 2;
+    const int a_want = kind == HALO_F32 ? a_min : std::max(a_min, std::min(MAX_A, 1 + static_cast<int>(std::ceil(4500 / a_cyc))));
+    const int b_want = std::max(3, std::min(8, static_cast<int>(std::ceil(3000 / b_cyc))));
     bool ok = false;
-    for (int a = planes_bytes <= 24 * 1024 ? 3 : 2; a >= 1 && !ok; --a) ok = fit_b(a) && p.b_stages >= 3;
+    for (int a = a_want; a > a_min && !ok; --a) ok = fit_b(a) && p.b_stages >= b_want;
+    for (int a = a_min; a >= 1 && !ok; --a) ok = fit_b(a) && p.b_stages >= 3;
     if (!ok) { err = "shared memory"; return false; }
   }
   if (p.split > 1 && 2 * 128 * (p.BN + 4) * 4 > p.a_stages * planes_bytes + RAW_STAGES * p.raw_bytes + p.b_stages * p.b_stage_bytes) {
@@ -998,16 +1050,34 @@ HaloKernel pick_kernel(const HaloPlan &hp) {
   }
   return nullptr;
 }
+// The issue loop's form for a geometry (before the weight stages are laid out); FORM_3X3_TAPS stands for all 3x3 ones.
+int tap_form(const HaloPlan &hp) {
+  const HaloParams &p = hp.p;
+  const int pairs = p.kch / 2, *r = p.tap_rows, *c = p.tap_cols;
+  int form = FORM_ANY;
+  if (hp.stride == 1 && r[0] == 3 && c[0] == 3) form = FORM_3X3_TAPS;
+  else if (p.planes == 4 && pairs && r[0] == 1 && c[0] == 1 && r[1] == 1 && c[1] == 2 && r[2] == 2 && c[2] == 1 && r[3] == 2 && c[3] == 2) form = FORM_3X3S2;
+  else if (p.planes == 1 && pairs && r[0] == 1 && c[0] == 1) form = FORM_1X1;
+  return p.pxw == pxw_of(form, hp.kind, pairs) ? form : FORM_ANY;
+}
+template <bool PAIR, bool SPLIT>
+HaloKernel pick_form(const HaloPlan &hp, int form) {
+  switch (form) {
+    case FORM_3X3_ROWS:
+      if constexpr (!PAIR) return pick_kernel<FORM_3X3_ROWS, false, SPLIT>(hp);
+      return nullptr;
+    case FORM_3X3_TAPS: return pick_kernel<FORM_3X3_TAPS, PAIR, SPLIT>(hp);
+    case FORM_3X3S2: return pick_kernel<FORM_3X3S2, PAIR, SPLIT>(hp);
+    case FORM_1X1: return pick_kernel<FORM_1X1, PAIR, SPLIT>(hp);
+  }
+  return pick_kernel<FORM_ANY, PAIR, SPLIT>(hp);
+}
 HaloKernel pick_kernel(const HaloPlan &hp) {
   const HaloParams &p = hp.p;
-  const bool s3x3 = hp.stride == 1 && p.tap_cols[0] == 3 && p.tap_rows[0] == 3 && p.pxw == pxw_3x3(hp.kind, p.kch / 2);
-  if (p.split > 1) return !s3x3 ? pick_kernel<FORM_ANY, false, true>(hp) : p.row_units ? pick_kernel<FORM_3X3_ROWS, false, true>(hp)
-                                                                                      : pick_kernel<FORM_3X3_TAPS, false, true>(hp);
-  if (p.pair) return s3x3 ? pick_kernel<FORM_3X3_TAPS, true>(hp) : pick_kernel<FORM_ANY, true>(hp);
-  if (!s3x3) return pick_kernel<FORM_ANY>(hp);
-  if (p.resident && p.b_stages == 3 * p.groups) return pick_kernel<FORM_3X3_RESIDENT>(hp);
-  if (p.resident) return pick_kernel<FORM_ANY>(hp);
-  return p.row_units ? pick_kernel<FORM_3X3_ROWS>(hp) : pick_kernel<FORM_3X3_TAPS>(hp);
+  int form = tap_form(hp);
+  if (p.resident) return form == FORM_3X3_TAPS && p.b_stages == 3 * p.groups ? pick_kernel<FORM_3X3_RESIDENT>(hp) : pick_kernel<FORM_ANY>(hp);
+  if (p.row_units) form = form == FORM_3X3_TAPS ? FORM_3X3_ROWS : FORM_ANY;
+  return p.split > 1 ? pick_form<false, true>(hp, form) : p.pair ? pick_form<true, false>(hp, form) : pick_form<false, false>(hp, form);
 }
 
 // Launch configuration: may overlap its set-up with the kernel before it (launch_overlapped), pairs as clusters of two.

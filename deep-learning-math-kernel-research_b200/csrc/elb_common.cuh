@@ -95,9 +95,10 @@ __device__ __forceinline__ float requant_one(int acc, float sc, float sh) {
 }
 
 // acc: 16 int32 accumulators; sc/sh: 16 per-channel constants; out/prev: address of the 16-channel
-// group in the output tensor (prev == out for the in-place sum).
+// group in the output tensor; prev: the stored 16 bytes the sum adds, where the caller has read them already.
 __device__ __forceinline__ void requant_store16(const int (&acc)[16], const float *__restrict__ sc,
-                                                const float *__restrict__ sh, void *out, const Requant &rq) {
+                                                const float *__restrict__ sh, void *out, const Requant &rq,
+                                                const uint4 *prev = nullptr) {
   float f[16];
   // the constants of the 16 channels are 64-byte aligned: four 16-byte loads per array
 #pragma unroll
@@ -126,7 +127,7 @@ __device__ __forceinline__ void requant_store16(const int (&acc)[16], const floa
     return;
   }
   if (rq.with_sum) {
-    const uint4 pv = *reinterpret_cast<const uint4 *>(out);
+    const uint4 pv = prev ? *prev : *reinterpret_cast<const uint4 *>(out);
     const uint32_t w[4] = {pv.x, pv.y, pv.z, pv.w};
 #pragma unroll
     for (int i = 0; i < 16; ++i) {

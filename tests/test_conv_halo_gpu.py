@@ -30,6 +30,12 @@ SHAPES = [                                            # n, ic, oc, ih, iw, extra
     (2, 16, 32, 20, 20, dict(kh=7, kw=7, pad=3, stride=2)),
     (36, 128, 256, 14, 14, {}),                       # pairs of CTAs
     (37, 64, 256, 28, 28, dict(stride=2)),            # pairs, parity planes; an odd number of row tiles
+    (3, 96, 300, 17, 19, dict(stride=2)),             # stride 2, taps as weight stages: six, four and two blocks per group
+    (2, 64, 260, 12, 30, dict(stride=2)),
+    (2, 32, 272, 15, 15, dict(stride=2)),
+    (2, 64, 260, 16, 15, dict(stride=2, pad=0)),
+    (3, 160, 272, 9, 9, dict(kh=1, kw=1, pad=0, stride=2)),
+    (3, 160, 272, 13, 9, dict(stride=2, sum=True, sscale=0.5)),
     (1, 512, 64, 14, 14, {}),                         # a tile's K loop shared by the CTAs of a cluster
     (2, 1024, 256, 7, 7, dict(kh=1, kw=1, pad=0, algo="1x1")),
     (1, 304, 40, 9, 9, dict(kh=1, kw=1, pad=0, algo="1x1")),
