@@ -735,14 +735,15 @@ int alignup(int v, int a) { return (v + a - 1) / a * a; }
 // Modelled cycles of one K step: the tensor pipe (N / 2 per MMA of 128 or 256 x N x 32 bytes), the shared-memory
 // port at 128 B/clk (operand reads of the MMAs, incoming copies, fp32: the split), the SM's intake from L2 at
 // about 48 B/clk.  b: bytes of weights an SM takes in per K step (0: resident), a: of input.
-double kstep_cycles(int kind, int BN, bool pair, double b, double a) {
+double kstep_cycles(int kind, int BN, bool pair, double b, double a, bool strided = false) {
   const double read_n = BN / (pair ? 8.0 : 4.0);
   double tensor, port;
   if (kind == HALO_I8) { tensor = BN / 2.0; port = 32 + read_n; }
   else if (!pair && BN <= 128) { tensor = 1.5 * BN; port = 64 + 3 * read_n; }      // (stacked hi / lo rows)
   else { tensor = 1.5 * BN; port = 3 * (32 + read_n); }
   port += (b + a * (kind == HALO_F32 ? 4 : 1)) / 128;
-  return std::max(std::max(tensor, port), (b + a) / 48);
+  // (a parity plane of int8 arrives 16 bytes at a time)
+  return std::max(std::max(tensor, port), b / 48 + a / (strided && kind == HALO_I8 ? 16 : 48));
 }
 
 int tap_form(const HaloPlan &hp);
@@ -854,10 +855,11 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
     const double epilogue = kind == HALO_I8 ? 400 + 128.0 * BN / 9 : 0;
     for (int pair = 0; pair < 2; ++pair) {
       // pairs take the weights tap by tap, in rows of 512 bytes per half
-      // (fp32 with a stride: each CTA waits for the slower of the two splits of a stage, 150 -> 180 us on 128 -> 256, 56x56)
-      if (pair && ((kind == HALO_F32 && stride > 1) || pairs < 2 || BN % 32 || stays || m_tiles < 2 || kb * pairs > 48 * 1024 || kb * pairs * 3 <= 24 * 1024)) continue;
+      // (with a stride the CTAs wait for one another at every parity plane: 128 -> 256, 56x56: fp32 150 -> 180 us, int8
+      // with a residual 27.8 -> 29.9; 512 -> 512, 14x14: 13.3 -> 17.5)
+      if (pair && (stride > 1 || pairs < 2 || BN % 32 || stays || m_tiles < 2 || kb * pairs > 48 * 1024 || kb * pairs * 3 <= 24 * 1024)) continue;
       const double b = stays ? 0.0 : pair ? kb / 2 : kb;
-      const double tile = std::max(kstep_cycles(kind, BN, pair != 0, b, ab) * p.ksteps * p.groups + 600, epilogue);
+      const double tile = std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps * p.groups + 600, epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
       if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; }
@@ -867,7 +869,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
     for (int split = 2; split <= 8 && split <= p.groups && m_tiles * nt * split <= num_sms * (split == 8 ? 0.8 : 0.88); split *= 2) {
       const double parts = 128.0 * (BN + 4) * 4;
       if (kch == 1 || 2 * parts > 150 * 1024) continue;
-      const double t = kstep_cycles(kind, BN, false, kb, ab) * p.ksteps * ((p.groups + split - 1) / split) + 600 + 4000 + 2000 + parts / 9;
+      const double t = kstep_cycles(kind, BN, false, kb, ab, stride > 1) * p.ksteps * ((p.groups + split - 1) / split) + 600 + 4000 + 2000 + parts / 9;
       if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; }
     }
   }
