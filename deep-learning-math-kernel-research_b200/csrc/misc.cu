@@ -44,48 +44,133 @@ __global__ void __launch_bounds__(256) reorder_kernel(T *__restrict__ dst, const
   }
 }
 
-// u8 nchw -> nChw16c when a plane is a whole number of 4-pixel groups: one thread = 4 pixels of one
-// channel block.  It reads one 32-bit word per real channel (a warp: 128 contiguous bytes of a plane)
-// and writes the four pixels' 16-byte blocks, padding lanes zero.  (The byte-wise kernel above moves
-// one byte per access: measured 43 us for 32 RGB images of 224x224 against a few us of traffic.)
-__global__ void __launch_bounds__(256) reorder_u8_planes_kernel(uint4 *__restrict__ dst, const uint8_t *__restrict__ src,
-                                                                int c, int hw4, long long total) {
+// u8 nchw <-> nChw16c: one thread = 4 pixels of one channel block.  The plane side is one 32-bit word per real
+// channel (a warp: 128 contiguous bytes of a plane; WORDS = false, planes of another length: four bytes), the
+// blocked side four 16-byte pixels, padding lanes zero.  (The byte-wise kernel above moves one byte per access:
+// 43 us for 32 RGB images of 224x224 against a few us of traffic.)
+template <bool TO_BLOCKED, bool WORDS>
+__global__ void __launch_bounds__(256) reorder_u8_planes_kernel(void *__restrict__ dst_, const void *__restrict__ src_,
+                                                                int c, int hw, int groups, long long total) {
   griddep_launch_dependents();      // an INT8 kernel behind this one may set itself up (see launch_overlapped)
   const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   const int C2 = (c + 15) / 16;
-  const int q = static_cast<int>(idx % hw4);
-  const int cb = static_cast<int>((idx / hw4) % C2);
-  const long long n = idx / (static_cast<long long>(hw4) * C2);
-  uint32_t pl[16];
+  const int q = static_cast<int>(idx % groups);
+  const int cb = static_cast<int>((idx / groups) % C2);
+  const long long n = idx / (static_cast<long long>(groups) * C2);
+  const int px0 = 4 * q, cnt = min(4, hw - px0);
+  const long long plane0 = (n * c + cb * 16) * hw + px0;
+  const long long pix0 = (n * C2 + cb) * hw + px0;
+  if constexpr (TO_BLOCKED) {
+    const uint8_t *src = static_cast<const uint8_t *>(src_) + plane0;
+    uint32_t pl[16];
 #pragma unroll
-  for (int ch = 0; ch < 16; ++ch) {
-    const int cc = cb * 16 + ch;
-    pl[ch] = cc < c ? __ldg(reinterpret_cast<const uint32_t *>(src) + (n * c + cc) * hw4 + q) : 0u;
-  }
-  uint4 *o = dst + ((n * C2 + cb) * hw4 + q) * 4;
-#pragma unroll
-  for (int px = 0; px < 4; ++px) {
-    uint32_t w[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      // byte px of the four planes 4j .. 4j+3, in channel order
-      const uint32_t lo = __byte_perm(pl[4 * j], pl[4 * j + 1], 0x0040 + px * 0x0011);
-      const uint32_t hi = __byte_perm(pl[4 * j + 2], pl[4 * j + 3], 0x0040 + px * 0x0011);
-      w[j] = __byte_perm(lo, hi, 0x5410);
+    for (int ch = 0; ch < 16; ++ch) {
+      pl[ch] = 0u;
+      if (cb * 16 + ch >= c) continue;
+      const uint8_t *p = src + static_cast<long long>(ch) * hw;
+      if (WORDS) pl[ch] = __ldg(reinterpret_cast<const uint32_t *>(p));
+      else
+        for (int i = 0; i < cnt; ++i) pl[ch] |= static_cast<uint32_t>(__ldg(p + i)) << (8 * i);
     }
-    o[px] = make_uint4(w[0], w[1], w[2], w[3]);
+    uint4 *o = static_cast<uint4 *>(dst_) + pix0;
+#pragma unroll
+    for (int px = 0; px < 4; ++px) {
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // byte px of the four planes 4j .. 4j+3, in channel order
+        const uint32_t lo = __byte_perm(pl[4 * j], pl[4 * j + 1], 0x0040 + px * 0x0011);
+        const uint32_t hi = __byte_perm(pl[4 * j + 2], pl[4 * j + 3], 0x0040 + px * 0x0011);
+        w[j] = __byte_perm(lo, hi, 0x5410);
+      }
+      if (px < cnt) o[px] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  } else {
+    const uint4 *src = static_cast<const uint4 *>(src_) + pix0;
+    uint32_t in[4][4];      // [pixel][four channels]
+#pragma unroll
+    for (int px = 0; px < 4; ++px) {
+      const uint4 v = px < cnt ? __ldg(src + px) : make_uint4(0, 0, 0, 0);
+      in[px][0] = v.x; in[px][1] = v.y; in[px][2] = v.z; in[px][3] = v.w;
+    }
+    uint8_t *dst = static_cast<uint8_t *>(dst_) + plane0;
+#pragma unroll
+    for (int ch = 0; ch < 16; ++ch) {
+      if (cb * 16 + ch >= c) continue;
+      const int j = ch >> 2, e = ch & 3;
+      const uint32_t lo = __byte_perm(in[0][j], in[1][j], 0x0040 + e * 0x0011);
+      const uint32_t hi = __byte_perm(in[2][j], in[3][j], 0x0040 + e * 0x0011);
+      const uint32_t w = __byte_perm(lo, hi, 0x5410);
+      uint8_t *p = dst + static_cast<long long>(ch) * hw;
+      if (WORDS) *reinterpret_cast<uint32_t *>(p) = w;
+      else
+        for (int i = 0; i < cnt; ++i) p[i] = static_cast<uint8_t>(w >> (8 * i));
+    }
   }
+}
+
+// nhwc <-> nChw16c: both sides hold the 16 channels of a pixel and block as PER contiguous words W, so this is a copy
+// of 16- to 64-byte pieces.  Consecutive lanes take the words of a piece, CBS channel blocks of a pixel (so that
+// they cover whole 32-byte sectors of the nhwc side), then pixels (whole sectors of the blocked side); a thread
+// moves four pixels.  The general converter below does five divisions per element: fp32 8 x 200 channels 45x27
+// 32 -> 4 us.
+template <typename W, int PER, int CBS, bool TO_BLOCKED>
+__global__ void __launch_bounds__(256) reorder_nhwc_kernel(W *__restrict__ dst, const W *__restrict__ src, int c_words, int c2, int hw) {
+  griddep_launch_dependents();
+  constexpr int PIX = 256 / (PER * CBS), ITER = 4;
+  const int word = threadIdx.x % PER, cb = blockIdx.y * CBS + (threadIdx.x / PER) % CBS;
+  const int px0 = blockIdx.x * (PIX * ITER) + threadIdx.x / (PER * CBS);
+  if (cb >= c2) return;
+  const bool real = cb * PER + word < c_words;
+  const size_t n = blockIdx.z;
+  const size_t plain = n * hw * c_words + cb * PER + word, blocked = (n * c2 + cb) * static_cast<size_t>(hw) * PER + word;
+  W v[ITER];
+#pragma unroll
+  for (int i = 0; i < ITER; ++i) {
+    const int px = px0 + i * PIX;
+    v[i] = W{};
+    if (px < hw && real) v[i] = TO_BLOCKED ? __ldg(src + plain + static_cast<size_t>(px) * c_words) : __ldg(src + blocked + static_cast<size_t>(px) * PER);
+  }
+#pragma unroll
+  for (int i = 0; i < ITER; ++i) {
+    const int px = px0 + i * PIX;
+    if (px >= hw) continue;
+    if (TO_BLOCKED) dst[blocked + static_cast<size_t>(px) * PER] = v[i];
+    else if (real) dst[plain + static_cast<size_t>(px) * c_words] = v[i];
+  }
+}
+template <typename W, int PER, int CBS, bool TO_BLOCKED>
+cudaError_t launch_nhwc(void *dst, const void *src, int n, int c, int hw, int eb, cudaStream_t s) {
+  const int c2 = (c + 15) / 16, pix = 256 / (PER * CBS) * 4;
+  const dim3 grid((hw + pix - 1) / pix, (c2 + CBS - 1) / CBS, n);
+  reorder_nhwc_kernel<W, PER, CBS, TO_BLOCKED><<<grid, 256, 0, s>>>(static_cast<W *>(dst), static_cast<const W *>(src),
+                                                                   c * eb / static_cast<int>(sizeof(W)), c2, hw);
+  return cudaGetLastError();
+}
+// The widest word that the channel count and both addresses allow.
+template <bool TO_BLOCKED>
+cudaError_t launch_nhwc(void *dst, const void *src, int n, int c, int hw, int eb, cudaStream_t s) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | static_cast<uintptr_t>(c * eb);
+  if (eb == 4) return all % 16 == 0 ? launch_nhwc<uint4, 4, 1, TO_BLOCKED>(dst, src, n, c, hw, eb, s)
+                                    : launch_nhwc<uint32_t, 16, 1, TO_BLOCKED>(dst, src, n, c, hw, eb, s);
+  if (all % 16 == 0) return launch_nhwc<uint4, 1, 2, TO_BLOCKED>(dst, src, n, c, hw, eb, s);
+  if (all % 4 == 0) return launch_nhwc<uint32_t, 4, 2, TO_BLOCKED>(dst, src, n, c, hw, eb, s);
+  return launch_nhwc<uint8_t, 16, 2, TO_BLOCKED>(dst, src, n, c, hw, eb, s);
 }
 
 template <bool TO_BLOCKED>
 cudaError_t launch(void *dst, const void *src, int n, int c, int h, int w, int eb, cudaStream_t s) {
   const int hw = h * w;
-  if (TO_BLOCKED && eb == 1 && hw % 4 == 0 && ((reinterpret_cast<uintptr_t>(src) & 3) == 0) &&
-      ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-    const long long total = static_cast<long long>(n) * ((c + 15) / 16) * (hw / 4);
+  const void *blocked = TO_BLOCKED ? dst : src, *plain = TO_BLOCKED ? src : dst;
+  if (eb == 1 && reinterpret_cast<uintptr_t>(blocked) % 16 == 0) {
+    const int groups = (hw + 3) / 4;
+    const long long total = static_cast<long long>(n) * ((c + 15) / 16) * groups;
     const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
-    reorder_u8_planes_kernel<<<blocks, 256, 0, s>>>((uint4 *)dst, (const uint8_t *)src, c, hw / 4, total);
+    if (hw % 4 == 0 && reinterpret_cast<uintptr_t>(plain) % 4 == 0)
+      reorder_u8_planes_kernel<TO_BLOCKED, true><<<blocks, 256, 0, s>>>(dst, src, c, hw, groups, total);
+    else
+      reorder_u8_planes_kernel<TO_BLOCKED, false><<<blocks, 256, 0, s>>>(dst, src, c, hw, groups, total);
     return cudaGetLastError();
   }
   dim3 grid((hw + 127) / 128, (c + 15) / 16, n);
@@ -223,6 +308,10 @@ cudaError_t launch_reorder(void *dst, int dst_fmt, const void *src, int src_fmt,
   // fast paths for activations
   if (dst_fmt == ELB_NCHW16C && src_fmt == ELB_NCHW) return launch<true>(dst, src, a, b, h, w, eb, s);
   if (dst_fmt == ELB_NCHW && src_fmt == ELB_NCHW16C) return launch<false>(dst, src, a, b, h, w, eb, s);
+  if (a <= 65535 && static_cast<long long>(h) * w < (1ll << 31) && (b + 15) / 16 <= 65535) {
+    if (dst_fmt == ELB_NCHW16C && src_fmt == ELB_NHWC) return launch_nhwc<true>(dst, src, a, b, h * w, eb, s);
+    if (dst_fmt == ELB_NHWC && src_fmt == ELB_NCHW16C) return launch_nhwc<false>(dst, src, a, b, h * w, eb, s);
+  }
   if ((dst_fmt == ELB_NCHW && src_fmt == ELB_NHWC) || (dst_fmt == ELB_NHWC && src_fmt == ELB_NCHW)) {
     const int rows = src_fmt == ELB_NCHW ? b : h * w, cols = src_fmt == ELB_NCHW ? h * w : b;
     if (a <= 65535 && (rows + 31) / 32 <= 65535) {
