@@ -9,12 +9,14 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include "../../include/euler_b200.h"
 #include "elb_common.cuh"
 #include "conv_halo.cuh"
+#include "host_pipe.hpp"
 #include "host_prep.hpp"
 #include "wino.cuh"
 #include "depthwise.cuh"
@@ -170,6 +172,8 @@ struct elb_conv {
   // host-pointer callers: copy streams and events of the chunked, overlapped execute
   cudaStream_t s_h2d = nullptr, s_d2h = nullptr;
   std::vector<cudaEvent_t> ev_in, ev_done;
+  std::shared_ptr<HostPipe> pipe;       // pageable host tensors: pinned slots and helper threads
+  HostPipe::Events pipe_ev;
   // winograd
   WinoPlan wino{};
   // int8 depthwise
@@ -644,9 +648,14 @@ void perf_line(const elb_conv &pl, double ms) {
   log_line(LOG_PERF, buf);
 }
 
-bool is_device_ptr(const void *p) {
+bool is_device_ptr(const void *p, bool *pageable = nullptr) {
   cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    if (pageable) *pageable = true;
+    return false;
+  }
+  if (pageable) *pageable = a.type == cudaMemoryTypeUnregistered;
   return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
@@ -830,7 +839,8 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
     pl.pending_d2h = pl.pending_d2h || used_d2h;
     return wait_pending(pl);
   };
-  const bool in_dev = is_device_ptr(input), out_dev = is_device_ptr(output);
+  bool in_page = false, out_page = false;
+  const bool in_dev = is_device_ptr(input, &in_page), out_dev = is_device_ptr(output, &out_page);
   if (in_dev && out_dev) {
     if (verbose) CUDA_TRY(cudaEventRecord(t0, pl.stream));
     rc = do_enqueue(pl, output, input, pl.stream);
@@ -867,8 +877,43 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
       CUDA_TRY(cudaStreamWaitEvent(pl.s_h2d, pl.ev_call_done, 0));
       if (pl.pending_d2h) CUDA_TRY(cudaStreamWaitEvent(pl.stream, pl.ev_d2h_done, 0));
     }
+    // Pageable tensors of a waiting call go through pinned slots that helper threads fill and empty (host_pipe.hpp);
+    // below a megabyte their start costs more than it gives.  A pipe busy with another thread's call is not waited for.
+    const bool pageable = wait && (in_dev || in_page) && (out_dev || out_page) && moved >= (size_t(1) << 20);
+    if (pageable && !pl.pipe) pl.pipe = HostPipe::get();
     if (verbose) CUDA_TRY(cudaEventRecord(t0, pl.stream));
-    if (chunks == 1) {
+    if (pageable && pl.pipe && pl.pipe->try_lock()) {
+      // chunks of about 1.5 MB: what nothing overlaps is the first one's copy in and the last one's copy out
+      if (!getenv("ELB_HOST_CHUNKS")) chunks = (int)std::min<size_t>(std::min<size_t>(16, N), std::max<size_t>(1, moved / (size_t(3) << 19)));
+      if (pl.pending && (rc = wait_pending(pl)) != ELB_OK) { pl.pipe->unlock(); return rc; }
+      std::vector<HostPipe::Piece> pin, pout;
+      auto cut = [](std::vector<HostPipe::Piece> &v, void *host, void *dev, size_t bytes, int chunk) {
+        for (size_t at = 0; at < bytes; at += HostPipe::SLOT_BYTES)
+          v.push_back({(uint8_t *)host + at, (uint8_t *)dev + at, std::min(HostPipe::SLOT_BYTES, bytes - at), chunk});
+      };
+      auto first_of = [&](int k) { return (int)((long long)N * k / chunks); };
+      for (int k = 0; k < chunks; ++k) {
+        const size_t n0 = first_of(k), cnt = first_of(k + 1) - n0;
+        if (!in_dev) cut(pin, const_cast<uint8_t *>((const uint8_t *)input + n0 * in_img), (uint8_t *)pl.d_in_stage + n0 * in_img, cnt * in_img, k);
+        if (!out_dev && pl.d.with_ip_sum) cut(pin, (uint8_t *)output + n0 * out_img, (uint8_t *)pl.d_out_stage + n0 * out_img, cnt * out_img, k);
+        if (!out_dev) cut(pout, (uint8_t *)output + n0 * out_img, (uint8_t *)pl.d_out_stage + n0 * out_img, cnt * out_img, k);
+      }
+      int launch_rc = ELB_OK;
+      const cudaError_t e = pl.pipe->run(pl.pipe_ev, pin, pout, chunks, pl.s_h2d, pl.s_d2h, [&](int k) -> cudaError_t {
+        cudaError_t le = cudaEventRecord(pl.ev_call_done, pl.s_h2d);
+        if (le == cudaSuccess) le = cudaStreamWaitEvent(pl.stream, pl.ev_call_done, 0);
+        if (le != cudaSuccess) return le;
+        launch_rc = do_enqueue_range(pl, dout, din, first_of(k), first_of(k + 1) - first_of(k), pl.stream);
+        if (launch_rc != ELB_OK) return cudaErrorUnknown;
+        le = cudaEventRecord(pl.ev_d2h_done, pl.stream);
+        return le == cudaSuccess ? cudaStreamWaitEvent(pl.s_d2h, pl.ev_d2h_done, 0) : le;
+      });
+      pl.pipe->unlock();
+      if (launch_rc != ELB_OK) { cudaDeviceSynchronize(); return launch_rc; }
+      CUDA_TRY(e);
+      if (verbose) CUDA_TRY(cudaEventRecord(t1, pl.stream));
+      rc = finish(false);
+    } else if (chunks == 1) {
       if (!in_dev) CUDA_TRY(cudaMemcpyAsync(pl.d_in_stage, input, pl.uinfo.bytes_input, cudaMemcpyHostToDevice, pl.stream));
       if (!out_dev && pl.d.with_ip_sum)
         CUDA_TRY(cudaMemcpyAsync(pl.d_out_stage, output, pl.uinfo.bytes_output, cudaMemcpyHostToDevice, pl.stream));
