@@ -137,11 +137,13 @@ def last_error() -> str:
 
 def _ptr(x):
     """Address of a torch tensor / numpy array / int / None."""
+    if x is None:
+        return None
     try:
         return x.data_ptr()                 # (first: what the calls of a running program pass)
     except AttributeError:
         pass
-    if x is None or isinstance(x, int):
+    if isinstance(x, int):
         return x
     if hasattr(x, "ctypes"):
         return x.ctypes.data

@@ -843,6 +843,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   if (m_tiles * p.OCB > 1e9 || OCP > HALO_MAX_OC) { err = "size"; return false; }
   const int planes_bytes = p.a_bytes * (kind == HALO_F32 ? 2 : 1);
   const int pairs = kch / 2;
+  const double group_min = kind == HALO_F32 ? 1900 : 0;      // the way of a stage through the split, where a filter has few taps to hide it
   double best = 0;
   p.BN = 0;
   for (int nt = (OCP + 255) / 256; nt <= p.OCB; ++nt) {
@@ -859,7 +860,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       // with a residual 27.8 -> 29.9; 512 -> 512, 14x14: 13.3 -> 17.5)
       if (pair && (stride > 1 || pairs < 2 || BN % 32 || stays || m_tiles < 2 || kb * pairs > 48 * 1024 || kb * pairs * 3 <= 24 * 1024)) continue;
       const double b = stays ? 0.0 : pair ? kb / 2 : kb;
-      const double tile = std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps * p.groups + 600, epilogue);
+      const double tile = std::max(std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps, group_min) * p.groups + 600, epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
       if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; }
@@ -869,7 +870,8 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
     for (int split = 2; split <= 8 && split <= p.groups && m_tiles * nt * split <= num_sms * (split == 8 ? 0.8 : 0.88); split *= 2) {
       const double parts = 128.0 * (BN + 4) * 4;
       if (kch == 1 || 2 * parts > 150 * 1024) continue;
-      const double t = kstep_cycles(kind, BN, false, kb, ab, stride > 1) * p.ksteps * ((p.groups + split - 1) / split) + 600 + 4000 + 2000 + parts / 9;
+      const double t = std::max(kstep_cycles(kind, BN, false, kb, ab, stride > 1) * p.ksteps, group_min) * ((p.groups + split - 1) / split) + 600 +
+                       4000 + 2000 + parts / 9;
       if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; }
     }
   }
@@ -944,12 +946,15 @@ template <typename PutChunk>
 static void pack_walk(const HaloPlan &hp, uint8_t *dst, PutChunk put) {
   const HaloParams &p = hp.p;
   const int halves = p.pair ? 2 : 1, rows = p.BN / halves, unit = p.pair ? (hp.kind == HALO_F32 ? 2 : p.kch / 2) : 1;
-  for (int nt = 0; nt < p.n_tiles; ++nt)
-    for (int g = 0; g < p.groups; ++g)
-      for (int k0 = 0; k0 < p.ksteps; k0 += unit)
-        for (int h = 0; h < halves; ++h)
-          for (int k = k0; k < k0 + unit; ++k, dst += p.kstep_bytes)
-            for (int j = 0; j < 2; ++j) put(dst, j, hp.order[2 * k + j], g, nt * p.BN + h * rows, rows);
+  const size_t group_bytes = static_cast<size_t>(p.ksteps) * p.kstep_bytes * halves;
+  host::parallel_for(p.n_tiles * p.groups, group_bytes * p.n_tiles * p.groups, [&](int i) {
+    const int nt = i / p.groups, g = i - nt * p.groups;
+    uint8_t *at = dst + i * group_bytes;
+    for (int k0 = 0; k0 < p.ksteps; k0 += unit)
+      for (int h = 0; h < halves; ++h)
+        for (int k = k0; k < k0 + unit; ++k, at += p.kstep_bytes)
+          for (int j = 0; j < 2; ++j) put(at, j, hp.order[2 * k + j], g, nt * p.BN + h * rows, rows);
+  });
 }
 
 std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP) {
@@ -973,9 +978,8 @@ std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, 
       const float *src = u + (static_cast<size_t>(o0 + r) * taps + c.tap) * ICP + g * 16 + c.cb * 4;
       for (int e = 0; e < 4; ++e) {
         const float h = host::tf32_rna(src[e]);
-        volatile float l = src[e] - h;
         hi[r * 4 + e] = h;
-        lo[r * 4 + e] = l;
+        lo[r * 4 + e] = src[e] - h;      // (exact)
       }
     }
   });

@@ -4,9 +4,12 @@
 // bit-exactness of every later output, so nothing here may be re-associated or fused except where
 // the reference build itself fuses (written as an explicit fmaf).
 #pragma once
+#include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -14,6 +17,27 @@ namespace elb {
 namespace host {
 
 inline int alignup(int x, int a) { return (x + a - 1) / a * a; }
+
+// body(i) for i in [0, n) on up to eight threads; `work` = rough number of values touched (small jobs stay on the
+// calling thread: a thread costs about 30 us).  Every index is independent, so the results do not depend on it.
+template <typename Body>
+inline void parallel_for(int n, size_t work, Body body) {
+  int threads = static_cast<int>(std::thread::hardware_concurrency()) / 2;
+  threads = std::min(std::min(threads, 8), std::min(n, static_cast<int>(std::min<size_t>(work >> 15, 8))));
+  if (threads <= 1) {
+    for (int i = 0; i < n; ++i) body(i);
+    return;
+  }
+  std::atomic<int> next{0};
+  auto run = [&] { for (int i = next++; i < n; i = next++) body(i); };
+  std::vector<std::thread> th;
+  try {
+    for (int t = 1; t < threads; ++t) th.emplace_back(run);
+  } catch (...) {      // no more threads: the others do the work
+  }
+  run();
+  for (std::thread &t : th) t.join();
+}
 
 // OIhw16i16o index: [O/16][I/16][kh][kw][16 i][16 o]   (reference: src/elx_conv.hpp:10-12)
 inline size_t w_index(int I2, int KH, int KW, int o, int i, int kh, int kw) {
@@ -50,7 +74,8 @@ inline I8Weights quantize_weights_i8(const float *w, int oc, int ic, int kh, int
   r.absmax.assign(r.OCP, 0.0f);
   r.qsum.assign(r.OCP, 0);
   r.qsum_tap.assign((size_t)r.OCP * r.taps, 0);
-  for (int o = 0; o < r.OCP; ++o) {
+  parallel_for(r.OCP, (size_t)oc * ic * r.taps * 4, [&](int o) {
+    if (o >= oc) return;
     float m = 0.0f;
     for (int i = 0; i < ic; ++i)
       for (int a = 0; a < kh; ++a)
@@ -59,7 +84,7 @@ inline I8Weights quantize_weights_i8(const float *w, int oc, int ic, int kh, int
           if (v > m) m = v;
         }
     r.absmax[o] = m;
-    if (m == 0.0f) continue;
+    if (m == 0.0f) return;
     int32_t s = 0;
     for (int a = 0; a < kh; ++a)
       for (int b = 0; b < kw; ++b)
@@ -72,7 +97,7 @@ inline I8Weights quantize_weights_i8(const float *w, int oc, int ic, int kh, int
           s += qv;
         }
     r.qsum[o] = s;
-  }
+  });
   return r;
 }
 

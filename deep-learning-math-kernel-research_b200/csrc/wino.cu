@@ -1598,7 +1598,7 @@ inline void weights_tile4(const float (&g)[3][3], float (&u)[4][4]) {
 std::vector<float> transform_weights(const float *w, int oc, int ic, int OCP, int ICP, int A) {
   std::vector<float> u(static_cast<size_t>(A) * A * OCP * ICP, 0.0f);
   const int I2 = ICP / 16;
-  for (int o = 0; o < oc; ++o)
+  host::parallel_for(oc, static_cast<size_t>(oc) * ic * 36, [&](int o) {
     for (int i = 0; i < ic; ++i) {
       float g[3][3], m[6][3], r[6];
       for (int kh = 0; kh < 3; ++kh)
@@ -1619,6 +1619,7 @@ std::vector<float> transform_weights(const float *w, int oc, int ic, int OCP, in
         for (int b = 0; b < 6; ++b) u[(static_cast<size_t>(a * 6 + b) * OCP + o) * ICP + i] = r[b];
       }
     }
+  });
   return u;
 }
 
@@ -1878,11 +1879,12 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
   if (w->direct || w->halo) {
     // U[oc][tap][ic]: K runs over (kh, kw) taps, then the input channels
     u.assign(static_cast<size_t>(w->OCP) * taps * w->ICP, 0.0f);
-    for (int o = 0; o < d.oc; ++o)
+    host::parallel_for(d.oc, u.size(), [&](int o) {
       for (int tap = 0; tap < taps; ++tap)
         for (int i = 0; i < d.ic; ++i)
           u[(static_cast<size_t>(o) * taps + tap) * w->ICP + i] =
               hw[host::w_index(w->ICP / 16, d.kh, d.kw, o, i, tap / d.kw, tap % d.kw)];
+    });
   } else {
     u = transform_weights(hw.data(), d.oc, d.ic, w->OCP, w->ICP, g.A);
   }
@@ -1903,8 +1905,8 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
   if (w->kind == KIND_F32) {
     // [a][nt][ks = channel block][plane][chunk j = 4 channels][BN rows][4 floats]
     float *dst = reinterpret_cast<float *>(img.data());
-    for (int a = 0; a < AA; ++a)
-      for (int nt = 0; nt < w->n_tiles; ++nt)
+    host::parallel_for(AA * w->n_tiles, u.size(), [&](int an) {
+      const int a = an / w->n_tiles, nt = an - a * w->n_tiles;
         for (int ks = 0; ks < KS; ++ks)
           for (int r = 0; r < BN; ++r) {
             const int o = nt * BN + r;
@@ -1926,11 +1928,12 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
               }
             }
           }
+    });
   } else {
     // per (a, oc): abs-max over ic, q = rne((U*127)/absmax), scale = (absmax/127)*tS,
     // shift = -(sum q * scale) * ceil(tz)      (src/elx_conv_wino_trans_weights.cpp:437-535)
     std::vector<float> scale(static_cast<size_t>(AA) * w->OCP, 0.0f), shift(scale.size(), 0.0f);
-    for (int a = 0; a < AA; ++a)
+    host::parallel_for(AA, u.size(), [&](int a) {
       for (int o = 0; o < w->OCP; ++o) {
         const float *src = &u[(static_cast<size_t>(a) * w->OCP + o) * w->ICP];
         float m = 0.0f;
@@ -1957,6 +1960,7 @@ int wino_prepare(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, 
         scale[static_cast<size_t>(a) * w->OCP + o] = sc;
         shift[static_cast<size_t>(a) * w->OCP + o] = zw;
       }
+    });
     W_TRY(cudaMalloc(&w->d_scale, scale.size() * 4));
     W_TRY(cudaMalloc(&w->d_shift, shift.size() * 4));
     W_TRY(cudaMemcpy(w->d_scale, scale.data(), scale.size() * 4, cudaMemcpyHostToDevice));
