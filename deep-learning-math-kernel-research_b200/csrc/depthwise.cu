@@ -21,6 +21,7 @@
 // are floored (round toward minus infinity, no saturation) and packed four at a time with
 // additions that g++ compiles as 64-bit adds over channel pairs, the remaining L % 4 pixels are
 // rounded to nearest even and saturated; s8 outputs are always rounded to nearest and saturated.
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <string>
@@ -29,6 +30,7 @@
 #include "depthwise.cuh"
 #include "elb_common.cuh"
 #include "host_prep.hpp"
+#include "umma.cuh"
 
 namespace elb {
 
@@ -47,6 +49,7 @@ struct DwParams {
   int groups_full;         // floored 4-pixel groups in a full chunk  (T / 4, or 0 without floor mode)
   int floored_row;         // floored groups per output row
   int rest_row;            // nearest-rounded items per output row (chunk remainders, or ceil(OW/4))
+  int rest_pairs;          // the remainders (at most two pixels) of two chunks make one item (dw_fast_kernel)
   int rest_every_chunk;    // floor mode: 1 when full chunks have a remainder (T % 4 != 0)
   int rows_strip;          // output rows per thread
   int strips;              // ceil(OH / rows_strip)
@@ -152,11 +155,6 @@ __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ f32x2 add2_rm(f32x2 a, f32x2 b) {      // round toward minus infinity
-  f32x2 d;
-  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
@@ -169,14 +167,9 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 constexpr uint32_t MAGIC_BITS = 0x4B400000u;      // bit pattern of 1.5 * 2^23
 constexpr float MAGIC = 12582912.0f;              // 1.5 * 2^23: float(MAGIC_BITS + i) == MAGIC + i for |i| < 2^22
 
-// FAST: every value the epilogue can produce is known (from the folded constants) to lie inside
-// (-2^22, 2^22), and either the output is s8 or ReLU with a non-negative lower bound is on.  Then
-// int <-> float conversions can be done exactly on the FMA pipe by adding 1.5 * 2^23 (the
-// accumulators even start at that bit pattern), rounding toward minus infinity is an add with
-// the .rm modifier, and a floored group whose four values all fit a byte is packed with three
-// multiply-adds; a group with a value above 255 (possible only with an overflowing output scale)
-// takes the exact 64-bit path of the general epilogue instead.
-template <int S, bool FAST>
+// The general kernel: accumulator dumps, and plans whose values the fast kernel below cannot take (u8 without ReLU,
+// scales beyond 2^22).
+template <int S>
 __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_constant__ DwParams p) {
   const int quad = threadIdx.x & 3;
   // Blocks are split by rounding rule so that a warp never has to run both epilogues.
@@ -236,7 +229,6 @@ __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_con
   const int oh0 = strip * p.rows_strip;
   const int oh1 = min(p.OH, oh0 + p.rows_strip);
   const bool clamp_hi = p.relu_hi < 3.0e38f;
-  constexpr int ACC0 = FAST ? static_cast<int>(MAGIC_BITS) : 0;
   // rows[k] = input row oh*S - pad_t + k of the current output row
   RowWin<S> rows[3];
   load_row<S>(col, oh0 * S - p.pad_t, p.IH, row_words, rows[0]);
@@ -254,7 +246,7 @@ __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_con
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[k][c] = ACC0;
+      for (int c = 0; c < 4; ++c) acc[k][c] = 0;
 #pragma unroll
     for (int kh = 0; kh < 3; ++kh) mac_row<S>(rows[kh], filt[kh], acc);
 
@@ -265,26 +257,13 @@ __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_con
       for (int k = 0; k < 4; ++k)
         if (k < width)
           *reinterpret_cast<int4 *>(p.acc_dump + (opix + k) * 16 + quad * 4) =
-              make_int4(acc[k][0] - ACC0, acc[k][1] - ACC0, acc[k][2] - ACC0, acc[k][3] - ACC0);
+              make_int4(acc[k][0], acc[k][1], acc[k][2], acc[k][3]);
     }
     float f[4][4];
-    if (FAST) {
-      // channel pairs: (acc - magic) * scale + shift in two packed instructions per pair
-      const f32x2 magic2 = pack2(MAGIC, MAGIC);
-      const f32x2 sc2[2] = {pack2(sc[0], sc[1]), pack2(sc[2], sc[3])}, sh2[2] = {pack2(sh[0], sh[1]), pack2(sh[2], sh[3])};
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+    for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const f32x2 a = sub2(pack2(__int_as_float(acc[k][2 * c]), __int_as_float(acc[k][2 * c + 1])), magic2);
-          unpack2(fma2(a, sc2[c], sh2[c]), f[k][2 * c], f[k][2 * c + 1]);
-        }
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) f[k][c] = __fmaf_rn(__int2float_rn(acc[k][c]), sc[c], sh[c]);
-    }
+      for (int c = 0; c < 4; ++c) f[k][c] = __fmaf_rn(__int2float_rn(acc[k][c]), sc[c], sh[c]);
     if (p.relu) {
 #pragma unroll
       for (int k = 0; k < 4; ++k)
@@ -295,72 +274,31 @@ __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_con
         }
     }
     uint32_t cw[4] = {0u, 0u, 0u, 0u};       // per channel: bytes = pixels 0..3
-    bool packed = false;
-    if (FAST) {
-      if (floored) {
-        uint32_t any = 0u, bits[4][4];
-        const f32x2 magic2 = pack2(MAGIC, MAGIC);
+    if (floored) {
+      // word = u0 + (u1 << 8) + (u2 << 16) + (u3 << 24) with 64-bit adds over channel pairs
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+      for (int e = 0; e < 2; ++e) {
+        unsigned long long sum = 0ull;
 #pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            float b0, b1;
-            unpack2(add2_rm(pack2(f[k][2 * c], f[k][2 * c + 1]), magic2), b0, b1);     // MAGIC_BITS + floor(f)
-            bits[k][2 * c] = __float_as_uint(b0);
-            bits[k][2 * c + 1] = __float_as_uint(b1);
-            any |= bits[k][2 * c] | bits[k][2 * c + 1];
-          }
-        if ((any & 0x003FFF00u) == 0u) {      // all sixteen floored values fit a byte: no carries anywhere
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            cw[c] = bits[0][c] + (bits[1][c] << 8) + (bits[2][c] << 16) + (bits[3][c] << 24) -
-                    MAGIC_BITS * 0x01010101u;
-          packed = true;
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t lo = static_cast<uint32_t>(cvt_x86(floorf(f[k][2 * e]))) << (8 * k);
+          const uint32_t hi = static_cast<uint32_t>(cvt_x86(floorf(f[k][2 * e + 1]))) << (8 * k);
+          sum += static_cast<unsigned long long>(lo) | (static_cast<unsigned long long>(hi) << 32);
         }
-      } else {
+        cw[2 * e] = static_cast<uint32_t>(sum);
+        cw[2 * e + 1] = static_cast<uint32_t>(sum >> 32);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          uint32_t b[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int r = static_cast<int>(__float_as_uint(__fadd_rn(f[k][c], MAGIC)));   // MAGIC_BITS + rne(f)
-            b[k] = static_cast<uint32_t>(p.out_type == OUT_U8
-                                             ? min(r, static_cast<int>(MAGIC_BITS) + 255)
-                                             : max(static_cast<int>(MAGIC_BITS) - 128, min(static_cast<int>(MAGIC_BITS) + 127, r)));
-          }
-          // low bytes of the four words (the low byte of MAGIC_BITS is zero)
-          cw[c] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+          const int r = cvt_x86(rintf(f[k][c]));
+          uint32_t b;
+          if (p.out_type == OUT_U8) b = static_cast<uint32_t>(r) > 255u ? 255u : static_cast<uint32_t>(r);
+          else b = static_cast<uint32_t>(max(-128, min(127, r))) & 0xFFu;
+          cw[c] |= b << (8 * k);
         }
-        packed = true;
-      }
-    }
-    if (!packed) {
-      if (floored) {
-        // word = u0 + (u1 << 8) + (u2 << 16) + (u3 << 24) with 64-bit adds over channel pairs
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          unsigned long long sum = 0ull;
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint32_t lo = static_cast<uint32_t>(cvt_x86(floorf(f[k][2 * e]))) << (8 * k);
-            const uint32_t hi = static_cast<uint32_t>(cvt_x86(floorf(f[k][2 * e + 1]))) << (8 * k);
-            sum += static_cast<unsigned long long>(lo) | (static_cast<unsigned long long>(hi) << 32);
-          }
-          cw[2 * e] = static_cast<uint32_t>(sum);
-          cw[2 * e + 1] = static_cast<uint32_t>(sum >> 32);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int r = cvt_x86(rintf(f[k][c]));
-            uint32_t b;
-            if (p.out_type == OUT_U8) b = static_cast<uint32_t>(r) > 255u ? 255u : static_cast<uint32_t>(r);
-            else b = static_cast<uint32_t>(max(-128, min(127, r))) & 0xFFu;
-            cw[c] |= b << (8 * k);
-          }
-      }
     }
     uint32_t pw[4];
     transpose4(cw, pw);
@@ -375,13 +313,271 @@ __global__ void __launch_bounds__(256, DW_MIN_BLOCKS) dw_kernel(const __grid_con
   }
 }
 
+// Saturating conversions: u8 toward minus infinity (the reference's floored pixels; negative values become 0, which is
+// ReLU), u8 and s8 to nearest even.
+__device__ __forceinline__ uint32_t cvt_floor_u8(float f) {
+  uint32_t r;
+  asm("{\n\t.reg .u8 b;\n\tcvt.rmi.u8.f32 b, %1;\n\tcvt.u32.u8 %0, b;\n\t}" : "=r"(r) : "f"(f));
+  return r;
+}
+__device__ __forceinline__ uint32_t cvt_near_u8(float f) {
+  uint32_t r;
+  asm("{\n\t.reg .u8 b;\n\tcvt.rni.u8.f32 b, %1;\n\tcvt.u32.u8 %0, b;\n\t}" : "=r"(r) : "f"(f));
+  return r;
+}
+__device__ __forceinline__ uint32_t cvt_near_s8(float f) {
+  int r;
+  asm("{\n\t.reg .s8 b;\n\tcvt.rni.s8.f32 b, %1;\n\tcvt.s32.s8 %0, b;\n\t}" : "=r"(r) : "f"(f));
+  return static_cast<uint32_t>(r);
+}
+
+// The kernel of plans whose epilogue values are provably inside (-2^22, 2^22) (DwImpl::fast) and whose u8 outputs are
+// ReLU'd.  Bound by instruction issue at few warps (registers): 64 images of 128 channels 56x56 take 26 % fewer
+// instructions than before and 57 % of the issue slots are used (43 % when rows were loaded straight into registers,
+// the rest waited for them).  What it does for that:
+//   * the accumulators start at the bit pattern of 1.5 * 2^23 and convert to float by one subtraction, two at a time;
+//   * a row's four pixels are converted by one saturating conversion per value (on the conversion unit, 30 % busy) and
+//     packed pixel by pixel: nothing is transposed back.  Only a floored group with a value of 256 or more (an
+//     overflowing output scale) takes the reference's packing with carries;
+//   * the input rows come through a small ring in shared memory, two rows ahead (four: 25.5 us instead of 24.6 from a
+//     cold L2), and the window of three rows rotates by unrolling instead of moving registers;
+//   * the nearest-rounded remainders of two chunks, at most two pixels each, share a thread.
+// Measured: 30.9 -> 24.6 us (that case, L2 cold), 14.3 -> 12.2 (100 x 512 x 14x14), 15.7 -> 14.8 (stride 2, 8 x 64 x
+// 223x211), 4.7 -> 3.3 (1 x 1024 x 7x7).
+constexpr int DW_DEPTH = 2;
+template <int S, bool OUT8S>
+__global__ void __launch_bounds__(128, 4) dw_fast_kernel(const __grid_constant__ DwParams p) {
+  const int quad = threadIdx.x & 3;
+  const bool floored = static_cast<long long>(blockIdx.x) < p.blocks_floored;
+  const int per_row = floored ? p.floored_row : p.rest_row;
+  const unsigned per_plane = static_cast<unsigned>(p.strips) * per_row;
+  const unsigned lin = (floored ? blockIdx.x : blockIdx.x - static_cast<unsigned>(p.blocks_floored)) * 32u + (threadIdx.x >> 2);
+  if (lin >= per_plane * static_cast<unsigned>(p.N * p.CB)) return;
+  const int plane_idx = static_cast<int>(lin / per_plane);
+  const int rem = static_cast<int>(lin - plane_idx * per_plane);
+  const int strip = rem / per_row;
+  const int item = rem - strip * per_row;
+  // two pairs of output pixels: xa, xa + 1 and xb, xb + 1; wa / wb of them are real
+  int xa, xb, wa, wb;
+  if (floored) {
+    const int chunk = min(item / p.groups_full, p.chunks - 1);        // the last chunk may hold fewer groups
+    xa = chunk * p.T + 4 * (item - chunk * p.groups_full);
+    xb = xa + 2; wa = wb = 2;
+  } else if (p.floor_mode) {
+    auto left = [&](int c) { return c < p.chunks ? min(p.T, p.OW - c * p.T) & 3 : 0; };
+    auto start = [&](int c) { return c * p.T + (min(p.T, p.OW - c * p.T) & ~3); };
+    if (p.rest_pairs) {
+      const int c = p.rest_every_chunk ? 2 * item : p.chunks - 1;
+      xa = start(c); wa = left(c);
+      const bool two = p.rest_every_chunk && c + 1 < p.chunks;
+      wb = two ? left(c + 1) : 0;
+      xb = wb ? start(c + 1) : xa;
+    } else {
+      const int c = p.rest_every_chunk ? item : p.chunks - 1;
+      xa = start(c); xb = xa + 2;
+      wa = min(left(c), 2); wb = left(c) - wa;
+    }
+  } else {
+    xa = 4 * item; xb = xa + 2;
+    wa = min(2, p.OW - xa); wb = max(0, min(2, p.OW - xb));
+  }
+  const int ch0 = (plane_idx % p.CB) * 16 + quad * 4;
+
+  uint32_t f0[3][4];
+  f32x2 sc2[2], sh2[2];
+  {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int kh = 0; kh < 3; ++kh) f0[kh][c] = __ldg(p.wq + (ch0 + c) * 3 + kh);
+    const float4 sc = __ldg(reinterpret_cast<const float4 *>(p.scale + ch0)), sh = __ldg(reinterpret_cast<const float4 *>(p.shift + ch0));
+    sc2[0] = pack2(sc.x, sc.y); sc2[1] = pack2(sc.z, sc.w);
+    sh2[0] = pack2(sh.x, sh.y); sh2[1] = pack2(sh.z, sh.w);
+  }
+  const uint32_t *plane = reinterpret_cast<const uint32_t *>(p.in + static_cast<size_t>(plane_idx) * p.IH * p.IW * 16) + quad;
+  // columns base + k of a window; bit k: inside the image
+  constexpr int NPIX = S == 1 ? 6 : 9;
+  const int base_a = xa * S - p.pad_l, base_b = xb * S - p.pad_l;
+  uint32_t in_a = 0, in_b = 0;
+#pragma unroll
+  for (int k = 0; k < NPIX; ++k) {
+    in_a |= (base_a + k >= 0 && base_a + k < p.IW ? 1u : 0u) << k;
+    if (k < 4) in_b |= (base_b + k >= 0 && base_b + k < p.IW ? 1u : 0u) << k;
+  }
+  const bool joined = S == 2 || xb == xa + 2;      // window b follows window a: its first columns are a's last
+  const long long off_a = static_cast<long long>(base_a) * 4, off_b = static_cast<long long>(base_b) * 4;
+  const int row_words = p.IW * 4;
+  const int oh0 = strip * p.rows_strip, oh1 = min(p.OH, oh0 + p.rows_strip);
+
+  // Input rows travel through a ring of DW_DEPTH rows in shared memory, private to the thread (no barrier): asynchronous
+  // copies keep that many rows in flight without a register.  Words outside the image stay the zeros written here.
+  constexpr int NW = S == 1 ? 8 : 9;               // words 6 and 7 at stride 1: the first two columns of a window b of its own
+  __shared__ uint32_t ring[DW_DEPTH][NW][128];
+#pragma unroll
+  for (int d = 0; d < DW_DEPTH; ++d)
+#pragma unroll
+    for (int k = 0; k < NW; ++k) ring[d][k][threadIdx.x] = 0u;
+  const int last_ih = (oh1 - 1) * S - p.pad_t + 2;
+  int next_ih = oh0 * S - p.pad_t, put = 0, take = 0;
+  const uint32_t *src_a = plane + static_cast<long long>(next_ih) * row_words + off_a;
+  const long long b_from_a = off_b - off_a;
+  const uint32_t ring0 = smem_u32(&ring[0][0][threadIdx.x]);
+  auto copy = [](uint32_t dst, const uint32_t *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+  };
+  auto load = [&]() {                              // the next input row, if one is left; always one group
+    const uint32_t dst = ring0 + put * (NW * 512);
+    if (next_ih <= last_ih) {
+      if (next_ih >= 0 && next_ih < p.IH) {
+        if (S == 2 || joined) {
+#pragma unroll
+          for (int k = 0; k < NPIX; ++k)
+            if ((in_a >> k) & 1u) copy(dst + k * 512, src_a + 4 * k);
+        } else {
+          const uint32_t *src_b = src_a + b_from_a;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if ((in_a >> k) & 1u) copy(dst + k * 512, src_a + 4 * k);
+            if ((in_b >> k) & 1u) copy(dst + (k < 2 ? 6 + k : 2 + k) * 512, src_b + 4 * k);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NW; ++k) ring[put][k][threadIdx.x] = 0u;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ++next_ih;
+    src_a += row_words;
+    put = (put + 1) & (DW_DEPTH - 1);
+  };
+  auto window = [&](RowWin<S> &w) {                // the oldest row of the ring; its place takes the next one
+    asm volatile("cp.async.wait_group %0;" ::"n"(DW_DEPTH - 1) : "memory");
+    uint32_t px[NPIX];
+#pragma unroll
+    for (int k = 0; k < NPIX; ++k) px[k] = ring[take][k][threadIdx.x];
+    if constexpr (S == 1) {
+      uint32_t b0 = px[2], b1 = px[3];
+      if (!joined) { b0 = ring[take][6][threadIdx.x]; b1 = ring[take][7][threadIdx.x]; }
+      const uint32_t wa4[4] = {px[0], px[1], px[2], px[3]}, wb4[4] = {b0, b1, px[4], px[5]};
+      transpose4(wa4, w.a);
+      transpose4(wb4, w.b);
+    } else {
+      const uint32_t wa4[4] = {px[0], px[1], px[2], px[3]}, wb4[4] = {px[4], px[5], px[6], px[7]};
+      transpose4(wa4, w.a);
+      transpose4(wb4, w.b);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) w.c[c] = (px[NPIX - 1] >> (8 * c)) & 0xFFu;
+    }
+    take = (take + 1) & (DW_DEPTH - 1);
+    load();
+  };
+  const bool clamp = p.relu && (OUT8S || p.relu_lo > 0.0f || p.relu_hi < 3.0e38f);      // (else the conversion is the ReLU)
+  uint32_t *dst_a = reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(p.out) + ((static_cast<size_t>(plane_idx) * p.OH + oh0) * p.OW + xa) * 16) + quad;
+  const int to_b = (xb - xa) * 4;
+  auto row = [&](const RowWin<S> &w0, const RowWin<S> &w1, const RowWin<S> &w2) {
+    int acc[4][4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[k][c] = static_cast<int>(MAGIC_BITS);
+#pragma unroll
+    for (int kh = 0; kh < 3; ++kh) {
+      FilterRow f;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        f.f0[c] = f0[kh][c];
+        f.f1[c] = S == 1 ? f0[kh][c] << 8 : f0[kh][c] << 16;
+        f.f2[c] = (f0[kh][c] >> 16) & 0xFFu;
+      }
+      mac_row<S>(kh == 0 ? w0 : kh == 1 ? w1 : w2, f, acc);
+    }
+    float f[4][4];
+    const f32x2 magic2 = pack2(MAGIC, MAGIC);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const f32x2 a = sub2(pack2(__int_as_float(acc[k][2 * c]), __int_as_float(acc[k][2 * c + 1])), magic2);
+        unpack2(fma2(a, sc2[c], sh2[c]), f[k][2 * c], f[k][2 * c + 1]);
+      }
+    if (clamp) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) f[k][c] = fminf(fmaxf(f[k][c], p.relu_lo), p.relu_hi);
+    }
+    uint32_t pw[4];
+    bool done = false;
+    if (!OUT8S && floored) {
+      float top = f[0][0];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) top = fmaxf(top, f[k][c]);
+      if (top >= 256.0f) {
+        // word = u0 + (u1 << 8) + (u2 << 16) + (u3 << 24) with 64-bit adds over channel pairs
+        uint32_t cw[4];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          unsigned long long sum = 0ull;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint32_t lo = static_cast<uint32_t>(cvt_x86(floorf(fmaxf(f[k][2 * e], 0.0f)))) << (8 * k);
+            const uint32_t hi = static_cast<uint32_t>(cvt_x86(floorf(fmaxf(f[k][2 * e + 1], 0.0f)))) << (8 * k);
+            sum += static_cast<unsigned long long>(lo) | (static_cast<unsigned long long>(hi) << 32);
+          }
+          cw[2 * e] = static_cast<uint32_t>(sum);
+          cw[2 * e + 1] = static_cast<uint32_t>(sum >> 32);
+        }
+        transpose4(cw, pw);
+        done = true;
+      }
+    }
+    if (!done) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t b[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) b[c] = OUT8S ? cvt_near_s8(f[k][c]) : floored ? cvt_floor_u8(f[k][c]) : cvt_near_u8(f[k][c]);
+        pw[k] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+      }
+    }
+    if (wa > 0) dst_a[0] = pw[0];
+    if (wa > 1) dst_a[4] = pw[1];
+    if (wb > 0) dst_a[to_b] = pw[2];
+    if (wb > 1) dst_a[to_b + 4] = pw[3];
+    dst_a += p.OW * 4;
+  };
+
+  RowWin<S> w[3];
+#pragma unroll
+  for (int d = 0; d < DW_DEPTH; ++d) load();
+  window(w[0]);
+  if constexpr (S == 1) window(w[1]);
+  for (int oh = oh0; oh < oh1;) {
+#pragma unroll
+    for (int u = 0; u < 3; ++u) {                  // (the rows' registers take turns instead of moving)
+      if constexpr (S == 1) {
+        window(w[(u + 2) % 3]);
+        row(w[u], w[(u + 1) % 3], w[(u + 2) % 3]);
+      } else {
+        window(w[(2 * u + 1) % 3]);
+        window(w[(2 * u + 2) % 3]);
+        row(w[(2 * u) % 3], w[(2 * u + 1) % 3], w[(2 * u + 2) % 3]);
+      }
+      if (++oh >= oh1) break;
+    }
+  }
+}
+
 }  // namespace
 
 struct DwImpl {
   DwParams p{};
-  int stride = 1;
+  int stride = 1, num_sms = 148;
   int G = 0;
-  bool fast = false;       // epilogue values provably inside (-2^22, 2^22), see dw_kernel
+  bool fast = false;       // epilogue values provably inside (-2^22, 2^22), see dw_fast_kernel
   void *d_wq = nullptr, *d_scale = nullptr, *d_shift = nullptr;
 };
 
@@ -410,6 +606,7 @@ int dw_setup(DwPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, int nu
   pl.impl = w;
   w->stride = d.stride_h;
   w->G = host::alignup(d.g, V);
+  w->num_sms = num_sms;
   DwParams &p = w->p;
   p.N = d.n; p.CB = w->G / V; p.IH = d.ih; p.IW = d.iw; p.OH = d.oh; p.OW = d.ow;
   p.pad_t = d.pad_t; p.pad_l = d.pad_l;
@@ -523,17 +720,43 @@ int dw_run(DwPlan &pl, void *out, const void *in, void *acc_dump, int first, int
   p.out = static_cast<uint8_t *>(out) + first * out_img;
   p.acc_dump = acc_dump ? static_cast<int32_t *>(acc_dump) + first * out_img : nullptr;
   p.N = count;
+  if (w->fast && !p.acc_dump) {
+    const int last = p.OW - (p.chunks - 1) * p.T;
+    p.rest_pairs = w->stride == 1 && p.floor_mode && (p.T & 3) <= 2 && (last & 3) <= 2;
+    if (p.rest_pairs && p.rest_every_chunk) p.rest_row = (p.chunks + 1) / 2;
+    // Rows per thread: whole waves of four resident blocks per SM; a strip's start and its first rows cost about 1.3
+    // (stride 2: 1) rows of work.
+    const long long planes = static_cast<long long>(count) * p.CB, slots = 4ll * w->num_sms;
+    double best = 0;
+    for (int rs = std::min(2, p.OH); rs <= 14 && rs <= p.OH; ++rs) {
+      const int strips = (p.OH + rs - 1) / rs;
+      const long long blocks = (planes * strips * p.floored_row + 31) / 32 + (planes * strips * p.rest_row + 31) / 32;
+      const double t = static_cast<double>((blocks + slots - 1) / slots) * (rs + (w->stride == 1 ? 1.3 : 1.0));
+      if (best == 0 || t < best * 0.99) { best = t; p.rows_strip = rs; p.strips = strips; }
+    }
+    p.blocks_floored = (static_cast<long long>(count) * p.CB * p.strips * p.floored_row + 31) / 32;
+    const long long rest = (static_cast<long long>(count) * p.CB * p.strips * p.rest_row + 31) / 32;
+    if ((p.blocks_floored + rest) * 32 > 0x7FFFFFFFll) { err = "depthwise: problem too large for one launch"; return ELB_UNIMPLEMENTED; }
+    const dim3 g(static_cast<unsigned>(p.blocks_floored + rest));
+    const bool s8 = p.out_type == OUT_S8;
+    if (w->stride == 1) {
+      if (s8) dw_fast_kernel<1, true><<<g, 128, 0, s>>>(p);
+      else dw_fast_kernel<1, false><<<g, 128, 0, s>>>(p);
+    } else {
+      if (s8) dw_fast_kernel<2, true><<<g, 128, 0, s>>>(p);
+      else dw_fast_kernel<2, false><<<g, 128, 0, s>>>(p);
+    }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) { err = std::string("depthwise launch failed: ") + cudaGetErrorString(e); return ELB_GENERAL_ERROR; }
+    launches = 1;
+    return ELB_OK;
+  }
   p.blocks_floored = (static_cast<long long>(count) * p.CB * p.strips * p.floored_row + 63) / 64;
   const long long blocks_rest = (static_cast<long long>(p.N) * p.CB * p.strips * p.rest_row + 63) / 64;
   if ((p.blocks_floored + blocks_rest) * 64 > 0x7FFFFFFFll) { err = "depthwise: problem too large for one launch"; return ELB_UNIMPLEMENTED; }
   dim3 grid(static_cast<unsigned>(p.blocks_floored + blocks_rest));
-  if (w->stride == 1) {
-    if (w->fast) dw_kernel<1, true><<<grid, 256, 0, s>>>(p);
-    else dw_kernel<1, false><<<grid, 256, 0, s>>>(p);
-  } else {
-    if (w->fast) dw_kernel<2, true><<<grid, 256, 0, s>>>(p);
-    else dw_kernel<2, false><<<grid, 256, 0, s>>>(p);
-  }
+  if (w->stride == 1) dw_kernel<1><<<grid, 256, 0, s>>>(p);
+  else dw_kernel<2><<<grid, 256, 0, s>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) { err = std::string("depthwise launch failed: ") + cudaGetErrorString(e); return ELB_GENERAL_ERROR; }
   launches = 1;

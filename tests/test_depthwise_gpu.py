@@ -58,6 +58,32 @@ def test_depthwise_bit_exact(pkg, case):
         d.close()
 
 
+# Without an accumulator dump the layers run on the kernel whose epilogue works on the FMA pipe (stride 1 and 2): strips
+# of 2 and more rows, pairs of chunk remainders (T % 4 and the last chunk's up to 2, with even and odd chunk counts, or 3),
+# groups with values above 255, both signs of the output, images narrower than a window.
+FAST_CASES = CASES + [
+    _dw("dw_fast_pairs_odd", 2, 32, 30, 42, 14),
+    _dw("dw_fast_pairs_last_only", 1, 48, 9, 30, 8),
+    _dw("dw_fast_rest3", 1, 32, 11, 21, 7),
+    _dw("dw_fast_narrow", 2, 32, 5, 3, 0),
+    _dw("dw_fast_s2_s8", 2, 48, 31, 33, 5, stride=2, types="u8f32s8f32"),
+    _dw("dw_fast_s2_rows", 8, 64, 57, 40, 20, stride=2),
+    _dw("dw_fast_many", 8, 256, 14, 14, 0),
+]
+
+
+@pytest.mark.parametrize("case", FAST_CASES, ids=lambda c: c.name)
+def test_depthwise_without_dump(pkg, case):
+    import gpuutil as G
+    t = R.make_tensors(case)
+    want = R.oracle_int8_depthwise(case, t)
+    got, d = G.run_gpu(case, t)
+    d.close()
+    cb = case.oc // 16
+    bad = int((got[:, :cb] != want[:, :cb]).sum())
+    assert bad == 0, f"{bad} of {want[:, :cb].size} output bytes differ"
+
+
 def test_depthwise_host_buffers_and_repeat(pkg):
     """The drop-in call with host memory, twice (weights are only read on the first call)."""
     import gpuutil as G
