@@ -332,8 +332,8 @@ __device__ __forceinline__ uint32_t cvt_near_s8(float f) {
 }
 
 // The kernel of plans whose epilogue values are provably inside (-2^22, 2^22) (DwImpl::fast) and whose u8 outputs are
-// ReLU'd.  Bound by instruction issue at few warps (registers): 64 images of 128 channels 56x56 take 26 % fewer
-// instructions than before and 57 % of the issue slots are used (43 % when rows were loaded straight into registers,
+// ReLU'd.  Bound by instruction issue at few warps (registers): 64 images of 128 channels 56x56 take 44 % fewer
+// instructions than before and 58 % of the issue slots are used (40 % when rows were loaded straight into registers,
 // the rest waited for them).  What it does for that:
 //   * the accumulators start at the bit pattern of 1.5 * 2^23 and convert to float by one subtraction, two at a time;
 //   * a row's four pixels are converted by one saturating conversion per value (on the conversion unit, 30 % busy) and
@@ -342,11 +342,12 @@ __device__ __forceinline__ uint32_t cvt_near_s8(float f) {
 //   * the input rows come through a small ring in shared memory, two rows ahead (four: 25.5 us instead of 24.6 from a
 //     cold L2), and the window of three rows rotates by unrolling instead of moving registers;
 //   * the nearest-rounded remainders of two chunks, at most two pixels each, share a thread.
-// Measured: 30.9 -> 24.6 us (that case, L2 cold), 14.3 -> 12.2 (100 x 512 x 14x14), 15.7 -> 14.8 (stride 2, 8 x 64 x
-// 223x211), 4.7 -> 3.3 (1 x 1024 x 7x7).
+// Measured: 31.6 -> 22.4 us (that case, L2 cold; 2.5 us of it from starting under the kernel before), 14.3 -> 12.2 (100 x 512 x
+// 14x14), 15.7 -> 14.8 (stride 2, 8 x 64 x 223x211), 4.7 -> 2.5 (1 x 1024 x 7x7).
 constexpr int DW_DEPTH = 2;
 template <int S, bool OUT8S>
 __global__ void __launch_bounds__(128, 4) dw_fast_kernel(const __grid_constant__ DwParams p) {
+  griddep_launch_dependents();
   const int quad = threadIdx.x & 3;
   const bool floored = static_cast<long long>(blockIdx.x) < p.blocks_floored;
   const int per_row = floored ? p.floored_row : p.rest_row;
@@ -551,6 +552,7 @@ __global__ void __launch_bounds__(128, 4) dw_fast_kernel(const __grid_constant__
   };
 
   RowWin<S> w[3];
+  griddep_wait();                                  // (everything above read constants of the plan)
 #pragma unroll
   for (int d = 0; d < DW_DEPTH; ++d) load();
   window(w[0]);
@@ -739,14 +741,9 @@ int dw_run(DwPlan &pl, void *out, const void *in, void *acc_dump, int first, int
     if ((p.blocks_floored + rest) * 32 > 0x7FFFFFFFll) { err = "depthwise: problem too large for one launch"; return ELB_UNIMPLEMENTED; }
     const dim3 g(static_cast<unsigned>(p.blocks_floored + rest));
     const bool s8 = p.out_type == OUT_S8;
-    if (w->stride == 1) {
-      if (s8) dw_fast_kernel<1, true><<<g, 128, 0, s>>>(p);
-      else dw_fast_kernel<1, false><<<g, 128, 0, s>>>(p);
-    } else {
-      if (s8) dw_fast_kernel<2, true><<<g, 128, 0, s>>>(p);
-      else dw_fast_kernel<2, false><<<g, 128, 0, s>>>(p);
-    }
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_overlapped(w->stride == 1 ? s8 ? dw_fast_kernel<1, true> : dw_fast_kernel<1, false>
+                                                           : s8 ? dw_fast_kernel<2, true> : dw_fast_kernel<2, false>,
+                                            g, dim3(128), 0, s, p);
     if (e != cudaSuccess) { err = std::string("depthwise launch failed: ") + cudaGetErrorString(e); return ELB_GENERAL_ERROR; }
     launches = 1;
     return ELB_OK;

@@ -33,9 +33,9 @@ __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("grid
 
 // Launch a kernel that may overlap its set-up with the tail of the kernel before it in the stream
 // (the kernel must contain griddep_wait).  Captured into a CUDA graph the
-// dependency becomes a programmatic edge.  Only the INT8 tensor-core kernels are launched this way:
+// dependency becomes a programmatic edge.  The INT8 tensor-core kernels are launched this way:
 // their set-up (barriers, tensor memory, per-channel constants, the copy table) is 2-3 us of a launch
-// that may last 10 us.  Measured on the fp32 Winograd path: overlapped launches of the GEMM and the
+// that may last 10 us; the depthwise kernel too (index arithmetic, weights, an empty ring).  Measured on the fp32 Winograd path: overlapped launches of the GEMM and the
 // input transform change nothing, and the output transform launched as an early dependent is SLOWER
 // (c1 0.506 -> 0.550 ms, with all three 0.592 ms; the fp32 stack 24.2 -> 28.5 ms), so those stay plain.
 template <typename... KArgs, typename... Args>
