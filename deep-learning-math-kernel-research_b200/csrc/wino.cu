@@ -622,10 +622,11 @@ struct WinoGemmParams {
 // loops are single threads bound by instruction latency -- as a run-time loop count the same code
 // measured 10-20 % slower at kmul = 1.
 // SPEC: 0 = every mode decided at run time from the parameters; 1 / 2 = fp32 with A in tensor memory
-// and stacked / plain weight rows, 3 = int8; none of them flat: the modes of the long launches,
+// and stacked / plain weight rows, 3 = int8, 4 / 5 = 1 / 2 in flat mode: the modes of the long launches,
 // compiled with their flags as constants (every instruction the one-thread role loops do not
 // execute is ~6 cycles; measured against the generic kernel on the same GPU: c1 GEMM 0.333 -> 0.265
-// ms, VGG conv1_2 0.45 -> 0.35 ms, conv4_2 0.19 -> 0.14 ms).
+// ms, VGG conv1_2 0.45 -> 0.35 ms, conv4_2 0.19 -> 0.14 ms; flat: 64 x 1024 -> 256 at 14x14 69 -> 40 us,
+// with two K stages per step 64 x 560 -> 96 at 14x14 26 -> 20 us, 125 x 512 -> 59 at 19x19 61 -> 43 us).
 // TBN: the tile's output channels as a constant (0 = p.BN): descriptors, ring geometry and the
 // epilogue's block loop then fold at compile time.
 template <bool CTA2, int KMUL = 1, int SPEC = 0, int TBN = 0>
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int BN = TBN != 0 ? TBN : p.BN;
   const int kind = SPEC == 3 ? static_cast<int>(KIND_I8) : SPEC != 0 ? static_cast<int>(KIND_F32) : p.kind;
-  const bool flat = SPEC != 0 ? false : p.flat != 0;
+  const bool flat = SPEC >= 4 ? true : SPEC != 0 ? false : p.flat != 0;
   const bool tracing = SPEC != 0 ? false : p.trace != nullptr;      // (timelines are taken from the generic kernel)
   const uint32_t rank = CTA2 ? cluster_ctarank() : 0u;
   const bool leader = rank == 0;
@@ -668,7 +669,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
   const bool a_in_tmem = SPEC == 3 ? false : SPEC != 0 ? true : (!CTA2 && kind == KIND_F32 && p.a_tmem != 0);
   // Stacked weights (see WinoGemmParams::stack): the accumulator is 2*BN columns wide, columns
   // [BN, 2*BN) collect hi*lo and are added to [0, BN) by the epilogue.
-  const bool stack = SPEC == 1 ? true : SPEC != 0 ? false : (!CTA2 && kind == KIND_F32 && p.stack != 0);
+  const bool stack = SPEC == 1 || SPEC == 4 ? true : SPEC != 0 ? false : (!CTA2 && kind == KIND_F32 && p.stack != 0);
   const int acc_width = stack ? 2 * BN : BN;
   // Accumulator buffers: two (the epilogue of a tile overlaps the next tile's MMAs) unless the A
   // slots in tensor memory leave room for one only: columns [0,256) hold the accumulators (two of at
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
   // deeper ring: 4 stages at BN = 256 (5 with A in tensor memory), 6 at 128, up to 8 below.
   // (Measured: the extra depth changes nothing on the 64- and 128-channel VGG layers, whose stages
   // land about 1400 cycles apart however many are in flight.)
-  constexpr int kmul = KMUL;                      // (KMUL > 1 is launched only with A in tensor memory, not in flat mode)
+  constexpr int kmul = KMUL;                      // (KMUL > 1 is launched only with A in tensor memory)
   const int ksteps = p.k_stages / kmul;           // pipeline steps per tile
   const int stage_bytes = a_in_tmem ? kmul * (A_RAW_BYTES + 128 * BN) : CTA2 ? STAGE_BYTES : A_STAGE_BYTES + 128 * BN;
   const int b_off = a_in_tmem ? kmul * A_RAW_BYTES : A_STAGE_BYTES;
@@ -740,8 +741,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
     };
     bool ok = pw < np;
     if (flat) {
-      // flat mode: lanes 0..3 fetch the four 16-byte channel chunks of a stage (boxes of 4 floats x
-      // 128 pixels, rows past the end of the plane arrive as zeros), lane 4 the weights
+      // flat mode: four lanes per K stage fetch its 16-byte channel chunks (boxes of 4 floats x 128 pixels, rows
+      // past the end of the plane arrive as zeros), one more lane the weights of the step
       if (lane == 0) tma_prefetch_desc(&p.tmap_a);
       for (int tile = first; tile < total_tiles && ok; tile += step) {
         const int nt = tile / p.m_tiles, mt = tile - nt * p.m_tiles;
@@ -749,18 +750,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
         const uint8_t *b_src = p.b_img + static_cast<size_t>(nt) * p.k_stages * b_stage_bytes;
         // CTAs that run side by side multiply by the same weights: each tile may start its K loop at a
         // different stage so that they do not all ask the same L2 lines at the same moment
-        const int rot = p.rotate_k ? tile % p.k_stages : 0;
-        for (int ks = 0; ks < p.k_stages; ++ks, next_stage()) {
+        const int rot = (SPEC == 0 && p.rotate_k) ? tile % ksteps : 0;
+        for (int ks = 0; ks < ksteps; ++ks, next_stage()) {
           if (turn != pw) continue;
-          const int ksr = ks + rot < p.k_stages ? ks + rot : ks + rot - p.k_stages;     // rotated K stage
+          const int ksr = ks + rot < ksteps ? ks + rot : ks + rot - ksteps;     // rotated step
           int w_ok = 1;
           if (lane == 0) w_ok = mbar_wait(&empty[s], ph ^ 1u, abort_flag) ? 1 : 0;
           if (!__all_sync(0xFFFFFFFFu, w_ok)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
           uint8_t *stage = smem + s * stage_bytes;
-          if (lane == 0) mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(A_RAW_BYTES) + b_stage_bytes);
+          if (lane == 0) mbar_arrive_expect_tx(&full[s], kmul * (static_cast<uint32_t>(A_RAW_BYTES) + b_stage_bytes));
           __syncwarp();
-          if (lane < 4) tma_tile_3d(stage + lane * 2048, &p.tmap_a, 4 * lane, ptile * BM, n * p.CB + ksr, &full[s]);
-          else if (lane == 4) tma_bulk_g2s(stage + b_off, b_src + static_cast<size_t>(ksr) * b_stage_bytes, b_stage_bytes, &full[s]);
+          if (lane < 4 * kmul) tma_tile_3d(stage + lane * 2048, &p.tmap_a, 4 * (lane & 3), ptile * BM, n * p.CB + ksr * kmul + (lane >> 2), &full[s]);
+          else if (lane == 4 * kmul) tma_bulk_g2s(stage + b_off, b_src + static_cast<size_t>(ksr) * b_stage_bytes * kmul, b_stage_bytes * kmul, &full[s]);
           __syncwarp();
         }
       }
@@ -1265,16 +1266,32 @@ inline cudaError_t gemm_set_attributes() {
   set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 2, 1, 128>));
   set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 1, 2, 256>));
   set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 1, 3, 256>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 1, 4>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 2, 4>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 2, 4, 64>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 2, 4, 128>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 1, 5>));
+  set(reinterpret_cast<const void *>(wino_gemm_kernel<false, 1, 5, 256>));
   return e;
 }
 inline void gemm_launch(const WinoGemmParams &gp, int ctas, cudaStream_t s) {
-  // specialised kernels: fp32, A in tensor memory, not flat, no timeline requested
-  const bool plain = !gp.flat && !gp.trace && !gp.ablate && !gp.rotate_k && gp.producers == GEMM_PRODUCERS_DEFAULT;
+  // specialised kernels: fp32, A in tensor memory, no timeline requested
+  const bool plain = !gp.trace && !gp.ablate && !gp.rotate_k && gp.producers == GEMM_PRODUCERS_DEFAULT;
   if (plain && gp.kind == KIND_I8 && gp.BN == 256 && !gp.acc_dump) {
     wino_gemm_kernel<false, 1, 3, 256><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     return;
   }
-  const int spec = (plain && gp.kind == KIND_F32 && gp.a_tmem) ? (gp.stack ? 1 : 2) : 0;
+  const int spec = (plain && gp.kind == KIND_F32 && gp.a_tmem) ? (gp.stack ? 1 : 2) + (gp.flat ? 3 : 0) : 0;
+  if (spec >= 4) {
+    if (spec == 4 && gp.kmul == 2 && gp.BN == 64) wino_gemm_kernel<false, 2, 4, 64><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else if (spec == 4 && gp.kmul == 2 && gp.BN == 128) wino_gemm_kernel<false, 2, 4, 128><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else if (spec == 4 && gp.kmul == 2) wino_gemm_kernel<false, 2, 4><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else if (spec == 4) wino_gemm_kernel<false, 1, 4><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else if (gp.kmul == 2) wino_gemm_kernel<false, 2, 0><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else if (gp.BN == 256) wino_gemm_kernel<false, 1, 5, 256><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    else wino_gemm_kernel<false, 1, 5><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
+    return;
+  }
   if (gp.kmul == 2) {
     if (spec == 1 && gp.BN == 64) wino_gemm_kernel<false, 2, 1, 64><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else if (spec == 1 && gp.BN == 128) wino_gemm_kernel<false, 2, 1, 128><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
@@ -2058,7 +2075,7 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     gp.stack = w->stack ? 1 : 0;
     gp.a_tmem = tune_a_tmem(KIND_F32, gp.k_stages, static_cast<long long>(gp.m_tiles) * gp.n_tiles, num_sms,
                             w->stack ? 2 * w->BN : w->BN, true);
-    gp.kmul = 1;
+    gp.kmul = tune_kmul(KIND_F32, gp.a_tmem, gp.k_stages, w->BN);
     gp.bias = static_cast<const float *>(w->d_bias);
     gp.out = static_cast<float *>(out) + static_cast<size_t>(first) * (w->out_img_bytes / 4);
     gp.with_bias = w->with_bias; gp.with_relu = w->with_relu; gp.with_sum = w->with_sum;
