@@ -682,7 +682,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
   // (Measured: the extra depth changes nothing on the 64- and 128-channel VGG layers, whose stages
   // land about 1400 cycles apart however many are in flight.)
   constexpr int kmul = KMUL;                      // (KMUL > 1 is launched only with A in tensor memory)
-  const int ksteps = p.k_stages / kmul;           // pipeline steps per tile
+  // pipeline steps per tile; in flat mode the last one may hold a single K stage
+  const int ksteps = kmul == 1 ? p.k_stages : flat ? (p.k_stages + kmul - 1) / kmul : p.k_stages / kmul;
+  const bool half_last = kmul > 1 && flat && (p.k_stages & 1) != 0;
   const int stage_bytes = a_in_tmem ? kmul * (A_RAW_BYTES + 128 * BN) : CTA2 ? STAGE_BYTES : A_STAGE_BYTES + 128 * BN;
   const int b_off = a_in_tmem ? kmul * A_RAW_BYTES : A_STAGE_BYTES;
   // the ring may also use the area of the int8 epilogue constants when the kernel runs fp32
@@ -758,10 +760,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
           if (lane == 0) w_ok = mbar_wait(&empty[s], ph ^ 1u, abort_flag) ? 1 : 0;
           if (!__all_sync(0xFFFFFFFFu, w_ok)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; break; }
           uint8_t *stage = smem + s * stage_bytes;
-          if (lane == 0) mbar_arrive_expect_tx(&full[s], kmul * (static_cast<uint32_t>(A_RAW_BYTES) + b_stage_bytes));
+          const int parts = half_last && ksr + 1 == ksteps ? 1 : kmul;
+          if (lane == 0) mbar_arrive_expect_tx(&full[s], parts * (static_cast<uint32_t>(A_RAW_BYTES) + b_stage_bytes));
           __syncwarp();
-          if (lane < 4 * kmul) tma_tile_3d(stage + lane * 2048, &p.tmap_a, 4 * (lane & 3), ptile * BM, n * p.CB + ksr * kmul + (lane >> 2), &full[s]);
-          else if (lane == 4 * kmul) tma_bulk_g2s(stage + b_off, b_src + static_cast<size_t>(ksr) * b_stage_bytes * kmul, b_stage_bytes * kmul, &full[s]);
+          if (lane < 4 * parts) tma_tile_3d(stage + lane * 2048, &p.tmap_a, 4 * (lane & 3), ptile * BM, n * p.CB + ksr * kmul + (lane >> 2), &full[s]);
+          else if (lane == 4 * kmul) tma_bulk_g2s(stage + b_off, b_src + static_cast<size_t>(ksr) * b_stage_bytes * kmul, b_stage_bytes * parts, &full[s]);
           __syncwarp();
         }
       }
@@ -887,6 +890,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
             // (j: the K stages of this pipeline step; more than one only with A in tensor memory)
 #pragma unroll
             for (int j = 0; j < kmul; ++j) {
+            if (j > 0 && half_last && last_ks) break;      // (what the splitters made of the stage's old bytes is not multiplied)
             const uint64_t st_desc = st_desc_hi | ((b_addr + j * 128 * BN) >> 4);
 #pragma unroll
             for (int k2 = 0; k2 < 2; ++k2) {
@@ -918,6 +922,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) wino_gemm_kernel(const __grid
             // planes: A hi at +0, lo at +8 KB; B hi at +0, lo at +4 chunks.  K step = 2 chunks.
 #pragma unroll
             for (int j = 0; j < kmul; ++j) {
+            if (j > 0 && half_last && last_ks) break;      // (what the splitters made of the stage's old bytes is not multiplied)
 #pragma unroll
             for (int k2 = 0; k2 < 2; ++k2) {
               const uint64_t ahi = a_desc + ((k2 * 4096) >> 4);
@@ -1643,15 +1648,11 @@ std::vector<float> transform_weights(const float *w, int oc, int ic, int OCP, in
 // Tuning switches of the GEMM kernel (tune_env: overridable only in -DELB_TUNING builds).
 // fp32: A in tensor memory relieves the shared-memory port and deepens the ring; with an accumulator
 // wider than 128 columns it leaves room for one accumulator buffer only, whose epilogue therefore
-// hands tensor memory back before it stores (see the kernel).  The Winograd / direct GEMMs (not flat)
-// always use it: they then run the kernels specialised for it, which beat the generic kernel with A
+// hands tensor memory back before it stores (see the kernel).  // It is always used: such layers run the kernels specialised for it, which beat the generic kernel with A
 // in shared memory on every layer of the VGG-16 stack (same GPU, 32 images: conv2_1 GEMM 0.176 ->
-// 0.126 ms, conv3_1 0.116 -> 0.087 ms; the layers from 256 input channels up had it before).  The
-// flat 1x1 kernel keeps the rule it was measured with: long K loops, or a CTA that runs a single tile
-// (1x1 benchmark layer 68.9 -> 55.9 us), or accumulators of at most 128 columns.
-inline int tune_a_tmem(int kind, int k_stages, long long total_tiles, int num_sms, int acc_width, bool flat) {
-  const int dflt = kind != KIND_F32 ? 0 : !flat ? 1 : (k_stages >= 16 || total_tiles <= num_sms || acc_width <= 128) ? 1 : 0;
-  return tune_env("ELB_F32_A_TMEM", dflt) > 0 ? 1 : 0;
+// 0.126 ms, conv3_1 0.116 -> 0.087 ms; the layers from 256 input channels up had it before).
+inline int tune_a_tmem(int kind) {
+  return tune_env("ELB_F32_A_TMEM", kind == KIND_F32 ? 1 : 0) > 0 ? 1 : 0;
 }
 // K rotation spreads the weight reads of CTAs running side by side over L2; measured without effect
 // on this kernel (the weights of one position are 0.5 MB and stay hot), so it is off.
@@ -1662,11 +1663,11 @@ inline int tune_rotate_k() {
 // more time handing a stage from role to role than multiplying it, so they move two stages at a
 // time (VGG conv1_2, 64 -> 64 channels: GEMM 0.610 -> 0.447 ms); 256-wide tiles are bound by their
 // MMAs and keep the deeper ring of single stages.
-inline int tune_kmul(int kind, int a_tmem, int k_stages, int BN) {
+inline int tune_kmul(int kind, int a_tmem, int k_stages, int BN, bool flat = false) {
   int v = tune_env("ELB_WINO_KMUL", (kind == KIND_F32 && a_tmem && BN <= 128) ? 2 : 1);
   if (kind != KIND_F32 || !a_tmem || v != 2) return 1;
   const int ring_bytes = GEMM_STAGES_1 * (A_STAGE_BYTES + B_STAGE_MAX) + EPI_CONST_BYTES;
-  while (v > 1 && (k_stages % v != 0 || ring_bytes / (v * (A_RAW_BYTES + 128 * BN)) < 2)) v /= 2;
+  while (v > 1 && ((!flat && k_stages % v != 0) || k_stages < v || ring_bytes / (v * (A_RAW_BYTES + 128 * BN)) < 2)) v /= 2;
   return v;
 }
 // Producer warps taking turns on the stages (1..GEMM_PRODUCERS).
@@ -2073,9 +2074,8 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     gp.producers = tune_producers();
     gp.rotate_k = tune_rotate_k();
     gp.stack = w->stack ? 1 : 0;
-    gp.a_tmem = tune_a_tmem(KIND_F32, gp.k_stages, static_cast<long long>(gp.m_tiles) * gp.n_tiles, num_sms,
-                            w->stack ? 2 * w->BN : w->BN, true);
-    gp.kmul = tune_kmul(KIND_F32, gp.a_tmem, gp.k_stages, w->BN);
+    gp.a_tmem = tune_a_tmem(KIND_F32);
+    gp.kmul = tune_kmul(KIND_F32, gp.a_tmem, gp.k_stages, w->BN, true);
     gp.bias = static_cast<const float *>(w->d_bias);
     gp.out = static_cast<float *>(out) + static_cast<size_t>(first) * (w->out_img_bytes / 4);
     gp.with_bias = w->with_bias; gp.with_relu = w->with_relu; gp.with_sum = w->with_sum;
@@ -2145,8 +2145,7 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     gp.rotate_k = tune_rotate_k();
     gp.ablate = tune_env("ELB_ABL", 0);
     gp.stack = w->stack ? 1 : 0;
-    gp.a_tmem = tune_a_tmem(w->kind, gp.k_stages, static_cast<long long>(gp.positions) * gp.m_tiles * gp.n_tiles, num_sms,
-                            w->stack ? 2 * w->BN : w->BN, false);
+    gp.a_tmem = tune_a_tmem(w->kind);
     gp.kmul = tune_kmul(w->kind, gp.a_tmem, gp.k_stages, w->BN);
     if (w->cta2) {
       const int pairs = gp.positions * ((gp.m_tiles + 1) / 2) * gp.n_tiles;

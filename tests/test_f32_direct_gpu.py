@@ -52,6 +52,30 @@ def test_fp32_direct_matches_oracle(pkg, case):
         d.close()
 
 
+# 1x1 layers of enough tiles for the GEMM kernel's flat mode: one K stage, odd and even counts of them (two per step on
+# tiles of at most 128 output channels), tile widths 32 to 256, two N tiles, pixels that do not fill the last tile.
+FLAT_CASES = [
+    _c("f32_flat_one_stage", 90, 16, 32, 30, 30, kh=1, kw=1, pad=0),
+    _c("f32_flat_odd", 90, 48, 24, 31, 27, kh=1, kw=1, pad=0),
+    _c("f32_flat_odd_64_sum", 60, 80, 64, 28, 30, kh=1, kw=1, pad=0, sum=True),
+    _c("f32_flat_even_128", 50, 64, 128, 28, 28, kh=1, kw=1, pad=0),
+    _c("f32_flat_208", 40, 96, 200, 28, 28, kh=1, kw=1, pad=0),
+    _c("f32_flat_256", 40, 64, 256, 28, 28, kh=1, kw=1, pad=0, relu=False),
+    _c("f32_flat_two_n_tiles", 40, 112, 320, 20, 20, kh=1, kw=1, pad=0),
+]
+
+
+@pytest.mark.parametrize("case", FLAT_CASES, ids=lambda c: c.name)
+def test_fp32_flat_matches_oracle(pkg, case):
+    import gpuutil as G
+    t = R.make_tensors(case)
+    want = R.oracle_direct_f64(case, t)
+    got, d = G.run_gpu(case, t)
+    assert d.device_status() == 0
+    d.close()
+    assert R.rel_l2(got, want) <= F32_TOL
+
+
 def test_fp32_direct_host_buffers_and_repeat(pkg):
     import gpuutil as G
     case = CASES[7]
