@@ -92,7 +92,8 @@ __device__ __forceinline__ void requant_relu_u8(const int (&acc)[16], const floa
   *reinterpret_cast<uint4 *>(out) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// 32 bytes in one store: a lane's two 16-byte stores into one 32-byte sector would be two partial writes
+// 32 bytes in one store: a lane's two 16-byte stores into one 32-byte sector would be two partial writes.  The address
+// must be 32-byte aligned (HaloParams::wide).
 __device__ __forceinline__ void store_v8(float *p, const float (&f)[16], int at) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + at), "f"(f[at]), "f"(f[at + 1]),
                "f"(f[at + 2]), "f"(f[at + 3]), "f"(f[at + 4]), "f"(f[at + 5]), "f"(f[at + 6]), "f"(f[at + 7])
@@ -249,8 +250,13 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) f[i] = fminf(fmaxf(f[i], p.rq.relu_lo), p.rq.relu_hi);
       }
-      store_v8(o, f, 0);
-      store_v8(o, f, 8);
+      if (p.wide) {
+        store_v8(o, f, 0);
+        store_v8(o, f, 8);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) reinterpret_cast<float4 *>(o)[i] = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+      }
     }
   };
   const int part_pitch = p.BN / 4 + 1;      // SPLIT: 16-byte words per row of partial sums (odd: no bank conflicts)
@@ -1147,6 +1153,7 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   }
   std::memcpy(p.tmap, hit->m, sizeof(p.tmap[0]) * p.planes);
   p.b_img = static_cast<const uint8_t *>(hp.d_b);
+  p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const bool fast = p.rq.out_type == OUT_U8 && p.rq.relu && p.rq.relu_lo == 0.0f && p.rq.relu_hi >= 3.0e38f && !p.rq.with_sum &&
                     !p.shift_tbl;
   p.fast = !fast ? 0 : p.OCB * 16 <= HALO_PARAM_OC ? 1 : 2;

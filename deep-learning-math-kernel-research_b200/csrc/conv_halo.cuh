@@ -54,6 +54,7 @@ struct HaloParams {
   int a_bytes, raw_bytes, a_stages;  // one ring stage of operand rows (f32: of its hi or lo half), of raw f32 rows; ring depth
   int ksteps;                        // K steps of a channel group, all planes
   int b_per_tile;                    // weight stages of a tile
+  int wide;                          // fp32: `out` is 32-byte aligned (the library promises 16)
   int fast;                          // int8: u8 result, ReLU at 0, no residual, one shift vector (1: constants in cst)
   int row_units;                     // a weight stage holds a filter row's taps (1) or one tap (0) of a plane
   int kstep_bytes, b_stages, b_stage_bytes;

@@ -94,3 +94,47 @@ def test_direct_kernel_reads_its_input_with_a_step(pkg):
     torch.cuda.synchronize()
     assert d.launch_count() == 1 and R.rel_l2(out.cpu().numpy(), want) <= 1e-5
     d.close()
+
+
+ALIGN_CASES = [
+    R.ConvCase("al_direct", 2, 48, 40, 13, 11, stride=2, types="fp32", algo="direct", relu=True, bias=True, sum=True),
+    R.ConvCase("al_split", 1, 256, 64, 14, 14, types="fp32", algo="direct", bias=True),
+    R.ConvCase("al_wino", 16, 64, 64, 24, 24, types="fp32", algo="wino", tile=6, relu=True, bias=True),
+    R.ConvCase("al_u8_f32", 2, 64, 40, 13, 11, types="u8f32f32f32", algo="direct", relu=True, bias=True),
+]
+
+
+@pytest.mark.parametrize("case", ALIGN_CASES, ids=lambda c: c.name)
+def test_tensors_sixteen_bytes_into_an_allocation(pkg, case):
+    """16-byte alignment is all that the library asks of a tensor; 32-byte stores need a look at the address."""
+    sixteen_bytes_into_an_allocation(case)
+
+
+def sixteen_bytes_into_an_allocation(case, planar=False):
+    import torch
+    import gpuutil as G
+    E = G.package()
+    t = R.make_tensors(case)
+    oracle = R.oracle_int8_conv if case.types != "fp32" else R.oracle_wino_f32 if case.algo == "wino" else R.oracle_direct_f64
+    want = oracle(case, t)
+    first = t["residual"] if case.sum else np.zeros(R.out_shape(case), case.out_dtype)
+
+    def shifted(a):
+        raw = torch.full((a.nbytes + 4096 + 16,), 0xA5, dtype=torch.uint8, device="cuda")
+        raw[16:16 + a.nbytes] = torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1)).cuda()
+        return raw, raw.data_ptr() + 16
+
+    d = G.make_desc(case)
+    assert d.setup() == E.ELD_OK, E.last_error()
+    x, x_ptr = shifted(t["input"])
+    y, y_ptr = shifted(first)
+    assert x_ptr % 32 == 16 and y_ptr % 32 == 16
+    assert E.elx_conv(d, y_ptr, x_ptr, torch.from_numpy(t["weights"]).cuda(), torch.from_numpy(t["bias"]).cuda()) == E.ELX_OK, E.last_error()
+    raw = y.cpu().numpy()
+    got = raw[16:16 + first.nbytes].view(case.out_dtype).reshape(first.shape)
+    assert (raw[:16] == 0xA5).all() and (raw[16 + first.nbytes:] == 0xA5).all() and d.device_status() == 0
+    if case.types == "fp32":
+        assert R.rel_l2(got, want) <= 1e-5
+    else:
+        assert np.array_equal(got, want)
+    d.close()
