@@ -260,7 +260,12 @@ __global__ void __launch_bounds__(RGB_THREADS, 1) f32_rgb_umma_kernel(const __gr
               v[i] = __fadd_rn(sum[b][half * 8 + i], s_bias[b * 16 + half * 8 + i]);
               if (p.with_relu) v[i] = fmaxf(v[i], 0.0f);
             }
-            st_global_v8(dst + half * 8, v);
+            if (p.wide) {
+              st_global_v8(dst + half * 8, v);
+            } else {
+              reinterpret_cast<float4 *>(dst)[2 * half] = make_float4(v[0], v[1], v[2], v[3]);
+              reinterpret_cast<float4 *>(dst)[2 * half + 1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
           }
         }
       }
@@ -285,7 +290,9 @@ bool f32_rgb_umma_supported(const SmallIcParams &p) {
   return p.planar && p.OCB * 16 == RGB_BN && !p.with_sum && p.ic >= 1 && p.ic <= 4;
 }
 
-cudaError_t launch_f32_rgb_umma(const SmallIcParams &p, int num_sms, int *status, cudaStream_t s) {
+cudaError_t launch_f32_rgb_umma(const SmallIcParams &params, int num_sms, int *status, cudaStream_t s) {
+  SmallIcParams p = params;
+  p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const long long tiles = static_cast<long long>(p.N) * ((p.W + RGB_TW - 1) / RGB_TW) * ((p.H + RGB_TH - 1) / RGB_TH);
   const int grid = static_cast<int>(tiles < num_sms ? tiles : num_sms);
   switch (p.ic) {

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(SI_THREADS, 3) f32_small_ic_kernel(const Small
       const int ow = ow0 + px;
       if (ow < p.W) {
         float4 *dst = reinterpret_cast<float4 *>(p.out + (((static_cast<size_t>(n) * p.OCB + ocb) * p.H + oh) * p.W + ow) * 16) + half * 2;
-        if (!p.with_sum) {                         // the eight channels are one 32-byte sector: one store
+        if (!p.with_sum && p.wide) {               // the eight channels are one 32-byte sector: one store
           float v[8];
 #pragma unroll
           for (int i = 0; i < 4; ++i) unpack2(acc[px][i], v[2 * i], v[2 * i + 1]);
@@ -211,7 +211,9 @@ cudaError_t init_f32_small_ic(int OCB) {
   return e;
 }
 
-cudaError_t launch_f32_small_ic(const SmallIcParams &p, cudaStream_t s) {
+cudaError_t launch_f32_small_ic(const SmallIcParams &params, cudaStream_t s) {
+  SmallIcParams p = params;
+  p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const long long threads = static_cast<long long>(p.N) * p.H * ((p.W + 3) / 4);
   const unsigned blocks = static_cast<unsigned>((threads + SI_THREADS - 1) / SI_THREADS);
   const size_t smem = f32_small_ic_smem_bytes(p.OCB);

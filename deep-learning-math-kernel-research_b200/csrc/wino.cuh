@@ -41,6 +41,7 @@ struct SmallIcParams {
   int N, H, W, CB, OCB, ic;
   int with_bias, with_relu, with_sum;
   int planar;           // the input is the caller's nchw tensor
+  int wide;             // set by the launch functions: `out` is 32-byte aligned (the library promises 16)
   long long *trace;     // optional per-CTA timeline of the tensor-core kernel (64 slots per CTA), else null
 };
 size_t f32_small_ic_smem_bytes(int OCB);

@@ -1,5 +1,7 @@
 """The halo-tiled kernel (conv_halo.cu) at the edges of its tiles, channel groups and weight-stage forms, against
 the C restatement: INT8 bit-exact (accumulators and outputs), fp32 to the direct path's tolerance."""
+import dataclasses
+
 import numpy as np
 import pytest
 
@@ -100,6 +102,9 @@ ALIGN_CASES = [
     R.ConvCase("al_direct", 2, 48, 40, 13, 11, stride=2, types="fp32", algo="direct", relu=True, bias=True, sum=True),
     R.ConvCase("al_split", 1, 256, 64, 14, 14, types="fp32", algo="direct", bias=True),
     R.ConvCase("al_wino", 16, 64, 64, 24, 24, types="fp32", algo="wino", tile=6, relu=True, bias=True),
+    R.ConvCase("al_small_ic", 2, 3, 40, 19, 21, types="fp32", algo="wino", tile=6, relu=True, bias=True),
+    R.ConvCase("al_small_ic_image", 2, 3, 40, 19, 20, types="fp32", algo="wino", tile=6, bias=True, ifmt="nchw"),
+    R.ConvCase("al_rgb", 2, 3, 64, 19, 40, types="fp32", algo="wino", tile=6, relu=True, bias=True, ifmt="nchw"),
     R.ConvCase("al_u8_f32", 2, 64, 40, 13, 11, types="u8f32f32f32", algo="direct", relu=True, bias=True),
 ]
 
@@ -107,16 +112,14 @@ ALIGN_CASES = [
 @pytest.mark.parametrize("case", ALIGN_CASES, ids=lambda c: c.name)
 def test_tensors_sixteen_bytes_into_an_allocation(pkg, case):
     """16-byte alignment is all that the library asks of a tensor; 32-byte stores need a look at the address."""
-    sixteen_bytes_into_an_allocation(case)
-
-
-def sixteen_bytes_into_an_allocation(case, planar=False):
     import torch
     import gpuutil as G
     E = G.package()
-    t = R.make_tensors(case)
+    blocked = dataclasses.replace(case, ifmt="")
+    t = R.make_tensors(blocked)
     oracle = R.oracle_int8_conv if case.types != "fp32" else R.oracle_wino_f32 if case.algo == "wino" else R.oracle_direct_f64
-    want = oracle(case, t)
+    want = oracle(blocked, t)
+    t = R.user_tensors(case, t)
     first = t["residual"] if case.sum else np.zeros(R.out_shape(case), case.out_dtype)
 
     def shifted(a):
