@@ -1785,7 +1785,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     if (take) {
       w->halo = hp;
       w->flat = false;
-      if (wino_f32) { w->relu_lo = 0.0f; w->relu_hi = 3.402823466e38f; }      // (relu_bound is not used on this path)
+      if (wino_f32) { w->relu_lo = 0.0f; w->relu_hi = INFINITY; }      // (relu_bound is not used on this path)
     } else {
       delete hp;
     }

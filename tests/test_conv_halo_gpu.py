@@ -79,6 +79,20 @@ def test_winograd_request_on_the_direct_kernel(pkg, shape, tile, total):
     d.close()
 
 
+def test_winograd_request_keeps_infinities(pkg):
+    """The Winograd path's ReLU is a plain maximum with zero: an infinite sum stays infinite."""
+    import gpuutil as G
+    case = R.ConvCase("halo_inf", 1, 512, 512, 14, 14, types="fp32", algo="wino", tile=6, relu=True, bias=True)
+    t = R.make_tensors(case)
+    t["bias"] = t["bias"].copy()
+    t["bias"][[3, 500]], t["bias"][4] = np.inf, -np.inf
+    got, d = G.run_gpu(case, t)
+    assert d.launch_count() == 1
+    got = R.from_nChw16c(got, 512)
+    assert np.isposinf(got[:, [3, 500]]).all() and (got[:, 4] == 0).all() and np.isfinite(np.delete(got, [3, 500], 1)).all()
+    d.close()
+
+
 def test_direct_kernel_reads_its_input_with_a_step(pkg):
     import torch
     import gpuutil as G
