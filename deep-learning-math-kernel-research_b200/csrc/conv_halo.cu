@@ -127,7 +127,12 @@ __host__ __device__ constexpr int pxw_of(int form, int kind, int pairs) {
 // sums meet in the CTAs' own shared memory (always added in the same order).  For problems of a few tiles: a
 // 3x3 layer of one 14x14 image is two pixel tiles, whose K loop alone would keep a few SMs busy for longer than the
 // whole call should take.
-template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT>
+// FINE: fp32, 3x3 stride 1, BN <= 128.  The tensor core cuts the sum off when it adds to an accumulator in tensor memory, so
+// the error of a sum grows with the number of MMAs that add into it (against 64 bits 1.9e-8 of the result each, always
+// toward zero): 144 of them for 128 channels, where the transform kernels' GEMM has 32.  So the K loop runs in parts of
+// p.chunk_groups channel groups, each afresh in the other accumulator buffer, and up to 64 output channels the two K steps of a tap
+// have accumulators of their own; the epilogue adds all that up in registers, rounding to nearest.
+template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE>
 __global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
 conv_halo_kernel(const __grid_constant__ HaloParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -389,6 +394,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     const uint32_t b_lbo = static_cast<uint32_t>(STACK ? 2 * BN : PAIR ? BN / 2 : BN) << 16;
     const uint32_t ks16 = uni(p.kstep_bytes) >> 4, lo16 = uni(p.a_bytes) >> 4, a16 = lo16 * PLANES, b16 = uni(p.b_stage_bytes) >> 4;
     const uint32_t a_lbo = static_cast<uint32_t>(PAIRS == 0 ? 1 : pair16 >> 1) << 16;      // (one pixel / one chunk further)
+    const uint32_t d_lo = KIND == HALO_F32 && uni(p.sep) != 0 ? BN : 0;      // columns of the lo products behind the others'
+    const uint32_t d_alt = FINE && BN <= 64 ? 2 * BN : 0;                      // and of a tap's second K step
     auto desc = [](uint32_t lo, uint32_t hi) { return static_cast<uint64_t>(lo) | (static_cast<uint64_t>(hi) << 32); };
     const uint32_t el = elect_one() ? 1u : 0u;
     auto commit = [](uint64_t *b, uint32_t e) {
@@ -397,22 +404,38 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     };
     const int me = warp >> 1;      // this issuer takes tiles me, me + 2, ... of the CTA's
     // ring positions; the stages of the other issuer's tiles are skipped
-    const int skip_a = groups * planes, skip_b = resident ? 0 : uni(p.b_per_tile);
-    int as = 0, bs = 0;
+    // (FINE: units of work are parts of tiles; part c has the groups from g0 + c * chunk_groups)
+    const int own = SPLIT ? g1 - g0 : groups, chunk_groups = FINE ? uni(p.chunk_groups) : own, chunks = FINE ? (own + chunk_groups - 1) / chunk_groups : 1;
+    const int b_tile = resident ? 0 : uni(p.b_per_tile), b_group = FINE ? b_tile / groups : 0;
+    int as = 0, bs = 0, chunk = 0;
     uint32_t aph = 0, bph = 0;
-    auto skip = [&]() {
-      as += skip_a;
+    auto skip = [&]() {      // the unit behind this one
+      const int next = FINE && chunk + 1 < chunks ? chunk + 1 : 0, n = FINE ? min(chunk_groups, own - next * chunk_groups) : groups;
+      as += n * planes;
       while (as >= a_stages) { as -= a_stages; aph ^= 1u; }
-      bs += skip_b;
+      bs += FINE ? n * b_group : b_tile;
       while (bs >= b_stages) { bs -= b_stages; bph ^= 1u; }
     };
     auto next_b = [&]() {
       if (++bs == b_stages) { bs = 0; bph ^= 1u; }
     };
-    if (me) skip();
+    int tile = first;
+    auto advance = [&](int units) {
+      if (FINE) {
+        for (chunk += units; chunk >= chunks; chunk -= chunks) tile += step;
+      } else {
+        tile += units * step;
+      }
+    };
+    if (me) {
+      chunk = chunks - 1;      // (behind which comes the first unit)
+      skip();
+      chunk = 0;
+      advance(1);
+    }
     bool ok = true, b_ready = false;
     int t = me;
-    for (int tile = first + me * step; tile < total && ok; tile += 2 * step, t += 2, skip()) {
+    for (; tile < total && ok; t += 2, skip(), advance(2)) {
       const uint32_t buf = t & (bufs - 1), tph = (bufs == 4 ? t >> 2 : t >> 1) & 1u, my_ph = (t >> 1) & 1u;
       const uint32_t d_tmem = tmem_base + buf * (bufs == 4 ? 128u : 256u);
       // An issuer looks at the rings only once the other has seen every stage of the tile before: a barrier tells
@@ -420,30 +443,32 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       if ((t > 0 && !wait_all(&bar.turn[me], my_ph ^ (me ^ 1u), abort_flag)) ||
           !wait_all(&bar.tempty[buf], tph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
       uint32_t acc = 0;
-      for (int g = g0; g < (SPLIT ? g1 : groups) && ok; ++g)
+      const int gb = (SPLIT ? g0 : 0) + (FINE ? chunk * chunk_groups : 0), ge = FINE ? min(SPLIT ? g1 : groups, gb + chunk_groups) : SPLIT ? g1 : groups;
+      for (int g = gb; g < ge && ok; ++g)
       for (int q = 0; q < planes && ok; ++q) {
         if (!wait_all(&bar.afull[as], aph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_MMA; break; }
-        if (resident && g == groups - 1 && q == planes - 1 && el) mbar_arrive(&bar.turn[me ^ 1u]);
+        if (resident && g == ge - 1 && q == planes - 1 && el) mbar_arrive(&bar.turn[me ^ 1u]);
         tc_fence_after_sync();
         uint32_t a_row = (a_base + as * a16) | a_lbo, b_lo = 0;
-        auto mma = [&](uint32_t al, uint32_t bl, uint32_t accumulate) {
+        auto mma = [&](uint32_t d, uint32_t al, uint32_t bl, uint32_t accumulate) {
           if (KIND == HALO_I8) {
-            if (PAIR) umma_i8_2cta_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
-            else umma_i8_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
+            if (PAIR) umma_i8_2cta_el(d, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
+            else umma_i8_el(d, desc(al, a_hi), desc(bl, b_hi), idesc, accumulate, el);
           } else if (STACK) {
-            // hi * [hi; lo] in one MMA of 2 * BN columns, lo * hi in one of BN (the first BN rows are hi)
-            umma_tf32_el(d_tmem, desc(al, a_hi), desc(bl, b_hi), idesc2, accumulate, el);
-            umma_tf32_el(d_tmem, desc(al + lo16, a_hi), desc(bl, b_hi), idesc, 1u, el);
+            // hi * [hi; lo] in one MMA of 2 * BN columns, lo * hi in one of BN (the first BN rows are hi), added to the
+            // other lo products: the hi sum takes one addition per K step, and what is cut off the lo sum is 2^-11 of that
+            umma_tf32_el(d, desc(al, a_hi), desc(bl, b_hi), idesc2, accumulate, el);
+            umma_tf32_el(d + BN, desc(al + lo16, a_hi), desc(bl, b_hi), idesc, 1u, el);
           } else {
             // planes: the two hi chunks, then the two lo chunks
             const uint64_t bh = desc(bl, b_hi), blo = desc(bl + (ks16 >> 1), b_hi);
-            auto one = [&](uint64_t ad, uint64_t bd, uint32_t ac) {
-              if (PAIR) umma_tf32_2cta_el(d_tmem, ad, bd, idesc, ac, el);
-              else umma_tf32_el(d_tmem, ad, bd, idesc, ac, el);
+            auto one = [&](uint32_t dd, uint64_t ad, uint64_t bd, uint32_t ac) {
+              if (PAIR) umma_tf32_2cta_el(dd, ad, bd, idesc, ac, el);
+              else umma_tf32_el(dd, ad, bd, idesc, ac, el);
             };
-            one(desc(al + lo16, a_hi), bh, accumulate);
-            one(desc(al, a_hi), blo, 1u);
-            one(desc(al, a_hi), bh, 1u);
+            one(d + d_lo, desc(al + lo16, a_hi), bh, accumulate);
+            one(d + d_lo, desc(al, a_hi), blo, 1u);
+            one(d, desc(al, a_hi), bh, d_lo ? accumulate : 1u);
           }
         };
         // `n` taps from column c of the row at a_row (PAIRS = 0: n pairs of taps), unrolled
@@ -453,7 +478,8 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
           for (int i = 0; i < N; ++i)
 #pragma unroll
             for (int j = 0; j < P; ++j)
-              mma(a_row + c + i * (PAIRS ? 1 : 2) + j * pair16, b_lo + (i * P + j) * ks16, (i | j) == 0 ? acc : 1u);
+              mma(FINE && j ? d_tmem + d_alt : d_tmem, a_row + c + i * (PAIRS ? 1 : 2) + j * pair16, b_lo + (i * P + j) * ks16,
+                  (i | j) == 0 || (FINE && i == 0 && d_alt) ? acc : 1u);
           acc = 1u;
           b_lo += N * P * ks16;
         };
@@ -603,42 +629,97 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     // ---------------------------------------------------------------- epilogue: one output pixel per thread
     // int8: group g of four warps serves accumulator g of four, or column half g & 1 of accumulator g >> 1 of two
     const int quarter = warp & 3, group = (warp - EPI_WARP0) >> 2;
-    const bool whole = p.bufs == 4;
+    const bool whole = p.bufs == 4, sep = STACK || (KIND == HALO_F32 && PAIR && p.sep);
     const int half = whole ? 0 : group & 1, blk_step = whole ? 1 : 2;
     const int row = quarter * 32 + lane;
     const int nb16 = p.BN >> 4, cnt = whole ? nb16 : (nb16 - half + 1) >> 1;
     const int t_step = KIND == HALO_F32 ? 1 : p.bufs, t_shift = whole ? 2 : 1;
     int t = KIND == HALO_F32 ? 0 : whole ? group : group >> 1;
     bool ok = true;
+    // the residual this tile adds: on its way to L2 while the MMAs run
+    auto prefetch_residual = [&](const Pixel &px, int nt) {
+      if (!p.rq.with_sum || !px.valid) return;
+      const int elt = KIND == HALO_F32 || p.rq.out_type == OUT_F32 ? 4 : 1;
+      for (int k = 0; k < cnt; ++k) {
+        const int ocb = nt * nb16 + half + blk_step * k;
+        if (ocb < p.OCB)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.out) +
+                                                        (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16 * elt));
+      }
+    };
+    auto release = [&](uint32_t buf) {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR && rank) mbar_arrive_cluster(mapa_u32(&bar.tempty[buf], 0));
+        else mbar_arrive(&bar.tempty[buf]);
+      }
+    };
+    auto finish = [&](const Pixel &px, int nt, int blk, uint32_t (&r)[16], const uint4 *pv) {
+      if (SPLIT) {      // (every copy into the rings has landed and every MMA has read them: the space is free)
+        uint4 *d = reinterpret_cast<uint4 *>(smem) + row * part_pitch + blk * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+      } else {
+        emit(px, nt * nb16 + blk, r, pv);
+      }
+    };
+    if constexpr (FINE) {
+      for (int tile = first; tile < p.total_tiles && ok; tile += step) {
+        const int mu = p.div_n.div(tile), nt = tile - mu * p.n_tiles, mt = PAIR ? 2 * mu + rank : mu;
+        const Pixel px = SPLIT ? Pixel{} : locate(mt, row);
+        if (!SPLIT) prefetch_residual(px, nt);
+        float sum[4][16];      // (BN <= 128: at most four blocks per warp)
+        const int ways = p.BN <= 64 ? 2 : 1;
+        for (int g = g0, c = 0; g < g1; g += p.chunk_groups, ++c, ++t) {
+          const uint32_t buf = t & 1;
+          if (!wait_all(&bar.tfull[buf], (t >> 1) & 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
+          tc_fence_after_sync();
+          const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * 256u + half * 16;
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (k >= cnt) continue;
+#pragma unroll 1
+            for (int w = 0; w < ways; ++w) {
+              uint32_t r[16], q[16];
+              tmem_ld16(t_addr + 2 * w * p.BN + k * 32, r);
+              tmem_ld16(t_addr + (2 * w + 1) * p.BN + k * 32, q);
+              tmem_ld_wait16(r);
+              tmem_ld_wait16(q);
+#pragma unroll
+              for (int i = 0; i < 16; ++i) {
+                const float v = __fadd_rn(__uint_as_float(r[i]), __uint_as_float(q[i]));
+                sum[k][i] = (c | w) == 0 ? v : __fadd_rn(sum[k][i], v);
+              }
+            }
+          }
+          release(buf);
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (k >= cnt) continue;
+          uint32_t r[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(sum[k][i]);
+          finish(px, nt, half + 2 * k, r, nullptr);
+        }
+      }
+    } else
     for (int tile = first + t * step; tile < p.total_tiles && ok; tile += t_step * step, t += t_step) {
       const int mu = p.div_n.div(tile), nt = tile - mu * p.n_tiles, mt = PAIR ? 2 * mu + rank : mu;
       const Pixel px = SPLIT ? Pixel{} : locate(mt, row);
       const uint32_t buf = t & (p.bufs - 1), tph = (t >> t_shift) & 1u;
-      if (!SPLIT && p.rq.with_sum && px.valid) {
-        // the residual this tile adds: on its way to L2 while the MMAs run
-        const int elt = KIND == HALO_F32 || p.rq.out_type == OUT_F32 ? 4 : 1;
-        for (int k = 0; k < cnt; ++k) {
-          const int ocb = nt * nb16 + half + blk_step * k;
-          if (ocb < p.OCB)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const uint8_t *>(p.out) +
-                                                          (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16 * elt));
-        }
-      }
+      if (!SPLIT) prefetch_residual(px, nt);
       if (!wait_all(&bar.tfull[buf], tph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
       tc_fence_after_sync();
       const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (whole ? 128u : 256u) + half * 16;
       auto take = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16], const uint4 &pv) {
-        if (STACK) {
+        if (sep) {
 #pragma unroll
           for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(r[i]), __uint_as_float(r2[i])));
         }
-        if (SPLIT) {      // (every copy into the rings has landed and every MMA has read them: the space is free)
-          uint4 *d = reinterpret_cast<uint4 *>(smem) + row * part_pitch + blk * 4;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) d[i] = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
-        } else {
-          emit(px, nt * nb16 + blk, r, KIND == HALO_I8 ? &pv : nullptr);
-        }
+        finish(px, nt, blk, r, KIND == HALO_I8 ? &pv : nullptr);
       };
       // int8: the stored output that block k adds, fetched a block ahead
       const bool add = KIND == HALO_I8 && !SPLIT && p.rq.with_sum && px.valid;
@@ -647,39 +728,30 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         if (add && ocb < p.OCB)
           pv = *reinterpret_cast<const uint4 *>(static_cast<const uint8_t *>(p.out) + (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16);
       };
-      auto release = [&]() {
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) {
-          if (PAIR && rank) mbar_arrive_cluster(mapa_u32(&bar.tempty[buf], 0));
-          else mbar_arrive(&bar.tempty[buf]);
-        }
-      };
       {
       // blocks half, half + blk_step, ... of this warp, two in flight: while one is converted and stored the next is
         // on its way out of tensor memory
         uint32_t r0[16], r1[16], q0[16], q1[16];
         uint4 pv0 = make_uint4(0, 0, 0, 0), pv1 = pv0;
-        constexpr bool pair = STACK;
         auto load = [&](int k, uint32_t (&r)[16], uint32_t (&q)[16]) {
           tmem_ld16(t_addr + k * (16 * blk_step), r);
-          if (pair) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
+          if (sep) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
         };
         if (cnt > 0) { load(0, r0, q0); residual(0, pv0); }
 #pragma unroll 1
         for (int k = 0; k < cnt; k += 2) {
           tmem_ld_wait16(r0);
-          if (pair) tmem_ld_wait16(q0);
+          if (sep) tmem_ld_wait16(q0);
           if (k + 1 < cnt) { load(k + 1, r1, q1); residual(k + 1, pv1); }
           take(half + blk_step * k, r0, q0, pv0);
           if (k + 1 < cnt) {
             tmem_ld_wait16(r1);
-            if (pair) tmem_ld_wait16(q1);
+            if (sep) tmem_ld_wait16(q1);
             if (k + 2 < cnt) { load(k + 2, r0, q0); residual(k + 2, pv0); }
             take(half + blk_step * (k + 1), r1, q1, pv1);
           }
         }
-        release();
+        release(buf);
       }
     }
   }
@@ -757,7 +829,7 @@ int tap_form(const HaloPlan &hp);
 }  // namespace
 
 bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, int oh, int ow, int kh, int kw, int stride,
-               int pad_t, int pad_l, int num_sms, std::string &err) {
+               int pad_t, int pad_l, int num_sms, std::string &err, int max_acc) {
   HaloParams &p = hp.p;
   hp.kind = kind; hp.stride = stride; hp.IH = ih; hp.IW = iw;
   hp.CB = (ic + 15) / 16;
@@ -860,29 +932,42 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
     const bool stays = nt == 1 && all + 2.0 * planes_bytes + 8192 + BN * 8 <= SMEM_LIMIT - RAW_STAGES * p.raw_bytes;
     // (int8: the epilogue, about 9 outputs per clock)
     const double epilogue = kind == HALO_I8 ? 400 + 128.0 * BN / 9 : 0;
+    // fp32: does max_acc allow `groups` channel groups per CTA, and if only in parts (FINE), how many groups in each?
+    struct Parts { bool ok; int fine, groups, count; };
+    auto parts_of = [&](int groups) -> Parts {
+      if (!max_acc || p.ksteps * (BN <= 128 ? 1 : 3) * groups <= max_acc) return {true, 0, groups, 1};
+      const int each = std::min(groups, max_acc / (BN <= 64 ? p.ksteps / 2 : p.ksteps));
+      if (BN > 128 || stride != 1 || kh != 3 || kw != 3 || each == 0) return {false, 0, 0, 0};
+      return {true, 1, each, (groups + each - 1) / each};
+    };
     for (int pair = 0; pair < 2; ++pair) {
       // pairs take the weights tap by tap, in rows of 512 bytes per half
       // (with a stride the CTAs wait for one another at every parity plane: 128 -> 256, 56x56: fp32 150 -> 180 us, int8
       // with a residual 27.8 -> 29.9; 512 -> 512, 14x14: 13.3 -> 17.5)
       if (pair && (stride > 1 || pairs < 2 || BN % 32 || stays || m_tiles < 2 || kb * pairs > 48 * 1024 || kb * pairs * 3 <= 24 * 1024)) continue;
+      const Parts parts = parts_of(p.groups);
+      if (!parts.ok) continue;
       const double b = stays ? 0.0 : pair ? kb / 2 : kb;
-      const double tile = std::max(std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps, group_min) * p.groups + 600, epilogue);
+      const double tile = std::max(std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps, group_min) * p.groups + 600 + 300 * (parts.count - 1), epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
-      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; }
+      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; p.fine = parts.fine; p.chunk_groups = parts.groups; }
     }
     // few tiles: several CTAs share the K loop of each.  Partial sums cross shared memories at about 9 B/clk.  An SM
     // holds one CTA, and the device no more clusters than its GPCs have room for (15 of 8, 33 of 4).
     for (int split = 2; split <= 8 && split <= p.groups && m_tiles * nt * split <= num_sms * (split == 8 ? 0.8 : 0.88); split *= 2) {
-      const double parts = 128.0 * (BN + 4) * 4;
-      if (kch == 1 || 2 * parts > 150 * 1024) continue;
+      const double sums = 128.0 * (BN + 4) * 4;
+      const Parts parts = parts_of((p.groups + split - 1) / split);
+      if (kch == 1 || 2 * sums > 150 * 1024 || !parts.ok) continue;
       const double t = std::max(kstep_cycles(kind, BN, false, kb, ab, stride > 1) * p.ksteps, group_min) * ((p.groups + split - 1) / split) + 600 +
-                       4000 + 2000 + parts / 9;
-      if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; }
+                       4000 + 2000 + sums / 9 + 300 * (parts.count - 1);
+      if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; p.fine = parts.fine; p.chunk_groups = parts.groups; }
     }
   }
+  if (p.BN == 0) { err = "precision"; return false; }
   hp.est_us = best / 1750;
   p.stack = kind == HALO_F32 && p.BN <= 128 && !p.pair;
+  p.sep = kind == HALO_F32 && p.BN <= 128;
   p.bufs = kind == HALO_I8 && p.BN <= 128 ? 4 : 2;      // accumulators in the 512 columns of tensor memory
   p.div_n.set(p.n_tiles);
   p.div_col.set(p.col_tiles);
@@ -1047,18 +1132,21 @@ typedef void (*HaloKernel)(HaloParams);
 template <int FORM, bool PAIR = false, bool SPLIT = false>
 HaloKernel pick_kernel(const HaloPlan &hp) {
   if (hp.kind == HALO_F32) {
+    if constexpr (FORM == FORM_3X3_TAPS || (!PAIR && (FORM == FORM_3X3_ROWS || (!SPLIT && FORM == FORM_3X3_RESIDENT))))
+      if (hp.p.fine) return conv_halo_kernel<HALO_F32, 2, FORM, !PAIR, PAIR, SPLIT, true>;
+    if (hp.p.fine) return nullptr;      // (halo_plan() makes no such plan)
     if constexpr (!PAIR)
-      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false, SPLIT>;
-    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR, SPLIT>;
+      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false, SPLIT, false>;
+    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR, SPLIT, false>;
   }
   switch (hp.p.kch) {
-    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR, SPLIT>;
-    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR, SPLIT>;
-    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR, SPLIT>;
+    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR, SPLIT, false>;
+    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR, SPLIT, false>;
+    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR, SPLIT, false>;
   }
   if constexpr (!PAIR) {
-    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false, SPLIT>;
-    if constexpr (!SPLIT) return conv_halo_kernel<HALO_I8, 0, FORM, false, false, false>;
+    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false, SPLIT, false>;
+    if constexpr (!SPLIT) return conv_halo_kernel<HALO_I8, 0, FORM, false, false, false, false>;
   }
   return nullptr;
 }

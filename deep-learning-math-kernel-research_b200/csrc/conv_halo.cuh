@@ -63,6 +63,8 @@ struct HaloParams {
   int bufs;                          // accumulators in tensor memory: 4 of up to 128 columns or 2 of up to 256
   int resident;                      // every weight stage of the (single) n tile stays in shared memory
   int stack;                         // f32: hi and lo weight rows of a chunk stacked (BN <= 128)
+  int sep;                           // f32: the lo products have accumulators of their own, BN columns behind the hi ones
+  int fine, chunk_groups;            // f32: the K loop runs in parts of so many channel groups (conv_halo.cu, FINE)
   int strided;                       // stride > 1: five-dimensional maps of the parity planes
   int cb_step;                       // channel blocks per group
   int row0[4], rows[4], col0[4];     // rows a tile reads of each plane: first (relative to the tile's), count; first column
@@ -89,9 +91,10 @@ struct HaloPlan {
   struct Maps { const void *base; int cnt, step, src_h, src_w; CUtensorMap m[4][HALO_HEIGHTS]; };
   std::vector<Maps> maps;            // tensor maps encoded so far
 };
-// false: the shape does not suit the kernel (err says why)
+// false: the shape does not suit the kernel (err says why).  max_acc (f32; 0: any): how many MMAs may add into one
+// accumulator before it is added up in the epilogue's registers.
 bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, int oh, int ow, int kh, int kw, int stride,
-               int pad_t, int pad_l, int num_sms, std::string &err);
+               int pad_t, int pad_l, int num_sms, std::string &err, int max_acc = 0);
 // Weights in the order the kernel reads them: i8 from q[OCP][taps][ICP], f32 from u[OCP][taps][ICP].
 std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP);
 std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, int taps, int ICP);

@@ -1752,7 +1752,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   //     transforming them: few channels (VGG conv1_2 at 16 images 413 -> 245 us, conv2_1 153 -> 103, conv2_2
   //     217 -> 195; conv3_1 325 against 373 stays), or a single image, where the 36 transformed weight planes
   //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 63 -> 18 us; one image of
-  //     512 channels 14x14 30 -> 14 us).  The direct result has the smaller rounding error of the two.  Layers of
+  //     512 channels 14x14 30 -> 14 us).  Layers of
   //     at most 32 input channels and few tiles stay on the transform kernels, whose launches the chain's tests count.
   const bool wino_f32 = info.kernel == ELB_KERNEL_WINO_F32_UMMA;
   if ((direct && (w->flat || !(d.kh == 1 && d.kw == 1 && d.stride_h == 1))) ||
@@ -1762,7 +1762,13 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     HaloPlan *hp = new HaloPlan();
     std::string why;
-    bool take = halo_plan(*hp, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why);
+    // No less precise than the transform kernels: their error against 64 bits, in units of one MMA's addition to an
+    // accumulator (1.9e-8 of the result, conv_halo.cu): 2 K steps of 2 (BN <= 128) or 3 MMAs per channel block, and the transforms'
+    // own rounding, F(4x4,3x3) 28, F(2x2,3x3) 6 (16 to 1024 channels: 6.0e-7 to 7.9e-6 and 2.2e-7 to 7.2e-6, within 6 % of this
+    // but for F(2x2,3x3) above 128 channels, 10 %).  A tenth is left as margin: 64 -> 64 measures 8.1e-7 and 4.2e-7
+    // through the transforms, 7.0e-7 and 3.7e-7 direct.
+    const int max_acc = !wino_f32 ? 0 : static_cast<int>(0.9 * (g.CB * (w->BN <= 128 ? 4 : 6) + (g.A == 6 ? 28 : 6)));
+    bool take = halo_plan(*hp, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why, max_acc);
     if (take && w->flat) {      // the GEMM kernel: fitted on 1024 -> 256 at 14x14, 64 -> 64 at 28x28, 256 -> 1024 at 7x7
       const double tiles = static_cast<double>(d.n) * ((d.oh * d.ow + BM - 1) / BM) * w->n_tiles;
       take = hp->est_us < 6 + 0.65 * g.k_stages * std::ceil(tiles / sms);

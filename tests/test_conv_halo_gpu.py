@@ -1,5 +1,6 @@
 """The halo-tiled kernel (conv_halo.cu) at the edges of its tiles, channel groups and weight-stage forms, against
 the C restatement: INT8 bit-exact (accumulators and outputs), fp32 to the direct path's tolerance."""
+import ctypes
 import dataclasses
 
 import numpy as np
@@ -77,6 +78,34 @@ def test_winograd_request_on_the_direct_kernel(pkg, shape, tile, total):
     assert d.kernel == "wino_f32_umma" and d.launch_count() == 1 and d.device_status() == 0
     assert R.rel_l2(got, R.oracle_wino_f32(case, t)) <= 1e-5
     d.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 32, 48, 28, 31), (2, 64, 64, 56, 56), (1, 96, 112, 40, 31), (24, 64, 128, 28, 28), (4, 128, 128, 28, 27),
+                                   (1, 144, 64, 60, 60), (1, 256, 256, 14, 14)], ids=str)
+def test_winograd_request_is_no_less_precise_than_the_transform_kernels(pkg, shape):
+    """Whatever kernel a plan chooses, its error against 64 bits is at most that of the three transform kernels.
+    F(4x4,3x3): the allocation-free entry point always runs those.  F(2x2,3x3): their error as it was measured, 1.9e-8 of the
+    result for each MMA that adds into an accumulator (4 or 6 per channel block) and 5 to 7 times that for the transforms."""
+    import torch
+    import gpuutil as G
+    E = G.package()
+    n, ic, oc, ih, iw = shape
+    case = R.ConvCase("halo_precision", n, ic, oc, ih, iw, types="fp32", algo="wino", tile=6, bias=True)
+    t = R.make_tensors(case)
+    want = R.oracle_direct_f64(case, t)
+    desc = G.make_desc(case)._c_desc()
+    x, w, b = (torch.from_numpy(t[k]).cuda() for k in ("input", "weights", "bias"))
+    y = torch.zeros(R.out_shape(case), device="cuda")
+    rc = E.lib.elb_wino_f32_conv_noalloc(ctypes.byref(desc), y.data_ptr(), x.data_ptr(), w.data_ptr(), b.data_ptr(), None)
+    assert rc == 0, E.last_error()
+    torch.cuda.synchronize()
+    limit = R.rel_l2(y.cpu().numpy(), want)
+    got, d6 = G.run_gpu(case, t)
+    assert R.rel_l2(got, want) <= 1.02 * limit
+    got, d4 = G.run_gpu(dataclasses.replace(case, tile=4), t)
+    assert R.rel_l2(got, want) <= 2.2e-8 * ((4 if oc <= 128 else 6) * ((ic + 15) // 16) + 7)
+    d6.close()
+    d4.close()
 
 
 def test_winograd_request_keeps_infinities(pkg):
