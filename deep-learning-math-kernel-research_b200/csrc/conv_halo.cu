@@ -1079,6 +1079,34 @@ std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, 
 
 namespace {
 
+// First byte of parity plane q of the tensor at `in` (one plane: the tensor itself)
+void *plane_base(const HaloPlan &hp, const void *in, int q) {
+  const int s = hp.stride, ph = hp.parity[q] / s, pw = hp.parity[q] % s;
+  return const_cast<uint8_t *>(static_cast<const uint8_t *>(in)) + (static_cast<size_t>(ph) * hp.IW + pw) * (hp.kind == HALO_F32 ? 64 : 16);
+}
+
+// Which copies the tiles of `images` images take of plane q (bit i: of HaloParams::tmap[q][i]'s height): the walk of the
+// kernel's row warp.  The tiles' offsets in an image repeat after at most `period` tiles.
+int copy_heights(const HaloParams &p, int images, int q) {
+  const long long row_tiles = (static_cast<long long>(images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
+  int seen = 0;
+  for (int rt = 0; rt < row_tiles && rt <= p.period; ++rt) {
+    const int v0 = rt * TILE_H + p.row0[q], rows = p.rows[q];
+    if ((v0 > 0 ? v0 % p.period : v0) + rows <= p.period) {
+      seen |= 1 << (HALO_HEIGHTS - 1);
+      continue;
+    }
+    for (int r = 0; r < rows;) {
+      const int v = v0 + r, left = v > 0 ? p.period - v % p.period : p.period - v;      // rows of this image from here
+      const int len = std::min(left, rows - r);
+      if (len >= 8) seen |= 8;
+      seen |= len & 7;
+      r += len;
+    }
+  }
+  return seen;
+}
+
 // Tensor maps of `cnt` images at `in`.
 bool encode_maps(const HaloPlan &hp, const void *in, int cnt, int step, int src_h, int src_w, CUtensorMap (*out)[HALO_HEIGHTS],
                  std::string &err) {
@@ -1110,11 +1138,11 @@ bool encode_maps(const HaloPlan &hp, const void *in, int cnt, int step, int src_
                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
       } else {
         const int s = hp.stride, ph = hp.parity[q] / s, pw = hp.parity[q] % s;
+        void *base = plane_base(hp, in, q);
         cuuint64_t dims[5] = {16, static_cast<cuuint64_t>((hp.IW - pw + s - 1) / s), CB,
                               static_cast<cuuint64_t>((hp.IH - ph + s - 1) / s), static_cast<cuuint64_t>(cnt)};
         cuuint64_t strides[4] = {s * px, IH * IW * px, s * IW * px, CB * IH * IW * px};
         cuuint32_t box[5] = {16, static_cast<cuuint32_t>(p.pxw), blocks, height, 1};
-        uint8_t *base = const_cast<uint8_t *>(static_cast<const uint8_t *>(in)) + (static_cast<size_t>(ph) * IW + pw) * px;
         r = enc(&out[q][i], hp.kind == HALO_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 5, base, dims,
                 strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1230,16 +1258,28 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
                  int step, int src_h, int src_w) {
   const HaloPlan::Maps *hit = nullptr;
   for (const auto &m : hp.maps)
-    if (m.base == in && m.cnt == images && m.step == step && (step == 1 || (m.src_h == src_h && m.src_w == src_w))) { hit = &m; break; }
+    if (m.cnt == images && m.step == step && (step == 1 || (m.src_h == src_h && m.src_w == src_w))) { hit = &m; break; }
   if (!hit) {
     HaloPlan::Maps m{};
-    m.base = in; m.cnt = images; m.step = step; m.src_h = src_h; m.src_w = src_w;
+    m.cnt = images; m.step = step; m.src_h = src_h; m.src_w = src_w;
+    for (int q = 0; q < p.planes; ++q) m.heights[q] = static_cast<uint8_t>(copy_heights(p, images, q));
     if (!encode_maps(hp, in, images, step, src_h, src_w, m.m, err)) return false;
-    if (hp.maps.size() >= 64) hp.maps.erase(hp.maps.begin());
-    hp.maps.push_back(m);
-    hit = &hp.maps.back();
+    if (hp.maps.size() < 16) hp.maps.push_back(m);
+    else hp.maps[hp.next_map] = m;
+    hit = &hp.maps[hp.next_map];
+    hp.next_map = (hp.next_map + 1) % 16;
   }
   std::memcpy(p.tmap, hit->m, sizeof(p.tmap[0]) * p.planes);
+  // (with five maps per plane encoded for every new address a call took 7.2 us of host time, strided 8.3, against 4.4)
+  const PFN_replaceAddress set_address = get_replace_address();
+  if (!set_address) { err = "cuTensorMapReplaceAddress is not available from the driver"; return false; }
+  for (int q = 0; q < p.planes; ++q)
+    for (int i = 0; i < HALO_HEIGHTS; ++i)
+      if ((hit->heights[q] >> i) & 1)
+        if (set_address(&p.tmap[q][i], step > 1 ? const_cast<void *>(in) : plane_base(hp, in, q)) != CUDA_SUCCESS) {
+          err = "cuTensorMapReplaceAddress failed";
+          return false;
+        }
   p.b_img = static_cast<const uint8_t *>(hp.d_b);
   p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const bool fast = p.rq.out_type == OUT_U8 && p.rq.relu && p.rq.relu_lo == 0.0f && p.rq.relu_hi >= 3.0e38f && !p.rq.with_sum &&

@@ -88,8 +88,11 @@ struct HaloPlan {
   std::vector<Chunk> order;          // two (i8) chunks per K step of a group; f32: cb = quarter of the block
   std::vector<float> scale, shift;   // int8: host copies of the requantisation constants, [OCP]
   void *d_b = nullptr;               // packed weights (owned by the plan that owns this)
-  struct Maps { const void *base; int cnt, step, src_h, src_w; CUtensorMap m[4][HALO_HEIGHTS]; };
-  std::vector<Maps> maps;            // tensor maps encoded so far
+  // Tensor maps of the image counts (and input steps) seen so far, whatever the address: a launch copies them and sets its
+  // input's address in those that its tiles use (`heights`: bit i = the maps of HaloParams::tmap[plane][i]).
+  struct Maps { int cnt, step, src_h, src_w; uint8_t heights[4]; CUtensorMap m[4][HALO_HEIGHTS]; };
+  std::vector<Maps> maps;            // at most 16, the oldest replaced
+  size_t next_map = 0;
 };
 // false: the shape does not suit the kernel (err says why).  max_acc (f32; 0: any): how many MMAs may add into one
 // accumulator before it is added up in the epilogue's registers.

@@ -262,6 +262,20 @@ inline PFN_encodeTiled get_encode_tiled() {
   return fn;
 }
 
+// Points an encoded map at another tensor of the same shape.
+typedef CUresult (*PFN_replaceAddress)(CUtensorMap *, void *);
+inline PFN_replaceAddress get_replace_address() {
+  static PFN_replaceAddress fn = nullptr;
+  if (!fn) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapReplaceAddress", &p, cudaEnableDefault, &qr) == cudaSuccess &&
+        qr == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<PFN_replaceAddress>(p);
+  }
+  return fn;
+}
+
 // Any reorder<T, dst, src> of the reference; supported = false when the pair is not one of them.
 cudaError_t launch_reorder(void *dst, int dst_fmt, const void *src, int src_fmt, int g, int a, int b, int h,
                            int w, int eb, cudaStream_t s, bool &supported);

@@ -184,3 +184,30 @@ def test_tensors_sixteen_bytes_into_an_allocation(pkg, case):
     else:
         assert np.array_equal(got, want)
     d.close()
+
+
+@pytest.mark.parametrize("case", [
+    _c("turns_i8_s2", 3, 64, 48, 15, 13, stride=2),
+    _c("turns_i8_small_images", 5, 32, 32, 7, 7),
+    _c("turns_f32", 3, 32, 48, 9, 20, types="fp32"),
+], ids=lambda c: c.name)
+def test_inputs_taking_turns(pkg, case):
+    """A plan keeps its tensor maps per image count, not per address: every call reads the tensor it is given."""
+    import torch
+    import gpuutil as G
+    E = G.package()
+    sets = [R.make_tensors(dataclasses.replace(case, name=f"{case.name}{k}")) for k in range(4)]
+    w, b = (torch.from_numpy(sets[0][k]).cuda() for k in ("weights", "bias"))
+    d = G.make_desc(case)
+    assert d.setup() == E.ELD_OK and d.prepare(w, b) == 0
+    xs = [torch.from_numpy(t["input"]).cuda() for t in sets]
+    oracle = R.oracle_direct_f64 if case.types == "fp32" else R.oracle_int8_conv
+    wants = [oracle(case, dict(sets[0], input=t["input"])) for t in sets]
+    ys = [torch.zeros(R.out_shape(case), dtype=torch.from_numpy(wants[0]).dtype, device="cuda") for _ in range(12)]
+    for k, y in enumerate(ys):
+        assert d.enqueue(y, xs[(5 * k) % 4], stream=torch.cuda.current_stream().cuda_stream) == 0, E.last_error()
+    torch.cuda.synchronize()
+    for k, y in enumerate(ys):
+        want = wants[(5 * k) % 4]
+        assert (R.rel_l2(y.cpu().numpy(), want) <= 1e-5) if case.types == "fp32" else np.array_equal(y.cpu().numpy(), want)
+    d.close()
