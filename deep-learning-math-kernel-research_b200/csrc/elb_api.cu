@@ -174,6 +174,7 @@ struct elb_conv {
   std::vector<cudaEvent_t> ev_in, ev_done;
   std::shared_ptr<HostPipe> pipe;       // pageable host tensors: pinned slots and helper threads
   HostPipe::Events pipe_ev;
+  size_t paged_bytes = 0;               // moved from and to pageable memory without it
   // winograd
   WinoPlan wino{};
   // int8 depthwise
@@ -880,7 +881,7 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
     // Pageable tensors of a waiting call go through pinned slots that helper threads fill and empty (host_pipe.hpp);
     // below a megabyte their start costs more than it gives.  A pipe busy with another thread's call is not waited for.
     const bool pageable = wait && (in_dev || in_page) && (out_dev || out_page) && moved >= (size_t(1) << 20);
-    if (pageable && !pl.pipe) pl.pipe = HostPipe::get();
+    if (pageable && !pl.pipe && !(pl.pipe = HostPipe::get(pl.paged_bytes >= HostPipe::EARN_BYTES))) pl.paged_bytes += moved;
     if (verbose) CUDA_TRY(cudaEventRecord(t0, pl.stream));
     if (pageable && pl.pipe && pl.pipe->try_lock()) {
       // chunks of about 1.5 MB: what nothing overlaps is the first one's copy in and the last one's copy out

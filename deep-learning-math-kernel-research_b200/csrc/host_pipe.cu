@@ -3,7 +3,10 @@
 // of a 64-image INT8 1x1 layer whose kernel takes 9 us, where the bus would take 0.25 ms.
 #include "host_pipe.hpp"
 
+#include <sys/mman.h>
+
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 
 #if defined(__x86_64__)
@@ -30,12 +33,12 @@ HostPipe::Events::~Events() {
   }
 }
 
-std::shared_ptr<HostPipe> HostPipe::get() {
+std::shared_ptr<HostPipe> HostPipe::get(bool make) {
   static std::mutex m;
   static std::weak_ptr<HostPipe> current;
   std::lock_guard<std::mutex> lock(m);
   std::shared_ptr<HostPipe> p = current.lock();
-  if (!p) {
+  if (!p && make) {
     p.reset(new HostPipe());
     if (!p->start()) return nullptr;
     current = p;
@@ -44,10 +47,16 @@ std::shared_ptr<HostPipe> HostPipe::get() {
 }
 
 bool HostPipe::start() {
-  // (mapped into every device's context: plans of several GPUs share the slots)
-  if (cudaHostAlloc(reinterpret_cast<void **>(&slots_), 2 * SLOTS * SLOT_BYTES, cudaHostAllocPortable) != cudaSuccess) {
+  // Mapped into every device's context: plans of several GPUs share the slots.  On huge pages, where there are any:
+  // touching and pinning 16 MB takes 3.5 ms, from cudaHostAlloc 7 to 20.
+  constexpr size_t HUGE_PAGE = size_t(2) << 20, bytes = 2 * SLOTS * SLOT_BYTES;
+  slots_ = static_cast<unsigned char *>(std::aligned_alloc(HUGE_PAGE, bytes));
+  if (!slots_) return false;
+  madvise(slots_, bytes, MADV_HUGEPAGE);
+  std::memset(slots_, 0, bytes);
+  pinned_ = cudaHostRegister(slots_, bytes, cudaHostRegisterPortable) == cudaSuccess;
+  if (!pinned_) {
     cudaGetLastError();
-    slots_ = nullptr;
     return false;
   }
   // the calling thread copies too; half of the cores at most, and no more than saturate the memory
@@ -66,7 +75,8 @@ HostPipe::~HostPipe() {
   }
   cv_.notify_all();
   for (std::thread &t : threads_) t.join();
-  if (slots_) cudaFreeHost(slots_);
+  if (pinned_) cudaHostUnregister(slots_);
+  std::free(slots_);
 }
 
 void HostPipe::begin() {

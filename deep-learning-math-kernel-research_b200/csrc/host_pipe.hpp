@@ -18,9 +18,12 @@ class HostPipe {
  public:
   static constexpr size_t SLOT_BYTES = size_t(1) << 20;
   static constexpr int SLOTS = 8;              // per direction
-  // The process's pipe: made by the first call that wants one, shared by all plans that hold it, given back (threads
-  // joined, memory freed) with the last of them.  Null when it cannot be had.
-  static std::shared_ptr<HostPipe> get();
+  // What a plan moves the plain way before it asks for a pipe to be made: making and giving back one (pinning, threads)
+  // takes about 5 ms, what the pipe then saves about 25 us per MB, so a plan that runs a few times and goes never pays it.
+  static constexpr size_t EARN_BYTES = size_t(192) << 20;
+  // The process's pipe, shared by all plans that hold it and given back (threads joined, memory freed) with the last
+  // of them.  Null when there is none and `make` is false, or when it cannot be had.
+  static std::shared_ptr<HostPipe> get(bool make);
   ~HostPipe();
 
   // One piece of a transfer: `bytes` <= SLOT_BYTES
@@ -61,6 +64,7 @@ class HostPipe {
 
   std::mutex busy_;
   unsigned char *slots_ = nullptr;             // pinned: SLOTS for each direction
+  bool pinned_ = false;
   std::vector<std::thread> threads_;
   std::mutex m_;
   std::condition_variable cv_;

@@ -1,5 +1,6 @@
 """Pageable host tensors of more than a megabyte (pinned slots and helper threads), and the layout converters' word
 widths, at their edges."""
+import os
 import threading
 
 import numpy as np
@@ -27,6 +28,45 @@ def test_pageable_tensors(pkg, case):
     else:
         assert np.array_equal(got, R.oracle_int8_conv(case, t))
     d.close()
+
+
+def _threads():
+    return len(os.listdir("/proc/self/task"))
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c.name)
+def test_helpers_come_with_use_and_go_with_the_plan(pkg, case):
+    """Pinned slots and helper threads are made for a plan that has moved 192 MB the plain way, not for one that runs
+    once; another plan may use them meanwhile, and the last plan gives them back."""
+    import gpuutil as G
+    E = G.package()
+    t = R.make_tensors(case)
+    want = R.oracle_direct_f64(case, t) if case.types == "fp32" else R.oracle_int8_conv(case, t)
+    out = np.zeros(R.out_shape(case), case.out_dtype)
+
+    def run(d):
+        out[...] = t["residual"] if case.sum else 0
+        assert E.elx_conv(d, out, t["input"], t["weights"], t["bias"]) == E.ELX_OK, E.last_error()
+        assert R.rel_l2(out, want) <= 1e-5 if case.types == "fp32" else np.array_equal(out, want)
+
+    def plan():
+        d = G.make_desc(case)
+        assert d.setup() == E.ELD_OK
+        run(d)
+        return d
+
+    plan().close()                                  # (the driver starts threads of its own with the first call)
+    before = _threads()
+    d = plan()
+    assert _threads() == before
+    for _ in range((192 << 20) // (t["input"].nbytes + out.nbytes) + 2):
+        run(d)
+    assert _threads() > before or os.cpu_count() < 4
+    other = plan()
+    d.close()
+    run(other)
+    other.close()
+    assert _threads() == before
 
 
 def test_pageable_tensors_from_two_threads(pkg):
