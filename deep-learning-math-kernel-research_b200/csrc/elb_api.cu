@@ -881,12 +881,18 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
     // Pageable tensors of a waiting call go through pinned slots that helper threads fill and empty (host_pipe.hpp);
     // below a megabyte their start costs more than it gives.  A pipe busy with another thread's call is not waited for.
     const bool pageable = wait && (in_dev || in_page) && (out_dev || out_page) && moved >= (size_t(1) << 20);
-    if (pageable && !pl.pipe && !(pl.pipe = HostPipe::get(pl.paged_bytes >= HostPipe::EARN_BYTES))) pl.paged_bytes += moved;
+    if (pageable && !pl.pipe) {
+      const bool make = pl.paged_bytes >= HostPipe::EARN_BYTES;
+      pl.pipe = HostPipe::get(make);
+      if (!pl.pipe) pl.paged_bytes = (make ? 0 : pl.paged_bytes) + moved;
+    }
     if (verbose) CUDA_TRY(cudaEventRecord(t0, pl.stream));
-    if (pageable && pl.pipe && pl.pipe->try_lock()) {
+    std::unique_lock<std::mutex> pipe_lock;
+    if (pageable && pl.pipe) pipe_lock = pl.pipe->try_lock();
+    if (pipe_lock) {
       // chunks of about 1.5 MB: what nothing overlaps is the first one's copy in and the last one's copy out
       if (!getenv("ELB_HOST_CHUNKS")) chunks = (int)std::min<size_t>(std::min<size_t>(16, N), std::max<size_t>(1, moved / (size_t(3) << 19)));
-      if (pl.pending && (rc = wait_pending(pl)) != ELB_OK) { pl.pipe->unlock(); return rc; }
+      if (pl.pending && (rc = wait_pending(pl)) != ELB_OK) return rc;
       std::vector<HostPipe::Piece> pin, pout;
       auto cut = [](std::vector<HostPipe::Piece> &v, void *host, void *dev, size_t bytes, int chunk) {
         for (size_t at = 0; at < bytes; at += HostPipe::SLOT_BYTES)
@@ -909,7 +915,7 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
         le = cudaEventRecord(pl.ev_d2h_done, pl.stream);
         return le == cudaSuccess ? cudaStreamWaitEvent(pl.s_d2h, pl.ev_d2h_done, 0) : le;
       });
-      pl.pipe->unlock();
+      pipe_lock.unlock();
       if (launch_rc != ELB_OK) { cudaDeviceSynchronize(); return launch_rc; }
       CUDA_TRY(e);
       if (verbose) CUDA_TRY(cudaEventRecord(t1, pl.stream));

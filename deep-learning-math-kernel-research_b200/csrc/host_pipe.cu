@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 
 #if defined(__x86_64__)
 #include <immintrin.h>
@@ -23,7 +24,6 @@ inline void relax() {
   std::this_thread::yield();
 #endif
 }
-constexpr size_t PART = size_t(128) << 10;      // a slot is filled by several threads, in parts of this size
 }  // namespace
 
 HostPipe::Events::~Events() {
@@ -39,8 +39,8 @@ std::shared_ptr<HostPipe> HostPipe::get(bool make) {
   std::lock_guard<std::mutex> lock(m);
   std::shared_ptr<HostPipe> p = current.lock();
   if (!p && make) {
-    p.reset(new HostPipe());
-    if (!p->start()) return nullptr;
+    p.reset(new (std::nothrow) HostPipe());
+    if (!p || !p->start()) return nullptr;
     current = p;
   }
   return p;
@@ -96,7 +96,8 @@ void HostPipe::submit(void *dst, const void *src, size_t bytes, std::atomic<int>
   left->store(parts, std::memory_order_relaxed);
   std::lock_guard<std::mutex> lock(m_);
   for (size_t at = 0; at < bytes; at += PART)
-    tasks_.push_back({static_cast<char *>(dst) + at, static_cast<const char *>(src) + at, std::min(PART, bytes - at), left});
+    tasks_[(first_task_ + queued_++) % MAX_TASKS] = {static_cast<char *>(dst) + at, static_cast<const char *>(src) + at,
+                                                     bytes - at < PART ? bytes - at : PART, left};
   ready_.fetch_add(parts, std::memory_order_release);
 }
 
@@ -105,9 +106,10 @@ bool HostPipe::run_one() {
   Task t;
   {
     std::lock_guard<std::mutex> lock(m_);
-    if (tasks_.empty()) return false;
-    t = tasks_.front();
-    tasks_.pop_front();
+    if (queued_ == 0) return false;
+    t = tasks_[first_task_];
+    first_task_ = (first_task_ + 1) % MAX_TASKS;
+    --queued_;
     ready_.fetch_sub(1, std::memory_order_relaxed);
   }
   std::memcpy(t.dst, t.src, t.bytes);

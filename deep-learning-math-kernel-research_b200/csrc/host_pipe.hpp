@@ -4,7 +4,6 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstddef>
-#include <deque>
 #include <memory>
 #include <mutex>
 #include <thread>
@@ -35,20 +34,20 @@ class HostPipe {
   // What a plan keeps for its device: one event per slot.
   struct Events {
     cudaEvent_t in[SLOTS] = {}, out[SLOTS] = {};
-    bool made = false;
     ~Events();
   };
   // Run one call: every piece of `in` host -> device on s_in, `launch(chunk)` once a chunk's pieces have been enqueued,
   // every piece of `out` device -> host on s_out behind its chunk's launch (launch() orders the streams).  Returns when
-  // everything has arrived.  One call at a time: try_lock() first, unlock() afterwards.
+  // everything has arrived.  One call at a time: under try_lock().
   template <typename Launch>
   cudaError_t run(Events &ev, const std::vector<Piece> &in, const std::vector<Piece> &out, int chunks, cudaStream_t s_in,
                   cudaStream_t s_out, Launch launch);
-  bool try_lock() { return busy_.try_lock(); }
-  void unlock() { busy_.unlock(); }
+  std::unique_lock<std::mutex> try_lock() { return std::unique_lock<std::mutex>(busy_, std::try_to_lock); }
 
  private:
   HostPipe() = default;
+  static constexpr size_t PART = size_t(128) << 10;      // a slot is filled by several threads, in parts of this size
+  static constexpr int MAX_TASKS = 2 * SLOTS * static_cast<int>(SLOT_BYTES / PART);
   struct Task {
     void *dst;
     const void *src;
@@ -68,7 +67,8 @@ class HostPipe {
   std::vector<std::thread> threads_;
   std::mutex m_;
   std::condition_variable cv_;
-  std::deque<Task> tasks_;
+  Task tasks_[MAX_TASKS];                      // a ring: from first_task_, queued_ of them (it never allocates)
+  int first_task_ = 0, queued_ = 0;
   std::atomic<int> ready_{0}, active_{0};
   std::atomic<bool> stop_{false};
 };
@@ -77,14 +77,11 @@ template <typename Launch>
 cudaError_t HostPipe::run(Events &ev, const std::vector<Piece> &in, const std::vector<Piece> &out, int chunks, cudaStream_t s_in,
                           cudaStream_t s_out, Launch launch) {
   cudaError_t e = cudaSuccess;
-  if (!ev.made) {
-    for (int i = 0; i < SLOTS && e == cudaSuccess; ++i) {
-      e = cudaEventCreateWithFlags(&ev.in[i], cudaEventDisableTiming);
-      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev.out[i], cudaEventDisableTiming);
-    }
-    if (e != cudaSuccess) return e;
-    ev.made = true;
+  for (int i = 0; i < SLOTS && e == cudaSuccess; ++i) {
+    if (!ev.in[i]) e = cudaEventCreateWithFlags(&ev.in[i], cudaEventDisableTiming);
+    if (e == cudaSuccess && !ev.out[i]) e = cudaEventCreateWithFlags(&ev.out[i], cudaEventDisableTiming);
   }
+  if (e != cudaSuccess) return e;
   auto slot_in = [&](size_t i) { return slots_ + (i % SLOTS) * SLOT_BYTES; };
   auto slot_out = [&](size_t i) { return slots_ + (SLOTS + i % SLOTS) * SLOT_BYTES; };
   std::atomic<int> in_left[SLOTS], out_left[SLOTS];
