@@ -1754,9 +1754,13 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 63 -> 18 us; one image of
   //     512 channels 14x14 30 -> 14 us).  Layers of
   //     at most 32 input channels and few tiles stay on the transform kernels, whose launches the chain's tests count.
+  // ELB_WINO_CTA2=1 asks for the GEMM kernel on pairs of CTAs, which keeps these layers (flat ones have no such form).
   const bool wino_f32 = info.kernel == ELB_KERNEL_WINO_F32_UMMA;
-  if ((direct && (w->flat || !(d.kh == 1 && d.kw == 1 && d.stride_h == 1))) ||
-      (wino_f32 && (d.ic > 32 || static_cast<long long>(d.n) * d.oh * d.ow > 8192))) {
+  const char *on2 = getenv("ELB_WINO_CTA2");
+  const bool asks_pairs = on2 && atoi(on2) > 0;
+  if ((w->flat || !asks_pairs) &&
+      ((direct && (w->flat || !(d.kh == 1 && d.kw == 1 && d.stride_h == 1))) ||
+       (wino_f32 && (d.ic > 32 || static_cast<long long>(d.n) * d.oh * d.ow > 8192)))) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1836,8 +1840,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     // Pairs of CTAs are opt-in (ELB_WINO_CTA2=1): measured on B200 they are not faster than single
     // CTAs (VGG conv3_2 GEMM 0.417 ms either way, int8 0.152 vs 0.120 ms), because the kernel is
     // bound by the hi/lo splitter warps and the epilogue, not by the bytes of B.
-    const char *on2 = getenv("ELB_WINO_CTA2");
-    w->cta2 = g.m_tiles >= 4 && w->BN % 32 == 0 && on2 && atoi(on2) > 0 && !w->flat;
+    w->cta2 = g.m_tiles >= 4 && w->BN % 32 == 0 && asks_pairs && !w->flat;
     if (w->cta2) {
       int dev = 0, sms = 0;
       cudaGetDevice(&dev);

@@ -61,3 +61,18 @@ def test_winograd_pairs(pkg, pairs_on, case):
         assert R.rel_l2(got, want) <= 1e-5
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("case", [
+    R.ConvCase("p2_f32_three_kernels", 4, 64, 64, 40, 40, types="fp32", algo="wino", tile=6, relu=True, bias=True),
+    R.ConvCase("p2_f32_two_ntiles", 6, 48, 288, 30, 29, types="fp32", algo="wino", tile=6, bias=True),
+    R.ConvCase("p2_f32_direct", 4, 32, 64, 20, 20, types="fp32", algo="direct", relu=True, bias=True),
+], ids=lambda c: c.name)
+def test_pairs_run_the_gemm_kernel(pkg, pairs_on, case):
+    """Who asks for pairs gets the GEMM on pairs (at least four row tiles), between its two transforms, not another kernel."""
+    import gpuutil as G
+    t = R.make_tensors(case)
+    got, d = G.run_gpu(case, t)
+    assert d.launch_count() == 3 and d.device_status() == 0
+    assert R.rel_l2(got, R.oracle_wino_f32(case, t) if case.algo == "wino" else R.oracle_direct_f64(case, t)) <= 1e-5
+    d.close()
