@@ -1752,15 +1752,15 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   //     transforming them: few channels (VGG conv1_2 at 16 images 413 -> 245 us, conv2_1 153 -> 103, conv2_2
   //     217 -> 195; conv3_1 325 against 373 stays), or a single image, where the 36 transformed weight planes
   //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 63 -> 18 us; one image of
-  //     512 channels 14x14 30 -> 14 us).  Layers of
-  //     at most 32 input channels and few tiles stay on the transform kernels, whose launches the chain's tests count.
+  //     512 channels 14x14 30 -> 14 us), or so few tiles that the calls are launches (2 x 32 -> 32
+  //     at 14x14 12.0 -> 5.7 us).
   // ELB_WINO_CTA2=1 asks for the GEMM kernel on pairs of CTAs, which keeps these layers (flat ones have no such form).
   const bool wino_f32 = info.kernel == ELB_KERNEL_WINO_F32_UMMA;
   const char *on2 = getenv("ELB_WINO_CTA2");
   const bool asks_pairs = on2 && atoi(on2) > 0;
   if ((w->flat || !asks_pairs) &&
       ((direct && (w->flat || !(d.kh == 1 && d.kw == 1 && d.stride_h == 1))) ||
-       (wino_f32 && (d.ic > 32 || static_cast<long long>(d.n) * d.oh * d.ow > 8192)))) {
+       wino_f32)) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -7,6 +7,8 @@ library on the same input (the GPU's own previous activation, so one layer's rou
 charged to the next), and the whole chain within 1e-4 of the CPU chain (thirteen layers of
 ~1e-6 .. 3e-6 each compound; measured 2.3e-5 at the last layer).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -149,8 +151,8 @@ def test_stack_rejects_mismatched_layers(pkg):
 @pytest.mark.parametrize("int8", [False, True], ids=["fp32_folds_the_subsample", "int8_keeps_the_kernel"])
 def test_stack_subsample_between_layers(pkg, int8):
     """Two layers with a stride-2 subsample between them.  fp32 Winograd: the second layer reads every
-    second row and column of the first layer's full output itself (3 + 3 launches, no subsample
-    kernel); INT8 direct: one kernel per layer plus the subsample kernel.  Either way the chain equals
+    second row and column of the first layer's full output itself (the launches of the two layers, no
+    subsample kernel); INT8 direct: one kernel per layer plus the subsample kernel.  Either way the chain equals
     the CPU chain with an explicit subsample."""
     import torch
     E = G.package()
@@ -172,7 +174,12 @@ def test_stack_subsample_between_layers(pkg, int8):
     before = st.launch_count()
     assert st.enqueue(y, x, torch.cuda.current_stream().cuda_stream) == 0, E.last_error()
     torch.cuda.synchronize()
-    assert st.launch_count() - before == (3 if int8 else 6)
+    layers = 0
+    for k in range(2):
+        info = E.ElbConvInfo()
+        assert E.lib.elb_conv_info(st.layer_plan(k), ctypes.byref(info)) == 0
+        layers += info.launches_per_call
+    assert st.launch_count() - before == layers + (1 if int8 else 0)
     oracle = R.oracle_int8_conv if int8 else R.oracle_wino_f32
     mid = oracle(cases[0], {"input": x_np, "weights": tens[0]["weights"], "bias": tens[0]["bias"]})
     want = oracle(cases[1], {"input": np.ascontiguousarray(mid[:, :, ::2, ::2, :]), "weights": tens[1]["weights"],

@@ -181,3 +181,40 @@ def test_strided_input_is_refused_where_the_kernel_cannot_do_it(pkg):
         assert not d.input_step_supported()
     finally:
         d.close()
+
+
+@pytest.mark.parametrize("shape", [(4, 480, 128, 18, 18), (3, 464, 432, 11, 13), (5, 512, 256, 20, 12)], ids=str)
+@pytest.mark.parametrize("total", [False, True], ids=["plain", "sum"])
+def test_layers_that_stay_on_the_transform_kernels(pkg, shape, total):
+    """Many K stages, one and two channel tiles, stacked and plain weight rows, and an input read with a step."""
+    import torch
+    import gpuutil as G
+    E = G.package()
+    n, ic, oc, ih, iw = shape
+    case = _f32("wino_three", n, ic, oc, ih, iw, sum=total)
+    t = R.make_tensors(case)
+    want = R.oracle_wino_f32(case, t)
+    got, d = G.run_gpu(case, t)
+    assert d.launch_count() == 3 and d.device_status() == 0
+    assert R.rel_l2(got, want) <= 1e-5
+    if not total:
+        big = np.full((n, ic // 16, 2 * ih - 1, 2 * iw - 1, 16), 7.0, np.float32)
+        big[:, :, ::2, ::2] = t["input"]
+        out = torch.zeros(R.out_shape(case), device="cuda")
+        assert d.enqueue_strided(out, torch.from_numpy(big).cuda(), 2 * ih - 1, 2 * iw - 1, 2) == 0, E.last_error()
+        torch.cuda.synchronize()
+        assert d.launch_count() == 6 and np.array_equal(out.cpu().numpy(), got)
+    d.close()
+
+
+@pytest.mark.parametrize("case", [c for c in F32_CASES if c.ic > 4], ids=lambda c: c.name)
+def test_transform_kernels_at_their_edges(pkg, case, monkeypatch):
+    """The cases above on the transform kernels, whatever kernel their plans choose by themselves (the switch keeps a plan
+    with the GEMM kernel, on pairs of CTAs from four row tiles on)."""
+    import gpuutil as G
+    monkeypatch.setenv("ELB_WINO_CTA2", "1")
+    t = R.make_tensors(case)
+    got, d = G.run_gpu(case, t)
+    assert d.launch_count() == 3 and d.device_status() == 0
+    assert R.rel_l2(got, R.oracle_wino_f32(case, t)) <= 1e-5
+    d.close()
