@@ -1198,9 +1198,13 @@ ELB_API int elb_conv_set_stage_events(elb_conv_t *plan, void **cuda_events4) {
 int elb_conv_device_status(elb_conv_t *plan) {
   if (!plan) return -1;
   DeviceGuard guard(plan->device);
-  int st = -1;
-  if (cudaMemcpy(&st, plan->d_status, sizeof(int), cudaMemcpyDefault) != cudaSuccess) return -1;      // (behind the default stream's work)
-  return st;
+  // Behind the work of the default stream and of the streams that wait for it, as a copy of a word in device memory would
+  // be: a copy of the mapped word is one between host addresses, which waits for nothing.
+  cudaEvent_t ev = nullptr;
+  if (cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return -1;
+  const bool ok = cudaEventRecord(ev, cudaStreamLegacy) == cudaSuccess && cudaEventSynchronize(ev) == cudaSuccess;
+  cudaEventDestroy(ev);
+  return ok ? *reinterpret_cast<volatile int *>(plan->h_status) : -1;
 }
 
 }  // extern "C"

@@ -177,8 +177,9 @@ ELB_API int elb_conv_input_step_supported(elb_conv_t *plan);
 ELB_API int elb_conv_enqueue_strided(elb_conv_t *plan, void *output, const void *input, int src_h, int src_w, int step,
                                      void *cuda_stream);
 
-/* Device-side status word of the last launch: 0 = ok, otherwise the code of the bounded wait that
- * gave up (see csrc/elb_common.cuh).  Also returned as ELB_GENERAL_ERROR by execute. */
+/* Status word of the plan's launches: 0 = ok, otherwise the code of the bounded wait that gave up (see
+ * csrc/elb_common.cuh).  Also returned as ELB_GENERAL_ERROR by execute.  Waits for the default stream's
+ * work; what runs on a non-blocking stream has to be waited for first.  -1: it could not be read. */
 ELB_API int elb_conv_device_status(elb_conv_t *plan);
 
 /* Measurement hook, no counterpart in the reference: four cudaEvent_t handles which the Winograd

@@ -76,3 +76,23 @@ assert np.array_equal(out, R.oracle_int8_conv(case, t))
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env={k: v for k, v in os.environ.items() if k != "EULER_VERBOSE"},
                        capture_output=True, text=True, timeout=600)
     assert r.returncode == 0 and "euler-perf" not in r.stdout
+
+
+def test_device_status_waits_for_the_default_stream(pkg):
+    """The verdict is that of the work already queued on the default stream, not of whatever has finished by then."""
+    import torch
+    case = R.ConvCase("status_i8", 2, 64, 64, 14, 14, types="u8f32u8f32", algo="direct", relu=True, bias=True)
+    t = R.make_tensors(case)
+    d = G.make_desc(case)
+    assert d.setup() == 0
+    x, w, b = (torch.from_numpy(t[k]).cuda() for k in ("input", "weights", "bias"))
+    y = torch.zeros(R.out_shape(case), dtype=torch.uint8, device="cuda")
+    assert d.prepare(w, b) == 0
+    end = torch.cuda.Event()
+    torch.cuda._sleep(40_000_000)                   # some 20 ms of the default stream
+    assert d.enqueue(y, x) == 0
+    end.record()
+    assert not end.query()
+    assert d.device_status() == 0
+    assert end.query()
+    d.close()
