@@ -524,7 +524,7 @@ def run_layer(wid: str, ctx: Ctx, cpu_baseline: bool, steps: int | None = None):
                     "frac_of_tensor_peak": round(gemm_tf / tensor_peak(kind, ctx.peaks), 3)},
                    {"kernel": names[2], "ms": round(stage_ms[2], 5)}]
     else:
-        kernels = [{"kernel": d.kernel, "ms": round(ms_step_raw, 5)}]
+        kernels = [{"kernel": d.launched_kernel, "ms": round(ms_step_raw, 5)}]
     entry = {
         "metric": wl["metric"], "value": value, "unit": wl["unit"], "ms_per_step": ms_step, "steps": k_steps,
         "dtype": wl["dtype"],

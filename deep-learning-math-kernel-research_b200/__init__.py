@@ -34,7 +34,7 @@ forward_training, forward_inference, backward_data, backward_weights = range(4)
 FINE, COARSE, CALIBRATED = range(3)
 EL_NO_CALI = 3.4028234663852886e38
 KERNEL_NAMES = {0: "none", 1: "i8_gemm_umma", 2: "i8_conv_umma", 3: "i8_simt", 4: "wino_f32_umma",
-                5: "wino_i8_umma", 6: "i8_depthwise", 7: "f32_direct_umma", 8: "f32_small_ic"}
+                5: "wino_i8_umma", 6: "i8_depthwise", 7: "f32_direct_umma", 8: "f32_small_ic", 9: "conv_halo"}
 
 
 def build(verbose: bool = False) -> Path:
@@ -61,7 +61,7 @@ class ElbConvInfo(C.Structure):
     _fields_ = [("algorithm", C.c_int32), ("tile_size", C.c_int32), ("kernel", C.c_int32), ("device", C.c_int32)] + \
                [(k, C.c_uint64) for k in ("size_input", "size_weights", "size_output", "size_bias", "bytes_input",
                                           "bytes_weights", "bytes_output", "bytes_bias", "workspace_bytes")] + \
-               [("launches_per_call", C.c_int32), ("reserved", C.c_int32)]
+               [("launches_per_call", C.c_int32), ("launched_kernel", C.c_int32)]
 
 
 def _load():
@@ -231,6 +231,11 @@ class eld_conv_t:
     @property
     def kernel(self) -> str:
         return KERNEL_NAMES.get(self.info.kernel if self.info else 0, "?")
+
+    @property
+    def launched_kernel(self) -> str:
+        """The kernel that a call launches: ``kernel``, or "conv_halo" where the plan serves the request with it."""
+        return KERNEL_NAMES.get(self.info.launched_kernel if self.info else 0, "?")
 
     def prepare(self, weights, bias) -> int:
         return lib.elb_conv_prepare(self.xc, _ptr(weights), _ptr(bias))

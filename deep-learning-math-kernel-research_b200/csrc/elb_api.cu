@@ -1092,6 +1092,7 @@ int elb_conv_create(const elb_conv_desc_t *desc, elb_conv_t **plan) {
     pl->cvt_in = cvt_in = false;
   }
   // what the caller sees: the sizes of ITS formats, everything else from the internal plan
+  uinfo.launched_kernel = pl->halo || wino_on_halo(pl->wino) ? ELB_KERNEL_CONV_HALO : pl->info.kernel;
   uinfo.algorithm = pl->info.algorithm; uinfo.tile_size = pl->info.tile_size; uinfo.kernel = pl->info.kernel;
   uinfo.device = pl->info.device; uinfo.launches_per_call = pl->info.launches_per_call + (cvt_in ? 1 : 0) + (cvt_out ? 1 : 0);
   pl->uinfo = uinfo;

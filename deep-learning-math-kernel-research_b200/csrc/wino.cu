@@ -2202,6 +2202,8 @@ bool wino_input_step_supported(const WinoPlan &pl) {
   return w && w->kind == KIND_F32 && !w->small_ic && !w->flat && !w->direct && w->g.A == 6;
 }
 
+bool wino_on_halo(const WinoPlan &pl) { return pl.impl && pl.impl->halo; }
+
 void wino_release(WinoPlan &pl) {
   WinoImpl *w = pl.impl;
   if (!w) return;

@@ -21,6 +21,9 @@ struct WinoPlan {
 // Can this plan read its input with a step (fp32 Winograd F(4x4,3x3) through the transform kernels)?
 bool wino_input_step_supported(const WinoPlan &pl);
 
+// Does the halo-tiled direct kernel serve this plan?
+bool wino_on_halo(const WinoPlan &pl);
+
 // Build the launch geometry for pl from the descriptor (no device work).
 int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, std::string &err);
 // One-time weight transform / quantisation / packing into device memory.

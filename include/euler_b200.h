@@ -93,13 +93,14 @@ typedef struct elb_conv_desc {
 typedef struct elb_conv_info {
   int32_t algorithm;          /* resolved from ELB_CONV_AUTO                    src/eld_conv.cpp:148-159 */
   int32_t tile_size;          /* resolved Winograd tile (6 = F(4x4,3x3))        src/eld_conv.cpp:231-236 */
-  int32_t kernel;             /* ELB_KERNEL_* below                                                   */
+  int32_t kernel;             /* ELB_KERNEL_* below: the family that serves the request               */
   int32_t device;
   uint64_t size_input, size_weights, size_output, size_bias;           /* elements, src/eld_conv.cpp:99-112 */
   uint64_t bytes_input, bytes_weights, bytes_output, bytes_bias;       /* bytes,    src/eld_conv.cpp:123-126 */
   uint64_t workspace_bytes;   /* device memory the plan holds (packed weights, constants, t-buffers) */
   int32_t launches_per_call;  /* kernels one steady-state execute launches */
-  int32_t reserved;
+  int32_t launched_kernel;    /* ELB_KERNEL_* that a call of the plan launches: `kernel`, or ELB_KERNEL_CONV_HALO where the
+                                 plan serves the request with that one; 0 from elb_conv_sizes */
 } elb_conv_info_t;
 
 enum {
@@ -111,8 +112,11 @@ enum {
   ELB_KERNEL_WINO_I8_UMMA = 5,      /* int8 F(4x4,3x3): quantising transforms + tcgen05 kind::i8     */
   ELB_KERNEL_I8_DEPTHWISE = 6,      /* int8 depthwise 3x3: bandwidth-bound dp4a kernel               */
   ELB_KERNEL_F32_DIRECT_UMMA = 7,   /* fp32 1x1 / KxK direct: implicit GEMM on the 3xTF32 tcgen05 kernel */
-  ELB_KERNEL_F32_SMALL_IC = 8       /* fp32 3x3 s1 p1 Winograd request with <= 4 input channels: direct kernel (tcgen05
+  ELB_KERNEL_F32_SMALL_IC = 8,      /* fp32 3x3 s1 p1 Winograd request with <= 4 input channels: direct kernel (tcgen05
                                        implicit GEMM for an nchw image into 64 channels, CUDA cores otherwise) */
+  ELB_KERNEL_CONV_HALO = 9        /* launched_kernel only: the halo-tiled direct convolution (int8 as kind::i8, fp32 as 3xTF32),
+                                       one launch for KxK and strided layers, for 1x1 layers of few tiles and for fp32
+                                       Winograd requests where it is faster and no less precise */
 };
 
 typedef struct elb_conv elb_conv_t;      /* the plan; replaces `elx_conv_t *xc` (include/euler.hpp:186) */

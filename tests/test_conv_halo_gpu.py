@@ -56,11 +56,13 @@ def test_halo_matches_oracle(pkg, shape, types):
     if types == "fp32":
         got, d = G.run_gpu(case, t)
         assert d.launch_count() == 1 and d.device_status() == 0
+        assert d.launched_kernel == "conv_halo"
         assert R.rel_l2(got, R.oracle_direct_f64(case, t)) <= 1e-5
     else:
         want, want_acc = R.oracle_int8_conv(case, t, want_acc=True)
         got, d, acc = G.run_gpu(case, t, want_acc=True)
         assert d.launch_count() == 1 and d.device_status() == 0
+        assert d.launched_kernel == ("i8_gemm_umma" if shape[:3] == (1, 304, 40) else "conv_halo")      # (a 1x1 layer the GEMM kernel keeps)
         assert np.array_equal(acc, want_acc) and np.array_equal(got, want)
     d.close()
 
@@ -75,7 +77,7 @@ def test_winograd_request_on_the_direct_kernel(pkg, shape, tile, total):
     case = R.ConvCase("halo_wino", n, ic, oc, ih, iw, types="fp32", algo="wino", tile=tile, relu=True, bias=True, sum=total)
     t = R.make_tensors(case)
     got, d = G.run_gpu(case, t)
-    assert d.kernel == "wino_f32_umma" and d.launch_count() == 1 and d.device_status() == 0
+    assert d.kernel == "wino_f32_umma" and d.launched_kernel == "conv_halo" and d.launch_count() == 1 and d.device_status() == 0
     assert R.rel_l2(got, R.oracle_wino_f32(case, t)) <= 1e-5
     d.close()
 
