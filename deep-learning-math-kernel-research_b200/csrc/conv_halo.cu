@@ -869,6 +869,8 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   }
   p.period = period;
   p.div_period.set(period);
+  // (the kernel's row numbers, up to a tile and its halo past the last image, are 32-bit)
+  if (static_cast<long long>(n) * period + 64 > 0x7FFFFFFFll) { err = "size"; return false; }
   // Channel groups.  fp32: one 16-channel block (four chunks).  int8: an even number of blocks, at most eight,
   // that wastes the fewest chunks past the last block (narrow groups cost more hand-overs per MMA), or one.
   int kch = 4;
