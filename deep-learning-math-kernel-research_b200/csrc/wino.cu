@@ -1287,12 +1287,11 @@ inline void gemm_launch(const WinoGemmParams &gp, int ctas, cudaStream_t s) {
     return;
   }
   const int spec = (plain && gp.kind == KIND_F32 && gp.a_tmem) ? (gp.stack ? 1 : 2) + (gp.flat ? 3 : 0) : 0;
-  if (spec >= 4) {
+  if (spec == 4 || (spec == 5 && gp.kmul == 1)) {
     if (spec == 4 && gp.kmul == 2 && gp.BN == 64) wino_gemm_kernel<false, 2, 4, 64><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else if (spec == 4 && gp.kmul == 2 && gp.BN == 128) wino_gemm_kernel<false, 2, 4, 128><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else if (spec == 4 && gp.kmul == 2) wino_gemm_kernel<false, 2, 4><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else if (spec == 4) wino_gemm_kernel<false, 1, 4><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
-    else if (gp.kmul == 2) wino_gemm_kernel<false, 2, 0><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else if (gp.BN == 256) wino_gemm_kernel<false, 1, 5, 256><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     else wino_gemm_kernel<false, 1, 5><<<ctas, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(gp);
     return;
