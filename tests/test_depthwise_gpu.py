@@ -125,3 +125,45 @@ def test_depthwise_rejects_undefined_chunkings(pkg, case):
     assert d.setup() == pkg.ELD_UNIMPLEMENTED
     assert "one-pixel chunk" in pkg.last_error()
     d.close()
+
+
+@pytest.mark.parametrize("stride", [1, 2])
+def test_depthwise_between_its_neighbours(pkg, stride):
+    """The kernel may start under the one before it: directly behind the layer that writes its input, and directly behind
+    one that still reads the tensor it writes."""
+    import torch
+    import gpuutil as G
+    E = G.package()
+    before = R.ConvCase("dwn_before", 16, 32, 64, 56, 56, kh=1, kw=1, pad=0, types="u8f32u8f32", algo="1x1", relu=True, bias=True, oscale=0.5)
+    dw = _dw("dwn", 16, 64, 56, 56, 14, stride=stride)
+    after = R.ConvCase("dwn_after", 16, 64, 32, dw.oh, dw.ow, types="u8f32u8f32", algo="direct", relu=True, bias=True, oscale=0.5)
+    tens = [R.make_tensors(c) for c in (before, dw, after)]
+    descs = []
+    for c, t in zip((before, dw, after), tens):
+        d = G.make_desc(c)
+        assert d.setup() == E.ELD_OK, E.last_error()
+        assert d.prepare(torch.from_numpy(t["weights"]).cuda(), torch.from_numpy(t["bias"]).cuda()) == 0
+        descs.append(d)
+    rng = np.random.default_rng(R.seed_for("dwn", str(stride)))
+    images = [rng.integers(0, 256, tens[0]["input"].shape, dtype=np.uint8) for _ in range(2)]
+    plain = rng.integers(0, 256, tens[1]["input"].shape, dtype=np.uint8)      # a depthwise input of no producer
+
+    def chain(x):
+        return R.oracle_int8_conv(after, dict(tens[2], input=R.oracle_int8_depthwise(dw, dict(tens[1], input=x))))
+
+    want = [chain(R.oracle_int8_conv(before, dict(tens[0], input=x))) for x in images]
+    want_plain = chain(plain)
+    xs = [torch.from_numpy(x).cuda() for x in images]
+    xp = torch.from_numpy(plain).cuda()
+    b1 = torch.zeros(R.out_shape(before), dtype=torch.uint8, device="cuda")
+    b2 = torch.zeros(R.out_shape(dw), dtype=torch.uint8, device="cuda")
+    ys = [[torch.zeros(R.out_shape(after), dtype=torch.uint8, device="cuda") for _ in range(2)] for _ in range(10)]
+    s = torch.cuda.current_stream().cuda_stream
+    for k, (y, z) in enumerate(ys):
+        for d, o, i in ((descs[0], b1, xs[k % 2]), (descs[1], b2, b1), (descs[2], y, b2), (descs[1], b2, xp), (descs[2], z, b2)):
+            assert d.enqueue(o, i, stream=s) == 0, E.last_error()
+    torch.cuda.synchronize()
+    for k, (y, z) in enumerate(ys):
+        assert np.array_equal(y.cpu().numpy(), want[k % 2]) and np.array_equal(z.cpu().numpy(), want_plain), k
+    for d in descs:
+        d.close()
