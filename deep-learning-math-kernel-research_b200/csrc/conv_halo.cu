@@ -1,7 +1,7 @@
-// KxK convolution (INT8 u8 x s8 -> s32, and fp32 as 3xTF32) as an implicit GEMM whose activation operand
+// Convolution (INT8 u8 x s8 -> s32, and fp32 as 3xTF32) as an implicit GEMM whose activation operand
 // is fetched ONCE per channel group and reused by every filter tap.
 //
-// Replaces, for filters larger than one pixel or strides above one, the reference's
+// Replaces, for filters larger than one pixel, strides above one and 1x1 layers of few tiles, the reference's
 // elx_int8_conv_direct_t (src/elx_int8_conv_direct.cpp:502-571, kernels
 // src/kernel/elk_u8s8_conv.hxx:254-677) and elx_conv_direct_t (src/elx_conv_direct.cpp,
 // src/kernel/elk_conv.hxx).
@@ -25,8 +25,9 @@
 // Warp roles: 0 activation rows (TMA) | 1, 3 MMA issuers (even / odd tiles of the CTA, 1 owns tensor memory)
 // | 2 weights (bulk copies) | 4.. epilogue | (fp32) four warps that split the landed rows into tf32 hi / lo
 // planes in shared memory.
-// Two accumulators in tensor memory, each with its own issuer: one warp issues an MMA about every 40 cycles
-// (wait, addresses, descriptors), and on narrow tiles an MMA lasts no longer than that.
+// Two accumulators in tensor memory (int8 up to 128 channels per tile: four), filled by two issuers in turn.  An issuer
+// spends 8 cycles on an MMA while its warp stays converged (umma_i8_el), and some hundreds per tile and stage on
+// waits; two of them keep the pipe busy on tiles of 18 MMAs that last 864 cycles in all.
 #include "conv_halo.cuh"
 
 #include <algorithm>
@@ -728,31 +729,29 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         if (add && ocb < p.OCB)
           pv = *reinterpret_cast<const uint4 *>(static_cast<const uint8_t *>(p.out) + (px.pix + ocb * (static_cast<size_t>(p.OH) * p.OW)) * 16);
       };
-      {
       // blocks half, half + blk_step, ... of this warp, two in flight: while one is converted and stored the next is
-        // on its way out of tensor memory
-        uint32_t r0[16], r1[16], q0[16], q1[16];
-        uint4 pv0 = make_uint4(0, 0, 0, 0), pv1 = pv0;
-        auto load = [&](int k, uint32_t (&r)[16], uint32_t (&q)[16]) {
-          tmem_ld16(t_addr + k * (16 * blk_step), r);
-          if (sep) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
-        };
-        if (cnt > 0) { load(0, r0, q0); residual(0, pv0); }
+      // on its way out of tensor memory
+      uint32_t r0[16], r1[16], q0[16], q1[16];
+      uint4 pv0 = make_uint4(0, 0, 0, 0), pv1 = pv0;
+      auto load = [&](int k, uint32_t (&r)[16], uint32_t (&q)[16]) {
+        tmem_ld16(t_addr + k * (16 * blk_step), r);
+        if (sep) tmem_ld16(t_addr + p.BN + k * (16 * blk_step), q);
+      };
+      if (cnt > 0) { load(0, r0, q0); residual(0, pv0); }
 #pragma unroll 1
-        for (int k = 0; k < cnt; k += 2) {
-          tmem_ld_wait16(r0);
-          if (sep) tmem_ld_wait16(q0);
-          if (k + 1 < cnt) { load(k + 1, r1, q1); residual(k + 1, pv1); }
-          take(half + blk_step * k, r0, q0, pv0);
-          if (k + 1 < cnt) {
-            tmem_ld_wait16(r1);
-            if (sep) tmem_ld_wait16(q1);
-            if (k + 2 < cnt) { load(k + 2, r0, q0); residual(k + 2, pv0); }
-            take(half + blk_step * (k + 1), r1, q1, pv1);
-          }
+      for (int k = 0; k < cnt; k += 2) {
+        tmem_ld_wait16(r0);
+        if (sep) tmem_ld_wait16(q0);
+        if (k + 1 < cnt) { load(k + 1, r1, q1); residual(k + 1, pv1); }
+        take(half + blk_step * k, r0, q0, pv0);
+        if (k + 1 < cnt) {
+          tmem_ld_wait16(r1);
+          if (sep) tmem_ld_wait16(q1);
+          if (k + 2 < cnt) { load(k + 2, r0, q0); residual(k + 2, pv0); }
+          take(half + blk_step * (k + 1), r1, q1, pv1);
         }
-        release(buf);
       }
+      release(buf);
     }
   }
 
@@ -982,11 +981,11 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   const int row_steps = kch == 1 ? (most_c + 1) / 2 : most_c * pairs;
   // a stage costs its hand-over whatever it holds: whole filter rows while they are small
   auto set_units = [&](bool rows_of_taps) {
-  p.row_units = rows_of_taps;
-  b_per_group = 0;
-  for (int i = 0; i < p.planes; ++i) b_per_group += p.row_units ? p.tap_rows[i] : p.tap_rows[i] * p.tap_cols[i];
-  p.b_per_tile = b_per_group * p.groups;
-  p.b_stage_bytes = (p.row_units ? row_steps : pairs) * p.kstep_bytes;
+    p.row_units = rows_of_taps;
+    b_per_group = 0;
+    for (int i = 0; i < p.planes; ++i) b_per_group += p.row_units ? p.tap_rows[i] : p.tap_rows[i] * p.tap_cols[i];
+    p.b_per_tile = b_per_group * p.groups;
+    p.b_stage_bytes = (p.row_units ? row_steps : pairs) * p.kstep_bytes;
   };
   auto fit_b = [&](int a_stages) -> bool {
     p.a_stages = a_stages;
