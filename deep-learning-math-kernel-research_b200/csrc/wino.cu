@@ -1748,10 +1748,10 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   //     64 x 128 -> 256 channels 56x56: 231 MB of it, 252 -> 164 us);
   //   * plain 1x1 layers of so few tiles that most SMs would have none (1024 -> 256 at 14x14, one image 47 -> 13 us);
   //   * Winograd requests where nine products per output cost less than moving V and M through memory and
-  //     transforming them: few channels (VGG conv1_2 at 16 images 413 -> 245 us, conv2_1 153 -> 103, conv2_2
-  //     217 -> 195; conv3_1 325 against 373 stays), or a single image, where the 36 transformed weight planes
-  //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 63 -> 18 us; one image of
-  //     512 channels 14x14 30 -> 14 us), or so few tiles that the calls are launches (2 x 32 -> 32
+  //     transforming them: few channels (VGG conv1_2 at 64 images 1574 -> 1128 us, conv2_1 556 -> 400, conv2_2
+  //     867 -> 864; conv3_1 stays), or a single image, where the 36 transformed weight planes
+  //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 64 -> 21 us; one image of
+  //     512 channels 14x14 34 -> 15 us), or so few tiles that the calls are launches (2 x 32 -> 32
   //     at 14x14 12.0 -> 5.7 us).
   // ELB_WINO_CTA2=1 asks for the GEMM kernel on pairs of CTAs, which keeps these layers (flat ones have no such form).
   const bool wino_f32 = info.kernel == ELB_KERNEL_WINO_F32_UMMA;
