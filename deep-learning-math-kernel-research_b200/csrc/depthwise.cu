@@ -338,7 +338,8 @@ __device__ __forceinline__ uint32_t cvt_near_s8(float f) {
 //   * the accumulators start at the bit pattern of 1.5 * 2^23 and convert to float by one subtraction, two at a time;
 //   * a row's four pixels are converted by one saturating conversion per value (on the conversion unit, 30 % busy) and
 //     packed pixel by pixel: nothing is transposed back.  Only a floored group with a value of 256 or more (an
-//     overflowing output scale) takes the reference's packing with carries;
+//     overflowing output scale) takes the reference's packing with carries (22.2 us without any such value, 30.0 us with
+//     one in 250);
 //   * the input rows come through a small ring in shared memory, two rows ahead (four: 25.5 us instead of 24.6 from a
 //     cold L2), and the window of three rows rotates by unrolling instead of moving registers;
 //   * the nearest-rounded remainders of two chunks, at most two pixels each, share a thread.
