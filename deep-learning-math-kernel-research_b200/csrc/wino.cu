@@ -1748,8 +1748,8 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   //     64 x 128 -> 256 channels 56x56: 231 MB of it, 252 -> 164 us);
   //   * plain 1x1 layers of so few tiles that most SMs would have none (1024 -> 256 at 14x14, one image 47 -> 13 us);
   //   * Winograd requests where nine products per output cost less than moving V and M through memory and
-  //     transforming them: few channels (VGG conv1_2 at 64 images 1574 -> 1128 us, conv2_1 556 -> 400, conv2_2
-  //     867 -> 864; conv3_1 stays), or a single image, where the 36 transformed weight planes
+  //     transforming them: few channels (VGG conv1_2 at 64 images 1574 -> about 1150 us, conv2_1 556 -> 420;
+  //     conv2_2 within a few percent either way, conv3_1 stays), or a single image, where the 36 transformed weight planes
   //     (hi and lo, 8 bytes each) are the traffic (at 16 images 16 -> 64 channels 112x112 64 -> 21 us; one image of
   //     512 channels 14x14 34 -> 15 us), or so few tiles that the calls are launches (2 x 32 -> 32
   //     at 14x14 12.0 -> 5.7 us).
@@ -1767,10 +1767,12 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     std::string why;
     // No less precise than the transform kernels: their error against 64 bits, in units of one MMA's addition to an
     // accumulator (1.9e-8 of the result, conv_halo.cu): 2 K steps of 2 (BN <= 128) or 3 MMAs per channel block, and the transforms'
-    // own rounding, F(4x4,3x3) 28, F(2x2,3x3) 6 (16 to 1024 channels: 6.0e-7 to 7.9e-6 and 2.2e-7 to 7.2e-6, within 6 % of this
-    // but for F(2x2,3x3) above 128 channels, 10 %).  A tenth is left as margin: 64 -> 64 measures 8.1e-7 and 4.2e-7
-    // through the transforms, 7.0e-7 and 3.7e-7 direct.
-    const int max_acc = !wino_f32 ? 0 : static_cast<int>(0.9 * (g.CB * (w->BN <= 128 ? 4 : 6) + (g.A == 6 ? 28 : 6)));
+    // own rounding: F(4x4,3x3) 28 where the input's signs are mixed, 23 behind a ReLU, 9 to 13 where it is all positive; F(2x2,3x3) 6 (16
+    // to 1024 channels: 6.0e-7 to 7.9e-6 and 2.2e-7 to 7.2e-6 with mixed signs).  The smallest counts, and a tenth is left as
+    // margin: 64 -> 64 measures 8.1e-7 (all positive 4.9e-7) and 4.2e-7 (3.9e-7) through the transforms, 3.7e-7 (3.5e-7) direct.
+    // Counting 28 for F(4x4,3x3) the fp32 VGG-16 stack takes 5.60 ms instead of 5.69, at 1.4 times the transforms' error on all
+    // positive inputs.
+    const int max_acc = !wino_f32 ? 0 : static_cast<int>(0.9 * (g.CB * (w->BN <= 128 ? 4 : 6) + (g.A == 6 ? 9 : 6)));
     bool take = halo_plan(*hp, HALO_F32, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, sms, why, max_acc);
     if (take && w->flat) {      // the GEMM kernel: fitted on 1024 -> 256 at 14x14, 64 -> 64 at 28x28, 256 -> 1024 at 7x7
       const double tiles = static_cast<double>(d.n) * ((d.oh * d.ow + BM - 1) / BM) * w->n_tiles;
