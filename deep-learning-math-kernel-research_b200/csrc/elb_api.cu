@@ -764,7 +764,8 @@ int do_enqueue_range_inner(elb_conv &pl, void *out, const void *in, int n0, int 
 
 // The same in the caller's formats: plain activations (nchw / nhwc) are converted to nChw16c
 // before the kernels and the result back after them, image range by image range, on the same
-// stream (the residual of an in-place sum travels with the output tensor).
+// stream (the residual of an in-place sum travels with the output tensor).  The Winograd transform
+// kernels read and write nhwc tensors themselves where a pixel's channels are whole groups of four.
 int do_enqueue_range(elb_conv &pl, void *out, const void *in, int n0, int cnt, cudaStream_t s) {
   if (!pl.cvt_in && !pl.cvt_out) return do_enqueue_range_inner(pl, out, in, n0, cnt, s);
   const elb_conv_desc_t &d = pl.d;
@@ -773,20 +774,25 @@ int do_enqueue_range(elb_conv &pl, void *out, const void *in, int n0, int cnt, c
   const size_t u_out = pl.uinfo.bytes_output / N, b_out = pl.info.bytes_output / N;
   bool sup = false;
   cudaError_t e = cudaSuccess;
-  if (pl.cvt_in) {
+  const bool nhwc_in = pl.cvt_in && pl.ud.fmt_input == ELB_NHWC && wino_reads_nhwc(pl.wino, in);
+  const bool nhwc_out = pl.cvt_out && pl.ud.fmt_output == ELB_NHWC && wino_writes_nhwc(pl.wino, out);
+  const bool cvt_in = pl.cvt_in && !nhwc_in, cvt_out = pl.cvt_out && !nhwc_out;
+  if (cvt_in) {
     e = launch_reorder((uint8_t *)pl.d_cvt_in + n0 * b_in, ELB_NCHW16C, (const uint8_t *)in + n0 * u_in, pl.ud.fmt_input, 1, cnt,
                        d.ic, d.ih, d.iw, ebi, s, sup);
     ++pl.launches;
   }
-  if (e == cudaSuccess && pl.cvt_out && d.with_ip_sum) {
+  if (e == cudaSuccess && cvt_out && d.with_ip_sum) {
     e = launch_reorder((uint8_t *)pl.d_cvt_out + n0 * b_out, ELB_NCHW16C, (const uint8_t *)out + n0 * u_out, pl.ud.fmt_output, 1,
                        cnt, d.oc, d.oh, d.ow, ebo, s, sup);
     ++pl.launches;
   }
   if (e != cudaSuccess) return fail(ELB_GENERAL_ERROR, "format conversion launch failed: %s", cudaGetErrorString(e));
-  int rc = do_enqueue_range_inner(pl, pl.cvt_out ? pl.d_cvt_out : out, pl.cvt_in ? pl.d_cvt_in : in, n0, cnt, s);
+  pl.wino.in_nhwc = nhwc_in; pl.wino.out_nhwc = nhwc_out;
+  int rc = do_enqueue_range_inner(pl, cvt_out ? pl.d_cvt_out : out, cvt_in ? pl.d_cvt_in : in, n0, cnt, s);
+  pl.wino.in_nhwc = pl.wino.out_nhwc = false;
   if (rc != ELB_OK) return rc;
-  if (pl.cvt_out) {
+  if (cvt_out) {
     e = launch_reorder((uint8_t *)out + n0 * u_out, pl.ud.fmt_output, (const uint8_t *)pl.d_cvt_out + n0 * b_out, ELB_NCHW16C, 1, cnt,
                        d.oc, d.oh, d.ow, ebo, s, sup);
     ++pl.launches;
@@ -1094,7 +1100,9 @@ int elb_conv_create(const elb_conv_desc_t *desc, elb_conv_t **plan) {
   // what the caller sees: the sizes of ITS formats, everything else from the internal plan
   uinfo.launched_kernel = pl->halo || wino_on_halo(pl->wino) ? ELB_KERNEL_CONV_HALO : pl->info.kernel;
   uinfo.algorithm = pl->info.algorithm; uinfo.tile_size = pl->info.tile_size; uinfo.kernel = pl->info.kernel;
-  uinfo.device = pl->info.device; uinfo.launches_per_call = pl->info.launches_per_call + (cvt_in ? 1 : 0) + (cvt_out ? 1 : 0);
+  uinfo.device = pl->info.device;
+  uinfo.launches_per_call = pl->info.launches_per_call + (cvt_in && !(ud.fmt_input == ELB_NHWC && wino_reads_nhwc(pl->wino, nullptr)) ? 1 : 0) +
+                            (cvt_out && !(ud.fmt_output == ELB_NHWC && wino_writes_nhwc(pl->wino, nullptr)) ? 1 : 0);
   pl->uinfo = uinfo;
   if ((cvt_in && cudaMalloc(&pl->d_cvt_in, pl->info.bytes_input) != cudaSuccess) ||
       (cvt_out && cudaMalloc(&pl->d_cvt_out, pl->info.bytes_output) != cudaSuccess)) {

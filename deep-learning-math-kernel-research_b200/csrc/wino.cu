@@ -172,9 +172,20 @@ struct WinoInParams {
   WinoGeom g;
   float mrepS, tz;     // int8: u8 = sat(rne(fma(V, mrepS, tz)))
   int step, SH, SW;    // fp32 F(4x4,3x3): the input is a plane of SH x SW pixels read with this step (1: SH = IH, SW = IW)
+  int chans;           // nhwc (the kernels' NHWC): channels of a pixel, a multiple of 4
 };
 
-template <bool IN_U8>
+// Element of pixel (ih, iw) of image n, channel block `block`, channels 4 quad ..: in nChw16c planes of h x w pixels, or in the
+// caller's nhwc tensor of `chans` channels.  NHWC is a template argument of the transform kernels, and the nChw16c address is one
+// product chain from the image down: with a base per plane and the pitches as values the output transform of 64 x 256 channels
+// 56x56 was 8 us slower.
+template <bool NHWC>
+__device__ __forceinline__ size_t pixel_at(int n, int block, int quad, int ih, int iw, int blocks, int h, int w, int chans) {
+  return NHWC ? ((static_cast<size_t>(n) * h + ih) * w + iw) * chans + block * 16 + quad * 4
+              : (((static_cast<size_t>(n) * blocks + block) * h + ih) * w + iw) * 16 + quad * 4;
+}
+
+template <bool NHWC>
 __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_constant__ WinoInParams p) {
   const WinoGeom &g = p.g;
   const int quad = threadIdx.x & 3;
@@ -184,7 +195,7 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
   const int mt = t >> 7, row = t & 127;
 
   float m[6][6][4];   // first the 6x6 input patch d[h][w][channel], then (in place) the pass along h: m[i][w][channel]
-  const bool live = t < g.T;
+  const bool live = t < g.T && (!NHWC || cb * 16 + quad * 4 < p.chans);
   int n = 0, th = 0, tw = 0;
   if (live) {
     n = t / (g.ht * g.wt);
@@ -198,54 +209,32 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
   // All 36 loads of the patch are issued before the first use: the kernel is bandwidth-bound and
   // runs few warps per SM (the patch lives in registers), so the bytes in flight per thread are
   // what keeps HBM busy.
-  if (IN_U8) {
-    uint32_t raw[6][6];
+  // one base pointer per thread, row and column offsets added to it; tiles that do not touch the
+  // image border load without any bounds test (the address arithmetic and the predicates of 36
+  // separately addressed loads cost this kernel more than its transform)
+  const float4 *plane = reinterpret_cast<const float4 *>(static_cast<const float *>(p.in) +
+                                                         pixel_at<NHWC>(n, cb, quad, 0, 0, g.CB, p.SH, p.SW, p.chans));
+  const int col_pitch = p.step * (NHWC ? p.chans >> 2 : 4), row_pitch = p.SW * col_pitch;      // in float4 units
+  if (live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW) {
+    const float4 *p0 = plane + static_cast<size_t>(ih0) * row_pitch + iw0 * col_pitch;
+#pragma unroll
+    for (int h = 0; h < 6; ++h)
+#pragma unroll
+      for (int w = 0; w < 6; ++w) {
+        const float4 v = __ldg(p0 + h * row_pitch + w * col_pitch);
+        m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
+      }
+  } else {
 #pragma unroll
     for (int h = 0; h < 6; ++h)
 #pragma unroll
       for (int w = 0; w < 6; ++w) {
         const int ih = ih0 + h, iw = iw0 + w;
         const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-        const size_t pix = ((static_cast<size_t>(n) * g.CB + cb) * g.IH + (ok ? ih : 0)) * g.IW + (ok ? iw : 0);
-        raw[h][w] = ok ? __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(p.in) + pix * 16) + quad) : 0u;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ok) v = __ldg(plane + static_cast<size_t>(ih) * row_pitch + iw * col_pitch);
+        m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
       }
-    // u8 -> fp32 without the conversion unit: a byte permute builds the bit pattern of 2^23 + b,
-    // subtracting 2^23 is exact
-#pragma unroll
-    for (int h = 0; h < 6; ++h)
-#pragma unroll
-      for (int w = 0; w < 6; ++w)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-          m[h][w][c] = __fsub_rn(__uint_as_float(__byte_perm(raw[h][w], 0x4B000000u, 0x7650 + c)), 8388608.0f);
-  } else {
-    // one base pointer per thread, row and column offsets added to it; tiles that do not touch the
-    // image border load without any bounds test (the address arithmetic and the predicates of 36
-    // separately addressed loads cost this kernel more than its transform)
-    const float4 *plane = reinterpret_cast<const float4 *>(static_cast<const float *>(p.in) +
-                                                           (static_cast<size_t>(n) * g.CB + cb) * p.SH * p.SW * 16) + quad;
-    const int row_pitch = p.SW * p.step * 4, col_pitch = p.step * 4;      // in float4 units
-    if (live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW) {
-      const float4 *p0 = plane + static_cast<size_t>(ih0) * row_pitch + iw0 * col_pitch;
-#pragma unroll
-      for (int h = 0; h < 6; ++h)
-#pragma unroll
-        for (int w = 0; w < 6; ++w) {
-          const float4 v = __ldg(p0 + h * row_pitch + w * col_pitch);
-          m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
-        }
-    } else {
-#pragma unroll
-      for (int h = 0; h < 6; ++h)
-#pragma unroll
-        for (int w = 0; w < 6; ++w) {
-          const int ih = ih0 + h, iw = iw0 + w;
-          const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (ok) v = __ldg(plane + static_cast<size_t>(ih) * row_pitch + iw * col_pitch);
-          m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
-        }
-    }
   }
   // pass along h, in place.  (Two channels per instruction, as in the output transform, measured
   // SLOWER here: c1's input transform 0.127 -> 0.137 ms, VGG conv1_2's 0.245 -> 0.264 ms; and without
@@ -287,32 +276,10 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const int a = i * 6 + j;
-      if (IN_U8) {
-        // stage = 8 channel blocks; chunk = cb % 8; 4 bytes per thread
-        // sat_u8(rne(fma(V, mrepS, tz))): adding 1.5 * 2^23 rounds to nearest even and leaves the
-        // integer in the low bits; as an UNSIGNED number a negative result is huge, so one min()
-        // gives the reference's unsigned saturation (below zero -> 255, above 255 -> 255).  Exact
-        // while |fma| < 2^22; anything larger takes the plain conversion.
-        uint32_t b[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float f = __fmaf_rn(v[j][c], p.mrepS, p.tz);
-          const uint32_t u = __float_as_uint(__fadd_rn(f, 12582912.0f)) - 0x4B400000u;
-          b[c] = min(u, 255u);
-          if (!(fabsf(f) < 4194304.0f)) {
-            const float q = rintf(f);
-            b[c] = (q < 0.0f || q > 255.0f || q != q) ? 255u : static_cast<uint32_t>(q);
-          }
-        }
-        const uint32_t w = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
-        const size_t off = ((((static_cast<size_t>(a) * g.m_tiles + mt) * g.k_stages + (cb >> 3)) * 8 + (cb & 7)) * BM + row) * 16 + quad * 4;
-        *reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(p.a_img) + off) = live ? w : 0u;
-      } else {
-        // stage = this channel block, chunk = quad; plain fp32 (the GEMM kernel splits it into its
-        // tf32 hi / lo planes in shared memory, so V crosses HBM once, not twice)
-        // (one base address per thread + a constant step per position)
-        *reinterpret_cast<float4 *>(v_base + static_cast<size_t>(a) * v_step) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
-      }
+      // stage = this channel block, chunk = quad; plain fp32 (the GEMM kernel splits it into its
+      // tf32 hi / lo planes in shared memory, so V crosses HBM once, not twice)
+      // (one base address per thread + a constant step per position)
+      *reinterpret_cast<float4 *>(v_base + static_cast<size_t>(a) * v_step) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
     }
   }
 }
@@ -324,7 +291,7 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
 // FAST: the host has checked that |fma(V, mrepS, tz)| < 2^22 for every possible input (|V| <= 255 *
 // 5.28125^2, the largest absolute row sum of B^T squared), so the rounding by magic-number addition
 // is exact and the general conversion is not even compiled in.
-template <bool FAST>
+template <bool FAST, bool NHWC>
 __global__ void __launch_bounds__(TRANS_THREADS, 512 / TRANS_THREADS) wino_input_u8_kernel(const __grid_constant__ WinoInParams p) {
   const WinoGeom &g = p.g;
   const int quad = threadIdx.x & 3;
@@ -332,7 +299,7 @@ __global__ void __launch_bounds__(TRANS_THREADS, 512 / TRANS_THREADS) wino_input
   const int cb = blockIdx.y;
   if (t >= g.Tpad) return;
   const int mt = t >> 7, row = t & 127;
-  const bool live = t < g.T;
+  const bool live = t < g.T && (!NHWC || cb * 16 + quad * 4 < p.chans);
   int n = 0, th = 0, tw = 0;
   if (live) {
     n = t / (g.ht * g.wt);
@@ -345,13 +312,14 @@ __global__ void __launch_bounds__(TRANS_THREADS, 512 / TRANS_THREADS) wino_input
   uint32_t raw[6][6], outw[36];
   // one base pointer per thread; tiles inside the image load without bounds tests (see the fp32 kernel)
   const uint32_t *plane = reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(p.in) +
-                                                             (static_cast<size_t>(n) * g.CB + cb) * g.IH * g.IW * 16) + quad;
+                                                             pixel_at<NHWC>(n, cb, quad, 0, 0, g.CB, g.IH, g.IW, p.chans));
+  const int pix = NHWC ? p.chans >> 2 : 4;      // words of four channels from one pixel to the next
   if (live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW) {
-    const uint32_t *p0 = plane + (static_cast<size_t>(ih0) * g.IW + iw0) * 4;
+    const uint32_t *p0 = plane + (static_cast<size_t>(ih0) * g.IW + iw0) * pix;
 #pragma unroll
     for (int h = 0; h < 6; ++h)
 #pragma unroll
-      for (int w = 0; w < 6; ++w) raw[h][w] = __ldg(p0 + (h * g.IW + w) * 4);
+      for (int w = 0; w < 6; ++w) raw[h][w] = __ldg(p0 + (h * g.IW + w) * pix);
   } else {
 #pragma unroll
     for (int h = 0; h < 6; ++h)
@@ -359,7 +327,7 @@ __global__ void __launch_bounds__(TRANS_THREADS, 512 / TRANS_THREADS) wino_input
       for (int w = 0; w < 6; ++w) {
         const int ih = ih0 + h, iw = iw0 + w;
         const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-        raw[h][w] = ok ? __ldg(plane + (static_cast<size_t>(ih) * g.IW + iw) * 4) : 0u;
+        raw[h][w] = ok ? __ldg(plane + (static_cast<size_t>(ih) * g.IW + iw) * pix) : 0u;
       }
   }
 #pragma unroll
@@ -437,7 +405,7 @@ __device__ __forceinline__ void bt4(const float (&f)[4], float (&o)[4]) {
 // One thread = one 4x4 tile x 4 consecutive channels (64 values).  IN_U8: quantises to u8 like the
 // F(4x4,3x3) kernel; |V| <= 4 * 255, so the magic-number rounding is exact whenever the host found
 // 1020 * |mrepS| + |tz| < 2^22 (FAST), else the general conversion is kept.
-template <bool IN_U8, bool FAST>
+template <bool IN_U8, bool FAST, bool NHWC>
 __global__ void __launch_bounds__(128) wino4_input_kernel(const __grid_constant__ WinoInParams p) {
   const WinoGeom &g = p.g;
   const int quad = threadIdx.x & 3;
@@ -445,7 +413,7 @@ __global__ void __launch_bounds__(128) wino4_input_kernel(const __grid_constant_
   const int cb = blockIdx.y;
   if (t >= g.Tpad) return;
   const int mt = t >> 7, row = t & 127;
-  const bool live = t < g.T;
+  const bool live = t < g.T && (!NHWC || cb * 16 + quad * 4 < p.chans);
   int n = 0, th = 0, tw = 0;
   if (live) {
     n = t / (g.ht * g.wt);
@@ -461,15 +429,15 @@ __global__ void __launch_bounds__(128) wino4_input_kernel(const __grid_constant_
     for (int w = 0; w < 4; ++w) {
       const int ih = ih0 + h, iw = iw0 + w;
       const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-      const size_t pix = ((static_cast<size_t>(n) * g.CB + cb) * g.IH + (ok ? ih : 0)) * g.IW + (ok ? iw : 0);
+      const size_t at = pixel_at<NHWC>(n, cb, quad, ok ? ih : 0, ok ? iw : 0, g.CB, g.IH, g.IW, p.chans);
       if (IN_U8) {
-        const uint32_t raw = ok ? __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(p.in) + pix * 16) + quad) : 0u;
+        const uint32_t raw = ok ? __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(p.in) + at)) : 0u;
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           d[h][w][c] = __fsub_rn(__uint_as_float(__byte_perm(raw, 0x4B000000u, 0x7650 + c)), 8388608.0f);
       } else {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ok) v = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(p.in) + pix * 16) + quad);
+        if (ok) v = __ldg(reinterpret_cast<const float4 *>(static_cast<const float *>(p.in) + at));
         d[h][w][0] = v.x; d[h][w][1] = v.y; d[h][w][2] = v.z; d[h][w][3] = v.w;
       }
     }
@@ -1321,14 +1289,16 @@ struct WinoOutParams {
   int out_type, with_bias, with_relu, with_sum;
   float orepS, oz;
   float relu_lo, relu_hi;   // fp32 direct convolution only (the Winograd output transform uses a literal 0)
+  int chans;                // nhwc: channels of a pixel, a multiple of 4
 };
 
+template <bool NHWC>
 __global__ void __launch_bounds__(TRANS_THREADS) wino_output_kernel(const __grid_constant__ WinoOutParams p) {
   const WinoGeom &g = p.g;
   const int quad = threadIdx.x & 3;
   const int t = blockIdx.x * TRANS_TILES + (threadIdx.x >> 2);
   const int ocb = blockIdx.y;
-  if (t >= g.T) return;
+  if (t >= g.T || (NHWC && ocb * 16 + quad * 4 >= p.chans)) return;
   const int n = t / (g.ht * g.wt);
   const int r = t - n * g.ht * g.wt;
   const int th = r / g.wt, tw = r - th * g.wt;
@@ -1376,8 +1346,7 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_output_kernel(const __grid
     if (oh >= g.OH) continue;
     if (p.out_type == OUT_F32 && !p.with_sum) {
       // the common case (fp32 result, no residual): bias on channel pairs, one address per row
-      float *row0 = static_cast<float *>(p.out) +
-                    ((((static_cast<size_t>(n) * g.OCB + ocb) * g.OH + oh) * g.OW + 4 * tw) * 16 + quad * 4);
+      float *row0 = static_cast<float *>(p.out) + pixel_at<NHWC>(n, ocb, quad, oh, 4 * tw, g.OCB, g.OH, g.OW, p.chans);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         if (4 * tw + j >= g.OW) continue;
@@ -1389,7 +1358,7 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_output_kernel(const __grid
           v = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
         }
         if (p.with_relu) { v.x = fmaxf(v.x, 0.0f); v.y = fmaxf(v.y, 0.0f); v.z = fmaxf(v.z, 0.0f); v.w = fmaxf(v.w, 0.0f); }
-        *reinterpret_cast<float4 *>(row0 + j * 16) = v;
+        *reinterpret_cast<float4 *>(row0 + j * (NHWC ? p.chans : 16)) = v;
       }
       continue;
     }
@@ -1397,8 +1366,7 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_output_kernel(const __grid
     for (int j = 0; j < 4; ++j) {
       const int ow = 4 * tw + j;
       if (ow >= g.OW) continue;
-      const size_t pix = ((static_cast<size_t>(n) * g.OCB + ocb) * g.OH + oh) * g.OW + ow;
-      uint8_t *dst = static_cast<uint8_t *>(p.out) + (pix * 16 + quad * 4) * elt;
+      uint8_t *dst = static_cast<uint8_t *>(p.out) + pixel_at<NHWC>(n, ocb, quad, oh, ow, g.OCB, g.OH, g.OW, p.chans) * elt;
       float f[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -1448,12 +1416,13 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_output_kernel(const __grid
 // (src/kernel/elk_conv_wino_2x2_3x3_output.hxx:89-97); the epilogue is the one above except that
 // u8 / s8 results are rounded toward minus infinity (:145-153), where every other tile size
 // rounds to nearest even.
+template <bool NHWC>
 __global__ void __launch_bounds__(128) wino4_output_kernel(const __grid_constant__ WinoOutParams p) {
   const WinoGeom &g = p.g;
   const int quad = threadIdx.x & 3;
   const int t = blockIdx.x * 32 + (threadIdx.x >> 2);
   const int ocb = blockIdx.y;
-  if (t >= g.T) return;
+  if (t >= g.T || (NHWC && ocb * 16 + quad * 4 >= p.chans)) return;
   const int n = t / (g.ht * g.wt);
   const int r = t - n * g.ht * g.wt;
   const int th = r / g.wt, tw = r - th * g.wt;
@@ -1492,8 +1461,7 @@ __global__ void __launch_bounds__(128) wino4_output_kernel(const __grid_constant
     for (int j = 0; j < 2; ++j) {
       const int oh = 2 * th + i, ow = 2 * tw + j;
       if (oh >= g.OH || ow >= g.OW) continue;
-      const size_t pix = ((static_cast<size_t>(n) * g.OCB + ocb) * g.OH + oh) * g.OW + ow;
-      uint8_t *dst = static_cast<uint8_t *>(p.out) + (pix * 16 + quad * 4) * elt;
+      uint8_t *dst = static_cast<uint8_t *>(p.out) + pixel_at<NHWC>(n, ocb, quad, oh, ow, g.OCB, g.OH, g.OW, p.chans) * elt;
       float f[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -1691,7 +1659,7 @@ struct WinoImpl {
   HaloPlan *halo = nullptr;   // fp32 KxK / strided: the halo-tiled kernel (conv_halo.cu) does the whole convolution
   bool small_ic = false;   // fp32 Winograd asked for a layer with <= 4 input channels: the CUDA-core direct kernel
   void *d_w_small = nullptr;
-  int ic_real = 0;
+  int ic_real = 0, oc_real = 0;
   size_t in_img_bytes = 0, out_img_bytes = 0;
   size_t a_bytes = 0, b_bytes = 0, m_bytes = 0;
   bool cta2 = false;       // GEMM on pairs of CTAs (weight rows split over the pair)
@@ -1723,7 +1691,7 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   // the input and the output
   w->small_ic = info.kernel == ELB_KERNEL_WINO_F32_UMMA && d.ic <= 4 && host::alignup(d.oc, V) <= 256 &&
                 f32_small_ic_smem_bytes(host::alignup(d.oc, V) / V) <= 200 * 1024;
-  w->ic_real = d.ic;
+  w->ic_real = d.ic; w->oc_real = d.oc;
   if (w->small_ic) info.kernel = ELB_KERNEL_F32_SMALL_IC;
   if (w->kind == KIND_I8) {
     if (d.sampling_kind != ELB_CALIBRATED) { err = "int8 Winograd: only CALIBRATED sampling is implemented"; return ELB_UNIMPLEMENTED; }
@@ -2011,7 +1979,7 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
   WinoImpl *w = pl.impl;
   launches = 0;
   if (!w) { err = "plan not set up"; return ELB_GENERAL_ERROR; }
-  if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) {
+  if (((pl.in_nhwc ? 0 : reinterpret_cast<uintptr_t>(in)) | (pl.out_nhwc ? 0 : reinterpret_cast<uintptr_t>(out))) & 15) {
     err = "input/output tensors must be 16-byte aligned";
     return ELB_GENERAL_ERROR;
   }
@@ -2111,30 +2079,38 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     g.m_tiles = w->g.m_tiles;             // operand image pitch
     // 1. input transform (covers every row of the m-tiles that will be multiplied)
     WinoInParams ip{};
-    ip.in = static_cast<const uint8_t *>(in) + static_cast<size_t>(n0) * (stepped ? static_cast<size_t>(g.CB) * pl.src_h * pl.src_w * 64 : w->in_img_bytes);
+    const size_t in_img = stepped ? static_cast<size_t>(g.CB) * pl.src_h * pl.src_w * 64
+                        : pl.in_nhwc ? w->in_img_bytes / w->ICP * w->ic_real : w->in_img_bytes;
+    ip.in = static_cast<const uint8_t *>(in) + static_cast<size_t>(n0) * in_img;
     ip.a_img = w->d_a;
     ip.g = g;
     ip.step = stepped ? pl.in_step : 1; ip.SH = stepped ? pl.src_h : g.IH; ip.SW = stepped ? pl.src_w : g.IW;
     ip.g.Tpad = m_tiles_run * BM;
     ip.mrepS = w->mrepS; ip.tz = w->tz;
+    ip.chans = w->ic_real;
     dim3 gi((m_tiles_run * BM + TRANS_TILES - 1) / TRANS_TILES, g.CB);
     const bool timed = pl.stage_ev[0] != nullptr && n0 == first;
+    // the kernel for the tensor's layout
+    auto launch = [&](bool nhwc, auto blocked_kernel, auto nhwc_kernel, dim3 grid, int threads, const auto &params) {
+      if (nhwc) nhwc_kernel<<<grid, threads, 0, s>>>(params);
+      else blocked_kernel<<<grid, threads, 0, s>>>(params);
+    };
     if (timed) W_TRY(cudaEventRecord(pl.stage_ev[0], s));
     if (w->direct) {
       f32_gather_kernel<<<dim3((m_tiles_run * BM + 31) / 32, g.k_stages), 128, 0, s>>>(ip);
     } else if (g.A == 4) {
       dim3 g4((m_tiles_run * BM + 31) / 32, g.CB);
       const bool fast = 1020.0f * std::fabs(w->mrepS) + std::fabs(w->tz) < 4194304.0f;
-      if (w->kind != KIND_I8) wino4_input_kernel<false, true><<<g4, 128, 0, s>>>(ip);
-      else if (fast) wino4_input_kernel<true, true><<<g4, 128, 0, s>>>(ip);
-      else wino4_input_kernel<true, false><<<g4, 128, 0, s>>>(ip);
+      if (w->kind != KIND_I8) launch(pl.in_nhwc, wino4_input_kernel<false, true, false>, wino4_input_kernel<false, true, true>, g4, 128, ip);
+      else if (fast) launch(pl.in_nhwc, wino4_input_kernel<true, true, false>, wino4_input_kernel<true, true, true>, g4, 128, ip);
+      else launch(pl.in_nhwc, wino4_input_kernel<true, false, false>, wino4_input_kernel<true, false, true>, g4, 128, ip);
     } else if (w->kind == KIND_I8) {
       // largest |V| for u8 inputs: 255 * (largest absolute row sum of B^T = 5.28125)^2
       const bool fast = 255.0f * 27.8916f * std::fabs(w->mrepS) + std::fabs(w->tz) < 4194304.0f;
-      if (fast) wino_input_u8_kernel<true><<<gi, TRANS_THREADS, 0, s>>>(ip);
-      else wino_input_u8_kernel<false><<<gi, TRANS_THREADS, 0, s>>>(ip);
+      if (fast) launch(pl.in_nhwc, wino_input_u8_kernel<true, false>, wino_input_u8_kernel<true, true>, gi, TRANS_THREADS, ip);
+      else launch(pl.in_nhwc, wino_input_u8_kernel<false, false>, wino_input_u8_kernel<false, true>, gi, TRANS_THREADS, ip);
     }
-    else wino_input_kernel<false><<<gi, TRANS_THREADS, 0, s>>>(ip);
+    else launch(pl.in_nhwc, wino_input_kernel<false>, wino_input_kernel<true>, gi, TRANS_THREADS, ip);
     W_TRY(cudaGetLastError());
     if (timed) W_TRY(cudaEventRecord(pl.stage_ev[1], s));
     // 2. batched GEMM
@@ -2181,16 +2157,17 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
     WinoOutParams op{};
     op.m_in = static_cast<const float *>(w->d_m);
     op.bias = static_cast<const float *>(w->d_bias);
-    op.out = static_cast<uint8_t *>(out) + static_cast<size_t>(n0) * w->out_img_bytes;
+    op.out = static_cast<uint8_t *>(out) + static_cast<size_t>(n0) * (pl.out_nhwc ? w->out_img_bytes / w->OCP * w->oc_real : w->out_img_bytes);
     op.g = g;
+    op.chans = w->oc_real;
     op.g.Tpad = w->g.Tpad;
     op.out_type = w->out_type; op.with_bias = w->with_bias; op.with_relu = w->with_relu; op.with_sum = w->with_sum;
     op.orepS = w->orepS; op.oz = w->oz;
     op.relu_lo = w->relu_lo; op.relu_hi = w->relu_hi;
     dim3 go((g.T + TRANS_TILES - 1) / TRANS_TILES, g.OCB);
     if (w->direct) f32_epilogue_kernel<<<dim3((g.T + 31) / 32, g.OCB), 128, 0, s>>>(op);
-    else if (g.A == 4) wino4_output_kernel<<<dim3((g.T + 31) / 32, g.OCB), 128, 0, s>>>(op);
-    else wino_output_kernel<<<go, TRANS_THREADS, 0, s>>>(op);
+    else if (g.A == 4) launch(pl.out_nhwc, wino4_output_kernel<false>, wino4_output_kernel<true>, dim3((g.T + 31) / 32, g.OCB), 128, op);
+    else launch(pl.out_nhwc, wino_output_kernel<false>, wino_output_kernel<true>, go, TRANS_THREADS, op);
     W_TRY(cudaGetLastError());
     if (timed) W_TRY(cudaEventRecord(pl.stage_ev[3], s));
     launches += 3;
@@ -2201,6 +2178,18 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
 bool wino_input_step_supported(const WinoPlan &pl) {
   const WinoImpl *w = pl.impl;
   return w && w->kind == KIND_F32 && !w->small_ic && !w->flat && !w->direct && w->g.A == 6;
+}
+
+// The transform kernels move four channels at a time: whole groups of four, on their boundary.
+bool wino_reads_nhwc(const WinoPlan &pl, const void *in) {
+  const WinoImpl *w = pl.impl;
+  return w && !w->direct && !w->small_ic && !w->halo && w->ic_real % 4 == 0 &&
+         reinterpret_cast<uintptr_t>(in) % (w->kind == KIND_F32 ? 16 : 4) == 0;
+}
+bool wino_writes_nhwc(const WinoPlan &pl, const void *out) {
+  const WinoImpl *w = pl.impl;
+  return w && !w->direct && !w->small_ic && !w->halo && w->oc_real % 4 == 0 &&
+         reinterpret_cast<uintptr_t>(out) % (w->out_type == OUT_F32 ? 16 : 4) == 0;
 }
 
 bool wino_on_halo(const WinoPlan &pl) { return pl.impl && pl.impl->halo; }
@@ -2413,7 +2402,7 @@ extern "C" ELB_API int elb_wino_f32_conv_noalloc(const elb_conv_desc_t *desc, vo
   op.m_in = m_buf; op.bias = static_cast<const float *>(bias); op.out = output; op.g = g;
   op.out_type = OUT_F32; op.with_bias = d.with_bias; op.with_relu = d.with_relu; op.with_sum = d.with_ip_sum;
   op.orepS = 1.0f; op.oz = 0.0f;
-  wino_output_kernel<<<dim3((g.T + TRANS_TILES - 1) / TRANS_TILES, g.OCB), TRANS_THREADS, 0, s>>>(op);
+  wino_output_kernel<false><<<dim3((g.T + TRANS_TILES - 1) / TRANS_TILES, g.OCB), TRANS_THREADS, 0, s>>>(op);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(ELB_GENERAL_ERROR, std::string("kernel launch failed: ") + cudaGetErrorString(e));
   return ELB_OK;

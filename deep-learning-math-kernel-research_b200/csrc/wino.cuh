@@ -17,7 +17,13 @@ struct WinoPlan {
   // the input tensor is the caller's nchw tensor (only the direct kernel for at most four input
   // channels reads one; set by the C-ABI layer after wino_setup)
   bool in_planar = false;
+  // next call only: the tensor is the caller's nhwc tensor (wino_reads_nhwc / wino_writes_nhwc hold for it)
+  bool in_nhwc = false, out_nhwc = false;
 };
+// Do the transform kernels read / write this nhwc tensor themselves?  (null: any aligned one)
+bool wino_reads_nhwc(const WinoPlan &pl, const void *in);
+bool wino_writes_nhwc(const WinoPlan &pl, const void *out);
+
 // Can this plan read its input with a step (fp32 Winograd F(4x4,3x3) through the transform kernels)?
 bool wino_input_step_supported(const WinoPlan &pl);
 
