@@ -166,7 +166,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     }
     if (lane < RAW_STAGES) { mbar_init(&bar.rfull[lane], 1); mbar_init(&bar.rempty[lane], SPLIT_WARPS); }
     if (lane < 2) mbar_init(&bar.turn[lane], 1);
-    if (lane < MAX_BUFS) { mbar_init(&bar.tfull[lane], 1); mbar_init(&bar.tempty[lane], (p.bufs == 4 ? 4 : 8) * (PAIR ? 2 : 1)); }
+    if (lane < MAX_BUFS) { mbar_init(&bar.tfull[lane], 1); mbar_init(&bar.tempty[lane], (KIND == HALO_I8 && p.spread ? EPI_WARPS : p.bufs == 4 ? 4 : 8) * (PAIR ? 2 : 1)); }
     if (lane == 31) { mbar_init(&bar.parts, 1); *abort_flag = 0; }
     fence_barrier_init();
     fence_proxy_async_smem();
@@ -628,14 +628,17 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     }
   } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS) {
     // ---------------------------------------------------------------- epilogue: one output pixel per thread
-    // int8: group g of four warps serves accumulator g of four, or column half g & 1 of accumulator g >> 1 of two
+    // int8: group g of four warps serves accumulator g of four, or column half g & 1 of accumulator g >> 1 of two, or
+    // (HaloParams::spread) a quarter of the columns of every tile.  (A third value of the step, or this loop compiled twice,
+    // costs 2 to 4 % on other layers.)
     const int quarter = warp & 3, group = (warp - EPI_WARP0) >> 2;
-    const bool whole = p.bufs == 4, sep = STACK || (KIND == HALO_F32 && PAIR && p.sep);
-    const int half = whole ? 0 : group & 1, blk_step = whole ? 1 : 2;
+    const bool four = p.bufs == 4, spread = KIND == HALO_I8 && p.spread != 0, whole = four || spread, sep = STACK || (KIND == HALO_F32 && PAIR && p.sep);
     const int row = quarter * 32 + lane;
-    const int nb16 = p.BN >> 4, cnt = whole ? nb16 : (nb16 - half + 1) >> 1;
-    const int t_step = KIND == HALO_F32 ? 1 : p.bufs, t_shift = whole ? 2 : 1;
-    int t = KIND == HALO_F32 ? 0 : whole ? group : group >> 1;
+    const int nb16 = p.BN >> 4, share = (nb16 + 3) >> 2;
+    const int half = spread ? group * share : whole ? 0 : group & 1, blk_step = whole ? 1 : 2;      // first block of columns, step
+    const int cnt = spread ? min(share, nb16 - half) : whole ? nb16 : (nb16 - half + 1) >> 1;
+    const int t_step = KIND == HALO_F32 || spread ? 1 : p.bufs, t_shift = four ? 2 : 1;
+    int t = KIND == HALO_F32 || spread ? 0 : four ? group : group >> 1;
     bool ok = true;
     // the residual this tile adds: on its way to L2 while the MMAs run
     auto prefetch_residual = [&](const Pixel &px, int nt) {
@@ -714,7 +717,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
       if (!SPLIT) prefetch_residual(px, nt);
       if (!wait_all(&bar.tfull[buf], tph, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_EPILOGUE; break; }
       tc_fence_after_sync();
-      const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (whole ? 128u : 256u) + half * 16;
+      const uint32_t t_addr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * (four ? 128u : 256u) + half * 16;
       auto take = [&](int blk, uint32_t (&r)[16], uint32_t (&r2)[16], const uint4 &pv) {
         if (sep) {
 #pragma unroll
@@ -949,10 +952,11 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       const Parts parts = parts_of(p.groups);
       if (!parts.ok) continue;
       const double b = stays ? 0.0 : pair ? kb / 2 : kb;
-      const double tile = std::max(std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps, group_min) * p.groups + 600 + 300 * (parts.count - 1), epilogue);
+      const double loop = std::max(kstep_cycles(kind, BN, pair != 0, b, ab, stride > 1) * p.ksteps, group_min) * p.groups + 600 + 300 * (parts.count - 1);
+      const double tile = std::max(loop, epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
-      if (p.BN == 0 || t < best * 0.98) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; p.fine = parts.fine; p.chunk_groups = parts.groups; }
+      if (p.BN == 0 || t < best * 0.98) { best = t; hp.loop_ratio = loop / std::max(epilogue, 1.0); p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; p.fine = parts.fine; p.chunk_groups = parts.groups; }
     }
     // few tiles: several CTAs share the K loop of each.  Partial sums cross shared memories at about 9 B/clk.  An SM
     // holds one CTA, and the device no more clusters than its GPCs have room for (15 of 8, 33 of 4).
@@ -1293,7 +1297,16 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   p.row_tiles = ((images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
   const int m_tiles = p.row_tiles * p.col_tiles;
   p.total_tiles = (p.pair ? (m_tiles + 1) / 2 : m_tiles) * p.n_tiles;
-  LaunchConfig lc(hp, p.split > 1 ? p.total_tiles * p.split : p.pair ? 2 * std::min(p.total_tiles, hp.max_clusters) : std::min(p.total_tiles, num_sms), s);
+  const int units = p.split > 1 ? p.total_tiles : std::min(p.total_tiles, p.pair ? hp.max_clusters : num_sms);
+  // int8: sixteen epilogue warps on each tile finish it in a quarter (BN <= 128) or half of the time that a group's share of the
+  // warps takes, but every warp then pays a tile's fixed cost (locating its pixel, waits, releases).  So they share tiles
+  // where the last tile's epilogue is a good part of the launch (one or two tiles per CTA: 64 x 1024 -> 256 1x1 at 14x14
+  // 8.6 -> 8.05 us, 2 x 64 -> 256 1x1 at 56x56 3.95 -> 3.33) or where the K loop outlasts the epilogue anyway (128 -> 256 3x3
+  // stride 2 with a residual 28.4 -> 26.0, 30 x 96 -> 192 at 60x60 21.0 -> 16.2).  Elsewhere it loses: 64 -> 64 at 224x224
+  // 29.6 -> 36.2, 64 x 256 -> 1024 1x1 at 14x14 15.8 -> 16.9, 3 x 62 -> 640 at 99x99 16.1 -> 17.1 (ratio 0.77), and tiles of
+  // few blocks whatever the ratio (20 x 48 -> 48 at 100x100 9.4 -> 11.6; 16 x 128 -> 128 at 56x56 10.1 -> 9.7).
+  p.spread = hp.kind == HALO_I8 && (p.total_tiles <= 2 * units || (p.BN >= 112 && hp.loop_ratio > (p.bufs == 4 ? 1.2 : 0.9)));
+  LaunchConfig lc(hp, units * (p.split > 1 ? p.split : p.pair ? 2 : 1), s);
   const cudaError_t e = cudaLaunchKernelEx(&lc.cfg, pick_kernel(hp), p);
   if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
   return true;

@@ -61,6 +61,7 @@ struct HaloParams {
   int pair;                          // clusters of two CTAs multiply two row tiles by weights of which each holds half
   int split;                         // CTAs that share a tile's K loop (1: none; else one tile per cluster)
   int bufs;                          // accumulators in tensor memory: 4 of up to 128 columns or 2 of up to 256
+  int spread;                        // int8: all epilogue warps share each tile (halo_launch() says when)
   int resident;                      // every weight stage of the (single) n tile stays in shared memory
   int stack;                         // f32: hi and lo weight rows of a chunk stacked (BN <= 128)
   int sep;                           // f32: the lo products have accumulators of their own, BN columns behind the hi ones
@@ -81,6 +82,7 @@ struct HaloPlan {
   HaloParams p{};
   size_t smem_bytes = 0, b_bytes = 0;
   double est_us = 0;                 // modelled time of the whole batch
+  double loop_ratio = 0;             // int8: modelled time of a tile's K loop over its epilogue's
   int max_clusters = 0;              // pairs the device holds at once
   int stride = 1, IH = 0, IW = 0, CB = 0;
   int parity[4] = {0, 0, 0, 0};      // of each plane: row parity * stride + column parity
