@@ -212,10 +212,12 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
   // one base pointer per thread, row and column offsets added to it; tiles that do not touch the
   // image border load without any bounds test (the address arithmetic and the predicates of 36
   // separately addressed loads cost this kernel more than its transform)
+  // (rows and channels that are padding look at the tensor's first pixel)
   const float4 *plane = reinterpret_cast<const float4 *>(static_cast<const float *>(p.in) +
-                                                         pixel_at<NHWC>(n, cb, quad, 0, 0, g.CB, p.SH, p.SW, p.chans));
+                                                         pixel_at<NHWC>(n, live ? cb : 0, live ? quad : 0, 0, 0, g.CB, p.SH, p.SW, p.chans));
   const int col_pitch = p.step * (NHWC ? p.chans >> 2 : 4), row_pitch = p.SW * col_pitch;      // in float4 units
-  if (live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW) {
+  // (one path per warp: lanes on both would pay for both)
+  if (__all_sync(0xFFFFFFFFu, live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW)) {
     const float4 *p0 = plane + static_cast<size_t>(ih0) * row_pitch + iw0 * col_pitch;
 #pragma unroll
     for (int h = 0; h < 6; ++h)
@@ -225,16 +227,21 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
         m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
       }
   } else {
+    // every lane loads, from the nearest pixel inside the plane, so that no load waits for its bounds test
+    int col[6];
 #pragma unroll
-    for (int h = 0; h < 6; ++h)
+    for (int w = 0; w < 6; ++w) col[w] = min(max(iw0 + w, 0), g.IW - 1) * col_pitch;
+#pragma unroll
+    for (int h = 0; h < 6; ++h) {
+      const float4 *line = plane + static_cast<size_t>(min(max(ih0 + h, 0), g.IH - 1)) * row_pitch;
+      const bool row_ok = live && static_cast<unsigned>(ih0 + h) < static_cast<unsigned>(g.IH);
 #pragma unroll
       for (int w = 0; w < 6; ++w) {
-        const int ih = ih0 + h, iw = iw0 + w;
-        const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ok) v = __ldg(plane + static_cast<size_t>(ih) * row_pitch + iw * col_pitch);
-        m[h][w][0] = v.x; m[h][w][1] = v.y; m[h][w][2] = v.z; m[h][w][3] = v.w;
+        const float4 v = __ldg(line + col[w]);
+        const bool ok = row_ok && static_cast<unsigned>(iw0 + w) < static_cast<unsigned>(g.IW);
+        m[h][w][0] = ok ? v.x : 0.f; m[h][w][1] = ok ? v.y : 0.f; m[h][w][2] = ok ? v.z : 0.f; m[h][w][3] = ok ? v.w : 0.f;
       }
+    }
   }
   // pass along h, in place.  (Two channels per instruction, as in the output transform, measured
   // SLOWER here: c1's input transform 0.127 -> 0.137 ms, VGG conv1_2's 0.245 -> 0.264 ms; and without
@@ -284,10 +291,9 @@ __global__ void __launch_bounds__(TRANS_THREADS) wino_input_kernel(const __grid_
   }
 }
 
-// u8 variant (INT8 Winograd): the 36 input words of a thread stay packed (4 channels per word)
-// and the four channels are transformed ONE AFTER THE OTHER, so a thread needs ~36 + 36 + 36
-// registers instead of 36 + 144.  That doubles the warps an SM can hold; the kernel is bound by
-// instruction latency (few warps, long dependent fma chains), not by its 51 MB + 116 MB of traffic.
+// u8 variant (INT8 Winograd) for scales beyond the 16-bit bound of wino_input_u8_pairs_kernel: the 36 input words of a thread stay
+// packed (4 channels per word) and the four channels are transformed ONE AFTER THE OTHER, so a thread needs ~36 + 36 + 36
+// registers instead of 36 + 144.
 // FAST: the host has checked that |fma(V, mrepS, tz)| < 2^22 for every possible input (|V| <= 255 *
 // 5.28125^2, the largest absolute row sum of B^T squared), so the rounding by magic-number addition
 // is exact and the general conversion is not even compiled in.
@@ -387,6 +393,114 @@ __global__ void __launch_bounds__(TRANS_THREADS, 512 / TRANS_THREADS) wino_input
   const size_t v_step = static_cast<size_t>(g.m_tiles) * g.k_stages * 8 * BM * 4;                                        // words to the next one
 #pragma unroll
   for (int a = 0; a < 36; ++a) v_base[a * v_step] = live ? outw[a] : 0u;
+}
+
+
+// bt6 on two channels at once, operation for operation ((-a) * b and a * (-b) are the same product)
+__device__ __forceinline__ void bt6x2(const f32x2 (&f)[6], f32x2 (&o)[6]) {
+  auto k = [](float v) { return pack2(v, v); };
+  const f32x2 t0 = fma2(f[2], k(-2.25f), f[4]);
+  const f32x2 t1 = fma2(f[1], k(-2.25f), f[3]);
+  const f32x2 t2 = fma2(f[2], k(-0.390625f), f[4]);
+  const f32x2 t3 = fma2(f[1], k(-0.390625f), f[3]);
+  const f32x2 t4 = fma2(f[0], k(0.87890625f), f[4]);
+  const f32x2 t5 = fma2(f[1], k(0.87890625f), f[5]);
+  o[0] = fma2(f[2], k(-2.640625f), t4);
+  o[1] = fma2(t1, k(0.625f), t0);
+  o[2] = fma2(t1, k(-0.625f), t0);
+  o[3] = fma2(t3, k(1.5f), t2);
+  o[4] = fma2(t3, k(-1.5f), t2);
+  o[5] = fma2(f[3], k(-2.640625f), t5);
+}
+
+// The u8 transform where |fma(V, mrepS, tz)| < 2^15 for every possible input (the host checks; scales that use the eight bits are a
+// hundredth of that): one thread = one tile x TWO channels, as pairs in every instruction, and the rounded values saturate as
+// pairs of 16-bit integers.  Bound by instruction issue (64 % of the slots; 33 MB read and 58 MB written per 64 x 512 channels at
+// 28x28 take 36 us): with both paths of a border test in most warps it took 43 us, and the kernel below, one channel of four
+// after the other, 40.  The whole layer at 128 images 274 -> 266.6 us, 23 x 992 -> 48 at 71x71 226 -> 213, 3 x 32 -> 16 at 68x68 14.6 -> 13.8.
+constexpr int PAIR_TILES = TRANS_THREADS / 8;      // tiles per block (8 threads = the 16 channels of a block)
+template <bool NHWC>
+__global__ void __launch_bounds__(TRANS_THREADS, 10) wino_input_u8_pairs_kernel(const __grid_constant__ WinoInParams p) {
+  const WinoGeom &g = p.g;
+  const int pair = threadIdx.x & 7;
+  const int t = blockIdx.x * PAIR_TILES + (threadIdx.x >> 3);
+  const int cb = blockIdx.y;
+  if (t >= g.Tpad) return;
+  const int mt = t >> 7, row = t & 127;
+  const bool live = t < g.T && (!NHWC || cb * 16 + pair * 2 < p.chans);
+  int n = 0, th = 0, tw = 0;
+  if (live) {
+    n = t / (g.ht * g.wt);
+    const int r = t - n * g.ht * g.wt;
+    th = r / g.wt;
+    tw = r - th * g.wt;
+  }
+  const int ih0 = 4 * th - g.pad_t, iw0 = 4 * tw - g.pad_l;
+  const bool border = th == 0 || tw == 0 || th == g.ht - 1 || tw == g.wt - 1;   // src/elx_conv_wino_trans_input.hpp:247-249
+  uint32_t raw[6][6];
+  const uint16_t *plane = reinterpret_cast<const uint16_t *>(static_cast<const uint8_t *>(p.in) +
+                                                             pixel_at<NHWC>(n, live ? cb : 0, 0, 0, 0, g.CB, g.IH, g.IW, p.chans)) + (live ? pair : 0);
+  const int pix = NHWC ? p.chans >> 1 : 8;      // pairs of channels from one pixel to the next
+  // (one path per warp: eight tiles in a row hold a border tile on all but wide planes, and lanes on both paths pay for both)
+  if (__all_sync(0xFFFFFFFFu, live && ih0 >= 0 && iw0 >= 0 && ih0 + 5 < g.IH && iw0 + 5 < g.IW)) {
+    const uint16_t *p0 = plane + (static_cast<size_t>(ih0) * g.IW + iw0) * pix;
+#pragma unroll
+    for (int h = 0; h < 6; ++h)
+#pragma unroll
+      for (int w = 0; w < 6; ++w) raw[h][w] = __ldg(p0 + (h * g.IW + w) * pix);
+  } else {
+    // every lane loads, from the nearest pixel inside the plane, and masks what lies outside
+    int col[6];
+    uint32_t col_ok[6];
+#pragma unroll
+    for (int w = 0; w < 6; ++w) {
+      col[w] = min(max(iw0 + w, 0), g.IW - 1) * pix;
+      col_ok[w] = live && static_cast<unsigned>(iw0 + w) < static_cast<unsigned>(g.IW) ? 0xFFFFu : 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < 6; ++h) {
+      const uint16_t *line = plane + static_cast<size_t>(min(max(ih0 + h, 0), g.IH - 1)) * g.IW * pix;
+      const uint32_t row_ok = static_cast<unsigned>(ih0 + h) < static_cast<unsigned>(g.IH) ? 0xFFFFu : 0u;
+#pragma unroll
+      for (int w = 0; w < 6; ++w) raw[h][w] = __ldg(line + col[w]) & (row_ok & col_ok[w]);
+    }
+  }
+  f32x2 m[6][6];
+#pragma unroll
+  for (int w = 0; w < 6; ++w) {          // pass along h
+    f32x2 f[6], o[6];
+#pragma unroll
+    for (int h = 0; h < 6; ++h)          // u8 -> fp32: the permute builds 2^23 + b
+      f[h] = add2(pack2(__uint_as_float(__byte_perm(raw[h][w], 0x4B000000u, 0x7650)), __uint_as_float(__byte_perm(raw[h][w], 0x4B000000u, 0x7651))),
+                  pack2(-8388608.0f, -8388608.0f));
+    bt6x2(f, o);
+#pragma unroll
+    for (int i = 0; i < 6; ++i) m[i][w] = o[i];
+  }
+  uint8_t *v_base = static_cast<uint8_t *>(p.a_img) +
+                    (((static_cast<size_t>(mt) * g.k_stages + (cb >> 3)) * 8 + (cb & 7)) * BM + row) * 16 + pair * 2;      // position 0
+  const uint32_t v_step = static_cast<uint32_t>(g.m_tiles) * g.k_stages * (8 * BM * 16);      // bytes to the next one (the host checks that they fit)
+  const f32x2 rep2 = pack2(p.mrepS, p.mrepS), tz2 = pack2(p.tz, p.tz), magic = pack2(12582912.0f, 12582912.0f);
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {          // pass along w, quantise
+    f32x2 v[6];
+    bt6x2(m[i], v);
+    if ((i == 0 || i == 5) && border) {      // (two corner results of the reference's border kernel, see wino_input_kernel)
+      const f32x2 z2 = pack2(0.87890625f, 0.87890625f), z3 = pack2(-2.640625f, -2.640625f);
+      if (i == 0) v[5] = add2(mul2(m[i][3], z3), add2(mul2(m[i][1], z2), m[i][5]));
+      else v[0] = fma2(m[i][2], z3, add2(mul2(m[i][0], z2), m[i][4]));
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      // rne by the magic addition: the low 16 bits are the integer; as an UNSIGNED number a negative one is large, and one
+      // min() gives the reference's unsigned saturation (below zero -> 255, above 255 -> 255)
+      float lo, hi;
+      unpack2(add2(fma2(v[j], rep2, tz2), magic), lo, hi);
+      const uint32_t q = __vimin3_u16x2(__byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x5410), 0x00FF00FFu, 0x00FF00FFu);
+      // (rows that only fill up a row block and channels that are padding: whatever they hold is not used)
+      *reinterpret_cast<uint16_t *>(v_base + static_cast<size_t>(v_step) * (i * 6 + j)) = static_cast<uint16_t>(__byte_perm(q, 0u, 0x4420));
+    }
+  }
 }
 
 
@@ -2106,8 +2220,10 @@ int wino_run(WinoPlan &pl, void *out, const void *in, void *acc_dump, int *statu
       else launch(pl.in_nhwc, wino4_input_kernel<true, false, false>, wino4_input_kernel<true, false, true>, g4, 128, ip);
     } else if (w->kind == KIND_I8) {
       // largest |V| for u8 inputs: 255 * (largest absolute row sum of B^T = 5.28125)^2
-      const bool fast = 255.0f * 27.8916f * std::fabs(w->mrepS) + std::fabs(w->tz) < 4194304.0f;
-      if (fast) launch(pl.in_nhwc, wino_input_u8_kernel<true, false>, wino_input_u8_kernel<true, true>, gi, TRANS_THREADS, ip);
+      const float most = 255.0f * 27.8916f * std::fabs(w->mrepS) + std::fabs(w->tz);
+      const bool fast = most < 4194304.0f;
+      if (most < 32767.0f && w->a_bytes / 36 < (size_t(1) << 32)) launch(pl.in_nhwc, wino_input_u8_pairs_kernel<false>, wino_input_u8_pairs_kernel<true>, dim3(m_tiles_run * BM / PAIR_TILES, g.CB), TRANS_THREADS, ip);
+      else if (fast) launch(pl.in_nhwc, wino_input_u8_kernel<true, false>, wino_input_u8_kernel<true, true>, gi, TRANS_THREADS, ip);
       else launch(pl.in_nhwc, wino_input_u8_kernel<false, false>, wino_input_u8_kernel<false, true>, gi, TRANS_THREADS, ip);
     }
     else launch(pl.in_nhwc, wino_input_kernel<false>, wino_input_kernel<true>, gi, TRANS_THREADS, ip);
