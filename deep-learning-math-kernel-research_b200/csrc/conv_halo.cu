@@ -276,7 +276,9 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
     const int planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    const bool strided = FORM == FORM_3X3S2 || ((FORM == FORM_ANY || FORM == FORM_1X1 || KIND == HALO_F32) && uni(p.strided) != 0);
+    auto rows = [&](auto how) {      // 0 / 1: not strided / strided, 2: as the parameters say
+    constexpr int HOW = decltype(how)::value;
+    const bool strided = HOW == 2 ? uni(p.strided) != 0 : HOW != 0;
     // stride 1: 8-byte elements, so that the copy engine moves whole rows
     const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
     int s = 0;
@@ -342,6 +344,17 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
           if (++s == stages) { s = 0; ph ^= 1u; }
         }
       }
+    }
+    };
+    // (stride 1: an input read with a step.  A loop of its own for the int8 3x3 forms: tested at every copy it costs narrow
+    // tiles 2 to 3 %)
+    if constexpr (FORM == FORM_3X3S2) {
+      rows(std::integral_constant<int, 1>{});
+    } else if constexpr (FORM == FORM_ANY || FORM == FORM_1X1 || KIND == HALO_F32) {
+      rows(std::integral_constant<int, 2>{});
+    } else {
+      if (uni(p.strided)) rows(std::integral_constant<int, 1>{});
+      else rows(std::integral_constant<int, 0>{});
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- weights
@@ -956,7 +969,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       const double tile = std::max(loop, epilogue);
       const double waves = pair ? std::ceil(std::ceil(m_tiles / 2) * nt / (num_sms / 2)) : std::ceil(m_tiles * nt / num_sms);
       const double t = waves * tile + 4000;
-      if (p.BN == 0 || t < best * 0.98) { best = t; hp.loop_ratio = loop / std::max(epilogue, 1.0); p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; p.fine = parts.fine; p.chunk_groups = parts.groups; }
+      if (p.BN == 0 || t < best * 0.98) { best = t; hp.loop_ratio = loop / std::max(epilogue, 1.0); hp.gather_ratio = ab / 16 / kstep_cycles(kind, BN, pair != 0, 0, 0); p.BN = BN; p.n_tiles = nt; p.pair = pair; p.split = 1; p.fine = parts.fine; p.chunk_groups = parts.groups; }
     }
     // few tiles: several CTAs share the K loop of each.  Partial sums cross shared memories at about 9 B/clk.  An SM
     // holds one CTA, and the device no more clusters than its GPCs have room for (15 of 8, 33 of 4).
@@ -966,7 +979,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
       if (kch == 1 || 2 * sums > 150 * 1024 || !parts.ok) continue;
       const double t = std::max(kstep_cycles(kind, BN, false, kb, ab, stride > 1) * p.ksteps, group_min) * ((p.groups + split - 1) / split) + 600 +
                        4000 + 2000 + sums / 9 + 300 * (parts.count - 1);
-      if (t < best * 0.95) { best = t; p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; p.fine = parts.fine; p.chunk_groups = parts.groups; }
+      if (t < best * 0.95) { best = t; hp.gather_ratio = ab / 16 / kstep_cycles(kind, BN, false, 0, 0); p.BN = BN; p.n_tiles = nt; p.pair = 0; p.split = split; p.fine = parts.fine; p.chunk_groups = parts.groups; }
     }
   }
   if (p.BN == 0) { err = "precision"; return false; }

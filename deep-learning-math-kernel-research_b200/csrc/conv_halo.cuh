@@ -82,6 +82,7 @@ struct HaloPlan {
   HaloParams p{};
   size_t smem_bytes = 0, b_bytes = 0;
   double est_us = 0;                 // modelled time of the whole batch
+  double gather_ratio = 0;           // int8: time of a tile's rows pixel by pixel (16 bytes per clock) over that of its MMAs
   double loop_ratio = 0;             // int8: modelled time of a tile's K loop over its epilogue's
   int max_clusters = 0;              // pairs the device holds at once
   int stride = 1, IH = 0, IW = 0, CB = 0;

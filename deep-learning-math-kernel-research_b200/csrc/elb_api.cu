@@ -565,7 +565,9 @@ int run_i8_direct(elb_conv &pl, void *out, const void *in, int n0, int cnt, cuda
   if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15)
     return fail(ELB_GENERAL_ERROR, "input/output tensors must be 16-byte aligned");
   I8ConvParams p = pl.i8;
-  const size_t in_img = pl.info.bytes_input / pl.d.n, out_img = pl.info.bytes_output / pl.d.n;
+  const int step = pl.wino.in_step;      // (conv_enqueue_stepped)
+  const size_t in_img = step > 1 ? (size_t)p.CB * V * pl.wino.src_h * pl.wino.src_w : pl.info.bytes_input / pl.d.n;
+  const size_t out_img = pl.info.bytes_output / pl.d.n;
   p.in = (const uint8_t *)in + (size_t)n0 * in_img;
   p.out = (uint8_t *)out + (size_t)n0 * out_img;
   p.acc_dump = pl.d_acc_dump ? (int32_t *)pl.d_acc_dump + (size_t)n0 * p.OCB * V * pl.d.oh * pl.d.ow : nullptr;
@@ -580,7 +582,7 @@ int run_i8_direct(elb_conv &pl, void *out, const void *in, int n0, int cnt, cuda
     hp.shift_tbl = p.shift_tbl; hp.hclass = p.hclass; hp.wclass = p.wclass; hp.zp_nw = p.zp_nw; hp.zp_full = p.zp_full;
     hp.out = p.out; hp.acc_dump = p.acc_dump; hp.status = p.status; hp.rq = p.rq;
     std::string err;
-    if (!halo_launch(*pl.halo, hp, p.in, cnt, pl.num_sms, s, err)) return fail(ELB_GENERAL_ERROR, "%s", err.c_str());
+    if (!halo_launch(*pl.halo, hp, p.in, cnt, pl.num_sms, s, err, step, pl.wino.src_h, pl.wino.src_w)) return fail(ELB_GENERAL_ERROR, "%s", err.c_str());
     pl.launches += 1;
     return ELB_OK;
   }
@@ -983,6 +985,28 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
 }
 
 }  // namespace
+
+// What a stack asks of its layers beyond elb_conv_enqueue_strided: INT8 layers on the halo-tiled kernel read their input with a
+// step too, pixel by pixel, where that is hidden behind the tile's MMAs with a margin (64 -> 128 channels 0.6 of them, 128 -> 256
+// 0.3; 32 -> 48 1.1), and so need no subsampled tensor.
+namespace elb {
+bool conv_step_supported(elb_conv_t *plan) {
+  if (elb_conv_input_step_supported(plan)) return true;
+  return plan && plan->halo && !plan->cvt_in && plan->info.kernel == ELB_KERNEL_I8_CONV_UMMA && plan->halo->stride == 1 &&
+         plan->halo->gather_ratio <= 0.8;
+}
+int conv_enqueue_stepped(elb_conv_t *plan, void *output, const void *input, int src_h, int src_w, int step, cudaStream_t s) {
+  if (!conv_step_supported(plan) || (src_h + step - 1) / step != plan->d.ih || (src_w + step - 1) / step != plan->d.iw)
+    return fail(ELB_GENERAL_ERROR, "internal: this plan cannot read its input with a step of %d", step);
+  DeviceGuard guard(plan->device);
+  int rc = do_prepare(*plan, nullptr, nullptr);
+  if (rc != ELB_OK) return rc;
+  plan->wino.in_step = step; plan->wino.src_h = src_h; plan->wino.src_w = src_w;
+  rc = do_enqueue(*plan, output, input, s);
+  plan->wino.in_step = 1;
+  return rc;
+}
+}  // namespace elb
 
 // =============================================================================== C ABI
 extern "C" {
