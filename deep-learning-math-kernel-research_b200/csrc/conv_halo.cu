@@ -120,6 +120,12 @@ __host__ __device__ constexpr int pxw_of(int form, int kind, int pairs) {
                             : (kind == HALO_F32 || pairs == 2 || pairs == 4 ? 10 : pairs == 0 ? 16 : 12);
 }
 
+// Planes and channels of a kernel's HaloArgs
+__host__ __device__ constexpr int planes_of(int form) { return form == FORM_ANY || form == FORM_3X3S2 ? 4 : 1; }
+// (constants of 256 channels cost every call 0.4 us more and gain nothing: 16 x 80 -> 208 at 33x33 8.0 us, 7.6 without)
+constexpr int PARAM_OC = 128;
+__host__ __device__ constexpr int oc_of(int kind, bool split) { return kind == HALO_F32 || split ? 0 : PARAM_OC; }
+
 // PAIR: clusters of two CTAs.  One tcgen05.mma.cta_group::2 multiplies two row tiles (128 rows per CTA) by the BN
 // weight rows of which each CTA stages HALF: what an SM takes in per MMA from L2 and what the MMA reads from its
 // shared memory both fall by the weights' half, and these two (about 50 B/clk, 128 B/clk) bound the tiles of
@@ -135,7 +141,7 @@ __host__ __device__ constexpr int pxw_of(int form, int kind, int pairs) {
 // have accumulators of their own; the epilogue adds all that up in registers, rounding to nearest.
 template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE>
 __global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
-conv_halo_kernel(const __grid_constant__ HaloParams p) {
+conv_halo_kernel(const __grid_constant__ HaloArgs<planes_of(FORM), oc_of(KIND, SPLIT)> p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = smem_aligned(smem_raw);
   constexpr int PLANES = KIND == HALO_I8 ? 1 : 2, EPI_WARPS = KIND == HALO_I8 ? EPI_WARPS_I8 : EPI_WARPS_F32;
@@ -229,7 +235,7 @@ conv_halo_kernel(const __grid_constant__ HaloParams p) {
         for (int i = 0; i < 4; ++i) d[i] = make_int4(a[4 * i], a[4 * i + 1], a[4 * i + 2], a[4 * i + 3]);
       }
       if (p.fast == 2) requant_relu_u8(a, s_scale + ocb * 16, s_shift + ocb * 16, static_cast<uint8_t *>(p.out) + off);
-      else if (p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
+      else if (oc_of(KIND, SPLIT) > 0 && p.fast) requant_relu_u8(a, p.cst[0] + ocb * 16, p.cst[1] + ocb * 16, static_cast<uint8_t *>(p.out) + off);
       else requant_store16(a, s_scale + ocb * 16, px.shift_row + ocb * 16, static_cast<uint8_t *>(p.out) + off * (p.rq.out_type == OUT_F32 ? 4 : 1), p.rq, prev);
     } else {
       float f[16];
@@ -1174,27 +1180,35 @@ bool encode_maps(const HaloPlan &hp, const void *in, int cnt, int step, int src_
 
 namespace {
 
-typedef void (*HaloKernel)(HaloParams);
+// A kernel and what its parameters hold
+struct HaloKernel {
+  const void *fn = nullptr;
+  int planes = 0, oc = 0;
+};
+template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE>
+HaloKernel kernel_of() {
+  return {reinterpret_cast<const void *>(conv_halo_kernel<KIND, PAIRS, FORM, STACK, PAIR, SPLIT, FINE>), planes_of(FORM), oc_of(KIND, SPLIT)};
+}
 template <int FORM, bool PAIR = false, bool SPLIT = false>
 HaloKernel pick_kernel(const HaloPlan &hp) {
   if (hp.kind == HALO_F32) {
     if constexpr (FORM == FORM_3X3_TAPS || (!PAIR && (FORM == FORM_3X3_ROWS || (!SPLIT && FORM == FORM_3X3_RESIDENT))))
-      if (hp.p.fine) return conv_halo_kernel<HALO_F32, 2, FORM, !PAIR, PAIR, SPLIT, true>;
-    if (hp.p.fine) return nullptr;      // (halo_plan() makes no such plan)
+      if (hp.p.fine) return kernel_of<HALO_F32, 2, FORM, !PAIR, PAIR, SPLIT, true>();
+    if (hp.p.fine) return {};      // (halo_plan() makes no such plan)
     if constexpr (!PAIR)
-      if (hp.p.stack) return conv_halo_kernel<HALO_F32, 2, FORM, true, false, SPLIT, false>;
-    return conv_halo_kernel<HALO_F32, 2, FORM, false, PAIR, SPLIT, false>;
+      if (hp.p.stack) return kernel_of<HALO_F32, 2, FORM, true, false, SPLIT, false>();
+    return kernel_of<HALO_F32, 2, FORM, false, PAIR, SPLIT, false>();
   }
   switch (hp.p.kch) {
-    case 8: return conv_halo_kernel<HALO_I8, 4, FORM, false, PAIR, SPLIT, false>;
-    case 6: return conv_halo_kernel<HALO_I8, 3, FORM, false, PAIR, SPLIT, false>;
-    case 4: return conv_halo_kernel<HALO_I8, 2, FORM, false, PAIR, SPLIT, false>;
+    case 8: return kernel_of<HALO_I8, 4, FORM, false, PAIR, SPLIT, false>();
+    case 6: return kernel_of<HALO_I8, 3, FORM, false, PAIR, SPLIT, false>();
+    case 4: return kernel_of<HALO_I8, 2, FORM, false, PAIR, SPLIT, false>();
   }
   if constexpr (!PAIR) {
-    if (hp.p.kch == 2) return conv_halo_kernel<HALO_I8, 1, FORM, false, false, SPLIT, false>;
-    if constexpr (!SPLIT) return conv_halo_kernel<HALO_I8, 0, FORM, false, false, false, false>;
+    if (hp.p.kch == 2) return kernel_of<HALO_I8, 1, FORM, false, false, SPLIT, false>();
+    if constexpr (!SPLIT) return kernel_of<HALO_I8, 0, FORM, false, false, false, false>();
   }
-  return nullptr;
+  return {};
 }
 // The issue loop's form for a geometry (before the weight stages are laid out); FORM_3X3_TAPS stands for all 3x3 ones.
 int tap_form(const HaloPlan &hp) {
@@ -1211,7 +1225,7 @@ HaloKernel pick_form(const HaloPlan &hp, int form) {
   switch (form) {
     case FORM_3X3_ROWS:
       if constexpr (!PAIR) return pick_kernel<FORM_3X3_ROWS, false, SPLIT>(hp);
-      return nullptr;
+      return {};
     case FORM_3X3_TAPS: return pick_kernel<FORM_3X3_TAPS, PAIR, SPLIT>(hp);
     case FORM_3X3S2: return pick_kernel<FORM_3X3S2, PAIR, SPLIT>(hp);
     case FORM_1X1: return pick_kernel<FORM_1X1, PAIR, SPLIT>(hp);
@@ -1248,10 +1262,11 @@ struct LaunchConfig {
 }  // namespace
 
 cudaError_t halo_init(HaloPlan &hp) {
-  cudaError_t e = cudaFuncSetAttribute(pick_kernel(hp), cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
+  const HaloKernel k = pick_kernel(hp);
+  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
   if (e == cudaSuccess && hp.p.pair) {
     LaunchConfig lc(hp, 2, nullptr);
-    e = cudaOccupancyMaxActiveClusters(&hp.max_clusters, pick_kernel(hp), &lc.cfg);
+    e = cudaOccupancyMaxActiveClusters(&hp.max_clusters, k.fn, &lc.cfg);
     if (e == cudaSuccess && hp.max_clusters < 1) e = cudaErrorInvalidConfiguration;
   }
   return e;
@@ -1265,12 +1280,40 @@ bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err) {
   if (!enc) { err = "cuTensorMapEncodeTiled is not available from the driver"; return false; }
   cuuint64_t dims[2] = {64, hp.b_bytes / 512}, strides[1] = {512};
   cuuint32_t box[2] = {64, static_cast<cuuint32_t>(hp.p.b_stage_bytes / 512)}, estr[2] = {1, 1};
-  const CUresult r = enc(&hp.p.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, d_b, dims, strides, box, estr,
+  const CUresult r = enc(&hp.tmap_b, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, d_b, dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { err = "cuTensorMapEncodeTiled failed (" + std::to_string(static_cast<int>(r)) + ")"; return false; }
   return true;
 }
+
+namespace {
+// Launches `k` with the plan's maps (their addresses set to `base[plane]`) and constants behind p
+template <int PLANES, int OC>
+cudaError_t launch_args(const HaloPlan &hp, const HaloParams &p, const HaloPlan::Maps &maps, void *const *base, const HaloKernel &k,
+                        const cudaLaunchConfig_t &cfg, std::string &err) {
+  HaloArgs<PLANES, OC> a;
+  static_cast<HaloParams &>(a) = p;
+  const PFN_replaceAddress set_address = get_replace_address();
+  if (!set_address) { err = "cuTensorMapReplaceAddress is not available from the driver"; return cudaErrorUnknown; }
+  // (with five maps per plane encoded for every new address a call took 7.2 us of host time, strided 8.3, against 4.4)
+  for (int q = 0; q < p.planes; ++q)
+    for (int i = 0; i < HALO_HEIGHTS; ++i) {
+      a.tmap[q][i] = maps.m[q][i];
+      if (((maps.heights[q] >> i) & 1) && set_address(&a.tmap[q][i], base[q]) != CUDA_SUCCESS) {
+        err = "cuTensorMapReplaceAddress failed";
+        return cudaErrorUnknown;
+      }
+    }
+  if (p.pair) a.tmap_b = hp.tmap_b;
+  if (OC > 0 && p.fast == 1) {
+    std::copy_n(hp.scale.data(), p.OCB * 16, a.cst[0]);
+    std::copy_n(hp.shift.data(), p.OCB * 16, a.cst[1]);
+  }
+  void *args[] = {&a};
+  return cudaLaunchKernelExC(&cfg, k.fn, args);
+}
+}  // namespace
 
 bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err,
                  int step, int src_h, int src_w) {
@@ -1287,24 +1330,15 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
     hit = &hp.maps[hp.next_map];
     hp.next_map = (hp.next_map + 1) % 16;
   }
-  std::memcpy(p.tmap, hit->m, sizeof(p.tmap[0]) * p.planes);
-  // (with five maps per plane encoded for every new address a call took 7.2 us of host time, strided 8.3, against 4.4)
-  const PFN_replaceAddress set_address = get_replace_address();
-  if (!set_address) { err = "cuTensorMapReplaceAddress is not available from the driver"; return false; }
-  for (int q = 0; q < p.planes; ++q)
-    for (int i = 0; i < HALO_HEIGHTS; ++i)
-      if ((hit->heights[q] >> i) & 1)
-        if (set_address(&p.tmap[q][i], step > 1 ? const_cast<void *>(in) : plane_base(hp, in, q)) != CUDA_SUCCESS) {
-          err = "cuTensorMapReplaceAddress failed";
-          return false;
-        }
+  void *base[4];
+  for (int q = 0; q < p.planes; ++q) base[q] = step > 1 ? const_cast<void *>(in) : plane_base(hp, in, q);
+  const HaloKernel kernel = pick_kernel(hp);
+  if (p.planes > kernel.planes) { err = "internal: planes"; return false; }
   p.b_img = static_cast<const uint8_t *>(hp.d_b);
   p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;
   const bool fast = p.rq.out_type == OUT_U8 && p.rq.relu && p.rq.relu_lo == 0.0f && p.rq.relu_hi >= 3.0e38f && !p.rq.with_sum &&
                     !p.shift_tbl;
-  p.fast = !fast ? 0 : p.OCB * 16 <= HALO_PARAM_OC ? 1 : 2;
-  if (p.fast == 1)
-    for (int i = 0; i < p.OCB * 16; ++i) { p.cst[0][i] = hp.scale[i]; p.cst[1][i] = hp.shift[i]; }
+  p.fast = !fast ? 0 : p.OCB * 16 <= kernel.oc ? 1 : 2;
   p.N = images;
   if (step > 1) p.strided = 1;
   p.row_tiles = ((images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
@@ -1320,7 +1354,10 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   // few blocks whatever the ratio (20 x 48 -> 48 at 100x100 9.4 -> 11.6; 16 x 128 -> 128 at 56x56 10.1 -> 9.7).
   p.spread = hp.kind == HALO_I8 && (p.total_tiles <= 2 * units || (p.BN >= 112 && hp.loop_ratio > (p.bufs == 4 ? 1.2 : 0.9)));
   LaunchConfig lc(hp, units * (p.split > 1 ? p.split : p.pair ? 2 : 1), s);
-  const cudaError_t e = cudaLaunchKernelEx(&lc.cfg, pick_kernel(hp), p);
+  cudaError_t e;
+  if (kernel.planes == 1) e = kernel.oc ? launch_args<1, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<1, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
+  else e = kernel.oc ? launch_args<4, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<4, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
+  if (!err.empty()) return false;
   if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
   return true;
 }

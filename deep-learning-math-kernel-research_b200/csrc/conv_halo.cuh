@@ -10,7 +10,6 @@ namespace elb {
 
 enum : int { HALO_I8 = 0, HALO_F32 = 1 };
 constexpr int HALO_HEIGHTS = 5;
-constexpr int HALO_PARAM_OC = 256;
 constexpr int HALO_MAX_OC = 2048;      // per-channel constants kept in shared memory
 
 // n / d for 0 <= n < 2^31 as a multiply and a shift (the role loops divide once per tile)
@@ -29,10 +28,8 @@ struct FastDiv {
 #endif
 };
 
+// What a launch needs besides its tensor maps and constants (HaloArgs)
 struct HaloParams {
-  // [row / column parity plane of the input (stride 1: one)][rows a copy brings: 1, 2, 4, 8, all of a tile's]
-  alignas(64) CUtensorMap tmap[4][HALO_HEIGHTS];
-  CUtensorMap tmap_b;                // pairs of CTAs: the packed weights as rows of 512 bytes
   const uint8_t *b_img;              // packed weights [n tile][group][K step][...]
   const float *scale, *shift;        // int8: [OCP] requantisation constants; f32: shift = bias (null: none)
   const float *shift_tbl;            // int8, zero point with padding: shift vectors by (row class, column class)
@@ -69,11 +66,21 @@ struct HaloParams {
   int strided;                       // stride > 1: five-dimensional maps of the parity planes
   int cb_step;                       // channel blocks per group
   int row0[4], rows[4], col0[4];     // rows a tile reads of each plane: first (relative to the tile's), count; first column
-  // int8, up to HALO_PARAM_OC channels: {scale, shift} in the parameter space.  The epilogue reads its constants with
+  int tap_rows[4], tap_cols[4];      // the plane's taps: a rectangle, rows from row0, columns from col0
+};
+
+// Parameters of a kernel that reads up to PLANES planes and keeps the constants of up to OC channels here.  A launch costs the host
+// 0.4 us per kilobyte of parameters and a waiting call 0.5: with room for four planes and 256 channels in every kernel's
+// (5.4 KB) an empty launch took 7.0 us instead of 4.8, and 13.9 instead of 11.0 until it was waited for.
+template <int PLANES, int OC>
+struct HaloArgs : HaloParams {
+  // [row / column parity plane of the input (stride 1: one)][rows a copy brings: 1, 2, 4, 8, all of a tile's]
+  alignas(64) CUtensorMap tmap[PLANES][HALO_HEIGHTS];
+  CUtensorMap tmap_b;                // pairs of CTAs: the packed weights as rows of 512 bytes
+  // int8, up to OC channels: {scale, shift} in the parameter space.  The epilogue reads its constants with
   // every 16 outputs of a pixel, and from the constant bank those reads stay off the shared-memory port, which
   // the MMAs of narrow tiles fill (64 -> 128 channels at 112 x 112, 64 images: 63 -> 47 us without the loads).
-  alignas(16) float cst[2][HALO_PARAM_OC];
-  int tap_rows[4], tap_cols[4];      // the plane's taps: a rectangle, rows from row0, columns from col0
+  alignas(16) float cst[2][OC > 0 ? OC : 1];
 };
 
 // Geometry, packing order and launch parameters of one plan, filled by halo_plan().
@@ -89,10 +96,11 @@ struct HaloPlan {
   int parity[4] = {0, 0, 0, 0};      // of each plane: row parity * stride + column parity
   struct Chunk { int tap, cb; };     // tap -1: zero weights
   std::vector<Chunk> order;          // two (i8) chunks per K step of a group; f32: cb = quarter of the block
+  CUtensorMap tmap_b{};
   std::vector<float> scale, shift;   // int8: host copies of the requantisation constants, [OCP]
   void *d_b = nullptr;               // packed weights (owned by the plan that owns this)
   // Tensor maps of the image counts (and input steps) seen so far, whatever the address: a launch copies them and sets its
-  // input's address in those that its tiles use (`heights`: bit i = the maps of HaloParams::tmap[plane][i]).
+  // input's address in those that its tiles use (`heights`: bit i = the maps of HaloArgs::tmap[plane][i]).
   struct Maps { int cnt, step, src_h, src_w; uint8_t heights[4]; CUtensorMap m[4][HALO_HEIGHTS]; };
   std::vector<Maps> maps;            // at most 16, the oldest replaced
   size_t next_map = 0;
