@@ -373,16 +373,18 @@ int setup_i8_direct(elb_conv &pl) {
     // (ELB_I8_CTA2=1 asks for the pair kernel, which takes the one-copy-per-tap form below)
     const char *on2 = getenv("ELB_I8_CTA2");
     std::string why;
-    // A plain 1x1 layer goes the same way where the GEMM kernel below has few tiles of 128 pixels x BN channels (each
-    // its whole K loop on one SM) or small images half fill them.  Its time, fitted on 1024 -> 256 at 14x14, 256 ->
-    // 1024 at 7x7 and 64 -> 64 at 28x28, 1 to 64 images; one 14x14 image 8.1 -> 6.2 us, 16 of 7x7 6.6 -> 4.4 us.
+    // A plain 1x1 layer goes the same way unless the GEMM kernel below is modelled as fast within 0.85 us, which leaves it single tiles.
+    // Its time per wave of tiles of 128 pixels x BN channels is the K loop's or, up to about 1024 input channels, that of its
+    // eight epilogue warps, of which the direct kernel has sixteen: 32 x 64 -> 256 at 56x56 24.9 us there and 11.0 here (f32 results 36.0
+    // and 32.5, with a residual 42.0 and 23.8), 64 x 256 -> 1024 at 14x14 17.8 / 8.9, 16 x 96 -> 240 at 60x60 17.9 / 8.6,
+    // 5 x 128 -> 128 at 145x94 11.7 / 7.4, 16 x 1024 -> 1024 at 28x28 20.9 / 14.5, 11 x 621 -> 48 at 59x59 10.5 / 10.3.
     const int gemm_bn = p.OCB >= 16 ? 256 : p.OCB >= 8 ? 128 : 64;
     const double gemm_tiles = static_cast<double>(d.n) * ((d.oh * d.ow + 127) / 128) * ((p.OCB * V + gemm_bn - 1) / gemm_bn);
-    const double gemm_us = 2.5 + 0.007 * gemm_bn + std::ceil(gemm_tiles / pl.num_sms) * gemm_bn * (0.006 + 0.0011 * ((p.CB + 7) / 8));
+    const double gemm_us = 2.5 + 0.007 * gemm_bn + std::ceil(gemm_tiles / pl.num_sms) * gemm_bn * std::max(0.0149, 0.006 + 0.0011 * ((p.CB + 7) / 8));
     pl.halo = new HaloPlan();
     if (!(on2 && atoi(on2) > 0) &&
         halo_plan(*pl.halo, HALO_I8, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, pl.num_sms, why) &&
-        (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA || pl.halo->est_us + 1.5 < gemm_us)) {
+        (pl.info.kernel == ELB_KERNEL_I8_CONV_UMMA || pl.halo->est_us + 0.85 < gemm_us)) {
       CUDA_TRY(halo_init(*pl.halo));
       pl.info.launches_per_call = 1;
       return ELB_OK;
