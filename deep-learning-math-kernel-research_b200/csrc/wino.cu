@@ -1828,7 +1828,8 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
   // fp32 convolutions that the halo-tiled direct kernel (conv_halo.cu) runs as a whole:
   //   * direct KxK and strided ones, instead of an im2col tensor written and read once per tap (3x3 stride 2,
   //     64 x 128 -> 256 channels 56x56: 231 MB of it, 252 -> 164 us);
-  //   * plain 1x1 layers of so few tiles that most SMs would have none (1024 -> 256 at 14x14, one image 47 -> 13 us);
+  //   * plain 1x1 layers of so few tiles that most SMs would have none (1024 -> 256 at 14x14, one image 47 -> 13 us) or of few input
+  //     channels (16 x 64 -> 256 at 56x56 27 -> 18 us);
   //   * Winograd requests where nine products per output cost less than moving V and M through memory and
   //     transforming them: few channels (VGG conv1_2 at 64 images 1574 -> about 1150 us, conv2_1 556 -> 420;
   //     conv2_2 within a few percent either way, conv3_1 stays), or a single image, where the 36 transformed weight planes
@@ -1859,6 +1860,17 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     if (take && w->flat) {      // the GEMM kernel: fitted on 1024 -> 256 at 14x14, 64 -> 64 at 28x28, 256 -> 1024 at 7x7
       const double tiles = static_cast<double>(d.n) * ((d.oh * d.ow + BM - 1) / BM) * w->n_tiles;
       take = hp->est_us < 6 + 0.65 * g.k_stages * std::ceil(tiles / sms);
+      // With few input channels the GEMM kernel waits for its eight epilogue warps' scattered stores, 6.3 us per wave of 256-wide tiles;
+      // the direct kernel's rows pass through its splitters, 0.75 us per channel group.  Both fitted on 18 layers of 16 to 1024 input
+      // channels, within 10 %: 16 x 64 -> 256 at 56x56 27.2 us there and 18.1 here, 5 x 64 -> 403 at 94x145 57.0 / 37.9, 64 x 512 -> 2048 at
+      // 7x7 71.9 / 53.3; 16 x 256 -> 64 at 56x56 27.8 / 36.5, 64 x 1024 -> 256 at 14x14 42.4 / 52.3.
+      if (!take && hp->p.split == 1) {
+        const HaloParams &h = hp->p;
+        const double units = h.pair ? sms / 2 : sms, m = static_cast<double>(h.row_tiles) * h.col_tiles;
+        const double waves = std::ceil(std::ceil(m / (h.pair ? 2 : 1)) * h.n_tiles / units);
+        const double halo_us = 2.3 + waves * (0.75 * g.CB + 0.0075 * h.BN), gemm_us = 4 + std::ceil(tiles / sms) * (0.39 * g.CB + 0.0245 * w->BN);
+        take = halo_us < 0.95 * gemm_us;
+      }
     }
     if (take && wino_f32 && !w->small_ic) {
       // modelled time of the transform kernels: traffic at 5.8 TB/s, the GEMM at 3 x its operations in 0.8 PFLOP/s if
