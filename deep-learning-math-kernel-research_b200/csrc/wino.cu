@@ -104,7 +104,7 @@ __device__ __forceinline__ void bt6(const float (&f)[6], float (&o)[6]) {
 }
 
 // Two-lane fp32 arithmetic (add / mul / fma .f32x2: each lane rounds exactly as the scalar
-// instruction does).  The output transform runs few warps per SM and the four channels of a thread go
+// instruction does; but ptxas makes one fma of a mul2 whose result an add2 takes, .rn or not).  The output transform runs few warps per SM and the four channels of a thread go
 // through identical arithmetic: as two channel pairs the same work is half the instructions and,
 // as compiled, 136 registers instead of 181 (c1's output transform 0.147 -> 0.137 ms, VGG conv1_2's
 // 0.282 -> 0.259 ms).
@@ -486,9 +486,18 @@ __global__ void __launch_bounds__(TRANS_THREADS, 10) wino_input_u8_pairs_kernel(
     f32x2 v[6];
     bt6x2(m[i], v);
     if ((i == 0 || i == 5) && border) {      // (two corner results of the reference's border kernel, see wino_input_kernel)
-      const f32x2 z2 = pack2(0.87890625f, 0.87890625f), z3 = pack2(-2.640625f, -2.640625f);
-      if (i == 0) v[5] = add2(mul2(m[i][3], z3), add2(mul2(m[i][1], z2), m[i][5]));
-      else v[0] = fma2(m[i][2], z3, add2(mul2(m[i][0], z2), m[i][4]));
+      // As scalars: ptxas joins mul.rn.f32x2 and the add.rn.f32x2 behind it into one fma, which rounds once instead of twice.
+      const float z2 = 0.87890625f, z3 = -2.640625f;
+      float a[2], b[2], c[2], o[2];
+      unpack2(m[i][i == 0 ? 1 : 0], a[0], a[1]);
+      unpack2(m[i][i == 0 ? 3 : 2], b[0], b[1]);
+      unpack2(m[i][i == 0 ? 5 : 4], c[0], c[1]);
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const float t = __fadd_rn(__fmul_rn(a[l], z2), c[l]);
+        o[l] = i == 0 ? __fadd_rn(__fmul_rn(b[l], z3), t) : __fmaf_rn(b[l], z3, t);
+      }
+      v[i == 0 ? 5 : 0] = pack2(o[0], o[1]);
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
