@@ -1346,13 +1346,22 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   p.total_tiles = (p.pair ? (m_tiles + 1) / 2 : m_tiles) * p.n_tiles;
   const int units = p.split > 1 ? p.total_tiles : std::min(p.total_tiles, p.pair ? hp.max_clusters : num_sms);
   // int8: sixteen epilogue warps on each tile finish it in a quarter (BN <= 128) or half of the time that a group's share of the
-  // warps takes, but every warp then pays a tile's fixed cost (locating its pixel, waits, releases).  So they share tiles
-  // where the last tile's epilogue is a good part of the launch (one or two tiles per CTA: 64 x 1024 -> 256 1x1 at 14x14
-  // 8.6 -> 8.05 us, 2 x 64 -> 256 1x1 at 56x56 3.95 -> 3.33) or where the K loop outlasts the epilogue anyway (128 -> 256 3x3
-  // stride 2 with a residual 28.4 -> 26.0, 30 x 96 -> 192 at 60x60 21.0 -> 16.2).  Elsewhere it loses: 64 -> 64 at 224x224
-  // 29.6 -> 36.2, 64 x 256 -> 1024 1x1 at 14x14 15.8 -> 16.9, 3 x 62 -> 640 at 99x99 16.1 -> 17.1 (ratio 0.77), and tiles of
-  // few blocks whatever the ratio (20 x 48 -> 48 at 100x100 9.4 -> 11.6; 16 x 128 -> 128 at 56x56 10.1 -> 9.7).
-  p.spread = hp.kind == HALO_I8 && (p.total_tiles <= 2 * units || (p.BN >= 112 && hp.loop_ratio > (p.bufs == 4 ? 1.2 : 0.9)));
+  // warps takes, but every warp then pays a tile's fixed cost (locating its pixel, waits, releases).  Graph replays, us without / with:
+  //  * one tile per CTA (a split K loop too): the launch ends with it: 1 x 128 -> 544 1x1 at 27x27 with f32 results 3.64 / 3.44;
+  //  * two tiles, results of bytes: 42 x 298 -> 128 1x1 at 24x24 with a residual 10.8 / 8.7, 26 x 80 -> 128 3x3 at 27x31 10.2 / 8.7; with
+  //    more than 128 columns (half of the warps work on a tile as it is) only where the K loop is not much shorter than the epilogue:
+  //    7 x 25 -> 160 at 70x70 8.4 / 9.0 and 39 x 119 -> 528 at 14x14 5.7 / 6.1 (ratios 0.3, 0.5), 3 x 528 -> 192 at 101x107 9.0 / 8.8 (0.8);
+  //  * a K loop that outlasts the epilogue anyway: 128 -> 256 3x3 stride 2 with a residual 28.4 / 26.0, 5 x 176 -> 1439 3x3 at 41x41
+  //    28.1 / 26.0.  Not pairs on a 1x1 filter, where a tile's few K steps wait for 32 warps of two CTAs to hand an accumulator
+  //    back: 13 x 592 -> 1184 at 83x83 98 / 117, 13 x 704 -> 604 at 51x83 53 / 57.
+  // Elsewhere it loses: 64 -> 64 at 224x224 29.6 / 36.2, 64 x 256 -> 1024 1x1 at 14x14 15.8 / 16.9; so do f32 results, which are bound by
+  // their stores, behind the first tile (6 x 640 -> 297 1x1 at 74x62 18.2 / 19.7), one block of columns, which feeds a single group (16
+  // columns: 42 x 357 -> 16 at 24x26 5.5 / 5.8), and tiles of few blocks in a row (20 x 48 -> 48 at 100x100 9.4 / 11.6).
+  const bool bytes = p.rq.out_type != OUT_F32, long_loop = p.BN >= 112 && hp.loop_ratio > (p.bufs == 4 ? 1.2 : 0.9);
+  const bool pair_1x1 = p.pair && 2 * p.ksteps == p.kch;
+  p.spread = hp.kind == HALO_I8 && p.BN >= 32 &&
+             (p.total_tiles <= units ||
+              (bytes && ((p.total_tiles <= 2 * units && (p.BN <= 128 || hp.loop_ratio > 0.65)) || (long_loop && !pair_1x1))));
   LaunchConfig lc(hp, units * (p.split > 1 ? p.split : p.pair ? 2 : 1), s);
   cudaError_t e;
   if (kernel.planes == 1) e = kernel.oc ? launch_args<1, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<1, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
