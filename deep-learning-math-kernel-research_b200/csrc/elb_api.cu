@@ -373,14 +373,18 @@ int setup_i8_direct(elb_conv &pl) {
     // (ELB_I8_CTA2=1 asks for the pair kernel, which takes the one-copy-per-tap form below)
     const char *on2 = getenv("ELB_I8_CTA2");
     std::string why;
-    // A plain 1x1 layer goes the same way unless the GEMM kernel below is modelled as fast within 0.85 us, which leaves it single tiles.
-    // Its time per wave of tiles of 128 pixels x BN channels is the K loop's or, up to about 1024 input channels, that of its
-    // eight epilogue warps, of which the direct kernel has sixteen: 32 x 64 -> 256 at 56x56 24.9 us there and 11.0 here (f32 results 36.0
-    // and 32.5, with a residual 42.0 and 23.8), 64 x 256 -> 1024 at 14x14 17.8 / 8.9, 16 x 96 -> 240 at 60x60 17.9 / 8.6,
-    // 5 x 128 -> 128 at 145x94 11.7 / 7.4, 16 x 1024 -> 1024 at 28x28 20.9 / 14.5, 11 x 621 -> 48 at 59x59 10.5 / 10.3.
+    // A plain 1x1 layer goes the same way unless the GEMM kernel below is modelled as fast within 0.85 us, which leaves it layers
+    // of single tiles and those whose whole filter stays in shared memory in several channel groups, a form that the direct kernel is slow
+    // on (halo_plan()): 49 x 149 -> 16 at 41x66 10.6 us there and 20.9 here, 9 x 144 -> 32 at 72x114 7.2 / 12.2, 1 x 144 -> 32 at 13x13 3.6 / 4.7.
+    // Its time per wave of tiles of 128 pixels x BN channels is the K loop's (0.15 us a stage at least) or, up to about 1024 input channels, that
+    // of its eight epilogue warps, of which the direct kernel has sixteen: 32 x 64 -> 256 at 56x56 24.9 us there and 11.0 here (f32 results
+    // 36.0 and 32.5, with a residual 42.0 and 23.8), 64 x 256 -> 1024 at 14x14 17.8 / 8.9, 16 x 96 -> 240 at 60x60 17.9 / 8.6,
+    // 5 x 128 -> 128 at 145x94 11.7 / 7.4, 16 x 1024 -> 1024 at 28x28 20.9 / 14.5.  On 560 layers of 16 to 1024 input channels the rule's choice
+    // takes 0.7 % more than the faster of the two.
     const int gemm_bn = p.OCB >= 16 ? 256 : p.OCB >= 8 ? 128 : 64;
     const double gemm_tiles = static_cast<double>(d.n) * ((d.oh * d.ow + 127) / 128) * ((p.OCB * V + gemm_bn - 1) / gemm_bn);
-    const double gemm_us = 2.5 + 0.007 * gemm_bn + std::ceil(gemm_tiles / pl.num_sms) * gemm_bn * std::max(0.0149, 0.006 + 0.0011 * ((p.CB + 7) / 8));
+    const double gemm_tile = std::max(0.0149 * gemm_bn, 0.006 * gemm_bn + (p.CB + 7) / 8 * std::max(0.0011 * gemm_bn, 0.15));
+    const double gemm_us = 2.5 + 0.007 * gemm_bn + std::ceil(gemm_tiles / pl.num_sms) * gemm_tile;
     pl.halo = new HaloPlan();
     if (!(on2 && atoi(on2) > 0) &&
         halo_plan(*pl.halo, HALO_I8, d.n, d.ic, d.oc, d.ih, d.iw, d.oh, d.ow, d.kh, d.kw, d.stride_h, d.pad_t, d.pad_l, pl.num_sms, why) &&
