@@ -1358,16 +1358,19 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   //  * two tiles, results of bytes: 42 x 298 -> 128 1x1 at 24x24 with a residual 10.8 / 8.7, 26 x 80 -> 128 3x3 at 27x31 10.2 / 8.7; with
   //    more than 128 columns (half of the warps work on a tile as it is) only where the K loop is not much shorter than the epilogue:
   //    7 x 25 -> 160 at 70x70 8.4 / 9.0 and 39 x 119 -> 528 at 14x14 5.7 / 6.1 (ratios 0.3, 0.5), 3 x 528 -> 192 at 101x107 9.0 / 8.8 (0.8);
-  //  * a K loop that outlasts the epilogue anyway: 128 -> 256 3x3 stride 2 with a residual 28.4 / 26.0, 4 x 608 -> 144 1x1 at 104x97
-  //    11.7 / 11.2; of pairs by half as much again, because a tile waits for 32 warps of two CTAs to hand an accumulator back: 5 x 176 -> 1439
-  //    3x3 at 41x41 28.1 / 26.0 (ratio 1.85), 4 x 128 -> 640 3x3 at 41x41 11.6 / 12.1 (1.30), 13 x 592 -> 1184 1x1 at 83x83 98 / 117 (1.26).
+  //  * a K loop that outlasts the epilogue anyway: 128 -> 256 3x3 stride 2 with a residual 28.4 / 26.0, 4 x 608 -> 144 1x1 at 104x97 11.7 / 11.2;
+  //    of pairs by half as much again, because a tile waits for 32 warps of two CTAs to hand an accumulator back: 5 x 176 -> 1439
+  //    3x3 at 41x41 28.1 / 26.0 (ratio 1.85), 4 x 128 -> 640 3x3 at 41x41 11.6 / 12.1 (1.30);
+  //  * of pairs on a 1x1 filter, in launches of up to five tiles per CTA: 21 x 656 -> 848 at 15x14 with a residual 13.5 / 11.8, 6 x 656 -> 1264
+  //    at 40x40 17.8 / 16.7 (1.03); 44 x 560 -> 1035 at 57x57 (60 tiles) 122 / 142, 18 x 592 -> 305 at 46x49 (160 columns, 1.26) 21.8 / 23.2.
   // Elsewhere it loses: 64 -> 64 at 224x224 29.6 / 36.2, 63 x 336 -> 848 1x1 at 37x37 72.2 / 77.4 (ratio 0.95); so do f32 results, which are
   // bound by their stores, behind the first tile (6 x 640 -> 297 1x1 at 74x62 18.2 / 19.7), one block of columns, which feeds a single group
   // (16 columns: 42 x 357 -> 16 at 24x26 5.5 / 5.8), and tiles of few blocks in a row (20 x 48 -> 48 at 100x100 9.4 / 11.6).
-  const double need = p.pair ? 1.5 : p.bufs == 4 ? 1.2 : 1.0;
+  const bool pair_1x1 = p.pair && 2 * p.ksteps == p.kch;
+  const double need = pair_1x1 ? (p.BN >= 224 ? 1.0 : 1.4) : p.pair ? 1.5 : p.bufs == 4 ? 1.2 : 1.0;
   const bool two = p.total_tiles <= 2 * units && (p.pair ? hp.loop_ratio > need : p.BN <= 128 || hp.loop_ratio > 0.65);
-  p.spread = hp.kind == HALO_I8 && p.BN >= 32 &&
-             (p.total_tiles <= units || (p.rq.out_type != OUT_F32 && (two || (p.BN >= 112 && hp.loop_ratio > need))));
+  const bool loop = p.BN >= 112 && hp.loop_ratio > need && !(pair_1x1 && p.total_tiles > 5 * units);
+  p.spread = hp.kind == HALO_I8 && p.BN >= 32 && (p.total_tiles <= units || (p.rq.out_type != OUT_F32 && (two || loop)));
   LaunchConfig lc(hp, units * (p.split > 1 ? p.split : p.pair ? 2 : 1), s);
   cudaError_t e;
   if (kernel.planes == 1) e = kernel.oc ? launch_args<1, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<1, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
