@@ -1869,15 +1869,21 @@ int wino_setup(WinoPlan &pl, const elb_conv_desc_t &d, elb_conv_info_t &info, st
     if (take && w->flat) {      // the GEMM kernel: fitted on 1024 -> 256 at 14x14, 64 -> 64 at 28x28, 256 -> 1024 at 7x7
       const double tiles = static_cast<double>(d.n) * ((d.oh * d.ow + BM - 1) / BM) * w->n_tiles;
       take = hp->est_us < 6 + 0.65 * g.k_stages * std::ceil(tiles / sms);
-      // With few input channels the GEMM kernel waits for its eight epilogue warps' scattered stores, 6.3 us per wave of 256-wide tiles;
-      // the direct kernel's rows pass through its splitters, 0.75 us per channel group.  Both fitted on 18 layers of 16 to 1024 input
-      // channels, within 10 %: 16 x 64 -> 256 at 56x56 27.2 us there and 18.1 here, 5 x 64 -> 403 at 94x145 57.0 / 37.9, 64 x 512 -> 2048 at
-      // 7x7 71.9 / 53.3; 16 x 256 -> 64 at 56x56 27.8 / 36.5, 64 x 1024 -> 256 at 14x14 42.4 / 52.3.
+      // That one is about launches of few tiles, where the GEMM kernel's K loop is bare.  With few input channels it waits for its eight
+      // epilogue warps' scattered stores, 6.3 us per wave of 256-wide tiles; the direct kernel's rows pass through its splitters, 0.75 us per
+      // channel group.  Both fitted on 18 layers of 16 to 1024 input channels, within 10 %: 16 x 64 -> 256 at 56x56 27.2 us there and 18.1
+      // here, 5 x 64 -> 403 at 94x145 57.0 / 37.9, 64 x 512 -> 2048 at 7x7 71.9 / 53.3; 16 x 256 -> 64 at 56x56 27.8 / 36.5, 64 x 1024 -> 256 at
+      // 14x14 42.4 / 52.3.  What the two rules choose takes 0.3 % more than the faster kernel on 400 layers, and never 1 % more than
+      // the first rule's choice.
       if (!take && hp->p.split == 1) {
         const HaloParams &h = hp->p;
         const double units = h.pair ? sms / 2 : sms, m = static_cast<double>(h.row_tiles) * h.col_tiles;
         const double waves = std::ceil(std::ceil(m / (h.pair ? 2 : 1)) * h.n_tiles / units);
-        const double halo_us = 2.3 + waves * (0.75 * g.CB + 0.0075 * h.BN), gemm_us = 4 + std::ceil(tiles / sms) * (0.39 * g.CB + 0.0245 * w->BN);
+        // (A residual costs wide tiles behind the first more here than there: 24 x 32 -> 742 at 25x25 31.6 us there and 33.8 here,
+        // 14 x 144 -> 1392 at 32x32 52.6 / 55.6.)
+        const bool wide_sum = d.with_ip_sum && h.BN > 208 && waves > 1;
+        const double halo_us = 2.3 + waves * (0.75 * g.CB + (wide_sum ? 0.0245 : 0.0075) * h.BN);
+        const double gemm_us = 4 + std::ceil(tiles / sms) * (0.39 * g.CB + (wide_sum ? 0.0325 : 0.0245) * w->BN);
         take = halo_us < 0.95 * gemm_us;
       }
     }
