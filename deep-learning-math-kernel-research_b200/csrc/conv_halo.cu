@@ -1297,19 +1297,19 @@ bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err) {
 namespace {
 // Launches `k` with the plan's maps (their addresses set to `base[plane]`) and constants behind p
 template <int PLANES, int OC>
-cudaError_t launch_args(const HaloPlan &hp, const HaloParams &p, const HaloPlan::Maps &maps, void *const *base, const HaloKernel &k,
-                        const cudaLaunchConfig_t &cfg, std::string &err) {
+bool launch_args(const HaloPlan &hp, const HaloParams &p, const HaloPlan::Maps &maps, void *const *base, const HaloKernel &k,
+                 const cudaLaunchConfig_t &cfg, std::string &err) {
   HaloArgs<PLANES, OC> a;
   static_cast<HaloParams &>(a) = p;
   const PFN_replaceAddress set_address = get_replace_address();
-  if (!set_address) { err = "cuTensorMapReplaceAddress is not available from the driver"; return cudaErrorUnknown; }
+  if (!set_address) { err = "cuTensorMapReplaceAddress is not available from the driver"; return false; }
   // (with five maps per plane encoded for every new address a call took 7.2 us of host time, strided 8.3, against 4.4)
   for (int q = 0; q < p.planes; ++q)
     for (int i = 0; i < HALO_HEIGHTS; ++i) {
       a.tmap[q][i] = maps.m[q][i];
       if (((maps.heights[q] >> i) & 1) && set_address(&a.tmap[q][i], base[q]) != CUDA_SUCCESS) {
         err = "cuTensorMapReplaceAddress failed";
-        return cudaErrorUnknown;
+        return false;
       }
     }
   if (p.pair) a.tmap_b = hp.tmap_b;
@@ -1318,7 +1318,9 @@ cudaError_t launch_args(const HaloPlan &hp, const HaloParams &p, const HaloPlan:
     std::copy_n(hp.shift.data(), p.OCB * 16, a.cst[1]);
   }
   void *args[] = {&a};
-  return cudaLaunchKernelExC(&cfg, k.fn, args);
+  const cudaError_t e = cudaLaunchKernelExC(&cfg, k.fn, args);
+  if (e != cudaSuccess) err = std::string("kernel launch failed: ") + cudaGetErrorString(e);
+  return e == cudaSuccess;
 }
 }  // namespace
 
@@ -1372,12 +1374,9 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   const bool loop = p.BN >= 112 && hp.loop_ratio > need && !(pair_1x1 && p.total_tiles > 5 * units);
   p.spread = hp.kind == HALO_I8 && p.BN >= 32 && (p.total_tiles <= units || (p.rq.out_type != OUT_F32 && (two || loop)));
   LaunchConfig lc(hp, units * (p.split > 1 ? p.split : p.pair ? 2 : 1), s);
-  cudaError_t e;
-  if (kernel.planes == 1) e = kernel.oc ? launch_args<1, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<1, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
-  else e = kernel.oc ? launch_args<4, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<4, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
-  if (!err.empty()) return false;
-  if (e != cudaSuccess) { err = std::string("kernel launch failed: ") + cudaGetErrorString(e); return false; }
-  return true;
+  if (kernel.planes == 1)
+    return kernel.oc ? launch_args<1, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<1, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
+  return kernel.oc ? launch_args<4, PARAM_OC>(hp, p, *hit, base, kernel, lc.cfg, err) : launch_args<4, 0>(hp, p, *hit, base, kernel, lc.cfg, err);
 }
 
 }  // namespace elb
