@@ -282,85 +282,85 @@ conv_halo_kernel(const __grid_constant__ HaloArgs<planes_of(FORM), oc_of(KIND, S
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
     const int planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    auto rows = [&](auto how) {      // 0 / 1: not strided / strided, 2: as the parameters say
-    constexpr int HOW = decltype(how)::value;
-    const bool strided = HOW == 2 ? uni(p.strided) != 0 : HOW != 0;
-    // stride 1: 8-byte elements, so that the copy engine moves whole rows
-    const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
-    int s = 0;
-    uint32_t ph = 0;
-    bool ok = true;
-    for (int tile = first; tile < p.total_tiles && ok; tile += step) {
-      const int mt = PAIR ? 2 * p.div_n.div(tile) + rank : p.div_n.div(tile);
-      const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
-      // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
-      // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
-      // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
-      constexpr int Q = FORM == FORM_ANY || FORM == FORM_3X3S2 ? 4 : 1;      // planes the code is written out for
-      int idx[Q], img[Q], row[Q];
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        if (Q > 1 && q >= planes) continue;
-        const int rows = p.rows[q], v0 = rt * TILE_H + p.row0[q];
-        int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
-        if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
-        idx[q] = -1;
-        if (h + rows <= period) {
-          if (lane == 0) idx[q] = HALO_HEIGHTS - 1;
-        } else {
-          const int v = v0 + lane;
-          n = v > 0 ? p.div_period.div(v) : 0;
-          h = v - n * period;
-          const int n_prev = __shfl_up_sync(0xFFFFFFFFu, n, 1);
-          const uint32_t starts = __ballot_sync(0xFFFFFFFFu, lane == 0 || n != n_prev || lane == rows);
-          if (lane < rows) {
-            const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
-            const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
-            const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
-            if (at < (len & ~7)) {
-              if ((at & 7) == 0) idx[q] = 3;
-            } else {
-              const int sub = at & 7, rest = len - at;
-              if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx[q] = 31 - __clz(rest);
-            }
-          }
-        }
-        img[q] = n; row[q] = h;
-      }
-      for (int g = g0; g < g1 && ok; ++g) {
+    auto fetch_rows = [&](auto how) {      // 0 / 1: not strided / strided, 2: as the parameters say
+      constexpr int HOW = decltype(how)::value;
+      const bool strided = HOW == 2 ? uni(p.strided) != 0 : HOW != 0;
+      // stride 1: 8-byte elements, so that the copy engine moves whole rows
+      const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      for (int tile = first; tile < p.total_tiles && ok; tile += step) {
+        const int mt = PAIR ? 2 * p.div_n.div(tile) + rank : p.div_n.div(tile);
+        const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
+        // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
+        // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
+        // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
+        constexpr int Q = FORM == FORM_ANY || FORM == FORM_3X3S2 ? 4 : 1;      // planes the code is written out for
+        int idx[Q], img[Q], row[Q];
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-          if (Q > 1 && (q >= planes || !ok)) continue;
-          if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; continue; }
-          if (lane == 0 && (rank == 0 || !PAIR_A))
-            mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(p.rows[q] * pitch) * (PAIR_A ? 2u : 1u));
-          if (idx[q] >= 0) {
-            uint8_t *d = ring + s * stage_bytes + lane * pitch;
-            const int x = (ct * TILE_W + p.col0[q]) * x_unit, c = g * cb_step;
-            if (PAIR_A) {
-              const uint32_t pair_bar = mapa_u32(&full[s], 0);
-              if (!strided) tma_tile_4d_pair(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], pair_bar);
-              else tma_tile_5d_pair(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], pair_bar);
-            } else {
-              if (!strided) tma_tile_4d(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], &full[s]);
-              else tma_tile_5d(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], &full[s]);
+          if (Q > 1 && q >= planes) continue;
+          const int rows = p.rows[q], v0 = rt * TILE_H + p.row0[q];
+          int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
+          if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
+          idx[q] = -1;
+          if (h + rows <= period) {
+            if (lane == 0) idx[q] = HALO_HEIGHTS - 1;
+          } else {
+            const int v = v0 + lane;
+            n = v > 0 ? p.div_period.div(v) : 0;
+            h = v - n * period;
+            const int n_prev = __shfl_up_sync(0xFFFFFFFFu, n, 1);
+            const uint32_t starts = __ballot_sync(0xFFFFFFFFu, lane == 0 || n != n_prev || lane == rows);
+            if (lane < rows) {
+              const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
+              const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
+              const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
+              if (at < (len & ~7)) {
+                if ((at & 7) == 0) idx[q] = 3;
+              } else {
+                const int sub = at & 7, rest = len - at;
+                if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx[q] = 31 - __clz(rest);
+              }
             }
           }
-          __syncwarp();
-          if (++s == stages) { s = 0; ph ^= 1u; }
+          img[q] = n; row[q] = h;
+        }
+        for (int g = g0; g < g1 && ok; ++g) {
+#pragma unroll
+          for (int q = 0; q < Q; ++q) {
+            if (Q > 1 && (q >= planes || !ok)) continue;
+            if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; continue; }
+            if (lane == 0 && (rank == 0 || !PAIR_A))
+              mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(p.rows[q] * pitch) * (PAIR_A ? 2u : 1u));
+            if (idx[q] >= 0) {
+              uint8_t *d = ring + s * stage_bytes + lane * pitch;
+              const int x = (ct * TILE_W + p.col0[q]) * x_unit, c = g * cb_step;
+              if (PAIR_A) {
+                const uint32_t pair_bar = mapa_u32(&full[s], 0);
+                if (!strided) tma_tile_4d_pair(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], pair_bar);
+                else tma_tile_5d_pair(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], pair_bar);
+              } else {
+                if (!strided) tma_tile_4d(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], &full[s]);
+                else tma_tile_5d(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], &full[s]);
+              }
+            }
+            __syncwarp();
+            if (++s == stages) { s = 0; ph ^= 1u; }
+          }
         }
       }
-    }
     };
     // (stride 1: an input read with a step.  A loop of its own for the int8 3x3 forms: tested at every copy it costs narrow
     // tiles 2 to 3 %)
     if constexpr (FORM == FORM_3X3S2) {
-      rows(std::integral_constant<int, 1>{});
+      fetch_rows(std::integral_constant<int, 1>{});
     } else if constexpr (FORM == FORM_ANY || FORM == FORM_1X1 || KIND == HALO_F32) {
-      rows(std::integral_constant<int, 2>{});
+      fetch_rows(std::integral_constant<int, 2>{});
     } else {
-      if (uni(p.strided)) rows(std::integral_constant<int, 1>{});
-      else rows(std::integral_constant<int, 0>{});
+      if (uni(p.strided)) fetch_rows(std::integral_constant<int, 1>{});
+      else fetch_rows(std::integral_constant<int, 0>{});
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- weights
@@ -1116,7 +1116,7 @@ void *plane_base(const HaloPlan &hp, const void *in, int q) {
   return const_cast<uint8_t *>(static_cast<const uint8_t *>(in)) + (static_cast<size_t>(ph) * hp.IW + pw) * (hp.kind == HALO_F32 ? 64 : 16);
 }
 
-// Which copies the tiles of `images` images take of plane q (bit i: of HaloParams::tmap[q][i]'s height): the walk of the
+// Which copies the tiles of `images` images take of plane q (bit i: of HaloArgs::tmap[q][i]'s height): the walk of the
 // kernel's row warp.  The tiles' offsets in an image repeat after at most `period` tiles.
 int copy_heights(const HaloParams &p, int images, int q) {
   const long long row_tiles = (static_cast<long long>(images - 1) * p.period + p.OH + TILE_H - 1) / TILE_H;
