@@ -40,6 +40,6 @@ def test_direct_equals_gemm(pkg, shape, types, total, monkeypatch):
         assert d.prepare(wt, bias) == 0 and d.enqueue(y, x) == 0, E.last_error()
         torch.cuda.synchronize()
         assert d.device_status() == 0
-        got[gemm] = y.view(n, (oc + 15) // 16, -1)[:, :oc // 16]      # (channels that are padding are not compared)
+        got[gemm] = y      # (channels that are padding too: both write them)
         d.close()
     assert torch.equal(got[False], got[True])
