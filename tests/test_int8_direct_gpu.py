@@ -94,6 +94,22 @@ def test_int8_1x1_umma_matches_oracle(pkg, case):
     _check(case, "i8_gemm_umma")
 
 
+@pytest.mark.parametrize("case", [
+    _case("gemm_many_tiles", 20, 149, 16, 41, 66, kh=1, kw=1, pad=0, algo="1x1"),                 # 440 tiles: a persistent loop
+    _case("gemm_many_tiles_sum", 9, 144, 32, 52, 50, kh=1, kw=1, pad=0, algo="1x1", sum=True, sscale=0.5, oscale=0.5),
+    _case("gemm_ragged_s8", 5, 703, 30, 13, 11, kh=1, kw=1, pad=0, algo="1x1", types="u8f32s8f32", relu=False),
+    _case("gemm_f32_out", 12, 150, 17, 31, 30, kh=1, kw=1, pad=0, algo="1x1", types="u8f32f32f32"),
+    _case("gemm_single_tile", 1, 144, 48, 15, 13, kh=1, kw=1, pad=0, algo="1x1"),
+], ids=lambda c: c.name)
+def test_int8_1x1_layers_left_to_the_gemm_kernel(pkg, case):
+    """Layers that the direct kernel would be slower on: the single-CTA GEMM kernel is what runs."""
+    import gpuutil as G
+    d = G.make_desc(case)
+    assert d.setup() == 0 and d.launched_kernel == "i8_gemm_umma"
+    d.close()
+    _check(case, "i8_gemm_umma")
+
+
 @pytest.mark.parametrize("case", BOX_CASES, ids=lambda c: c.name)
 def test_int8_kxk_umma_matches_oracle(pkg, case):
     _check(case, "i8_conv_umma")
