@@ -66,3 +66,23 @@ def test_nhwc_channels_that_are_no_groups_of_four_are_converted(pkg, monkeypatch
     got, d = G.run_gpu(plain, R.user_tensors(plain, t))
     assert d.launch_count() == 5 and np.array_equal(got, R.act_to_user(blocked, case.oc, "nhwc"))
     d.close()
+
+
+@pytest.mark.parametrize("chunks", [2, 3])
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c.name)
+def test_image_ranges(pkg, case, chunks, monkeypatch):
+    """Host tensors cut into ranges of images: the kernels find each range in the nhwc tensors by the caller's pitch (channel counts that
+    are no multiple of 16), as the blocked tensor's result in one range."""
+    monkeypatch.setenv("ELB_WINO_CTA2", "1")
+    import gpuutil as G
+    t = R.make_tensors(case)
+    if case.types != "fp32":
+        case = R.calibrate_tinput(case, t)
+    blocked, d0 = G.run_gpu(case, t)
+    d0.close()
+    plain = dataclasses.replace(case, ifmt="nhwc", ofmt="nhwc")
+    monkeypatch.setenv("ELB_HOST_CHUNKS", str(chunks))
+    got, d = G.run_gpu(plain, R.user_tensors(plain, t), host_buffers=True)
+    assert d.launch_count() == 3 * min(chunks, case.n) and d.device_status() == 0      # no conversions
+    d.close()
+    assert np.array_equal(got, R.act_to_user(blocked, case.oc, "nhwc"))
