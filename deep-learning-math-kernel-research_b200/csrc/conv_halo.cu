@@ -122,7 +122,7 @@ __host__ __device__ constexpr int pxw_of(int form, int kind, int pairs) {
 
 // Planes and channels of a kernel's HaloArgs
 __host__ __device__ constexpr int planes_of(int form) { return form == FORM_ANY || form == FORM_3X3S2 ? 4 : 1; }
-// (constants of 256 channels cost every call 0.4 us more and gain nothing: 16 x 80 -> 208 at 33x33 8.0 us, 7.6 without)
+// (constants of 256 channels cost every call another kilobyte and gain nothing: 16 x 80 -> 208 at 33x33 8.0 us, 7.6 without)
 constexpr int PARAM_OC = 128;
 __host__ __device__ constexpr int oc_of(int kind, bool split) { return kind == HALO_F32 || split ? 0 : PARAM_OC; }
 
@@ -1031,7 +1031,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
   }
   if (kind == HALO_I8 && p.resident && taps == 1 && stride == 1 && p.groups > 1) {
     // The issuer's general loop serves these, and a channel group takes it 650 to 1000 cycles whatever the tile: 49 x 149 -> 16 at 41x66
-    // (five groups) modelled as 7.0 us takes 20.9, 9 x 144 -> 32 at 72x114 5.2 / 12.2, 13 x 81x129 512 -> 32 (four) 10.1 / 17.5.
+    // (five groups) modelled as 7.0 us takes 20.9, 9 x 144 -> 32 at 72x114 5.2 / 12.2.
     const double epilogue = 400 + 128.0 * p.BN / 9, loop = hp.loop_ratio * epilogue, slow = std::max(loop, 600.0 * p.groups);
     hp.est_us += std::ceil(m_tiles / num_sms) * (std::max(slow, epilogue) - std::max(loop, epilogue)) / 1750;
     hp.loop_ratio = slow / epilogue;

@@ -69,9 +69,10 @@ struct HaloParams {
   int tap_rows[4], tap_cols[4];      // the plane's taps: a rectangle, rows from row0, columns from col0
 };
 
-// Parameters of a kernel that reads up to PLANES planes and keeps the constants of up to OC channels here.  A launch costs the host
-// 0.4 us per kilobyte of parameters and a waiting call 0.5: with room for four planes and 256 channels in every kernel's
-// (5.4 KB) an empty launch took 7.0 us instead of 4.8, and 13.9 instead of 11.0 until it was waited for.
+// Parameters of a kernel that reads up to PLANES planes and keeps the constants of up to OC channels here: 1216, 2176, 3136 or 4096
+// bytes; with room for four planes and 256 channels every launch carried 5120.  An empty kernel that is waited for takes 9.3 us
+// with 64 bytes and 9.8 with 5120 (medians of 40 x 200 calls), enqueued back to back 2.7 and 2.8; on another host it was 11.0 and
+// 13.9, enqueued 4.8 and 7.0.
 template <int PLANES, int OC>
 struct HaloArgs : HaloParams {
   // [row / column parity plane of the input (stride 1: one)][rows a copy brings: 1, 2, 4, 8, all of a tile's]

@@ -415,9 +415,10 @@ __device__ __forceinline__ void bt6x2(const f32x2 (&f)[6], f32x2 (&o)[6]) {
 
 // The u8 transform where |fma(V, mrepS, tz)| < 2^15 for every possible input (the host checks; scales that use the eight bits are a
 // hundredth of that): one thread = one tile x TWO channels, as pairs in every instruction, and the rounded values saturate as
-// pairs of 16-bit integers.  Bound by instruction issue (64 % of the slots; 33 MB read and 58 MB written per 64 x 512 channels at
-// 28x28 take 36 us): with both paths of a border test in most warps it took 43 us, and the kernel below, one channel of four
-// after the other, 40.  The whole layer at 128 images 274 -> 266.6 us, 23 x 992 -> 48 at 71x71 226 -> 213, 3 x 32 -> 16 at 68x68 14.6 -> 13.8.
+// pairs of 16-bit integers.  Bound by instruction issue (65 % of the slots at 27 % of the warps; 26 MB read and 58 MB written per 64 x 512
+// channels at 28x28 take 36 us, a third of the copy bandwidth): with both paths of a border test in most warps it took 43 us, and
+// wino_input_u8_kernel, one channel of four after the other, 40.  The whole layer at 128 images 274 -> 266.6 us as graph replays on one
+// input (302 -> 297 with other inputs from call to call), 23 x 992 -> 48 at 71x71 226 -> 213, 3 x 32 -> 16 at 68x68 14.6 -> 13.8.
 constexpr int PAIR_TILES = TRANS_THREADS / 8;      // tiles per block (8 threads = the 16 channels of a block)
 template <bool NHWC>
 __global__ void __launch_bounds__(TRANS_THREADS, 10) wino_input_u8_pairs_kernel(const __grid_constant__ WinoInParams p) {
