@@ -139,7 +139,10 @@ __host__ __device__ constexpr int oc_of(int kind, bool split) { return kind == H
 // toward zero): 144 of them for 128 channels, where the transform kernels' GEMM has 32.  So the K loop runs in parts of
 // p.chunk_groups channel groups, each afresh in the other accumulator buffer, and up to 64 output channels the two K steps of a tap
 // have accumulators of their own; the epilogue adds all that up in registers, rounding to nearest.
-template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE>
+// STEPPED: an int8 3x3 form, stride 1, on every step-th pixel of a larger input.  Compiled apart: a second row loop beside the plain one
+// cost every call of these forms 0.1 us (7 x 64 -> 80 at 11x11 3.12 -> 3.25, 10 x 112 -> 64 at 13x9 3.57 -> 3.67), a test at every copy narrow
+// tiles 2 to 3 %.
+template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE, bool STEPPED>
 __global__ void __launch_bounds__(KIND == HALO_I8 ? THREADS_I8 : THREADS_F32, 1)
 conv_halo_kernel(const __grid_constant__ HaloArgs<planes_of(FORM), oc_of(KIND, SPLIT)> p) {
   extern __shared__ uint8_t smem_raw[];
@@ -282,85 +285,73 @@ conv_halo_kernel(const __grid_constant__ HaloArgs<planes_of(FORM), oc_of(KIND, S
     uint8_t *ring = KIND == HALO_I8 ? smem : raw;
     const int stage_bytes = KIND == HALO_I8 ? p.a_bytes : p.raw_bytes;
     const int planes = uni(p.planes), period = uni(p.period), pitch = uni(p.pitch), cb_step = uni(p.cb_step);
-    auto fetch_rows = [&](auto how) {      // 0 / 1: not strided / strided, 2: as the parameters say
-      constexpr int HOW = decltype(how)::value;
-      const bool strided = HOW == 2 ? uni(p.strided) != 0 : HOW != 0;
-      // stride 1: 8-byte elements, so that the copy engine moves whole rows
-      const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
-      int s = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int tile = first; tile < p.total_tiles && ok; tile += step) {
-        const int mt = PAIR ? 2 * p.div_n.div(tile) + rank : p.div_n.div(tile);
-        const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
-        // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
-        // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
-        // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
-        constexpr int Q = FORM == FORM_ANY || FORM == FORM_3X3S2 ? 4 : 1;      // planes the code is written out for
-        int idx[Q], img[Q], row[Q];
+    constexpr bool PLAIN = KIND == HALO_I8 && (FORM == FORM_3X3_ROWS || FORM == FORM_3X3_TAPS || FORM == FORM_3X3_RESIDENT);
+    const bool strided = FORM == FORM_3X3S2 || (PLAIN ? STEPPED : uni(p.strided) != 0);
+    // stride 1: 8-byte elements, so that the copy engine moves whole rows
+    const int x_unit = strided ? 1 : KIND == HALO_I8 ? 2 : 8;
+    int s = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int tile = first; tile < p.total_tiles && ok; tile += step) {
+      const int mt = PAIR ? 2 * p.div_n.div(tile) + rank : p.div_n.div(tile);
+      const int rt = p.div_col.div(mt), ct = mt - rt * p.col_tiles;
+      // Which copies bring this tile's rows, the same for every channel group; lane r stands for row r.  Rows of one
+      // image go in one copy (lane 0 issues it).  A tile across images takes each image's share in pieces of 8, 4, 2
+      // and 1 rows, issued by the lane of a piece's first row (a copy costs its issuer about 100 cycles).
+      constexpr int Q = FORM == FORM_ANY || FORM == FORM_3X3S2 ? 4 : 1;      // planes the code is written out for
+      int idx[Q], img[Q], row[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        if (Q > 1 && q >= planes) continue;
+        const int rows = p.rows[q], v0 = rt * TILE_H + p.row0[q];
+        int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
+        if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
+        idx[q] = -1;
+        if (h + rows <= period) {
+          if (lane == 0) idx[q] = HALO_HEIGHTS - 1;
+        } else {
+          const int v = v0 + lane;
+          n = v > 0 ? p.div_period.div(v) : 0;
+          h = v - n * period;
+          const int n_prev = __shfl_up_sync(0xFFFFFFFFu, n, 1);
+          const uint32_t starts = __ballot_sync(0xFFFFFFFFu, lane == 0 || n != n_prev || lane == rows);
+          if (lane < rows) {
+            const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
+            const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
+            const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
+            if (at < (len & ~7)) {
+              if ((at & 7) == 0) idx[q] = 3;
+            } else {
+              const int sub = at & 7, rest = len - at;
+              if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx[q] = 31 - __clz(rest);
+            }
+          }
+        }
+        img[q] = n; row[q] = h;
+      }
+      for (int g = g0; g < g1 && ok; ++g) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-          if (Q > 1 && q >= planes) continue;
-          const int rows = p.rows[q], v0 = rt * TILE_H + p.row0[q];
-          int n = 0, h = v0;                        // (rows in front of the first image: zeros, like its padding)
-          if (v0 > 0) { n = p.div_period.div(v0); h = v0 - n * period; }
-          idx[q] = -1;
-          if (h + rows <= period) {
-            if (lane == 0) idx[q] = HALO_HEIGHTS - 1;
-          } else {
-            const int v = v0 + lane;
-            n = v > 0 ? p.div_period.div(v) : 0;
-            h = v - n * period;
-            const int n_prev = __shfl_up_sync(0xFFFFFFFFu, n, 1);
-            const uint32_t starts = __ballot_sync(0xFFFFFFFFu, lane == 0 || n != n_prev || lane == rows);
-            if (lane < rows) {
-              const int seg = 31 - __clz(starts & (0xFFFFFFFFu >> (31 - lane)));      // first row of this lane's image
-              const uint32_t above = lane == 31 ? 0u : starts & (0xFFFFFFFEu << lane);
-              const int len = (above ? __ffs(above) - 1 : rows) - seg, at = lane - seg;
-              if (at < (len & ~7)) {
-                if ((at & 7) == 0) idx[q] = 3;
-              } else {
-                const int sub = at & 7, rest = len - at;
-                if (sub == 0 || (rest < (sub & -sub) && ((len & 7) & sub) == sub)) idx[q] = 31 - __clz(rest);
-              }
+          if (Q > 1 && (q >= planes || !ok)) continue;
+          if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; continue; }
+          if (lane == 0 && (rank == 0 || !PAIR_A))
+            mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(p.rows[q] * pitch) * (PAIR_A ? 2u : 1u));
+          if (idx[q] >= 0) {
+            uint8_t *d = ring + s * stage_bytes + lane * pitch;
+            const int x = (ct * TILE_W + p.col0[q]) * x_unit, c = g * cb_step;
+            if (PAIR_A) {
+              const uint32_t pair_bar = mapa_u32(&full[s], 0);
+              if (!strided) tma_tile_4d_pair(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], pair_bar);
+              else tma_tile_5d_pair(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], pair_bar);
+            } else {
+              if (!strided) tma_tile_4d(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], &full[s]);
+              else tma_tile_5d(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], &full[s]);
             }
           }
-          img[q] = n; row[q] = h;
-        }
-        for (int g = g0; g < g1 && ok; ++g) {
-#pragma unroll
-          for (int q = 0; q < Q; ++q) {
-            if (Q > 1 && (q >= planes || !ok)) continue;
-            if (!wait_all(&empty[s], ph ^ 1u, abort_flag)) { ok = false; fail_code = ST_WAIT_TIMEOUT_PRODUCER; continue; }
-            if (lane == 0 && (rank == 0 || !PAIR_A))
-              mbar_arrive_expect_tx(&full[s], static_cast<uint32_t>(p.rows[q] * pitch) * (PAIR_A ? 2u : 1u));
-            if (idx[q] >= 0) {
-              uint8_t *d = ring + s * stage_bytes + lane * pitch;
-              const int x = (ct * TILE_W + p.col0[q]) * x_unit, c = g * cb_step;
-              if (PAIR_A) {
-                const uint32_t pair_bar = mapa_u32(&full[s], 0);
-                if (!strided) tma_tile_4d_pair(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], pair_bar);
-                else tma_tile_5d_pair(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], pair_bar);
-              } else {
-                if (!strided) tma_tile_4d(d, &p.tmap[0][idx[q]], x, c, row[q], img[q], &full[s]);
-                else tma_tile_5d(d, &p.tmap[q][idx[q]], 0, x, c, row[q], img[q], &full[s]);
-              }
-            }
-            __syncwarp();
-            if (++s == stages) { s = 0; ph ^= 1u; }
-          }
+          __syncwarp();
+          if (++s == stages) { s = 0; ph ^= 1u; }
         }
       }
-    };
-    // (stride 1: an input read with a step.  A loop of its own for the int8 3x3 forms: tested at every copy it costs narrow
-    // tiles 2 to 3 %)
-    if constexpr (FORM == FORM_3X3S2) {
-      fetch_rows(std::integral_constant<int, 1>{});
-    } else if constexpr (FORM == FORM_ANY || FORM == FORM_1X1 || KIND == HALO_F32) {
-      fetch_rows(std::integral_constant<int, 2>{});
-    } else {
-      if (uni(p.strided)) fetch_rows(std::integral_constant<int, 1>{});
-      else fetch_rows(std::integral_constant<int, 0>{});
     }
   } else if (warp == 2) {
     // ---------------------------------------------------------------- weights
@@ -1193,11 +1184,14 @@ struct HaloKernel {
   int planes = 0, oc = 0;
 };
 template <int KIND, int PAIRS, int FORM, bool STACK, bool PAIR, bool SPLIT, bool FINE>
-HaloKernel kernel_of() {
-  return {reinterpret_cast<const void *>(conv_halo_kernel<KIND, PAIRS, FORM, STACK, PAIR, SPLIT, FINE>), planes_of(FORM), oc_of(KIND, SPLIT)};
+HaloKernel kernel_of(bool stepped = false) {
+  if constexpr (KIND == HALO_I8 && (FORM == FORM_3X3_ROWS || FORM == FORM_3X3_TAPS || FORM == FORM_3X3_RESIDENT))
+    if (stepped)
+      return {reinterpret_cast<const void *>(conv_halo_kernel<KIND, PAIRS, FORM, STACK, PAIR, SPLIT, FINE, true>), planes_of(FORM), oc_of(KIND, SPLIT)};
+  return {reinterpret_cast<const void *>(conv_halo_kernel<KIND, PAIRS, FORM, STACK, PAIR, SPLIT, FINE, false>), planes_of(FORM), oc_of(KIND, SPLIT)};
 }
 template <int FORM, bool PAIR = false, bool SPLIT = false>
-HaloKernel pick_kernel(const HaloPlan &hp) {
+HaloKernel pick_kernel(const HaloPlan &hp, bool stepped) {
   if (hp.kind == HALO_F32) {
     if constexpr (FORM == FORM_3X3_TAPS || (!PAIR && (FORM == FORM_3X3_ROWS || (!SPLIT && FORM == FORM_3X3_RESIDENT))))
       if (hp.p.fine) return kernel_of<HALO_F32, 2, FORM, !PAIR, PAIR, SPLIT, true>();
@@ -1207,13 +1201,13 @@ HaloKernel pick_kernel(const HaloPlan &hp) {
     return kernel_of<HALO_F32, 2, FORM, false, PAIR, SPLIT, false>();
   }
   switch (hp.p.kch) {
-    case 8: return kernel_of<HALO_I8, 4, FORM, false, PAIR, SPLIT, false>();
-    case 6: return kernel_of<HALO_I8, 3, FORM, false, PAIR, SPLIT, false>();
-    case 4: return kernel_of<HALO_I8, 2, FORM, false, PAIR, SPLIT, false>();
+    case 8: return kernel_of<HALO_I8, 4, FORM, false, PAIR, SPLIT, false>(stepped);
+    case 6: return kernel_of<HALO_I8, 3, FORM, false, PAIR, SPLIT, false>(stepped);
+    case 4: return kernel_of<HALO_I8, 2, FORM, false, PAIR, SPLIT, false>(stepped);
   }
   if constexpr (!PAIR) {
-    if (hp.p.kch == 2) return kernel_of<HALO_I8, 1, FORM, false, false, SPLIT, false>();
-    if constexpr (!SPLIT) return kernel_of<HALO_I8, 0, FORM, false, false, false, false>();
+    if (hp.p.kch == 2) return kernel_of<HALO_I8, 1, FORM, false, false, SPLIT, false>(stepped);
+    if constexpr (!SPLIT) return kernel_of<HALO_I8, 0, FORM, false, false, false, false>(stepped);
   }
   return {};
 }
@@ -1228,23 +1222,23 @@ int tap_form(const HaloPlan &hp) {
   return p.pxw == pxw_of(form, hp.kind, pairs) ? form : FORM_ANY;
 }
 template <bool PAIR, bool SPLIT>
-HaloKernel pick_form(const HaloPlan &hp, int form) {
+HaloKernel pick_form(const HaloPlan &hp, int form, bool stepped) {
   switch (form) {
     case FORM_3X3_ROWS:
-      if constexpr (!PAIR) return pick_kernel<FORM_3X3_ROWS, false, SPLIT>(hp);
+      if constexpr (!PAIR) return pick_kernel<FORM_3X3_ROWS, false, SPLIT>(hp, stepped);
       return {};
-    case FORM_3X3_TAPS: return pick_kernel<FORM_3X3_TAPS, PAIR, SPLIT>(hp);
-    case FORM_3X3S2: return pick_kernel<FORM_3X3S2, PAIR, SPLIT>(hp);
-    case FORM_1X1: return pick_kernel<FORM_1X1, PAIR, SPLIT>(hp);
+    case FORM_3X3_TAPS: return pick_kernel<FORM_3X3_TAPS, PAIR, SPLIT>(hp, stepped);
+    case FORM_3X3S2: return pick_kernel<FORM_3X3S2, PAIR, SPLIT>(hp, stepped);
+    case FORM_1X1: return pick_kernel<FORM_1X1, PAIR, SPLIT>(hp, stepped);
   }
-  return pick_kernel<FORM_ANY, PAIR, SPLIT>(hp);
+  return pick_kernel<FORM_ANY, PAIR, SPLIT>(hp, stepped);
 }
-HaloKernel pick_kernel(const HaloPlan &hp) {
+HaloKernel pick_kernel(const HaloPlan &hp, bool stepped) {
   const HaloParams &p = hp.p;
   int form = tap_form(hp);
-  if (p.resident) return form == FORM_3X3_TAPS && p.b_stages == 3 * p.groups ? pick_kernel<FORM_3X3_RESIDENT>(hp) : pick_kernel<FORM_ANY>(hp);
+  if (p.resident) return form == FORM_3X3_TAPS && p.b_stages == 3 * p.groups ? pick_kernel<FORM_3X3_RESIDENT>(hp, stepped) : pick_kernel<FORM_ANY>(hp, stepped);
   if (p.row_units) form = form == FORM_3X3_TAPS ? FORM_3X3_ROWS : FORM_ANY;
-  return p.split > 1 ? pick_form<false, true>(hp, form) : p.pair ? pick_form<true, false>(hp, form) : pick_form<false, false>(hp, form);
+  return p.split > 1 ? pick_form<false, true>(hp, form, stepped) : p.pair ? pick_form<true, false>(hp, form, stepped) : pick_form<false, false>(hp, form, stepped);
 }
 
 // Launch configuration: may overlap its set-up with the kernel before it (launch_overlapped), pairs as clusters of two.
@@ -1268,10 +1262,10 @@ struct LaunchConfig {
 
 }  // namespace
 
-cudaError_t halo_init(HaloPlan &hp) {
-  const HaloKernel k = pick_kernel(hp);
+cudaError_t halo_init(HaloPlan &hp, bool stepped) {
+  const HaloKernel k = pick_kernel(hp, stepped);
   cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_LIMIT + 1024);
-  if (e == cudaSuccess && hp.p.pair) {
+  if (e == cudaSuccess && hp.p.pair && !stepped) {
     LaunchConfig lc(hp, 2, nullptr);
     e = cudaOccupancyMaxActiveClusters(&hp.max_clusters, k.fn, &lc.cfg);
     if (e == cudaSuccess && hp.max_clusters < 1) e = cudaErrorInvalidConfiguration;
@@ -1341,7 +1335,7 @@ bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int nu
   }
   void *base[4];
   for (int q = 0; q < p.planes; ++q) base[q] = step > 1 ? const_cast<void *>(in) : plane_base(hp, in, q);
-  const HaloKernel kernel = pick_kernel(hp);
+  const HaloKernel kernel = pick_kernel(hp, step > 1);
   if (p.planes > kernel.planes) { err = "internal: planes"; return false; }
   p.b_img = static_cast<const uint8_t *>(hp.d_b);
   p.wide = reinterpret_cast<uintptr_t>(p.out) % 32 == 0;

@@ -90,6 +90,7 @@ struct HaloPlan {
   HaloParams p{};
   size_t smem_bytes = 0, b_bytes = 0;
   double est_us = 0;                 // modelled time of the whole batch
+  bool steps_ready = false;          // int8: halo_init() was called for launches with a step
   double gather_ratio = 0;           // int8: time of a tile's rows pixel by pixel (16 bytes per clock) over that of its MMAs
   double loop_ratio = 0;             // int8: modelled time of a tile's K loop over its epilogue's
   int max_clusters = 0;              // pairs the device holds at once
@@ -114,7 +115,7 @@ bool halo_plan(HaloPlan &hp, int kind, int n, int ic, int oc, int ih, int iw, in
 std::vector<uint8_t> halo_pack_i8(const HaloPlan &hp, const int8_t *q, int OCP, int taps, int ICP);
 std::vector<uint8_t> halo_pack_f32(const HaloPlan &hp, const float *u, int OCP, int taps, int ICP);
 bool halo_set_weights(HaloPlan &hp, void *d_b, std::string &err);      // the packed weights on the device
-cudaError_t halo_init(HaloPlan &hp);      // once per plan and device
+cudaError_t halo_init(HaloPlan &hp, bool stepped = false);      // once per plan and device; stepped: before launches with a step, too
 // Run `images` images: in / p.out address the first; p: a copy of hp.p with the per-call pointers set.
 // step > 1 (stride 1 only): the tensor holds src_h x src_w pixels per plane, of which every step-th row and column is read.
 bool halo_launch(HaloPlan &hp, HaloParams &p, const void *in, int images, int num_sms, cudaStream_t s, std::string &err,

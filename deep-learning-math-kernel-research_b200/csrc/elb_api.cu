@@ -998,8 +998,14 @@ int execute_common(elb_conv &pl, void *output, const void *input, const void *we
 namespace elb {
 bool conv_step_supported(elb_conv_t *plan) {
   if (elb_conv_input_step_supported(plan)) return true;
-  return plan && plan->halo && !plan->cvt_in && plan->info.kernel == ELB_KERNEL_I8_CONV_UMMA && plan->halo->stride == 1 &&
-         plan->halo->gather_ratio <= 0.8;
+  if (!plan || !plan->halo || plan->cvt_in || plan->info.kernel != ELB_KERNEL_I8_CONV_UMMA || plan->halo->stride != 1 ||
+      plan->halo->gather_ratio > 0.8)
+    return false;
+  if (!plan->halo->steps_ready) {
+    DeviceGuard guard(plan->device);
+    plan->halo->steps_ready = guard.ok && halo_init(*plan->halo, true) == cudaSuccess;
+  }
+  return plan->halo->steps_ready;
 }
 int conv_enqueue_stepped(elb_conv_t *plan, void *output, const void *input, int src_h, int src_w, int step, cudaStream_t s) {
   if (!conv_step_supported(plan) || (src_h + step - 1) / step != plan->d.ih || (src_w + step - 1) / step != plan->d.iw)
