@@ -546,6 +546,10 @@ __global__ void __launch_bounds__(128) wino4_input_kernel(const __grid_constant_
     tw = r - th * g.wt;
   }
   const int ih0 = 2 * th - g.pad_t, iw0 = 2 * tw - g.pad_l;
+  // u8: one base per thread and 32-bit pixel numbers (with whole addresses per pixel 29 x 144 -> 50 at 68x103 took 192 us instead of 184,
+  // 27 x 320 -> 64 at 49x33 73.4 / 69.7; fp32 the other way, 5 x 367 -> 65 at 34x34 36.8 / 37.2)
+  const size_t plane = pixel_at<NHWC>(n, cb, quad, 0, 0, g.CB, g.IH, g.IW, p.chans);
+  const int pitch = NHWC ? p.chans : 16;
   float d[4][4][4];
 #pragma unroll
   for (int h = 0; h < 4; ++h)
@@ -553,7 +557,8 @@ __global__ void __launch_bounds__(128) wino4_input_kernel(const __grid_constant_
     for (int w = 0; w < 4; ++w) {
       const int ih = ih0 + h, iw = iw0 + w;
       const bool ok = live && ih >= 0 && ih < g.IH && iw >= 0 && iw < g.IW;
-      const size_t at = pixel_at<NHWC>(n, cb, quad, ok ? ih : 0, ok ? iw : 0, g.CB, g.IH, g.IW, p.chans);
+      const size_t at = IN_U8 ? plane + static_cast<size_t>(ok ? ih * g.IW + iw : 0) * pitch
+                              : pixel_at<NHWC>(n, cb, quad, ok ? ih : 0, ok ? iw : 0, g.CB, g.IH, g.IW, p.chans);
       if (IN_U8) {
         const uint32_t raw = ok ? __ldg(reinterpret_cast<const uint32_t *>(static_cast<const uint8_t *>(p.in) + at)) : 0u;
 #pragma unroll
